@@ -5,31 +5,46 @@
 // Why: on this GPU the FP64 pipe issues 2 lanes per clock per SM and every
 // kernel of the path is bound by it; a hardware-style FP64 division
 // (reciprocal seed plus Newton steps in DFMA) costs several FP64 issue slots.
-// The same correctly rounded quotient can be formed from the operands' bits
-// with 32/64-bit integer multiplies, which run on a unit with far more lanes
-// and overlap with the FP64 work of other warps.  The quotient is the same
-// number (IEEE division is correctly rounded, so any correct method gives the
-// same bits): kernels that must match the reference bit for bit may use it.
+// The same correctly rounded results can be formed from the operands' bits
+// with 32-bit integer instructions, which run on units with far more lanes
+// and overlap with the FP64 work of other warps.  The results are the same
+// numbers (IEEE division, square root and multiplication are correctly
+// rounded, so any correct method gives the same bits): kernels that must
+// match the reference bit for bit may use them.
 //
-// Method (long division by a fixed-point reciprocal with Newton-Raphson
-// refinement and an exact remainder correction, as in integer division by
-// invariant divisors, Granlund & Montgomery 1994, Moller & Granlund 2011):
-//   significands ma, mb in [2^52, 2^53); d = mb * 2^11 in [2^63, 2^64)
-//   y0  ~ 2^127 / d from a correctly rounded FP32 reciprocal of d's top 24
-//       bits (relative error < 2^-22)
-//   y  <- y + y (2^127 - d y) / 2^127, twice (error squares each time; the
-//       truncations leave |y - 2^127/d| <= 4 units, relative < 2^-61)
-//   Q~ = floor((ma * 2^11) y / 2^74), within 1 of Q = floor(ma 2^53 / mb)
-//   R  = ma 2^53 - Q~ mb (exact in 64 bits since |R| < 2^54), one
-//       correction step each way gives Q and 0 <= R < mb
-//   Q in [2^53, 2^54): 54 quotient bits, the last one is the rounding bit and
-//       R != 0 the sticky bit; Q in [2^52, 2^53): 53 bits, rounding decided
-//       by comparing 2R with mb.
-// Domain: b normal and finite, and either a = +-0 (result +-0) or a normal
-// and finite with a result exponent that is normal with room for a rounding
-// carry; anything else (b zero, subnormal, infinite or NaN, a subnormal,
-// infinite or NaN, results that overflow or underflow) takes the hardware
-// division, so the function equals a / b for every input.
+// All three work on 32-bit words and multiply with 32 x 32 -> 64 bit
+// multiply-adds, and every exponent and sign is formed by adding the words'
+// upper 12 bits (the significand's carry then moves into the exponent by
+// itself).
+//
+// Product: the exact 106-bit product from four multiply-adds, the 53-bit
+// significand, rounding word and sticky bit by funnel shifts.
+//
+// Division and square root (long division in digits of 28-29 bits with a
+// 32-bit reciprocal estimate, Knuth, The Art of Computer Programming vol. 2,
+// 4.3.1, and the rounding test of Ziv, ACM TOMS 17(3), 1991): an FP32
+// reciprocal (reciprocal square root) seed of 22 bits and one Newton step in
+// 32-bit integers give v with a relative error below 2^-29, rounded down;
+// the first digit is a high product with v, the exact remainder follows in
+// 64-bit arithmetic, the second digit and remainder likewise, and a third
+// high product extends the quotient (root) to more than 80 bits.  Neither
+// operation has results half way between two doubles, so the truncated
+// 84-bit value decides the rounding unless it lies within a few units of
+// 2^-84 of a midpoint; that case (about one operand pair in 2^28) takes the
+// hardware operation.
+//
+// Domain: operands with exponents in the middle half of the range (about
+// 2^-503 .. 2^504), for the product +-0 too; anything else (subnormal,
+// infinite, NaN, results that could overflow or underflow) takes the
+// hardware operation, so each function equals its operator for every input.
+//
+// Bound: the integer pipes' issue rate.  Cycles per warp operation and SM with
+// 16 warps resident and nothing else running (GB300), against the earlier
+// form (64-bit fixed-point Newton iterations and a 128-bit product) and the
+// hardware operation: product 14 (29, 20), division 29 (80, 144), square root
+// 31 (81, 150); without the range checks (the *_core functions) 11 and 18.
+// Beside a saturated FP64 stream of 16 FMAs, four products cost 4% (hardware
+// products 30%) and four divisions 6% (earlier form 41%).
 #pragma once
 #include <stdint.h>
 
@@ -43,39 +58,75 @@
 
 namespace amrs {
 
-AMRS_HD uint64_t ddiv_mulhi(uint64_t a, uint64_t b) {
-#ifdef __CUDA_ARCH__
-  return __umul64hi(a, b);
-#else
-  return (uint64_t)(((unsigned __int128)a * b) >> 64);
-#endif
-}
+struct DWords {
+  uint32_t hi, lo;
+};
 
-// The bits of x.  On the device an opaque move: the compiler would otherwise
+// The words of x.  On the device an opaque move: the compiler would otherwise
 // turn integer tests on a reinterpreted double (an exponent field equal to
 // 0x7FF, (bits << 1) == 0) back into FP64 compares, each of which takes an
-// FP64 issue slot -- the very resource these functions exist to spare
-// (measured: 1 FP64 instruction per division and 4 per multiplication with a
-// plain reinterpretation, none with the move).
-AMRS_HD uint64_t ddiv_bits(double x) {
+// FP64 issue slot -- the very resource these functions exist to spare.
+AMRS_HD DWords dwords(double x) {
+  DWords w;
 #ifdef __CUDA_ARCH__
-  uint64_t u;
-  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
-  return u;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(w.lo), "=r"(w.hi) : "d"(x));
 #else
   uint64_t u;
   memcpy(&u, &x, 8);
-  return u;
+  w.hi = (uint32_t)(u >> 32);
+  w.lo = (uint32_t)u;
 #endif
+  return w;
 }
 
-AMRS_HD double ddiv_from_bits(uint64_t u) {
+AMRS_HD double dfrom(uint32_t hi, uint32_t lo) {
 #ifdef __CUDA_ARCH__
-  return __longlong_as_double((long long)u);
+  double x;
+  asm("mov.b64 %0, {%1, %2};" : "=d"(x) : "r"(lo), "r"(hi));
+  return x;
 #else
+  const uint64_t u = ((uint64_t)hi << 32) | lo;
   double x;
   memcpy(&x, &u, 8);
   return x;
+#endif
+}
+
+AMRS_HD uint32_t mulhi32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+AMRS_HD uint64_t madw(uint32_t a, uint32_t b, uint64_t c) { return (uint64_t)a * b + c; }
+// the upper word of (hi:lo) << s and the lower word of (hi:lo) >> s, 0 <= s < 32
+AMRS_HD uint32_t shl_hi(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, s);
+#else
+  return (uint32_t)((((uint64_t)hi << 32 | lo) << s) >> 32);
+#endif
+}
+AMRS_HD uint32_t shr_lo(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_r(lo, hi, s);
+#else
+  return (uint32_t)(((uint64_t)hi << 32 | lo) >> s);
+#endif
+}
+// (hi:lo) plus the carry of r + k, plus E in the upper word, as a double
+AMRS_HD double round_pack(uint32_t r, uint32_t k, uint32_t hi, uint32_t lo, uint32_t E) {
+#ifdef __CUDA_ARCH__
+  uint32_t l, h;
+  asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, %5, %6;\n\t}"
+      : "=r"(l), "=r"(h)
+      : "r"(r), "r"(k), "r"(lo), "r"(hi), "r"(E));
+  return dfrom(h, l);
+#else
+  const uint64_t c = ((uint64_t)r + k) >> 32;
+  const uint64_t u = ((((uint64_t)hi << 32) | lo) + c) + ((uint64_t)E << 32);
+  return dfrom((uint32_t)(u >> 32), (uint32_t)u);
 #endif
 }
 
@@ -93,13 +144,13 @@ inline double dmul_hw(double a, double b) { return a * b; }
 inline double dsqrt_hw(double x) { return ::sqrt(x); }
 #endif
 
-// Seeds of the Newton iterations.  They need about 22 correct bits, not
-// correct rounding: on the device the approximate FP32 reciprocal and
-// reciprocal square root (rcp.approx / rsqrt.approx, within 1 ulp and
-// 2^-22.9 relative), which run on the special-function unit and use no FP64
-// slot.  The host build perturbs the correctly rounded value by up to
-// +-2 ulps, so the host checks cover seeds at least that far off.
-AMRS_HD uint32_t ddiv_seed_perturb(uint32_t rb, uint32_t v) {
+// Seeds of the Newton steps.  They need about 22 correct bits, not correct
+// rounding: on the device the approximate FP32 reciprocal and reciprocal
+// square root (rcp.approx / rsqrt.approx, within 1 ulp and 2^-22.9 relative),
+// which run on the special-function unit and use no FP64 slot.  The host
+// build perturbs the correctly rounded value by up to +-2 ulps, so the host
+// checks cover seeds at least that far off.
+AMRS_HD uint32_t seed_perturb(uint32_t rb, uint32_t v) {
 #ifdef __CUDA_ARCH__
   (void)v;
   return rb;
@@ -107,188 +158,166 @@ AMRS_HD uint32_t ddiv_seed_perturb(uint32_t rb, uint32_t v) {
   return rb + (uint32_t)((int)((v ^ (v >> 7) ^ (v >> 13)) % 5u) - 2);
 #endif
 }
-
-// Reciprocal of a float holding an integer dt in [2^23, 2^24) (relative
-// error below 2^-22.5), returned as its bits.
-AMRS_HD uint32_t ddiv_rcp_bits(uint32_t dt) {
-  const uint32_t fb = 0x4B000000u | (dt & 0x7FFFFFu);  // the float equal to dt
+// a seed in (0.5, 1] (its bits, possibly an ulp or two outside) as a 32-bit
+// fraction: 2^32 times the value clamped to [0.5, 1)
+AMRS_HD uint32_t seed_fraction(uint32_t rb) {
+  rb = rb < 0x3F000000u ? 0x3F000000u : rb;
+  rb = rb > 0x3F7FFFFFu ? 0x3F7FFFFFu : rb;
+  return rb * 256u + 0x80000000u;
+}
+// 2^32 / f for the float f in [1, 2) with these bits, to 22 bits
+AMRS_HD uint32_t seed_rcp(uint32_t fb) {
 #ifdef __CUDA_ARCH__
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fb)));
-  return __float_as_uint(r);
+  return seed_fraction(__float_as_uint(r));
 #else
   float f, r;
   memcpy(&f, &fb, 4);
   r = 1.0f / f;
   uint32_t rb;
   memcpy(&rb, &r, 4);
-  return ddiv_seed_perturb(rb, dt);
+  return seed_fraction(seed_perturb(rb, fb));
 #endif
 }
-
-// One Newton-Raphson step of y ~ 2^127 / d (d in [2^63, 2^64)).
-AMRS_HD uint64_t ddiv_newton(uint64_t d, uint64_t y) {
-  const uint64_t plo = d * y, phi = ddiv_mulhi(d, y);
-  // e = 2^127 - d y as (ehi * 2^64 + elo), elo dropped: |ehi| < 2^43 here
-  const int64_t ehi = (int64_t)((1ull << 63) - phi - (plo != 0 ? 1ull : 0ull));
-  const uint64_t m = ehi < 0 ? (uint64_t)(-ehi) : (uint64_t)ehi;
-  const uint64_t lo = y * m, hi = ddiv_mulhi(y, m);
-  const uint64_t corr = (hi << 1) | (lo >> 63);  // y |e| / 2^127
-  if (ehi < 0) return y - corr;
-  const uint64_t s = y + corr;
-  return s < y ? ~0ull : s;  // 2^127 / d <= 2^64: clamp a carry
-}
-
-// a / b, correctly rounded; the integer path where its domain holds.
-AMRS_HD double ddiv_rn(double a, double b) {
-  const uint64_t ua = ddiv_bits(a), ub = ddiv_bits(b);
-  const int ea = (int)((ua >> 52) & 0x7FF), eb = (int)((ub >> 52) & 0x7FF);
-  const int E = ea - eb + 1023;  // biased exponent of the quotient when ma >= mb
-  const bool azero = (ua << 1) == 0;
-  if (eb == 0 || eb == 0x7FF || (!azero && (ea == 0 || ea == 0x7FF || E < 2 || E > 2045))) return ddiv_hw(a, b);
-  const uint64_t FRAC = (1ull << 52) - 1, HID = 1ull << 52;
-  const uint64_t ma = (ua & FRAC) | HID, mb = (ub & FRAC) | HID;
-  const uint64_t d = mb << 11;
-  // seed: y0 = r * 2^87 with r ~ 1/dt, dt = d >> 40: r = m 2^(er - 23) gives
-  // y0 = m << (er + 64); r lies near (2^-24, 2^-23], an approximate r may sit
-  // just outside, and a y0 of 2^64 or more is clamped
-  const uint32_t rb = ddiv_rcp_bits((uint32_t)(d >> 40));
-  const int rsh = (int)((rb >> 23) & 0xFFu) - 127 + 64;
-  const uint64_t y0 = rsh >= 41 ? ~0ull : ((uint64_t)((rb & 0x7FFFFFu) | 0x800000u) << rsh);
-  const uint64_t y = ddiv_newton(d, ddiv_newton(d, y0));
-  // quotient of X = ma 2^53 by mb
-  uint64_t q = ddiv_mulhi(ma << 11, y) >> 10;
-  int64_t r = (int64_t)((ma << 53) - q * mb);
-  if (r < 0) {
-    q -= 1;
-    r += (int64_t)mb;
-  } else if (r >= (int64_t)mb) {
-    q += 1;
-    r -= (int64_t)mb;
-  }
-  uint64_t sig, inc;
-  int ebias;
-  if (q >= (1ull << 53)) {
-    sig = q >> 1;
-    const uint64_t round = q & 1ull, sticky = r != 0 ? 1ull : 0ull;
-    inc = round & (sticky | (sig & 1ull));
-    ebias = E;
-  } else {
-    sig = q;
-    const uint64_t twor = (uint64_t)r << 1;
-    inc = (twor > mb || (twor == mb && (sig & 1ull))) ? 1ull : 0ull;
-    ebias = E - 1;
-  }
-  // (ebias - 1) << 52 plus the 53-bit significand (hidden bit included);
-  // a rounding carry to 2^53 moves into the exponent by itself
-  const uint64_t mag = azero ? 0ull : ((uint64_t)(ebias - 1) << 52) + sig + inc;
-  return ddiv_from_bits(mag | ((ua ^ ub) & (1ull << 63)));
-}
-
-// a * b, correctly rounded (IEEE round to nearest, ties to even), computed on
-// the integer pipe.  Significands ma, mb in [2^52, 2^53): the exact product
-// P = ma mb lies in [2^104, 2^106); (ma 2^11)(mb 2) = P 2^12 is formed as a
-// 128-bit integer whose high word is floor(P / 2^52) in [2^52, 2^54) and
-// whose low word holds the remaining bits of P.  A high word of 2^53 or more
-// gives the 53-bit significand P >> 53 with bit 52 of P as the rounding bit;
-// otherwise P >> 52 with bit 51; the bits below are the sticky bit.
-// Domain: a and b normal and finite with a normal result exponent, or either
-// one +-0 and the other finite (result +-0); anything else (subnormal,
-// infinite or NaN operands, products that underflow) takes the hardware
-// multiplication, so the function equals a * b for every input.  A product
-// that rounds up past the largest finite number becomes +-inf, as IEEE
-// rounding to nearest gives.
-AMRS_HD double dmul_rn(double a, double b) {
-  const uint64_t ua = ddiv_bits(a), ub = ddiv_bits(b);
-  const int ea = (int)((ua >> 52) & 0x7FF), eb = (int)((ub >> 52) & 0x7FF);
-  const int E = ea + eb - 1023;  // biased exponent of the product when P < 2^105
-  const bool fin = ea != 0x7FF && eb != 0x7FF;
-  const bool zero = fin && ((ua << 1) == 0 || (ub << 1) == 0);
-  if (!zero && (ea == 0 || eb == 0 || !fin || E < 1 || E > 2045)) return dmul_hw(a, b);
-  const uint64_t X = (ua << 11) | (1ull << 63);                     // ma 2^11
-  const uint64_t Y = ((ub << 1) & ((1ull << 53) - 2)) | (1ull << 53);  // mb 2
-  const uint64_t hi = ddiv_mulhi(X, Y), lo = X * Y;
-  const bool top = (hi >> 53) != 0;
-  const uint64_t sig = top ? (hi >> 1) : hi;
-  const uint64_t round = top ? (hi & 1ull) : (lo >> 63);
-  const uint64_t sticky = (top ? lo : (lo << 1)) != 0 ? 1ull : 0ull;
-  const uint64_t inc = round & (sticky | (sig & 1ull));
-  const int eres = top ? E + 1 : E;
-  const uint64_t mag = zero ? 0ull : ((uint64_t)(eres - 1) << 52) + sig + inc;
-  return ddiv_from_bits(mag | ((ua ^ ub) & (1ull << 63)));
-}
-
-// Reciprocal square root of a float holding an integer v in [2^22, 2^24)
-// (relative error below 2^-22.5), returned as its bits.
-AMRS_HD uint32_t dsqrt_rsqrt_bits(uint32_t v) {
-  // v as a float without a conversion instruction: 2^23 + low bits, or
-  // 2^22 + low bits for v below 2^23
-  const uint32_t fb = (v >> 23) ? (0x4B000000u | (v & 0x7FFFFFu)) : (0x4A800000u | ((v << 1) & 0x7FFFFFu));
+// 2^32 / sqrt(f) for the float f in [1, 4) with these bits, to 22 bits
+AMRS_HD uint32_t seed_rsqrt(uint32_t fb) {
 #ifdef __CUDA_ARCH__
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fb)));
-  return __float_as_uint(r);
+  return seed_fraction(__float_as_uint(r));
 #else
   float f;
   memcpy(&f, &fb, 4);
   const float r = (float)(1.0 / sqrt((double)f));
   uint32_t rb;
   memcpy(&rb, &r, 4);
-  return ddiv_seed_perturb(rb, v);
+  return seed_fraction(seed_perturb(rb, fb));
 #endif
 }
+// the Newton correction v e / 2^31 for |e| < 2^11
+AMRS_HD uint32_t seed_corr(uint32_t v, int32_t e) { return (uint32_t)(((int32_t)(v >> 12) * e) >> 19); }
 
-// One Newton-Raphson step of y ~ 2^95 / sqrt(n) (n in [2^62, 2^64)):
-// y <- y + y (1 - n y^2 / 2^190) / 2.
-AMRS_HD uint64_t dsqrt_newton(uint64_t n, uint64_t y) {
-  const uint64_t t = ddiv_mulhi(y, y);             // y^2 / 2^64
-  const uint64_t u = ddiv_mulhi(n, t);             // n y^2 / 2^128, ~2^62
-  const int64_t e = (int64_t)((1ull << 62) - u);   // 2^62 (1 - n y^2 / 2^190)
-  const uint64_t m = e < 0 ? (uint64_t)(-e) : (uint64_t)e;
-  const uint64_t lo = y * m, hi = ddiv_mulhi(y, m);
-  const uint64_t corr = (hi << 1) | (lo >> 63);    // y |e| / 2^63
-  if (e < 0) return y - corr;
-  const uint64_t s = y + corr;
-  return s < y ? ~0ull : s;
+// exponent of the word in [520, 1528)
+AMRS_HD bool mid_range(uint32_t hi) { return hi * 2u - 0x41000000u < 0x7E000000u; }
+
+// a / b for words in the domain; *slow is set when the truncated quotient
+// cannot decide the rounding.  ma/mb in (1/2, 2), digits q1, q2, q3 of
+// ma 2^86 / mb = q1 2^58 + q2 2^29 + q3, each rounded down (v is):
+//   q1 <= ma 2^28 / mb,   R1 = ma 2^28 - q1 mb in [0, 2.3 mb)
+//   q2 <= R1 2^29 / mb,   R2 = R1 2^29 - q2 mb in [0, 3.8 mb)
+//   q3 <= R2 2^29 / mb    within 5 units
+AMRS_HD double ddiv_core(DWords a, DWords b, bool* slow) {
+  const uint32_t mah = (a.hi & 0xFFFFFu) | 0x100000u, mbh = (b.hi & 0xFFFFFu) | 0x100000u;
+  // v ~ 2^63 / dh, dh = the top 32 bits of mb 2^11; one Newton step
+  const uint32_t dh = shl_hi(b.lo, mbh, 11);
+  const uint32_t v0 = seed_rcp(((dh >> 8) & 0x7FFFFFu) | 0x3F800000u);
+  const int32_t e = (int32_t)(0x7FFFFFFFu - mulhi32(v0, dh));
+  const uint32_t v = v0 + seed_corr(v0, e) - 3u;  // < 2^95 / (mb 2^11)
+  const uint64_t nmb = 0ull - (((uint64_t)mbh << 32) | b.lo);
+  const uint32_t nl = (uint32_t)nmb, nh = (uint32_t)(nmb >> 32);
+  const uint32_t q1 = mulhi32(shl_hi(a.lo, mah, 11), v) >> 3;
+  uint64_t R = madw(q1, nl, ((uint64_t)shl_hi(a.lo, mah, 28) << 32) | (a.lo << 28));
+  uint32_t rl = (uint32_t)R, rh = (uint32_t)(R >> 32) + q1 * nh;
+  const uint32_t q2 = mulhi32(shr_lo(rl, rh, 23), v);
+  R = madw(q2, nl, ((uint64_t)shl_hi(rl, rh, 29) << 32) | (rl << 29));
+  rl = (uint32_t)R;
+  rh = (uint32_t)(R >> 32) + q2 * nh;
+  const uint32_t q3 = mulhi32(shr_lo(rl, rh, 23), v);
+  const uint64_t T = madw(q2, 1u << 29, q3);
+  const uint64_t W = madw(q1, 1u << 26, T >> 32);  // in (2^53, 2^55)
+  const uint32_t Wh = (uint32_t)(W >> 32), Wl = (uint32_t)W;
+  const uint32_t top = Wh >> 22, s = 1u + top;
+  const uint32_t r = shr_lo((uint32_t)T, Wl, s);
+  *slow = r - 0x7FFFFFF8u < 8u;
+  return round_pack(r, 0x80000000u, Wh >> s, shr_lo(Wl, Wh, s),
+                    (a.hi & 0xFFF00000u) - (b.hi & 0xFFF00000u) + (1021u << 20) + (top << 20));
 }
 
-// sqrt(x), correctly rounded (IEEE round to nearest even), computed on the
-// integer pipe for positive normal x (and +-0); anything else takes the
-// hardware square root, so the function equals sqrt(x) for every input.
-// Method: x = M 2^(2k) with N = M 2^104 an integer in [2^104, 2^106); a
-// fixed-point reciprocal square root y ~ 2^95 / sqrt(N / 2^42) from a
-// correctly rounded FP32 rsqrt seed and two Newton-Raphson steps (relative
-// error < 2^-60); S~ = floor(sqrt(N)) within 1 from (N / 2^42) y / 2^74; the
-// exact remainder R = N - S^2 (|R| < 2^55, exact in 64-bit arithmetic) fixes
-// S and decides the rounding: up iff R > S (N is an integer, so it never
-// equals (S + 1/2)^2).
-AMRS_HD double dsqrt_rn(double x) {
-  const uint64_t ux = ddiv_bits(x);
-  const int ex = (int)(ux >> 52);  // sign bit included: negative x lands above 0x7FF
-  if ((ux << 1) == 0) return x;     // +-0
-  if (ex == 0 || ex >= 0x7FF) return dsqrt_hw(x);
-  const int e = ex - 1023;
-  const uint64_t mx = (ux & ((1ull << 52) - 1)) | (1ull << 52);
-  const uint64_t N_lo = (e & 1) ? (mx << 53) : (mx << 52);  // N mod 2^64
-  const uint64_t n64 = (e & 1) ? (mx << 11) : (mx << 10);   // N / 2^42, in [2^62, 2^64)
-  const uint32_t rb = dsqrt_rsqrt_bits((uint32_t)(n64 >> 40));
-  // y0 = rsqrt * 2^75 = m << (er + 52) for rsqrt = m 2^(er - 23) near (2^-12, 2^-11];
-  // an approximate value may sit just outside, and 2^64 or more is clamped
-  const int rsh = (int)((rb >> 23) & 0xFFu) - 127 + 52;
-  const uint64_t y0 = rsh >= 41 ? ~0ull : ((uint64_t)((rb & 0x7FFFFFu) | 0x800000u) << rsh);
-  const uint64_t y = dsqrt_newton(n64, dsqrt_newton(n64, y0));
-  uint64_t S = ddiv_mulhi(n64, y) >> 10;
-  int64_t R = (int64_t)(N_lo - S * S);
-  if (R < 0) {
-    S -= 1;
-    R += (int64_t)(2 * S + 1);
-  } else if (R > (int64_t)(2 * S)) {
-    R -= (int64_t)(2 * S + 1);
-    S += 1;
+// a / b, correctly rounded; the integer path where its domain holds.
+AMRS_HD double ddiv_rn(double a, double b) {
+  const DWords A = dwords(a), B = dwords(b);
+  bool slow;
+  double x = ddiv_core(A, B, &slow);
+  if (!mid_range(A.hi) || !mid_range(B.hi) || slow) {
+    // +-0 / b with b in range is +-0
+    if (((A.hi << 1) | A.lo) == 0u && mid_range(B.hi)) x = dfrom((A.hi ^ B.hi) & 0x80000000u, 0u);
+    else x = ddiv_hw(a, b);
   }
-  const uint64_t inc = R > (int64_t)S ? 1ull : 0ull;
-  const int eb = (e >> 1) + 1023;  // floor(e / 2), biased
-  return ddiv_from_bits(((uint64_t)(eb - 1) << 52) + S + inc);
+  return x;
+}
+
+// a * b for words in the domain (any exponents whose sum gives a normal
+// product).  v:t:p is the 106-bit product ma mb, p3 its upper word in
+// [2^8, 2^10); the rounding word r holds the bits below the significand with
+// the last word's sticky bit or-ed in, and r + 0x7FFFFFFF + lsb carries
+// exactly when rounding to nearest even goes up.
+AMRS_HD double dmul_core(DWords a, DWords b) {
+  const uint32_t mah = (a.hi & 0xFFFFFu) | 0x100000u, mbh = (b.hi & 0xFFFFFu) | 0x100000u;
+  const uint64_t p = madw(a.lo, b.lo, 0ull);
+  const uint64_t t = madw(mah, b.lo, madw(a.lo, mbh, p >> 32));
+  const uint64_t v = madw(mah, mbh, t >> 32);
+  const uint32_t p3 = (uint32_t)(v >> 32), p2 = (uint32_t)v, p1 = (uint32_t)t, p0 = (uint32_t)p;
+  const uint32_t top = p3 >> 9, s = 12u - top;
+  const uint32_t r = shl_hi(p0, p1, s) | (p0 < 1u ? p0 : 1u);
+  const uint32_t lo = shl_hi(p1, p2, s);
+  return round_pack(r, 0x7FFFFFFFu + (lo & 1u), shl_hi(p2, p3, s), lo,
+                    (a.hi & 0xFFF00000u) + (b.hi & 0xFFF00000u) - 0x40000000u + (top << 20));
+}
+
+// a * b, correctly rounded; the integer path where its domain holds.
+AMRS_HD double dmul_rn(double a, double b) {
+  const DWords A = dwords(a), B = dwords(b);
+  double x = dmul_core(A, B);
+  if (!mid_range(A.hi) || !mid_range(B.hi)) {
+    const bool za = ((A.hi << 1) | A.lo) == 0u, zb = ((B.hi << 1) | B.lo) == 0u;
+    if ((za && (zb || mid_range(B.hi))) || (zb && mid_range(A.hi))) x = dfrom((A.hi ^ B.hi) & 0x80000000u, 0u);
+    else x = dmul_hw(a, b);
+  }
+  return x;
+}
+
+// sqrt(x) for words in the domain (positive).  x = M 2^(2k), n' = M 2^60 in
+// [2^60, 2^62); digits S1 (31 bits), s2, s3 of sqrt(n') 2^54 = S1 2^54 +
+// s2 2^27 + s3 with v ~ 2^62 / sqrt(n') a few units below:
+//   S1 < sqrt(n') by 0.5 .. 8,    R1 = n' - S1^2 > 0
+//   s2 < R1 2^27 / (2 sqrt(n')) by 2 .. 9 (the 3 outweighs the omitted
+//   second-order term),           R2 = R1 2^54 - s2 (S1 2^28 + s2) in (0, 2^63)
+//   s3 ~ R2 / (2 sqrt(n')) within 4 units.
+AMRS_HD double dsqrt_core(DWords x, bool* slow) {
+  const uint32_t odd = (~x.hi >> 20) & 1u;  // the unbiased exponent is odd
+  const uint32_t mxh = (x.hi & 0xFFFFFu) | 0x100000u;
+  const uint32_t nh = shl_hi(x.lo, mxh, 10u + odd);  // top word of 4 n'
+  const uint32_t v0 = seed_rsqrt((shl_hi(x.lo, x.hi, 3) & 0x7FFFFFu) | (0x3F800000u + (odd << 23)));
+  const int32_t e = (int32_t)(0x3FFFFFFFu - mulhi32(mulhi32(v0, v0), nh));
+  const uint32_t v = v0 + seed_corr(v0, e) - 4u;
+  const uint32_t S1 = mulhi32(nh, v);
+  const uint64_t n4 = ((uint64_t)shl_hi(x.lo, mxh, 8u + odd) << 32) | (x.lo << (8u + odd));
+  const uint64_t R1 = n4 - (uint64_t)S1 * S1;
+  const uint32_t s2 = mulhi32((uint32_t)(R1 >> 4), v) - 3u;
+  const uint64_t M = madw(S1, 1u << 28, s2);
+  const uint64_t P = madw(s2, (uint32_t)M, (uint64_t)(s2 * (uint32_t)(M >> 32)) << 32);
+  const uint64_t R2 = ((uint64_t)((uint32_t)R1 << 22) << 32) - P;
+  const uint32_t s3 = mulhi32((uint32_t)(R2 >> 31), v);
+  const uint64_t T = madw(s2, 1u << 27, s3);
+  const uint64_t W = madw(S1, 1u << 22, T >> 32);
+  const uint32_t r = (uint32_t)T;
+  *slow = r - 0x7FFFFFF0u < 32u;
+  return round_pack(r, 0x80000000u, (uint32_t)(W >> 32), (uint32_t)W,
+                    (((x.hi + 0x100000u) >> 1) & 0x7FF00000u) + (510u << 20));
+}
+
+// sqrt(x), correctly rounded; the integer path for positive x in its domain,
+// +-0 directly, anything else by the hardware square root.
+AMRS_HD double dsqrt_rn(double x) {
+  const DWords X = dwords(x);
+  bool slow;
+  double y = dsqrt_core(X, &slow);
+  if (X.hi - (520u << 20) >= (1008u << 20) || slow) {
+    if (((X.hi << 1) | X.lo) == 0u) y = x;
+    else y = dsqrt_hw(x);
+  }
+  return y;
 }
 
 }  // namespace amrs
