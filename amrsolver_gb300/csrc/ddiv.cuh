@@ -92,6 +92,8 @@ AMRS_HD double dfrom(uint32_t hi, uint32_t lo) {
 #endif
 }
 
+AMRS_HD double dfrom(DWords w) { return dfrom(w.hi, w.lo); }
+
 AMRS_HD uint32_t mulhi32(uint32_t a, uint32_t b) {
 #ifdef __CUDA_ARCH__
   return __umulhi(a, b);
@@ -115,18 +117,18 @@ AMRS_HD uint32_t shr_lo(uint32_t lo, uint32_t hi, uint32_t s) {
   return (uint32_t)(((uint64_t)hi << 32 | lo) >> s);
 #endif
 }
-// (hi:lo) plus the carry of r + k, plus E in the upper word, as a double
-AMRS_HD double round_pack(uint32_t r, uint32_t k, uint32_t hi, uint32_t lo, uint32_t E) {
+// (hi:lo) plus the carry of r + k, plus E in the upper word
+AMRS_HD DWords round_pack(uint32_t r, uint32_t k, uint32_t hi, uint32_t lo, uint32_t E) {
 #ifdef __CUDA_ARCH__
   uint32_t l, h;
   asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, %5, %6;\n\t}"
       : "=r"(l), "=r"(h)
       : "r"(r), "r"(k), "r"(lo), "r"(hi), "r"(E));
-  return dfrom(h, l);
+  return DWords{h, l};
 #else
   const uint64_t c = ((uint64_t)r + k) >> 32;
   const uint64_t u = ((((uint64_t)hi << 32) | lo) + c) + ((uint64_t)E << 32);
-  return dfrom((uint32_t)(u >> 32), (uint32_t)u);
+  return DWords{(uint32_t)(u >> 32), (uint32_t)u};
 #endif
 }
 
@@ -207,7 +209,7 @@ AMRS_HD bool mid_range(uint32_t hi) { return hi * 2u - 0x41000000u < 0x7E000000u
 //   q1 <= ma 2^28 / mb,   R1 = ma 2^28 - q1 mb in [0, 2.3 mb)
 //   q2 <= R1 2^29 / mb,   R2 = R1 2^29 - q2 mb in [0, 3.8 mb)
 //   q3 <= R2 2^29 / mb    within 5 units
-AMRS_HD double ddiv_core(DWords a, DWords b, bool* slow) {
+AMRS_HD DWords ddiv_core(DWords a, DWords b, bool* slow) {
   const uint32_t mah = (a.hi & 0xFFFFFu) | 0x100000u, mbh = (b.hi & 0xFFFFFu) | 0x100000u;
   // v ~ 2^63 / dh, dh = the top 32 bits of mb 2^11; one Newton step
   const uint32_t dh = shl_hi(b.lo, mbh, 11);
@@ -238,7 +240,7 @@ AMRS_HD double ddiv_core(DWords a, DWords b, bool* slow) {
 AMRS_HD double ddiv_rn(double a, double b) {
   const DWords A = dwords(a), B = dwords(b);
   bool slow;
-  double x = ddiv_core(A, B, &slow);
+  double x = dfrom(ddiv_core(A, B, &slow));
   if (!mid_range(A.hi) || !mid_range(B.hi) || slow) {
     // +-0 / b with b in range is +-0
     if (((A.hi << 1) | A.lo) == 0u && mid_range(B.hi)) x = dfrom((A.hi ^ B.hi) & 0x80000000u, 0u);
@@ -252,7 +254,7 @@ AMRS_HD double ddiv_rn(double a, double b) {
 // [2^8, 2^10); the rounding word r holds the bits below the significand with
 // the last word's sticky bit or-ed in, and r + 0x7FFFFFFF + lsb carries
 // exactly when rounding to nearest even goes up.
-AMRS_HD double dmul_core(DWords a, DWords b) {
+AMRS_HD DWords dmul_core(DWords a, DWords b) {
   const uint32_t mah = (a.hi & 0xFFFFFu) | 0x100000u, mbh = (b.hi & 0xFFFFFu) | 0x100000u;
   const uint64_t p = madw(a.lo, b.lo, 0ull);
   const uint64_t t = madw(mah, b.lo, madw(a.lo, mbh, p >> 32));
@@ -268,7 +270,7 @@ AMRS_HD double dmul_core(DWords a, DWords b) {
 // a * b, correctly rounded; the integer path where its domain holds.
 AMRS_HD double dmul_rn(double a, double b) {
   const DWords A = dwords(a), B = dwords(b);
-  double x = dmul_core(A, B);
+  double x = dfrom(dmul_core(A, B));
   if (!mid_range(A.hi) || !mid_range(B.hi)) {
     const bool za = ((A.hi << 1) | A.lo) == 0u, zb = ((B.hi << 1) | B.lo) == 0u;
     if ((za && (zb || mid_range(B.hi))) || (zb && mid_range(A.hi))) x = dfrom((A.hi ^ B.hi) & 0x80000000u, 0u);
@@ -284,7 +286,7 @@ AMRS_HD double dmul_rn(double a, double b) {
 //   s2 < R1 2^27 / (2 sqrt(n')) by 2 .. 9 (the 3 outweighs the omitted
 //   second-order term),           R2 = R1 2^54 - s2 (S1 2^28 + s2) in (0, 2^63)
 //   s3 ~ R2 / (2 sqrt(n')) within 4 units.
-AMRS_HD double dsqrt_core(DWords x, bool* slow) {
+AMRS_HD DWords dsqrt_core(DWords x, bool* slow) {
   const uint32_t odd = (~x.hi >> 20) & 1u;  // the unbiased exponent is odd
   const uint32_t mxh = (x.hi & 0xFFFFFu) | 0x100000u;
   const uint32_t nh = shl_hi(x.lo, mxh, 10u + odd);  // top word of 4 n'
@@ -312,7 +314,7 @@ AMRS_HD double dsqrt_core(DWords x, bool* slow) {
 AMRS_HD double dsqrt_rn(double x) {
   const DWords X = dwords(x);
   bool slow;
-  double y = dsqrt_core(X, &slow);
+  double y = dfrom(dsqrt_core(X, &slow));
   if (X.hi - (520u << 20) >= (1008u << 20) || slow) {
     if (((X.hi << 1) | X.lo) == 0u) y = x;
     else y = dsqrt_hw(x);

@@ -168,21 +168,15 @@ __global__ void __launch_bounds__(256) weno_flux_lambda_kernel(BoxTable tb, Face
 // separate multiply and add.  The four divisions are correctly rounded on
 // the integer pipe (ddiv_rn): the same quotients as the reference's, at a
 // fraction of the FP64 issue slots.
-// Products formed on the integer pipe (kmul), by bit: 0 the shared 3 s2,
+// Products formed on the integer pipe (kmul), by bit of M: 0 the shared 3 s2,
 // 1 the (13/12) x^2 terms, 2 the quarter-scaled squares b^2 and f^2, 3 the
 // fourth power of beta1, 4 the squares of eps + beta, 5 the stencil
-// coefficients 7, 11, 5, 6 the final scaling, 7 the weight products,
-// 8 the LLF halves (0.5 me) U of the face kernel; bit 9 takes the maximum
-// wave speed of the face kernel as an integer maximum of the bit patterns.
-#ifndef AMRS_WENO_IMUL
-#define AMRS_WENO_IMUL 0x263
-#endif
-// The same for the reconstructions of the WENO5-Riemann face kernel, whose
-// serial solver leaves less room on the integer pipe.
+// coefficients 7, 11, 5, 6 the final scaling, 7 the weight products.
+// AMRS_WRREC_IMUL: the WENO5-Riemann face kernel's.
 #ifndef AMRS_WRREC_IMUL
 #define AMRS_WRREC_IMUL 0x001
 #endif
-template <int M = AMRS_WENO_IMUL>
+template <int M>
 __device__ __forceinline__ double weno5js(const double s0, const double s1, const double s2, const double s3,
                                           const double s4) {
   constexpr bool M0 = M & 1, M1 = (M >> 1) & 1, M2 = (M >> 2) & 1, M3 = (M >> 3) & 1, M4 = (M >> 4) & 1,
@@ -211,6 +205,82 @@ __device__ __forceinline__ double weno5js(const double s0, const double s1, cons
   const double vl2 = fma(2.0, s2, kmul<M5>(5.0, s3)) - s4;                   // 2 s2 + 5 s3 - s4
   return kmul<M6>(kmul<M6>(1.0 / 6.0, sum),
                   kmul<M7>(alpha0, vl0) + kmul<M7>(alpha1, vl1) + kmul<M7>(alpha2, vl2));
+}
+
+// The same reconstruction, same bits, with its products and quotients on the
+// integer pipe from end to end: they stay in the operands' words (dmul_core,
+// ddiv_core), and `ok` collects one range test per value that enters in place
+// of a test in every operation; where it ends up false the caller takes the
+// plain form.  The smoothness differences are zero or in [2^-100, 2^60); a
+// zero enters its square (or fourth power) as 2^-200, and the result, at most
+// 2^-400, changes no sum it enters.  eps + beta is beta from 2^-78 up (eps is
+// below half its last place) and eps below 2^-187 (the other way round); in
+// between the hardware adds them out of line.
+
+// A smoothness difference.
+__device__ __forceinline__ DWords weno_diff(double x, bool& ok) {
+  DWords w = dwords(x);
+  const bool zero = ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
+  ok = ok && (zero || w.hi * 2u - (923u << 21) < (160u << 21));
+  w.hi = zero ? (823u << 20) : w.hi;
+  return w;
+}
+static __device__ __noinline__ double dadd_hw(double a, double b) { return a + b; }
+// (eps + beta)^2
+__device__ __forceinline__ DWords weno_e2(double beta) {
+  DWords w = dwords(beta);
+  const bool big = w.hi >= (945u << 20), tiny = w.hi < (836u << 20);
+  if (!big) {
+    w = DWords{0x37A16C26u, 0x2777579Cu};  // 1e-40
+    if (!tiny) w = dwords(dadd_hw(1e-40, beta));
+  }
+  return dmul_core(w, w);
+}
+// A factor that may be zero: its words, and whether it is.
+struct ZWords {
+  DWords w;
+  bool zero;
+};
+__device__ __forceinline__ ZWords weno_fac(double x, bool& ok) {
+  ZWords z;
+  z.w = dwords(x);
+  z.zero = ((z.w.hi & 0x7FFFFFFFu) | z.w.lo) == 0u;
+  ok = ok && (z.zero || mid_range(z.w.hi));
+  return z;
+}
+// a * x for a nonzero a of the middle range.
+__device__ __forceinline__ double weno_mul(DWords a, const ZWords& x) {
+  const DWords r = dmul_core(a, x.w);
+  return dfrom(x.zero ? ((a.hi ^ x.w.hi) & 0x80000000u) : r.hi, x.zero ? 0u : r.lo);
+}
+
+__device__ __forceinline__ double weno5js_int(const double s0, const double s1, const double s2, const double s3,
+                                              const double s4, bool& ok) {
+  const DWords c1312{0x3FF15555u, 0x55555555u};
+  bool slow0, slow1, slow2, slow3;
+  const ZWords z2 = weno_fac(s2, ok);
+  const double s2x3 = weno_mul(DWords{0x40080000u, 0u}, z2);
+  const DWords a = weno_diff(fma(-2.0, s1, s0) + s2, ok), b = weno_diff(fma(-4.0, s1, s0) + s2x3, ok);
+  const double beta0 = fma(0.25, dfrom(dmul_core(b, b)), dfrom(dmul_core(dmul_core(c1312, a), a)));
+  const DWords alpha0 = ddiv_core(DWords{0x3FB99999u, 0x9999999Au}, weno_e2(beta0), &slow0);
+  const DWords c = weno_diff(fma(-2.0, s2, s1) + s3, ok), g = weno_diff(s1 - s3, ok);
+  const double beta1 = fma(0.25, dfrom(dmul_core(dmul_core(dmul_core(g, g), g), g)),
+                           dfrom(dmul_core(dmul_core(c1312, c), c)));
+  const DWords alpha1 = ddiv_core(DWords{0x3FE33333u, 0x33333333u}, weno_e2(beta1), &slow1);
+  const DWords d = weno_diff(fma(-2.0, s3, s2) + s4, ok), f = weno_diff(fma(-4.0, s3, s2x3) + s4, ok);
+  const double beta2 = fma(0.25, dfrom(dmul_core(f, f)), dfrom(dmul_core(dmul_core(c1312, d), d)));
+  const DWords alpha2 = ddiv_core(DWords{0x3FD33333u, 0x33333333u}, weno_e2(beta2), &slow2);
+  const DWords sum = ddiv_core(DWords{0x3FF00000u, 0u}, dwords(dfrom(alpha0) + dfrom(alpha1) + dfrom(alpha2)), &slow3);
+  const ZWords z1 = weno_fac(s1, ok), z3 = weno_fac(s3, ok);
+  const DWords c5{0x40140000u, 0u};
+  // 2 s0 - 7 s1 + 11 s2, -s1 + 5 s2 + 2 s3, 2 s2 + 5 s3 - s4
+  const double vl0 = fma(2.0, s0, -weno_mul(DWords{0x401C0000u, 0u}, z1)) + weno_mul(DWords{0x40260000u, 0u}, z2);
+  const double vl1 = fma(2.0, s3, -s1 + weno_mul(c5, z2));
+  const double vl2 = fma(2.0, s2, weno_mul(c5, z3)) - s4;
+  const double S = weno_mul(alpha0, weno_fac(vl0, ok)) + weno_mul(alpha1, weno_fac(vl1, ok)) +
+                   weno_mul(alpha2, weno_fac(vl2, ok));
+  ok = ok && !(slow0 || slow1 || slow2 || slow3);
+  return weno_mul(dmul_core(DWords{0x3FC55555u, 0x55555555u}, sum), weno_fac(S, ok));
 }
 
 // The same reconstruction with its weights over a common denominator, for
@@ -252,12 +322,41 @@ __device__ __forceinline__ double weno5js_cd(const double t0, const double t1, c
   return num / den;
 }
 
-// LLF-split WENO face flux for all components (src/rhs/High_resolution.h:162-246).
-// REF_ORDER: the reference's operation order; otherwise the split halves
-// 0.5 (f +- alpha U) enter weno5js_cd doubled as fma(+-alpha, U, f).
+// The plain form of one face and component, every operation on the FP64 pipe:
+// for the lanes whose values weno5js_int does not cover.
+static __device__ __noinline__ double weno_llf_plain(const double* p0, long long st, const double* u0, long long su,
+                                                    double me) {
+  const double hme = 0.5 * me;
+  double p[6], h[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    p[q] = p0[(q - 3) * st];
+    h[q] = hme * u0[(q - 3) * su];
+  }
+  return weno5js<0>(fma(0.5, p[0], h[0]), fma(0.5, p[1], h[1]), fma(0.5, p[2], h[2]), fma(0.5, p[3], h[3]),
+                    fma(0.5, p[4], h[4])) +
+         weno5js<0>(fma(0.5, p[5], -h[5]), fma(0.5, p[4], -h[4]), fma(0.5, p[3], -h[3]), fma(0.5, p[2], -h[2]),
+                    fma(0.5, p[1], -h[1]));
+}
+
+// LLF-split WENO face flux (src/rhs/High_resolution.h:162-246), one thread per
+// face and component (blockIdx.y).  REF_ORDER: the reference's operation
+// order; otherwise the split halves 0.5 (f +- alpha U) enter weno5js_cd doubled
+// as fma(+-alpha, U, f).
+//
+// Bound: the FP64 pipe (29 instructions per reconstruction: the differences,
+// sums and splits) with the integer pipes about as full (21 products and 4
+// quotients per reconstruction).  One component per thread instead of five in
+// a loop: the range test and the fallback then cover one flux, the kernel fits
+// three CTAs per SM (80 registers), and a small box fills the chip (256 x 8 x 8
+// tube: 1040 CTAs instead of 208).  Face kernel of the reference order, before
+// (11 of the products and the quotients on the integer pipe, one thread per
+// face) and after: 256^3 54.0 -> 29.4 ms, 64^3 874 -> 464 us, the tube 78 -> 41 us;
+// with 2 CTAs per SM 30.1 ms at 256^3, with 4 (64 registers) 32.6 ms.
 template <bool REF_ORDER>
-__global__ void __launch_bounds__(256) weno_face_kernel(BoxTable tb, FaceTable ft, int s_in, long long total) {
+__global__ void __launch_bounds__(256, 3) weno_face_kernel(BoxTable tb, FaceTable ft, int s_in, long long total) {
   if (list_idle(tb)) return;
+  const int n = blockIdx.y;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     FaceIdx f;
@@ -270,58 +369,42 @@ __global__ void __launch_bounds__(256) weno_face_kernel(BoxTable tb, FaceTable f
     const long long st = (f.d == 0) ? 1 : (f.d == 1 ? L.js : L.ks);
     const long long su = (f.d == 0) ? 1 : (f.d == 1 ? U.js : U.ks);
     const long long ol = L.off(f.i, f.j, f.k) + f.d * L.ns;
-    double me;
-    if (REF_ORDER && !((AMRS_WENO_IMUL >> 9) & 1)) {
-      me = rmax(L.p[ol - 3 * st], L.p[ol - 2 * st]);
-      me = rmax(me, L.p[ol - st]);
-      me = rmax(me, L.p[ol]);
-      me = rmax(me, L.p[ol + st]);
-      me = rmax(me, L.p[ol + 2 * st]);
-    } else {
-      // lambda = |u| + c > 0: the integer order of the bit patterns is the
-      // order of the values, and the maximum (the same value as the
-      // reference's chain of rmax) needs no FP64 instruction
-      long long m = __double_as_longlong(L.p[ol - 3 * st]);
+    // lambda = |u| + c > 0: the integer order of the bit patterns is the
+    // order of the values, and the maximum (the same value as the
+    // reference's chain of rmax) needs no FP64 instruction
+    long long m = __double_as_longlong(L.p[ol - 3 * st]);
 #pragma unroll
-      for (int q = -2; q <= 2; ++q) m = max(m, __double_as_longlong(L.p[ol + q * st]));
-      me = __longlong_as_double(m);
+    for (int q = -2; q <= 2; ++q) m = max(m, __double_as_longlong(L.p[ol + q * st]));
+    const double me = __longlong_as_double(m);
+    const double* u0 = U.p + U.off(f.i, f.j, f.k) + n * U.ns;
+    const double* p0 = PF.p + PF.off(f.i, f.j, f.k) + n * PF.ns;
+    double p[6], h[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      p[q] = p0[(q - 3) * st];
+      h[q] = u0[(q - 3) * su];
     }
-    const long long ou = U.off(f.i, f.j, f.k), opf = PF.off(f.i, f.j, f.k);
-    const DArr Fd = FR.f[f.d];
-    const long long of = Fd.off(f.i, f.j, f.k);
+    double flx;
     if (!REF_ORDER) {
-#pragma unroll 1
-      for (int n = 0; n < 5; ++n) {
-        double u[6], p[6];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          u[q] = U.p[ou + (q - 3) * su + n * U.ns];
-          p[q] = PF.p[opf + (q - 3) * su + n * PF.ns];
-        }
-        const double flx = weno5js_cd(fma(me, u[0], p[0]), fma(me, u[1], p[1]), fma(me, u[2], p[2]),
-                                      fma(me, u[3], p[3]), fma(me, u[4], p[4])) +
-                           weno5js_cd(fma(-me, u[5], p[5]), fma(-me, u[4], p[4]), fma(-me, u[3], p[3]),
-                                      fma(-me, u[2], p[2]), fma(-me, u[1], p[1]));
-        Fd.p[of + n * Fd.ns] = flx;
-      }
+      flx = weno5js_cd(fma(me, h[0], p[0]), fma(me, h[1], p[1]), fma(me, h[2], p[2]), fma(me, h[3], p[3]),
+                       fma(me, h[4], p[4])) +
+            weno5js_cd(fma(-me, h[5], p[5]), fma(-me, h[4], p[4]), fma(-me, h[3], p[3]), fma(-me, h[2], p[2]),
+                       fma(-me, h[1], p[1]));
     } else {
       // 0.5*(p + me*U) == fma(0.5, p, (0.5*me)*U): halving is exact, so the
       // split stencils round exactly as in the reference (normal range)
-      const double hme = 0.5 * me;
-      for (int n = 0; n < 5; ++n) {
-        double h[6], p[6];
+      const DWords hme = dwords(0.5 * me);
+      bool ok = mid_range(hme.hi);
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
-          h[q] = kmul<(AMRS_WENO_IMUL >> 8) & 1>(hme, U.p[ou + (q - 3) * su + n * U.ns]);
-          p[q] = PF.p[opf + (q - 3) * su + n * PF.ns];
-        }
-        double flx = weno5js(fma(0.5, p[0], h[0]), fma(0.5, p[1], h[1]), fma(0.5, p[2], h[2]),
-                             fma(0.5, p[3], h[3]), fma(0.5, p[4], h[4]));
-        flx += weno5js(fma(0.5, p[5], -h[5]), fma(0.5, p[4], -h[4]), fma(0.5, p[3], -h[3]),
-                       fma(0.5, p[2], -h[2]), fma(0.5, p[1], -h[1]));
-        Fd.p[of + n * Fd.ns] = flx;
-      }
+      for (int q = 0; q < 6; ++q) h[q] = weno_mul(hme, weno_fac(h[q], ok));
+      flx = weno5js_int(fma(0.5, p[0], h[0]), fma(0.5, p[1], h[1]), fma(0.5, p[2], h[2]), fma(0.5, p[3], h[3]),
+                        fma(0.5, p[4], h[4]), ok);
+      flx += weno5js_int(fma(0.5, p[5], -h[5]), fma(0.5, p[4], -h[4]), fma(0.5, p[3], -h[3]), fma(0.5, p[2], -h[2]),
+                         fma(0.5, p[1], -h[1]), ok);
+      if (!ok) flx = weno_llf_plain(p0, st, u0, su, me);
     }
+    const DArr Fd = FR.f[f.d];
+    Fd.p[Fd.off(f.i, f.j, f.k) + n * Fd.ns] = flx;
   }
 }
 
@@ -770,8 +853,9 @@ cudaError_t launch_weno_point(const BoxTable& tb, const FaceTable& ft, int s_in,
 cudaError_t launch_weno_faces(const BoxTable& tb, const FaceTable& ft, int s_in, long long nfaces[3], bool ref_order,
                               int nsm, cudaStream_t st) {
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
-  if (ref_order) weno_face_kernel<true><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, s_in, tot);
-  else weno_face_kernel<false><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, s_in, tot);
+  const dim3 grid(grid_for(tot, nsm), NCONS);
+  if (ref_order) weno_face_kernel<true><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
+  else weno_face_kernel<false><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
   return cudaGetLastError();
 }
 
