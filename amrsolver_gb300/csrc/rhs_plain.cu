@@ -409,26 +409,63 @@ __global__ void __launch_bounds__(256, 3) weno_face_kernel(BoxTable tb, FaceTabl
 }
 
 // ----------------------------------------------------------- Riemann ----
-// Square roots of the solver and the slopes, and the division of the
-// WENO5-Riemann kernel's solver: integer-pipe (dsqrt_rn, ddiv_rn) or
-// hardware, the same correctly rounded values; the defaults are the faster
-// forms at 128^3 and 256^3.
-#ifndef AMRS_RS_ISQRT
-#define AMRS_RS_ISQRT 0
-#endif
-#ifndef AMRS_SLOPE_ISQRT
-#define AMRS_SLOPE_ISQRT 1
-#endif
-#ifndef AMRS_WR_IDIV
-#define AMRS_WR_IDIV 0
-#endif
-template <bool I>
-__device__ __forceinline__ double sqrt_sel(double x) {
-  return I ? dsqrt_rn(x) : sqrt(x);
-}
+// Quotients, roots and products on the integer pipe without a range test
+// each: the caller tests the values that enter (pos, vel), so that every
+// operand and result is well inside the normal range, and takes a plain form
+// where ok ends up false.
+struct IntOps {
+  bool ok = true;
+  // a quotient of nonzero operands, the same with a dividend that may be
+  // zero (positive divisor), a root
+  __device__ __forceinline__ double div(double a, double b) {
+    bool slow;
+    const double q = dfrom(ddiv_core(dwords(a), dwords(b), &slow));
+    ok = ok && !slow;
+    return q;
+  }
+  __device__ __forceinline__ double divz(double a, double b) {
+    const DWords w = dwords(a);
+    bool slow;
+    const DWords q = ddiv_core(w, dwords(b), &slow);
+    const bool zero = ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
+    ok = ok && (zero || !slow);
+    return dfrom(zero ? w.hi : q.hi, zero ? w.lo : q.lo);
+  }
+  __device__ __forceinline__ double root(double a) {
+    bool slow;
+    const double q = dfrom(dsqrt_core(dwords(a), &slow));
+    ok = ok && !slow;
+    return q;
+  }
+  // products of nonzero factors, and of a positive factor a with any x
+  __device__ __forceinline__ double mul(double a, double b) const {
+    return dfrom(dmul_core(dwords(a), dwords(b)));
+  }
+  __device__ __forceinline__ double mulz(double a, double x) const {
+    const DWords w = dwords(x);
+    const DWords r = dmul_core(dwords(a), w);
+    const bool zero = ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
+    return dfrom(zero ? w.hi : r.hi, zero ? w.lo : r.lo);
+  }
+  // positive, in [2^-150, 2^150); zero or in [2^-100, 2^100)
+  __device__ __forceinline__ void pos(double x) {
+    ok = ok && dwords(x).hi - (873u << 20) < (300u << 20);
+  }
+  __device__ __forceinline__ void vel(double x) {
+    const DWords w = dwords(x);
+    ok = ok && (w.hi * 2u - (923u << 21) < (200u << 21) || ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u);
+  }
+  // max(x, smallp) for a finite x; the result below 2^150
+  __device__ __forceinline__ double floor_p(double x, double smallp) {
+    const long long b = __double_as_longlong(x), s = __double_as_longlong(smallp);
+    const long long m = b < s ? s : b;
+    ok = ok && dwords(x).hi * 2u < 0xFFE00000u && (uint32_t)(m >> 32) < (1173u << 20);
+    return __longlong_as_double(m);
+  }
+};
 
-__device__ __forceinline__ double mc_limiter(double dlft, double drgt) {
-  // src/rhs/Riemann.h:9-17
+// src/rhs/Riemann.h:9-17, with the hardware's operations.
+static __device__ __noinline__ double mc_limiter_plain(double dlft, double drgt) {
   const double dcen = 0.5 * (dlft + drgt);
   const double dsgn = copysign(1.0, dcen);
   const double slop = 2.0 * rmin(fabs(dlft), fabs(drgt));
@@ -436,8 +473,112 @@ __device__ __forceinline__ double mc_limiter(double dlft, double drgt) {
   return dsgn * rmin(dlim, fabs(dcen));
 }
 
-// Characteristic slopes in direction d (src/rhs/Riemann.h:19-120).
-__global__ void __launch_bounds__(256) slope_kernel(BoxTable tb, FaceTable ft, const long long* spre0,
+// The same with one FP64 instruction (the sum): the signs, the minima and the
+// scalings by 2 and 1/2 on the words.  In range: both slopes zero or in
+// [2^-400, 2^400), so that their product's sign is that of the signs and the
+// scalings are exact; a sum of two such is zero or above 2^-453.  (Slopes of
+// opposite sign, or a zero one: the limited slope is +-0 with the sign of the
+// sum.)
+__device__ __forceinline__ double mc_limiter(double dlft, double drgt) {
+  const DWords l = dwords(dlft), r = dwords(drgt), c = dwords(dlft + drgt);
+  const uint32_t lh = l.hi & 0x7FFFFFFFu, rh = r.hi & 0x7FFFFFFFu, ch = c.hi & 0x7FFFFFFFu;
+  const bool lz = (lh | l.lo) == 0u, rz = (rh | r.lo) == 0u;
+  if (!((lz || lh - (623u << 20) < (800u << 20)) && (rz || rh - (623u << 20) < (800u << 20))))
+    return mc_limiter_plain(dlft, drgt);
+  // 4 min(|l|, |r|) against |l + r|: the smaller half is the limited slope
+  const uint64_t al = ((uint64_t)lh << 32) | l.lo, ar = ((uint64_t)rh << 32) | r.lo;
+  const uint64_t m = al < ar ? al : ar, ac = ((uint64_t)ch << 32) | c.lo;
+  uint64_t d = m + (2ull << 52) < ac ? m + (2ull << 52) : ac;
+  d -= 1ull << 52;
+  // one zero: product +-0, min(0, .) = 0; opposite signs: dlim = 0; a zero sum
+  // comes with one of the two
+  if (lz || rz || (int32_t)(l.hi ^ r.hi) < 0) d = 0ull;
+  return dfrom((uint32_t)(d >> 32) | (c.hi & 0x80000000u), (uint32_t)d);
+}
+
+// Characteristic slopes in direction d (src/rhs/Riemann.h:19-120) and the
+// terms of the cell's extrapolations to its two faces (src/rhs/Riemann.h:251-337),
+// formed once per cell instead of once per face side: A = (d0+d2)/c + d1
+// (density), B = (d2-d0)/rho (normal velocity), C = (d0+d2)*c (pressure), d3,
+// d4, with c the cell's sqrt(gamma R T) + 1e-40; for z (`up`) also A and C
+// with the sound speed of the cell above the upper face, cell k + 2
+// (cns_riemann_z's left state reads q(i,j,k+1), src/rhs/Riemann.h:316).
+struct SlopeQ {
+  double rho[3], un[3], p[3], t1[3], t2[3], T, Tup;  // cells c-1, c, c+1
+};
+static __device__ __noinline__ void slope_plain(const SlopeQ& q, double gR, double tiny, bool up, double* o) {
+  const double c0 = sqrt(gR * q.T);
+  const double cspeed = c0 + tiny;
+  const double dpl = q.p[1] - q.p[0], dpr = q.p[2] - q.p[1];
+  const double hl = 0.5 * dpl / cspeed, hr = 0.5 * dpr / cspeed;
+  const double wl = 0.5 * q.rho[1] * (q.un[1] - q.un[0]), wr = 0.5 * q.rho[1] * (q.un[2] - q.un[1]);
+  const double cs2 = cspeed * cspeed;
+  const double d0 = mc_limiter_plain(hl - wl, hr - wr);
+  const double d1 = mc_limiter_plain((q.rho[1] - q.rho[0]) - dpl / cs2, (q.rho[2] - q.rho[1]) - dpr / cs2);
+  const double d2 = mc_limiter_plain(hl + wl, hr + wr);
+  const double csr = c0 + 1.e-40, s02 = d0 + d2;
+  o[SL_A] = s02 / csr + d1;
+  o[SL_B] = (d2 - d0) / q.rho[1];
+  o[SL_C] = s02 * csr;
+  o[SL_T1] = mc_limiter_plain(q.t1[1] - q.t1[0], q.t1[2] - q.t1[1]);
+  o[SL_T2] = mc_limiter_plain(q.t2[1] - q.t2[0], q.t2[2] - q.t2[1]);
+  if (up) {
+    const double csl = sqrt(gR * q.Tup) + 1.e-40;
+    o[SL_AL] = s02 / csl + d1;
+    o[SL_CL] = s02 * csl;
+  }
+}
+
+// 0.5 x for a zero or normal x well above the smallest
+__device__ __forceinline__ double half_of(double x) {
+  const DWords w = dwords(x);
+  return dfrom(((w.hi & 0x7FFFFFFFu) | w.lo) == 0u ? w.hi : w.hi - (1u << 20), w.lo);
+}
+
+// The same bits on the integer pipe where the ranges hold.  c0 >= 2^-78 makes
+// c0 + 1e-40 = c0 + 2e-40 = c0; the halves of d0 and d2 are taken at the end
+// (the limiter and the sums scale exactly), so dp / c and rho du enter whole.
+__device__ __forceinline__ void slope_terms(const SlopeQ& q, double gR, double tiny, bool up, double o[NSLOPE]) {
+  IntOps I;
+#pragma unroll
+  for (int n = 0; n < 3; ++n) { I.pos(q.rho[n]); I.pos(q.p[n]); I.vel(q.un[n]); I.vel(q.t1[n]); I.vel(q.t2[n]); }
+  I.pos(gR); I.pos(q.T);
+  const double c = I.root(I.mul(gR, q.T));
+  I.ok = I.ok && dwords(c).hi >= (945u << 20);
+  const double dpl = q.p[1] - q.p[0], dpr = q.p[2] - q.p[1];
+  const double hl = I.divz(dpl, c), hr = I.divz(dpr, c);
+  const double wl = I.mulz(q.rho[1], q.un[1] - q.un[0]), wr = I.mulz(q.rho[1], q.un[2] - q.un[1]);
+  const double cs2 = I.mul(c, c);
+  const double d0 = mc_limiter(hl - wl, hr - wr), d2 = mc_limiter(hl + wl, hr + wr);  // doubled
+  const double d1 = mc_limiter((q.rho[1] - q.rho[0]) - I.divz(dpl, cs2), (q.rho[2] - q.rho[1]) - I.divz(dpr, cs2));
+  const double s02 = d0 + d2;
+  o[SL_A] = fma(0.5, I.divz(s02, c), d1);
+  o[SL_B] = half_of(I.divz(d2 - d0, q.rho[1]));
+  o[SL_C] = half_of(I.mulz(c, s02));
+  o[SL_T1] = mc_limiter(q.t1[1] - q.t1[0], q.t1[2] - q.t1[1]);
+  o[SL_T2] = mc_limiter(q.t2[1] - q.t2[0], q.t2[2] - q.t2[1]);
+  if (up) {
+    I.pos(q.Tup);
+    const double cl = I.root(I.mul(gR, q.Tup));
+    I.ok = I.ok && dwords(cl).hi >= (945u << 20);
+    o[SL_AL] = fma(0.5, I.divz(s02, cl), d1);
+    o[SL_CL] = half_of(I.mulz(cl, s02));
+  }
+  if (!I.ok) {
+    const SlopeQ a = q;
+    double r[NSLOPE];
+    slope_plain(a, gR, tiny, up, r);
+#pragma unroll
+    for (int n = 0; n < SL_AL; ++n) o[n] = r[n];
+    if (up) { o[SL_AL] = r[SL_AL]; o[SL_CL] = r[SL_CL]; }
+  }
+}
+
+// Bound: both pipes (25 FP64 instructions, six quotients, a root and six
+// products per cell and direction; the limiters' comparisons and scalings by
+// two were 40 further FP64 instructions).  48^3, inviscid: 64 -> 28 us; four CTAs
+// per SM 2.5% faster than two over the step.
+__global__ void __launch_bounds__(256, 4) slope_kernel(BoxTable tb, FaceTable ft, const long long* spre0,
                                                     const long long* spre1, const long long* spre2,
                                                     long long tot0, long long tot1, long long tot2) {
   if (list_idle(tb)) return;
@@ -461,91 +602,68 @@ __global__ void __launch_bounds__(256) slope_kernel(BoxTable tb, FaceTable ft, c
     const DArr q = R.q;
     const DClosures& cl = tb.cls[R.cl];
     const long long s = (d == 0) ? 1 : (d == 1 ? q.js : q.ks);
-    const long long o = q.off(i, j, k);
+    const double* Q = q.p + q.off(i, j, k);
     const int QN = QU + d, QT1 = (d == 0) ? QV : QU, QT2 = (d == 2) ? QV : QW;
-    auto Q = [&](long long off, int n) { return q.p[off + n * q.ns]; };
-    const double c0 = sqrt_sel<AMRS_SLOPE_ISQRT>(cl.gamma * cl.Rspec * Q(o, QT));
-    const double cspeed = c0 + (d == 0 ? 2.e-40 : 1.e-40);
-    double dlft = ddiv_rn(0.5 * (Q(o, QPRES) - Q(o - s, QPRES)), cspeed) - 0.5 * Q(o, QRHO) * (Q(o, QN) - Q(o - s, QN));
-    double drgt = ddiv_rn(0.5 * (Q(o + s, QPRES) - Q(o, QPRES)), cspeed) - 0.5 * Q(o, QRHO) * (Q(o + s, QN) - Q(o, QN));
-    const double d0 = mc_limiter(dlft, drgt);
-    const double cs2 = cspeed * cspeed;
-    dlft = (Q(o, QRHO) - Q(o - s, QRHO)) - ddiv_rn(Q(o, QPRES) - Q(o - s, QPRES), cs2);
-    drgt = (Q(o + s, QRHO) - Q(o, QRHO)) - ddiv_rn(Q(o + s, QPRES) - Q(o, QPRES), cs2);
-    const double d1 = mc_limiter(dlft, drgt);
-    dlft = ddiv_rn(0.5 * (Q(o, QPRES) - Q(o - s, QPRES)), cspeed) + 0.5 * Q(o, QRHO) * (Q(o, QN) - Q(o - s, QN));
-    drgt = ddiv_rn(0.5 * (Q(o + s, QPRES) - Q(o, QPRES)), cspeed) + 0.5 * Q(o, QRHO) * (Q(o + s, QN) - Q(o, QN));
-    const double d2 = mc_limiter(dlft, drgt);
-    const double d3 = mc_limiter(Q(o, QT1) - Q(o - s, QT1), Q(o + s, QT1) - Q(o, QT1));
-    const double d4 = mc_limiter(Q(o, QT2) - Q(o - s, QT2), Q(o + s, QT2) - Q(o, QT2));
-    // The terms of this cell's extrapolations to its two faces
-    // (src/rhs/Riemann.h:251-337), formed once here instead of once per face
-    // side: A = (d0+d2)/c + d1 (density), B = (d2-d0)/rho (normal velocity),
-    // C = (d0+d2)*c (pressure), c the cell's sqrt(gamma R T) + 1e-40.
-    const double csr = c0 + 1.e-40;
-    const double s02 = d0 + d2;
+    const bool up = d == 2 && k <= R.hi[2];
+    SlopeQ v;
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      const double* c = Q + (n - 1) * s;
+      v.rho[n] = c[QRHO * q.ns];
+      v.un[n] = c[QN * q.ns];
+      v.p[n] = c[QPRES * q.ns];
+      v.t1[n] = c[QT1 * q.ns];
+      v.t2[n] = c[QT2 * q.ns];
+    }
+    v.T = Q[QT * q.ns];
+    v.Tup = up ? Q[2 * s + QT * q.ns] : v.T;
+    double o[NSLOPE];
+    slope_terms(v, cl.gamma * cl.Rspec, d == 0 ? 2.e-40 : 1.e-40, up, o);
     const DArr S = ft.fr[b].slope[d];
-    const long long os = S.off(i, j, k);
-    S.p[os + SL_A * S.ns] = ddiv_rn(s02, csr) + d1;
-    S.p[os + SL_B * S.ns] = ddiv_rn(d2 - d0, Q(o, QRHO));
-    S.p[os + SL_C * S.ns] = s02 * csr;
-    S.p[os + SL_T1 * S.ns] = d3;
-    S.p[os + SL_T2 * S.ns] = d4;
-    if (d == 2 && k <= R.hi[2]) {
-      // cns_riemann_z's left state takes its sound speed from q(i,j,k+1)
-      // (src/rhs/Riemann.h:316): for the face above this cell, cell k + 2
-      const double csl = sqrt_sel<AMRS_SLOPE_ISQRT>(cl.gamma * cl.Rspec * Q(o + 2 * s, QT)) + 1.e-40;
-      S.p[os + SL_AL * S.ns] = ddiv_rn(s02, csl) + d1;
-      S.p[os + SL_CL * S.ns] = s02 * csl;
+    double* so = S.p + S.off(i, j, k);
+#pragma unroll
+    for (int n = 0; n < SL_AL; ++n) so[n * S.ns] = o[n];
+    if (up) {
+      so[SL_AL * S.ns] = o[SL_AL];
+      so[SL_CL * S.ns] = o[SL_CL];
     }
   }
 }
 
-// Division of the two-shock solver: IDIV picks the integer-pipe form
-// (ddiv_rn) or the hardware one; both give the same correctly rounded bits.
-template <bool IDIV>
-__device__ __forceinline__ double rdiv(double a, double b) {
-  return IDIV ? ddiv_rn(a, b) : a / b;
-}
-
-// Two-shock approximate Riemann solver (src/rhs/Riemann.h:123-249).  Its
-// pressure iterations are one serial chain per face, so the choice of
-// division is the caller's: the MUSCL face kernel runs faster with the
-// integer-pipe division, the WENO5-Riemann kernel (whose reconstructions
-// already load the integer pipe) with the hardware one; the square roots are
-// the hardware's in both (AMRS_RS_ISQRT: their integer form lengthens the
-// chain at the 128^3 and 256^3 sizes, though it shortens it at 64^3).
-template <bool IDIV>
-__device__ void riemann_prob(const double gamma, const double smallp, const double rl, const double ul,
-                             const double pl, const double ut1l, const double ut2l, const double rr, const double ur,
-                             const double pr, const double ut1r, const double ut2r, double& flxrho, double& flxu,
-                             double& flxut, double& flxutt, double& flxe) {
+// Two-shock approximate Riemann solver (src/rhs/Riemann.h:123-249) with the
+// hardware's operations, out of line: for the faces riemann_prob does not
+// cover.  in = (rl, ul, pl, ut1l, ut2l, rr, ur, pr, ut1r, ut2r), out =
+// (flxrho, flxu, flxut, flxutt, flxe).
+static __device__ __noinline__ void riemann_plain(const double gamma, const double smallp, const double* in,
+                                                  double* out) {
+  const double rl = in[0], ul = in[1], pl = in[2], ut1l = in[3], ut2l = in[4];
+  const double rr = in[5], ur = in[6], pr = in[7], ut1r = in[8], ut2r = in[9];
   const double weakwv = 1.e-3;
   const double small = 1.e-6;
   const double clsql = gamma * pl * rl;
   const double clsqr = gamma * pr * rr;
-  double wl = sqrt_sel<AMRS_RS_ISQRT>(clsql);
-  double wr = sqrt_sel<AMRS_RS_ISQRT>(clsqr);
-  const double cleft = rdiv<IDIV>(wl, rl);
-  const double cright = rdiv<IDIV>(wr, rr);
+  double wl = sqrt(clsql);
+  double wr = sqrt(clsqr);
+  const double cleft = ((wl) / (rl));
+  const double cright = ((wr) / (rr));
   const double ccsmall = small * (cleft + cright);
-  double pstar = rdiv<IDIV>(wl * pr + wr * pl - wr * wl * (ur - ul), wl + wr);
+  double pstar = ((wl * pr + wr * pl - wr * wl * (ur - ul)) / (wl + wr));
   pstar = rmax(pstar, smallp);
   double pstnm1 = pstar;
   double wlsq = (0.5 * (gamma - 1.) * (pstar + pl) + pstar) * rl;
   double wrsq = (0.5 * (gamma - 1.) * (pstar + pr) + pstar) * rr;
-  wl = sqrt_sel<AMRS_RS_ISQRT>(wlsq);
-  wr = sqrt_sel<AMRS_RS_ISQRT>(wrsq);
-  double ustarp = ul - rdiv<IDIV>(pstar - pl, wl);
-  double ustarm = ur + rdiv<IDIV>(pstar - pr, wr);
-  pstar = rdiv<IDIV>(wl * pr + wr * pl - wr * wl * (ur - ul), wl + wr);
+  wl = sqrt(wlsq);
+  wr = sqrt(wrsq);
+  double ustarp = ul - ((pstar - pl) / (wl));
+  double ustarm = ur + ((pstar - pr) / (wr));
+  pstar = ((wl * pr + wr * pl - wr * wl * (ur - ul)) / (wl + wr));
   pstar = rmax(pstar, smallp);
   double ustar = 0.0;
   for (int iter = 0; iter < 3; ++iter) {
     wlsq = (0.5 * (gamma - 1.) * (pstar + pl) + pstar) * rl;
     wrsq = (0.5 * (gamma - 1.) * (pstar + pr) + pstar) * rr;
-    wl = rdiv<IDIV>(1., sqrt_sel<AMRS_RS_ISQRT>(wlsq));
-    wr = rdiv<IDIV>(1., sqrt_sel<AMRS_RS_ISQRT>(wrsq));
+    wl = ((1.) / (sqrt(wlsq)));
+    wr = ((1.) / (sqrt(wrsq)));
     const double ustnm1 = ustarm;
     const double ustnp1 = ustarp;
     ustarm = ur - (pr - pstar) * wr;
@@ -556,7 +674,7 @@ __device__ void riemann_prob(const double gamma, const double smallp, const doub
     double zm = fabs(ustarm - ustnm1);
     if (zm - weakwv * cright < 0.0) zm = dpditer * wr;
     const double zz = zp + zm;
-    const double denom = rdiv<IDIV>(dpditer, rmax(zz, ccsmall));
+    const double denom = ((dpditer) / (rmax(zz, ccsmall)));
     pstnm1 = pstar;
     pstar = pstar - denom * (ustarm - ustarp);
     pstar = rmax(pstar, smallp);
@@ -570,7 +688,7 @@ __device__ void riemann_prob(const double gamma, const double smallp, const doub
   } else {
     uo = 0.5 * (ur + ul);
     po = 0.5 * (pr + pl);
-    ro = rdiv<IDIV>(2. * (rl * rr), rl + rr);
+    ro = ((2. * (rl * rr)) / (rl + rr));
     sgnm = 1.;
     utrans1 = 0.5 * (ut1l + ut1r);
     utrans2 = 0.5 * (ut2l + ut2r);
@@ -584,25 +702,25 @@ __device__ void riemann_prob(const double gamma, const double smallp, const doub
   // (same operations, same values, same selection, NaN included).
   auto mixed = [&](double spin, double spout, double rstar) {
     const double ss = rmax(spout - spin, spout + spin);
-    const double frac = 0.5 * (1. + rdiv<IDIV>(spin + spout, rmax(ss, ccsmall)));
+    const double frac = 0.5 * (1. + ((spin + spout) / (rmax(ss, ccsmall))));
     rgdnv = frac * rstar + (1. - frac) * ro;
     ugdnv = frac * ustar + (1. - frac) * uo;
     pgdnv = frac * pstar + (1. - frac) * po;
   };
   if (pstar >= po) {
     // shock: spout == spin, so the side state or the star state
-    const double spin = rdiv<IDIV>(sqrt_sel<AMRS_RS_ISQRT>(wosq), ro) - suo;
+    const double spin = ((sqrt(wosq)) / (ro)) - suo;
     if (spin < 0.) {
       rgdnv = ro; ugdnv = uo; pgdnv = po;
     } else if (spin >= 0.) {
-      rgdnv = rdiv<IDIV>(ro, 1. - rdiv<IDIV>(ro * dpjmp, wosq)); ugdnv = ustar; pgdnv = pstar;
+      rgdnv = ((ro) / (1. - ((ro * dpjmp) / (wosq)))); ugdnv = ustar; pgdnv = pstar;
     } else {
-      mixed(spin, spin, rdiv<IDIV>(ro, 1. - rdiv<IDIV>(ro * dpjmp, wosq)));
+      mixed(spin, spin, ((ro) / (1. - ((ro * dpjmp) / (wosq)))));
     }
   } else {
-    const double rstar = rdiv<IDIV>(ro, 1. - rdiv<IDIV>(ro * dpjmp, wosq));
-    const double spout = sqrt_sel<AMRS_RS_ISQRT>(rdiv<IDIV>(gamma * po, ro)) - suo;
-    const double spin = sqrt_sel<AMRS_RS_ISQRT>(rdiv<IDIV>(gamma * pstar, rstar)) - suo;
+    const double rstar = ((ro) / (1. - ((ro * dpjmp) / (wosq))));
+    const double spout = sqrt(((gamma * po) / (ro))) - suo;
+    const double spin = sqrt(((gamma * pstar) / (rstar))) - suo;
     if (spout < 0.) {
       rgdnv = ro; ugdnv = uo; pgdnv = po;
     } else if (spin >= 0.) {
@@ -611,17 +729,131 @@ __device__ void riemann_prob(const double gamma, const double smallp, const doub
       mixed(spin, spout, rstar);
     }
   }
-  flxrho = rgdnv * ugdnv;
-  flxu = rgdnv * ugdnv * ugdnv + pgdnv;
-  flxut = rgdnv * ugdnv * utrans1;
-  flxutt = rgdnv * ugdnv * utrans2;
+  out[0] = rgdnv * ugdnv;
+  out[1] = rgdnv * ugdnv * ugdnv + pgdnv;
+  out[2] = rgdnv * ugdnv * utrans1;
+  out[3] = rgdnv * ugdnv * utrans2;
   // (0.5*r)*k + x == fma(0.5, r*k, x): the halving is exact (normal range)
-  flxe = ugdnv * (fma(0.5, rgdnv * (ugdnv * ugdnv + utrans1 * utrans1 + utrans2 * utrans2), rdiv<IDIV>(pgdnv, gamma - 1.)) +
+  out[4] = ugdnv * (fma(0.5, rgdnv * (ugdnv * ugdnv + utrans1 * utrans1 + utrans2 * utrans2), ((pgdnv) / (gamma - 1.))) +
                   pgdnv);
 }
 
-// MUSCL face states + Riemann flux (src/rhs/Riemann.h:251-337).
-__global__ void __launch_bounds__(256) riemann_face_kernel(BoxTable tb, FaceTable ft, long long total) {
+// The same solver, same bits, with its quotients and roots and most of its
+// products on the integer pipe.  The faces whose states are all in the tested
+// ranges (densities and pressures in 2^+-150, velocities zero or in 2^+-100, star
+// pressure finite and, after its floor, below 2^150) need no range test in any
+// operation: every intermediate then stays well inside the normal range.
+// Comparisons of values of known sign are integer comparisons of their bits.
+// A transonic fan, a star state outside the ranges and the one quotient or
+// root in 2^28 that the truncated value cannot round take riemann_plain.
+// 72 FP64 instructions (sums, the flux products) and 17 quotients, 11 roots and
+// 60 products on the integer pipe; with the products on the FP64 pipe the MUSCL
+// step at 96^3 takes 3.61 ms instead of 2.94, with any one group of them 2-13%
+// more.
+__device__ __forceinline__ void riemann_prob(const double gamma, const double smallp, const double in[10],
+                                             double out[5]) {
+  const double rl = in[0], ul = in[1], pl = in[2], ut1l = in[3], ut2l = in[4];
+  const double rr = in[5], ur = in[6], pr = in[7], ut1r = in[8], ut2r = in[9];
+  IntOps R;
+  R.pos(rl); R.pos(pl); R.pos(rr); R.pos(pr);
+  R.vel(ul); R.vel(ur); R.vel(ut1l); R.vel(ut2l); R.vel(ut1r); R.vel(ut2r);
+  auto bits = [](double x) { return __double_as_longlong(x); };
+  const double hg = 0.5 * (gamma - 1.);
+  R.pos(gamma); R.pos(hg);
+  double wl = R.root(R.mul(R.mul(gamma, pl), rl));
+  double wr = R.root(R.mul(R.mul(gamma, pr), rr));
+  const double cleft = R.div(wl, rl), cright = R.div(wr, rr);
+  const double wkl = R.mul(1.e-3, cleft), wkr = R.mul(1.e-3, cright);
+  const double ccsmall = R.mul(1.e-6, cleft + cright);
+  const double du = ur - ul;
+  auto star = [&]() {
+    const double num = R.mul(wl, pr) + R.mul(wr, pl) - R.mulz(R.mul(wr, wl), du);
+    return R.floor_p(R.divz(num, wl + wr), smallp);
+  };
+  auto wsq = [&](double ps, double p, double r) { return R.mul(R.mul(hg, ps + p) + ps, r); };
+  double pstar = star();
+  double pstnm1 = pstar;
+  wl = R.root(wsq(pstar, pl, rl));
+  wr = R.root(wsq(pstar, pr, rr));
+  double ustarp = ul - R.divz(pstar - pl, wl);
+  double ustarm = ur + R.divz(pstar - pr, wr);
+  pstar = star();
+#pragma unroll 1
+  for (int iter = 0; iter < 3; ++iter) {
+    wl = R.div(1., R.root(wsq(pstar, pl, rl)));
+    wr = R.div(1., R.root(wsq(pstar, pr, rr)));
+    const double ustnm1 = ustarm, ustnp1 = ustarp;
+    ustarm = ur - R.mulz(wr, pr - pstar);
+    ustarp = ul + R.mulz(wl, pl - pstar);
+    const double dpditer = fabs(pstnm1 - pstar);
+    // zp - weakwv * cleft < 0 exactly when zp < weakwv * cleft, both >= 0
+    double zp = fabs(ustarp - ustnp1), zm = fabs(ustarm - ustnm1);
+    if (bits(zp) < bits(wkl)) zp = R.mulz(wl, dpditer);
+    if (bits(zm) < bits(wkr)) zm = R.mulz(wr, dpditer);
+    const double zz = zp + zm;
+    const double denom = R.divz(dpditer, bits(zz) < bits(ccsmall) ? ccsmall : zz);
+    pstnm1 = pstar;
+    // (a product with a factor that may be zero on either side: on the FP64 pipe)
+    pstar = R.floor_p(pstar - denom * (ustarm - ustarp), smallp);
+  }
+  const double ustar = 0.5 * (ustarm + ustarp);
+  double ro, uo, po, utrans1, utrans2;
+  const bool right = bits(ustar) < 0 && (bits(ustar) << 1) != 0;
+  double suo;
+  if (right) {
+    ro = rr; uo = ur; po = pr; utrans1 = ut1r; utrans2 = ut2r;
+    suo = -uo;
+  } else {
+    ro = rl; uo = ul; po = pl; utrans1 = ut1l; utrans2 = ut2l;
+    if ((bits(ustar) << 1) == 0) {
+      uo = 0.5 * (ur + ul);
+      po = 0.5 * (pr + pl);
+      ro = R.div(2. * (rl * rr), rl + rr);
+      utrans1 = 0.5 * (ut1l + ut1r);
+      utrans2 = 0.5 * (ut2l + ut2r);
+    }
+    suo = uo;
+  }
+  const double wosq = wsq(pstar, po, ro);
+  const double dpjmp = pstar - po;
+  const double den = 1. - R.divz(R.mulz(ro, dpjmp), wosq);
+  const double rstar = R.div(ro, den);
+  R.pos(den); R.pos(rstar);
+  double spin, spout;
+  if (bits(pstar) >= bits(po)) {
+    spin = spout = R.div(R.root(wosq), ro) - suo;
+  } else {
+    spout = R.root(R.div(R.mul(gamma, po), ro)) - suo;
+    spin = R.root(R.div(R.mul(gamma, pstar), rstar)) - suo;
+  }
+  double rg = rstar, ug = ustar, pg = pstar;
+  if (bits(spout) < 0) {
+    rg = ro; ug = uo; pg = po;
+  } else if (bits(spin) < 0) {
+    R.ok = false;  // inside a transonic fan
+  }
+  const double m = R.mulz(rg, ug);
+  out[0] = m;
+  out[1] = m * ug + pg;
+  out[2] = m * utrans1;
+  out[3] = m * utrans2;
+  out[4] = ug * (fma(0.5, R.mulz(rg, ug * ug + utrans1 * utrans1 + utrans2 * utrans2), R.div(pg, gamma - 1.)) + pg);
+  if (!R.ok) {
+    double a[10], o[5];
+#pragma unroll
+    for (int n = 0; n < 10; ++n) a[n] = in[n];
+    riemann_plain(gamma, smallp, a, o);
+#pragma unroll
+    for (int n = 0; n < 5; ++n) out[n] = o[n];
+  }
+}
+
+// MUSCL face states + Riemann flux (src/rhs/Riemann.h:251-337).  Bound: the
+// solver's serial chain of quotients and roots, with both the FP64 and the
+// integer pipe about half full; two CTAs per SM (128 registers) beat three
+// (2.94 against 3.10 ms per step at 96^3).  48^3, with the hardware's roots and
+// products and checked integer quotients before: 194 -> 86 us.
+__global__ void __launch_bounds__(256, 2) riemann_face_kernel(BoxTable tb, FaceTable ft, long long total) {
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
@@ -644,25 +876,25 @@ __global__ void __launch_bounds__(256) riemann_face_kernel(BoxTable tb, FaceTabl
     // slope_kernel formed (z: the left terms with the quirk's sound speed);
     // q + 0.5*t == fma(0.5, t, q): the halving is exact (normal range)
     const int cA = (d == 2) ? SL_AL : SL_A, cC = (d == 2) ? SL_CL : SL_C;
-    const double rl = rmax(fma(0.5, D(osm, cA), Q(oqm, QRHO)), 1.0e-40);
-    const double ul = fma(0.5, D(osm, SL_B), Q(oqm, QN));
-    const double pl = rmax(fma(0.5, D(osm, cC), Q(oqm, QPRES)), 1.0e-40);
-    const double ut1l = fma(0.5, D(osm, SL_T1), Q(oqm, QT1));
-    const double ut2l = fma(0.5, D(osm, SL_T2), Q(oqm, QT2));
-    const double rr = rmax(fma(-0.5, D(os, SL_A), Q(oq, QRHO)), 1.0e-40);
-    const double ur = fma(-0.5, D(os, SL_B), Q(oq, QN));
-    const double pr = rmax(fma(-0.5, D(os, SL_C), Q(oq, QPRES)), 1.0e-40);
-    const double ut1r = fma(-0.5, D(os, SL_T1), Q(oq, QT1));
-    const double ut2r = fma(-0.5, D(os, SL_T2), Q(oq, QT2));
-    double frho, fu, fut, futt, fe;
-    riemann_prob<true>(gam, 1.0e-40, rl, ul, pl, ut1l, ut2l, rr, ur, pr, ut1r, ut2r, frho, fu, fut, futt, fe);
+    const double in[10] = {rmax(fma(0.5, D(osm, cA), Q(oqm, QRHO)), 1.0e-40),
+                           fma(0.5, D(osm, SL_B), Q(oqm, QN)),
+                           rmax(fma(0.5, D(osm, cC), Q(oqm, QPRES)), 1.0e-40),
+                           fma(0.5, D(osm, SL_T1), Q(oqm, QT1)),
+                           fma(0.5, D(osm, SL_T2), Q(oqm, QT2)),
+                           rmax(fma(-0.5, D(os, SL_A), Q(oq, QRHO)), 1.0e-40),
+                           fma(-0.5, D(os, SL_B), Q(oq, QN)),
+                           rmax(fma(-0.5, D(os, SL_C), Q(oq, QPRES)), 1.0e-40),
+                           fma(-0.5, D(os, SL_T1), Q(oq, QT1)),
+                           fma(-0.5, D(os, SL_T2), Q(oq, QT2))};
+    double F[5];
+    riemann_prob(gam, 1.0e-40, in, F);
     const DArr Fd = ft.fr[f.b].f[d];
     const long long of = Fd.off(f.i, f.j, f.k);
-    Fd.p[of + URHO * Fd.ns] = frho;
-    Fd.p[of + UN * Fd.ns] = fu;
-    Fd.p[of + UT1 * Fd.ns] = fut;
-    Fd.p[of + UT2 * Fd.ns] = futt;
-    Fd.p[of + UET * Fd.ns] = fe;
+    Fd.p[of + URHO * Fd.ns] = F[0];
+    Fd.p[of + UN * Fd.ns] = F[1];
+    Fd.p[of + UT1 * Fd.ns] = F[2];
+    Fd.p[of + UT2 * Fd.ns] = F[3];
+    Fd.p[of + UET * Fd.ns] = F[4];
   }
 }
 
@@ -698,16 +930,17 @@ __global__ void __launch_bounds__(256) weno_riemann_face_kernel(BoxTable tb, Fac
       lft[m] = weno5js<AMRS_WRREC_IMUL>(v[0], v[1], v[2], v[3], v[4]);
       rgt[m] = weno5js<AMRS_WRREC_IMUL>(v[5], v[4], v[3], v[2], v[1]);
     }
-    double frho, fu, fut, futt, fe;
-    riemann_prob<AMRS_WR_IDIV != 0>(cl.gamma, 1.0e-40, rmax(lft[0], 1.0e-40), lft[1], rmax(lft[2], 1.0e-40), lft[3], lft[4],
-                        rmax(rgt[0], 1.0e-40), rgt[1], rmax(rgt[2], 1.0e-40), rgt[3], rgt[4], frho, fu, fut, futt, fe);
+    const double in[10] = {rmax(lft[0], 1.0e-40), lft[1], rmax(lft[2], 1.0e-40), lft[3], lft[4],
+                           rmax(rgt[0], 1.0e-40), rgt[1], rmax(rgt[2], 1.0e-40), rgt[3], rgt[4]};
+    double F[5];
+    riemann_prob(cl.gamma, 1.0e-40, in, F);
     const DArr Fd = ft.fr[f.b].f[d];
     const long long of = Fd.off(f.i, f.j, f.k);
-    Fd.p[of + URHO * Fd.ns] = frho;
-    Fd.p[of + UN * Fd.ns] = fu;
-    Fd.p[of + UT1 * Fd.ns] = fut;
-    Fd.p[of + UT2 * Fd.ns] = futt;
-    Fd.p[of + UET * Fd.ns] = fe;
+    Fd.p[of + URHO * Fd.ns] = F[0];
+    Fd.p[of + UN * Fd.ns] = F[1];
+    Fd.p[of + UT1 * Fd.ns] = F[2];
+    Fd.p[of + UT2 * Fd.ns] = F[3];
+    Fd.p[of + UET * Fd.ns] = F[4];
   }
 }
 
