@@ -1,17 +1,11 @@
-"""Autotuner of the fused face kernel: tile shape per box-size class and the
-schedule's thread coarsening, timed on the real box list.
+"""Autotuner of the fused face kernels' schedule, timed on the real box list.
 
-The fused KEEP face kernel tiles each box's (x, y) extent into tx x ty
-columns (tx * ty <= 256 threads) and streams z through shared memory; a
-host-built schedule cuts the (tile column x plane) work of all boxes into
-`waves` x (resident CTAs) shares.  Two knobs therefore set how the work
-maps onto threads:
-
-* tile shape per (nx, ny) class: partial tiles idle lanes, narrow tiles
-  recompute more x/y pair terms at tile edges;
-* waves (z coarsening): one wave gives every CTA one long z run, so each
-  thread streams the most planes per z prologue; more waves give shorter
-  runs that CTAs pick up as others finish.
+The y and z marches of the fused KEEP path cut the (column block x cell) work
+of all boxes into equal shares, one per warp, up to `waves` x (resident warps):
+one wave gives every warp the longest run, so the fewest prologues; more waves
+give shorter runs that CTAs pick up as others finish.  The tile shapes of the
+sweep are recorded with the list; the kernels deal columns and rows to warps
+whatever they are, so only the waves change the time.
 
 The reference has no counterpart: its only tiling knob is MFIter over the
 boxes of max_grid_size (src/tim/CNS_advance.cpp:200).

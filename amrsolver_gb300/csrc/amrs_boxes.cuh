@@ -15,9 +15,9 @@ struct BoxRec {
   DArr slot[MAX_SLOTS];  // caller-owned ghosted state arrays (3 ghosts)
   DArr q;                // primitives scratch over grow(box,3), NQ comps
   DArr vf;               // viscous cell fluxes over grow(box,1), NVF comps
+  DArr div;              // KEEP path: y and z parts of the divergence, valid box, 2 NCONS comps
   int cl;                // closure index
-  int tx, ty, kc;        // tile shape and z chunk of the face kernel
-  int ntx, nty, nkz;     // tiles per direction
+  int tx, ty, kc;        // tile of the tuning interface (recorded; the marches deal columns to warps)
   // y walls of boundary code 6 that this box touches (walls == 0: none):
   // viscous cell fluxes of rows wrow_lo / wrow_hi use one-sided y
   // derivatives (ViscousWallFluxes); KEEP y faces j <= red_lo or
@@ -32,15 +32,21 @@ struct BoxTable {
   const BoxRec* box;
   const long long* pcell;  // prefix of primitive-region cells, size n+1
   const long long* vcell;  // prefix of viscous-region cells, size n+1
-  const int* fwork;        // prefix of face-kernel work items, size n+1 (unused by the balanced schedule)
-  const int4* seg;         // face-kernel segments: (box, tile index, k0, k1)
-  const int* cta_seg;      // segments of CTA c: [cta_seg[c], cta_seg[c+1])
+  const int* fwork;        // prefix of the KEEP x kernel's blocks, size n+1
+  const int4* seg;         // KEEP march segments: (box, 2 * column block + (dir - 1), m0, m1)
+  const int* share;        // segments of warp w: [share[w], share[w+1])
+  int nshare;
   const DClosures* cls;
   int n;
   int gq;                  // ghost depth of the primitive region
   // device-resident time loop: every kernel of a step returns at once while
   // *active == 0 (steps after the stop time); null outside such loops
   const int* active;
+  // raised by the primitives' kernel where a cell is outside keep_range; the
+  // face kernel of the same stage reads it (raised or null: every product on
+  // the FP64 pipe) and clears the other of the pair, the next stage's
+  int* range;
+  int* range_next;
 };
 
 __device__ __forceinline__ bool list_idle(const BoxTable& tb) { return tb.active && *tb.active == 0; }

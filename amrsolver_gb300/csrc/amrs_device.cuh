@@ -97,7 +97,7 @@ __device__ __forceinline__ double kmul(double a, double b) {
 #endif
 // Viscous cell-flux products on the integer pipe (see viscous_cell_dy).
 #ifndef AMRS_VISC_IMUL
-#define AMRS_VISC_IMUL 0x17
+#define AMRS_VISC_IMUL 0x3F
 #endif
 
 // cons2prim (src/rhs/CNS_hydro_K.h:15-34) plus QE = cv*T.
@@ -122,22 +122,43 @@ __device__ __forceinline__ void cons2prim(const double u[5], double q[NQ], const
   q[QE] = kmul<(M >> 3) & 1>(c.cv, q[QT]);
 }
 
+// Ranges in which keep_pair<D, true> holds, tested once per cell where the
+// primitives are formed: density, pressure and energy in [2^-100, 2^100),
+// velocities zero or in [2^-200, 2^100).  Every product of a pair then stays well
+// inside the normal range (the smallest, P times the velocity products' sum,
+// above 2^-810).
+__device__ __forceinline__ bool keep_range(const double q[NQ]) {
+  bool ok = true;
+#pragma unroll
+  for (int n = 0; n < NQ; ++n) {
+    const DWords w = dwords(q[n]);
+    if (n == QU || n == QV || n == QW)
+      ok = ok && (w.hi * 2u - (823u << 21) < (300u << 21) || ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u);
+    else if (n != QT)
+      ok = ok && w.hi - (923u << 20) < (200u << 20);
+  }
+  return ok;
+}
+
+__device__ __forceinline__ bool is_zero(double x) {
+  const DWords w = dwords(x);
+  return ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
+}
+// a * b on the integer pipe without range tests, +-0 where `zero`.
+__device__ __forceinline__ double mul_core(double a, double b) { return dfrom(dmul_core(dwords(a), dwords(b))); }
+__device__ __forceinline__ double mul_zero(double a, double b, bool zero) {
+  const DWords x = dwords(a), y = dwords(b);
+  const DWords r = dmul_core(x, y);
+  return dfrom(zero ? (x.hi ^ y.hi) & 0x80000000u : r.hi, zero ? 0u : r.lo);
+}
+
 // One KEEP pair term (src/rhs/CentralKEEP.h:19-36 helpers, :76-83 body),
 // already multiplied by its coefficient: the contribution of pair
 // (point 1 = larger index, point 2 = smaller index) to the face flux in
-// direction d.  q1/q2 give rho,u,v,w,T,p,e.
-//
-// IM selects, bit by bit, the products formed on the integer pipe
-// (dmul_rn, the same correctly rounded product): 0 P, 1-3 the three
-// products of s3, 4-7 the momentum and energy cubic products, 8-9 the two
-// products of pu, 10-14 the coefficient scalings of the five components,
-// 15 P s3.  The FP64 pipe is the bound of the kernels calling this, and the
-// integer pipe is otherwise idle in them, so moving part of the products
-// there shortens the FP64 stream without changing a bit of the result.
-#ifndef AMRS_KEEP_IMUL
-#define AMRS_KEEP_IMUL 0x7C00
-#endif
-template <int D, int IM = AMRS_KEEP_IMUL>
+// direction d.  q1/q2 give rho,u,v,w,T,p,e.  FAST: both points are in the ranges
+// of keep_range, and the sixteen products run on the integer pipe (the same
+// correctly rounded products); otherwise every operation on the FP64 pipe.
+template <int D, bool FAST = false>
 __device__ __forceinline__ void keep_pair(const double* q1, const double* q2, double coef, double T[5]) {
   constexpr int QN = QU + D;
   const double rhoS = q1[QRHO] + q2[QRHO];
@@ -153,20 +174,45 @@ __device__ __forceinline__ void keep_pair(const double* q1, const double* q2, do
   // So coef*(...) == (coef/8)*(...) with the eighths taken out, and no
   // FP64 instruction is spent on a power-of-two scaling.
   const double c8 = 0.125 * coef, c4 = 0.25 * coef;
-  const double P = kmul<(IM >> 0) & 1>(rhoS, unS);
-  const double s3 = kmul<(IM >> 1) & 1>(q1[QU], q2[QU]) + kmul<(IM >> 2) & 1>(q1[QV], q2[QV]) +
-                    kmul<(IM >> 3) & 1>(q1[QW], q2[QW]);
-  const double cx = kmul<(IM >> 4) & 1>(P, q1[QU] + q2[QU]);
-  const double cy = kmul<(IM >> 5) & 1>(P, q1[QV] + q2[QV]);
-  const double cz = kmul<(IM >> 6) & 1>(P, q1[QW] + q2[QW]);
-  const double ce = kmul<(IM >> 7) & 1>(P, q1[QE] + q2[QE]);
-  const double psum = q1[QPRES] + q2[QPRES];
-  const double pu = kmul<(IM >> 8) & 1>(q1[QPRES], q2[QN]) + kmul<(IM >> 9) & 1>(q2[QPRES], q1[QN]);
-  T[URHO] = kmul<(IM >> 10) & 1>(c4, P);
-  T[UMX] = kmul<(IM >> 11) & 1>(c8, D == 0 ? fma(4.0, psum, cx) : cx);
-  T[UMY] = kmul<(IM >> 12) & 1>(c8, D == 1 ? fma(4.0, psum, cy) : cy);
-  T[UMZ] = kmul<(IM >> 13) & 1>(c8, D == 2 ? fma(4.0, psum, cz) : cz);
-  T[UET] = kmul<(IM >> 14) & 1>(c8, fma(4.0, pu, kmul<(IM >> 15) & 1>(P, s3) + ce));
+  const double psum = q1[QPRES] + q2[QPRES], eS = q1[QE] + q2[QE];
+  if (FAST) {
+    // P is zero exactly when unS is, and with it every term but the pressure's;
+    // D's own momentum term P unS + 4 psum is positive
+    const bool zP = is_zero(unS);
+    const double P = mul_core(rhoS, unS);
+    double vS[3], s[3];
+    bool z[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double a = q1[QU + c], b = q2[QU + c];
+      s[c] = mul_zero(a, b, is_zero(a) || is_zero(b));
+      vS[c] = a + b;
+      z[c] = zP || is_zero(vS[c]);
+    }
+    const double s3 = s[0] + s[1] + s[2];
+    T[URHO] = mul_zero(c4, P, zP);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (c == D) T[UMX + c] = mul_core(c8, fma(4.0, psum, mul_zero(P, vS[c], zP)));
+      else T[UMX + c] = mul_zero(c8, mul_core(P, vS[c]), z[c]);
+    }
+    const double pu = mul_zero(q1[QPRES], q2[QN], is_zero(q2[QN])) + mul_zero(q2[QPRES], q1[QN], is_zero(q1[QN]));
+    const double en = fma(4.0, pu, mul_zero(P, s3, zP || is_zero(s3)) + mul_zero(P, eS, zP));
+    T[UET] = mul_zero(c8, en, is_zero(en));
+  } else {
+    const double P = rhoS * unS;
+    const double s3 = q1[QU] * q2[QU] + q1[QV] * q2[QV] + q1[QW] * q2[QW];
+    const double cx = P * (q1[QU] + q2[QU]);
+    const double cy = P * (q1[QV] + q2[QV]);
+    const double cz = P * (q1[QW] + q2[QW]);
+    const double ce = P * eS;
+    const double pu = q1[QPRES] * q2[QN] + q2[QPRES] * q1[QN];
+    T[URHO] = c4 * P;
+    T[UMX] = c8 * (D == 0 ? fma(4.0, psum, cx) : cx);
+    T[UMY] = c8 * (D == 1 ? fma(4.0, psum, cy) : cy);
+    T[UMZ] = c8 * (D == 2 ? fma(4.0, psum, cz) : cz);
+    T[UET] = c8 * fma(4.0, pu, P * s3 + ce);
+  }
 }
 
 // Cell-centred viscous fluxes (src/rhs/CNS_hydro_K.h:108-172) from the

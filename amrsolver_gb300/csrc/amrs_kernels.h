@@ -4,19 +4,23 @@
 #include <cuda_runtime.h>
 
 #include "amrs_boxes.cuh"
-#include "tma.cuh"
 
 namespace amrs {
 
 // ---- KEEP fused path (rhs_keep.cu)
 cudaError_t launch_prims(const BoxTable& tb, int s_in, long long ncells, int nsm, cudaStream_t st);
 cudaError_t launch_visc(const BoxTable& tb, long long ncells, int nsm, cudaStream_t st);
+// Launch shape of the KEEP face kernels over a list: the march's CTAs and
+// threads (its balanced schedule) and the x kernel's blocks and threads.
+struct KeepGrid {
+  int x_ctas = 0, x_threads = 256;
+  int march_ctas = 0, march_threads = 256;
+};
+int keep_x_blocks(int order, const int n[3], int threads);  // x blocks of a box
 cudaError_t launch_keep_face(int order, bool visc, bool src, const BoxTable& tb, int s_in, int s_s1, int s_out,
-                             const DProg& prog, int rhs_only, const TmaDesc& tma, int* err, int grid, int nsm,
-                             cudaStream_t st);
+                             const DProg& prog, int rhs_only, const KeepGrid& g, cudaStream_t st);
 bool keep_tile_fits(int order, int tx, int ty);
 int keep_ctas_per_sm(int order);
-template <int ORDER> int keep_smem_bytes();
 
 // ---- face-array (reference-structured) path (rhs_plain.cu)
 // Face flux scratch per box: three nodal arrays, described per box in FaceRec.

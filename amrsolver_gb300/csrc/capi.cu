@@ -5,10 +5,10 @@
 // sequence runs over a device box table, then the stage's BLAS-1 program is
 // applied in the last kernel's epilogue.  Nothing here synchronises the host
 // except where the header says so.
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -19,6 +19,7 @@
 
 #include "../../include/amrs_gb300.h"
 #include "amrs_kernels.h"
+#include "keep_schedule.h"
 
 using namespace amrs;
 
@@ -127,46 +128,6 @@ int prim_ghost(const amrs_scheme& s) {
 
 bool fused_path(const amrs_scheme& s) { return s.rhs_euler && s.flux_euler == 1 && !s.art_diss; }
 
-// Tile choice for one box (the autotuner can override per box size).
-void default_tile(const amrs_box& b, int order, int& tx, int& ty, int& kc, int nsm) {
-  const int nx = bn(b, 0), ny = bn(b, 1), nz = bn(b, 2);
-  static const int cand[][2] = {{32, 8}, {16, 16}, {24, 10}, {8, 30}, {16, 8}, {8, 16}, {8, 8}};
-  double best = 1e300;
-  tx = 16; ty = 8;
-  for (auto& c : cand) {
-    if (!keep_tile_fits(order, c[0], c[1])) continue;
-    const long long ntx = (nx + c[0] - 1) / c[0], nty = (ny + c[1] - 1) / c[1];
-    // cost: lanes issued per useful cell, plus the x/y halo pair overheads
-    const double lanes = (double)ntx * nty * F_THREADS;
-    const double useful = (double)nx * ny;
-    const double halo = 1.0 + (double)(order / 2) / c[0] + (double)(order / 2) / c[1];
-    const double cost = lanes / useful * halo;
-    if (cost < best) { best = cost; tx = c[0]; ty = c[1]; }
-  }
-  const long long ncol = (long long)((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
-  // enough z chunks to give every SM two tiles, but at least 8 planes each
-  long long want = (2LL * nsm + ncol - 1) / ncol;
-  kc = (int)std::max<long long>(8, (nz + want - 1) / std::max<long long>(want, 1));
-  kc = std::min(kc, nz);
-}
-
-// Time a CTA of the fused face kernel spends on one plane of a txw x tyw
-// tile column, in units of one KEEP pair evaluation by one thread.  The
-// kernel's phases are separated by barriers and deal their items
-// round-robin over F_THREADS threads, so a phase costs its rounds: phase 1
-// the H z pairs of a column plus the x/y stored pairs of separation >= 2,
-// phase 2 the x and y faces (~1.5 pairs each with their sums and viscous
-// averages), phase 3 the divergence (~0.5), plus a fixed ~1 per plane
-// (barriers, the wait for the plane's load).  A thin partial tile thus
-// costs about half a full one per plane, not its share of cells.
-double face_plane_cost(int H, int txw, int tyw) {
-  int nxy = 0;
-  for (int l = 2; l <= H; ++l) nxy += (txw + l) * tyw + txw * (tyw + l);
-  const int nf = (txw + 1) * tyw + txw * (tyw + 1);
-  auto rounds = [](int items) { return (double)((items + F_THREADS - 1) / F_THREADS); };
-  return 1.0 + H + rounds(nxy) + 1.5 * rounds(nf) + 0.5;
-}
-
 // Stage programs of CNS::advance (src/tim/CNS_advance.cpp:51-166) for
 // (order_rk, stages_rk): numeric coefficients for `dt` into `st`, and, when
 // `forms` is given, the same programs with every dt-dependent coefficient
@@ -271,14 +232,14 @@ struct List {
   size_t dtab_bytes = 0;
   void* dscr = nullptr;   // scratch fields in one allocation
   size_t dscr_bytes = 0;
-  CUtensorMap* dmaps = nullptr;
   BoxTable tb{};
   FaceTable ft{};
-  TmaDesc tma{};
   const long long* d_spre[3] = {nullptr, nullptr, nullptr};
   long long tot_p = 0, tot_v = 0, tot_g = 0, tot_valid = 0, tot_f[3] = {0, 0, 0}, tot_s[3] = {0, 0, 0};
   int tot_work = 0;
   int face_grid = 0;  // CTAs of the balanced face-kernel schedule
+  KeepGrid grid;      // launch shape of the fused path's face kernels
+  int* d_range = nullptr;  // the fused path's two range flags (BoxTable::range), used by turns
   int waves = 1;      // shares of the schedule per resident CTA (amrs_boxlist_set_schedule)
   cudaGraphExec_t graph = nullptr;
   int graph_key[6] = {0, 0, 0, 0, 0, 0};
@@ -326,8 +287,6 @@ struct amrs_handle {
   int* derr = nullptr;               // device flags: [0] bounded waits timed out, [1] non-finite result
   int check_nonfinite = 0;           // amrs_set_check_nonfinite
   unsigned long long* dred = nullptr;  // reduction cell
-  bool tma_ok = true;
-  void* encode_fn = nullptr;
   List* one = nullptr;               // reusable single-box list for per-box calls
   WallCfg wall{};                    // code-6 y walls of the per-box calls' domain (amrs_set_domain)
   int source = 0;                    // rhs_source with a body force (amrs_set_source)
@@ -350,31 +309,6 @@ struct amrs_boxlist {
 
 namespace {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// Tensor map of one box's primitive scratch: dims (x, y, z, comp) over
-// grow(box,3), box {tx+6, ty+2H, 1, NQ}.  Returns false when the layout
-// cannot be described (row pitch not a multiple of 16 bytes, etc.).
-bool make_qmap(amrs_handle* h, const BoxRec& R, int order, CUtensorMap* out) {
-  if (!h->encode_fn || !h->tma_ok) return false;
-  const int H = order / 2;
-  const cuuint64_t dims[4] = {(cuuint64_t)(R.hi[0] - R.lo[0] + 1 + 6), (cuuint64_t)(R.hi[1] - R.lo[1] + 1 + 6),
-                              (cuuint64_t)(R.hi[2] - R.lo[2] + 1 + 6), (cuuint64_t)NQ};
-  const cuuint64_t strides[3] = {(cuuint64_t)R.q.js * 8, (cuuint64_t)R.q.ks * 8, (cuuint64_t)R.q.ns * 8};
-  for (int i = 0; i < 3; ++i)
-    if (strides[i] % 16) return false;
-  if (((uintptr_t)R.q.p) % 16) return false;
-  const cuuint32_t box[4] = {(cuuint32_t)(R.tx + 6), (cuuint32_t)(R.ty + 2 * H), 1u, (cuuint32_t)NQ};
-  if ((box[0] * 8) % 16 || box[0] > 256 || box[1] > 256) return false;
-  const cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = reinterpret_cast<EncodeTiledFn>(h->encode_fn)(
-      out, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, R.q.p, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
-
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Build host tables and allocate/upload device tables + scratch.
@@ -386,6 +320,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   L.sc = h->sc;
   L.gq = prim_ghost(h->sc);
   L.fused = fused_path(h->sc);
+  L.grid = KeepGrid{};
   L.boxes.assign(boxes, boxes + n);
   L.hbox.assign(n, BoxRec{});
   L.cls.resize(std::max(ncl, 1));
@@ -407,12 +342,13 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   for (int d = 0; d < 3; ++d) { L.fpre[d].assign(n + 1, 0); L.spre[d].assign(n + 1, 0); }
   // scratch layout: per box, Q [NQ x grow3], VF [NVF x grow1], faces, pf, lam, sen, slopes
   size_t off = 0;
-  std::vector<size_t> q_off(n), vf_off(n), f_off(n * 3), pf_off(n), lam_off(n), sen_off(n), sl_off(n * 3);
+  std::vector<size_t> q_off(n), vf_off(n), div_off(n), f_off(n * 3), pf_off(n), lam_off(n), sen_off(n), sl_off(n * 3);
   for (int b = 0; b < n; ++b) {
     const amrs_box& B = boxes[b];
     if (!box_ok(B)) return AMRS_ERR_BOX;
     q_off[b] = off; off = align_up(off + grown_cells(B, 3) * NQ * 8, 256);
     if (need_visc) { vf_off[b] = off; off = align_up(off + grown_cells(B, 1) * NVF * 8, 256); }
+    if (L.fused) { div_off[b] = off; off = align_up(off + grown_cells(B, 0) * 2 * NCONS * 8, 256); }
     if (need_faces)
       for (int d = 0; d < 3; ++d) {
         const long long nf = (long long)(bn(B, 0) + (d == 0)) * (bn(B, 1) + (d == 1)) * (bn(B, 2) + (d == 2));
@@ -432,6 +368,16 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     L.dscr_bytes = off;
   }
   char* S = static_cast<char*>(L.dscr);
+  if (L.fused)
+    // x kernel: narrower blocks where 256 slots would leave SMs without one
+    for (L.grid.x_threads = 256; L.grid.x_threads > 64; L.grid.x_threads /= 2) {
+      long long blocks = 0;
+      for (int b = 0; b < n; ++b) {
+        const int nb[3] = {bn(boxes[b], 0), bn(boxes[b], 1), bn(boxes[b], 2)};
+        blocks += keep_x_blocks(order, nb, L.grid.x_threads);
+      }
+      if (blocks >= 4LL * h->nsm) break;
+    }
   L.hface.assign(need_faces ? n : 0, FaceRec{});
   for (int b = 0; b < n; ++b) {
     const amrs_box& B = boxes[b];
@@ -455,12 +401,11 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     };
     R.q = mk(q_off[b], 3, -1, NQ);
     if (need_visc) R.vf = mk(vf_off[b], 1, -1, NVF);
+    if (L.fused) R.div = mk(div_off[b], 0, -1, 2 * NCONS);
     R.cl = cidx ? cidx[b] : 0;
-    int tx, ty, kc;
-    if (tiles) { tx = tiles[3 * b]; ty = tiles[3 * b + 1]; kc = tiles[3 * b + 2]; }
-    else default_tile(B, order, tx, ty, kc, h->nsm);
-    R.tx = tx; R.ty = ty; R.kc = kc;
-    R.ntx = (bn(B, 0) + tx - 1) / tx; R.nty = (bn(B, 1) + ty - 1) / ty; R.nkz = (bn(B, 2) + kc - 1) / kc;
+    R.tx = tiles ? tiles[3 * b] : 32;
+    R.ty = tiles ? tiles[3 * b + 1] : 8;
+    R.kc = tiles ? tiles[3 * b + 2] : bn(B, 2);
     if (need_faces) {
       FaceRec& F = L.hface[b];
       for (int d = 0; d < 3; ++d) F.f[d] = mk(f_off[b * 3 + d], 0, d, NCONS);
@@ -477,7 +422,8 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     L.vcell[b + 1] = L.vcell[b] + (need_visc ? grown_cells(B, 1) : 0);
     L.gcell[b + 1] = L.gcell[b] + grown_cells(B, 3);
     L.valid[b + 1] = L.valid[b] + grown_cells(B, 0);
-    L.fwork[b + 1] = L.fwork[b] + R.ntx * R.nty * R.nkz;
+    const int nb[3] = {bn(B, 0), bn(B, 1), bn(B, 2)};
+    L.fwork[b + 1] = L.fwork[b] + (L.fused ? keep_x_blocks(order, nb, L.grid.x_threads) : 0);
     for (int d = 0; d < 3; ++d) {
       const long long nf = (long long)(bn(B, 0) + (d == 0)) * (bn(B, 1) + (d == 1)) * (bn(B, 2) + (d == 2));
       L.fpre[d][b + 1] = L.fpre[d][b] + nf;
@@ -489,66 +435,20 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   L.tot_work = L.fwork[n];
   for (int d = 0; d < 3; ++d) { L.tot_f[d] = L.fpre[d][n]; L.tot_s[d] = L.spre[d][n]; }
 
-  // Balanced static schedule of the fused face kernel: the (tile column x
-  // plane) work of all boxes, weighted by the time a CTA spends on one plane
-  // of that column (face_plane_cost), is cut into G equal shares (G =
-  // resident CTAs); a share is a run of segments (box, column, k0, k1),
-  // each segment costing one z-prologue.
+  // balanced static schedule of the y and z marches
   std::vector<int4> segs;
-  std::vector<int> cta_seg;
+  std::vector<int> share;
   L.face_grid = 0;
   if (L.fused) {
-    double total = 0.0;
-    long long colplanes = 0;
-    for (int b = 0; b < n; ++b) {
-      const BoxRec& R = L.hbox[b];
-      for (int c = 0; c < R.ntx * R.nty; ++c) {
-        const int txi = c % R.ntx, tyi = c / R.ntx;
-        const int txw = std::min(R.tx, R.hi[0] + 1 - (R.lo[0] + txi * R.tx));
-        const int tyw = std::min(R.ty, R.hi[1] + 1 - (R.lo[1] + tyi * R.ty));
-        total += face_plane_cost(order / 2, txw, tyw) * bn(boxes[b], 2);
-        colplanes += bn(boxes[b], 2);
-      }
-    }
-    const long long G = std::min<long long>((long long)L.waves * keep_ctas_per_sm(order) * h->nsm, colplanes);
-    const double per = total / (double)G;
-    int cta = 0;
-    double acc = 0.0;
-    cta_seg.push_back(0);
-    for (int b = 0; b < n; ++b) {
-      const BoxRec& R = L.hbox[b];
-      for (int c = 0; c < R.ntx * R.nty; ++c) {
-        const int txi = c % R.ntx, tyi = c / R.ntx;
-        const int txw = std::min(R.tx, R.hi[0] + 1 - (R.lo[0] + txi * R.tx));
-        const int tyw = std::min(R.ty, R.hi[1] + 1 - (R.lo[1] + tyi * R.ty));
-        const double w = face_plane_cost(order / 2, txw, tyw);
-        int k = R.lo[2];
-        while (k <= R.hi[2]) {
-          const double boundary = (cta + 1) * per;
-          long long fit = (long long)((boundary - acc) / w + 0.5);
-          if (fit < 1) fit = 1;
-          const int kend = (int)std::min<long long>(R.hi[2] + 1, k + fit);
-          segs.push_back(make_int4(b, c, k, kend));
-          acc += (kend - k) * w;
-          k = kend;
-          if (acc >= boundary - 0.5 * w && cta < G - 1) {
-            ++cta;
-            cta_seg.push_back((int)segs.size());
-          }
-        }
-      }
-    }
-    while ((long long)cta_seg.size() < G + 1) cta_seg.push_back((int)segs.size());
-    cta_seg[G] = (int)segs.size();
-    L.face_grid = (int)G;
-  }
-
-  // tensor maps (fused path only)
-  std::vector<CUtensorMap> maps;
-  bool tma_all = L.fused && h->tma_ok && h->encode_fn;
-  if (tma_all) {
-    maps.resize(n);
-    for (int b = 0; b < n && tma_all; ++b) tma_all = make_qmap(h, L.hbox[b], order, &maps[b]);
+    const long long resident = 8LL * keep_ctas_per_sm(order) * h->nsm;
+    const long long G = march_shares(march_items(L.hbox.data(), n), L.waves, resident, h->nsm);
+    share.push_back(0);
+    march_schedule(L.hbox.data(), n, G, [&](int4 v) { segs.push_back(v); }, [&] { share.push_back((int)segs.size()); });
+    const int w = march_cta_warps(G, h->nsm);
+    L.grid.march_threads = 32 * w;
+    L.grid.march_ctas = (int)((G + w - 1) / w);
+    L.face_grid = L.grid.march_ctas;
+    L.grid.x_ctas = L.fwork[n];
   }
 
   // device tables in one allocation
@@ -556,7 +456,6 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   const size_t o_box = t; t = align_up(t + sizeof(BoxRec) * n, 128);
   const size_t o_face = t; t = align_up(t + sizeof(FaceRec) * L.hface.size(), 128);
   const size_t o_cls = t; t = align_up(t + sizeof(DClosures) * L.cls.size(), 128);
-  const size_t o_maps = t; t = align_up(t + sizeof(CUtensorMap) * (tma_all ? n : 0), 128);
   const size_t o_p = t; t = align_up(t + 8 * (n + 1), 128);
   const size_t o_v = t; t = align_up(t + 8 * (n + 1), 128);
   const size_t o_g = t; t = align_up(t + 8 * (n + 1), 128);
@@ -566,7 +465,8 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   for (int d = 0; d < 3; ++d) { o_s[d] = t; t = align_up(t + 8 * (n + 1), 128); }
   const size_t o_w = t; t = align_up(t + 4 * (n + 1), 128);
   const size_t o_seg = t; t = align_up(t + sizeof(int4) * segs.size(), 128);
-  const size_t o_cs = t; t = align_up(t + 4 * cta_seg.size(), 128);
+  const size_t o_sh = t; t = align_up(t + 4 * share.size(), 128);
+  const size_t o_rng = t; t = align_up(t + 2 * sizeof(int), 128);
   if (t > L.dtab_bytes) {
     if (L.dtab) { cudaFree(L.dtab); L.dtab = nullptr; L.dtab_bytes = 0; }
     CK(cudaMalloc(&L.dtab, t));
@@ -576,7 +476,6 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   std::memcpy(&host[o_box], L.hbox.data(), sizeof(BoxRec) * n);
   if (!L.hface.empty()) std::memcpy(&host[o_face], L.hface.data(), sizeof(FaceRec) * L.hface.size());
   std::memcpy(&host[o_cls], L.cls.data(), sizeof(DClosures) * L.cls.size());
-  if (tma_all) std::memcpy(&host[o_maps], maps.data(), sizeof(CUtensorMap) * n);
   std::memcpy(&host[o_p], L.pcell.data(), 8 * (n + 1));
   std::memcpy(&host[o_v], L.vcell.data(), 8 * (n + 1));
   std::memcpy(&host[o_g], L.gcell.data(), 8 * (n + 1));
@@ -587,7 +486,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   }
   std::memcpy(&host[o_w], L.fwork.data(), 4 * (n + 1));
   if (!segs.empty()) std::memcpy(&host[o_seg], segs.data(), sizeof(int4) * segs.size());
-  if (!cta_seg.empty()) std::memcpy(&host[o_cs], cta_seg.data(), 4 * cta_seg.size());
+  if (!share.empty()) std::memcpy(&host[o_sh], share.data(), 4 * share.size());
   CK(cudaMemcpy(L.dtab, host.data(), t, cudaMemcpyHostToDevice));
   char* D = static_cast<char*>(L.dtab);
   L.tb.box = reinterpret_cast<const BoxRec*>(D + o_box);
@@ -595,10 +494,14 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   L.tb.vcell = reinterpret_cast<const long long*>(D + o_v);
   L.tb.fwork = reinterpret_cast<const int*>(D + o_w);
   L.tb.seg = reinterpret_cast<const int4*>(D + o_seg);
-  L.tb.cta_seg = reinterpret_cast<const int*>(D + o_cs);
+  L.tb.share = reinterpret_cast<const int*>(D + o_sh);
+  L.tb.nshare = share.empty() ? 0 : (int)share.size() - 1;
   L.tb.cls = reinterpret_cast<const DClosures*>(D + o_cls);
   L.tb.n = n;
   L.tb.gq = L.gq;
+  L.d_range = L.fused ? reinterpret_cast<int*>(D + o_rng) : nullptr;
+  L.tb.range = L.d_range;
+  L.tb.range_next = L.d_range ? L.d_range + 1 : nullptr;
   L.ft.fr = reinterpret_cast<const FaceRec*>(D + o_face);
   for (int d = 0; d < 3; ++d) {
     L.ft.fpre[d] = reinterpret_cast<const long long*>(D + o_f[d]);
@@ -606,8 +509,6 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   }
   L.ft.gpre = reinterpret_cast<const long long*>(D + o_g);
   L.ft.vpre = reinterpret_cast<const long long*>(D + o_va);
-  L.tma.maps = tma_all ? reinterpret_cast<const CUtensorMap*>(D + o_maps) : nullptr;
-  L.tma.enabled = tma_all ? 1 : 0;
   return AMRS_OK;
 }
 
@@ -629,14 +530,15 @@ amrs_status list_stage(amrs_handle* h, List& L, const DProg& prog, int s_in, int
                        cudaStream_t st) {
   const amrs_scheme& sc = L.sc;
   const int nsm = h->nsm;
+  if (L.d_range) std::swap(L.tb.range, L.tb.range_next);
   // 1. primitives over the grown boxes
   if (L.gq > 0 || sc.rhs_visc) CK(launch_prims(L.tb, s_in, L.tot_p, nsm, st));
   // 2. viscous cell fluxes
   if (sc.rhs_visc) CK(launch_visc(L.tb, L.tot_v, nsm, st));
   if (L.fused) {
     // 3. fused KEEP faces + viscous averages + divergence + stage program
-    CK(launch_keep_face(sc.order_keep, sc.rhs_visc != 0, L.source, L.tb, s_in, s_s1, s_out, prog, rhs_only, L.tma,
-                        h->derr, L.face_grid, nsm, st));
+    CK(launch_keep_face(sc.order_keep, sc.rhs_visc != 0, L.source, L.tb, s_in, s_s1, s_out, prog, rhs_only,
+                        L.grid, st));
     if (h->check_nonfinite) CK(launch_nonfinite_check(L.tb, L.ft.vpre, s_out, L.tot_valid, h->derr + 1, nsm, st));
     return AMRS_OK;
   }
@@ -779,13 +681,6 @@ amrs_status amrs_create(amrs_handle** out, const amrs_scheme* scheme, const amrs
     amrs_destroy(h);
     return s;
   }
-  const char* tma_env = std::getenv("AMRS_TMA");
-  h->tma_ok = !(tma_env && tma_env[0] == '0');
-  cudaDriverEntryPointQueryResult q;
-  void* fn = nullptr;
-  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-      q == cudaDriverEntryPointSuccess)
-    h->encode_fn = fn;
   *out = h;
   return AMRS_OK;
 }
@@ -2004,8 +1899,7 @@ amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const dou
     if (e == cudaSuccess && sc.rhs_visc) e = launch_visc(L.tb, L.tot_v, h->nsm, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[2], st);
     if (e == cudaSuccess && L.fused)
-      e = launch_keep_face(sc.order_keep, sc.rhs_visc != 0, L.source, L.tb, 0, 1, 2, p, 0, L.tma, h->derr,
-                           L.face_grid, h->nsm, st);
+      e = launch_keep_face(sc.order_keep, sc.rhs_visc != 0, L.source, L.tb, 0, 1, 2, p, 0, L.grid, st);
     else if (e == cudaSuccess && sc.flux_euler == 2)
       e = launch_weno_faces(L.tb, L.ft, 0, nf, sc.weno_fast == 0, h->nsm, st);
     else if (e == cudaSuccess && sc.flux_euler == 3)
@@ -2041,9 +1935,9 @@ amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const dou
   return AMRS_OK;
 }
 
-// Whether the fused face kernel of this handle's last single-box list stages
-// its planes with TMA (1) or with plain loads (0).
-int32_t amrs_debug_tma_enabled(amrs_handle* h) { return (h && h->one) ? h->one->tma.enabled : -1; }
-int32_t amrs_boxlist_tma_enabled(amrs_boxlist* bl) { return bl ? bl->L.tma.enabled : -1; }
+// Whether the fused face kernels stage primitives with TMA: they read them with
+// plain loads (0); -1 without a list.
+int32_t amrs_debug_tma_enabled(amrs_handle* h) { return (h && h->one) ? 0 : -1; }
+int32_t amrs_boxlist_tma_enabled(amrs_boxlist* bl) { return bl ? 0 : -1; }
 
 }  // extern "C"

@@ -11,7 +11,7 @@
 //
 // Limits and sharing rules:
 //  * boxes of at most 32 cells in every direction (the array holds
-//    NQ x 38^3 + 12 x 34^3 doubles plus a 64 KiB table region, 6.9 MB);
+//    NQ x 38^3 + 12 x 34^3 + 10 x 32^3 doubles plus a 96 KiB table region, 9.6 MB);
 //    larger boxes return AMRS_ERR_SIZE;
 //  * the array exists once per device that loads the library and stays
 //    allocated until the process exits;
@@ -30,6 +30,7 @@
 
 #include "../../include/amrs_gb300.h"
 #include "amrs_kernels.h"
+#include "keep_schedule.h"
 
 using namespace amrs;
 
@@ -38,8 +39,9 @@ namespace {
 constexpr int NA_MAX_EDGE = 32;
 constexpr size_t NA_Q = (size_t)NQ * (NA_MAX_EDGE + 6) * (NA_MAX_EDGE + 6) * (NA_MAX_EDGE + 6);
 constexpr size_t NA_VF = (size_t)NVF * (NA_MAX_EDGE + 2) * (NA_MAX_EDGE + 2) * (NA_MAX_EDGE + 2);
-constexpr size_t NA_TABLE_BYTES = 64 * 1024;
-constexpr size_t NA_DOUBLES = NA_Q + NA_VF + NA_TABLE_BYTES / 8;
+constexpr size_t NA_TABLE_BYTES = 96 * 1024;
+constexpr size_t NA_DIV = (size_t)2 * NCONS * NA_MAX_EDGE * NA_MAX_EDGE * NA_MAX_EDGE;
+constexpr size_t NA_DOUBLES = NA_Q + NA_VF + NA_DIV + NA_TABLE_BYTES / 8;
 
 }  // namespace
 
@@ -51,10 +53,10 @@ namespace {
 
 std::mutex g_na_mu;
 // host staging of the table region and of the schedule (no heap use)
-constexpr int NA_MAX_SEGS = 2048;
+constexpr int NA_MAX_SEGS = 4096;
 alignas(128) char g_na_host[NA_TABLE_BYTES];
 int4 g_na_segs[NA_MAX_SEGS];
-int g_na_cta[NA_MAX_SEGS + 1];
+int g_na_share[NA_MAX_SEGS + 1];
 constexpr int NA_MAX_DEVICES = 64;
 double* g_na_ptr[NA_MAX_DEVICES] = {nullptr};
 int g_na_nsm[NA_MAX_DEVICES] = {0};
@@ -152,7 +154,8 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   // scratch fields inside the static array
   double* qp = base;
   double* vfp = base + NA_Q;
-  char* tab = reinterpret_cast<char*>(base + NA_Q + NA_VF);
+  double* divp = vfp + NA_VF;
+  char* tab = reinterpret_cast<char*>(divp + NA_DIV);
   const int order = sc.order_keep;
 
   // box record, tile and balanced schedule (as the handle path builds them)
@@ -168,55 +171,32 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   R.slot[2] = na_user(dsdt);
   R.q = na_view(qp, *bx, 3);
   R.vf = na_view(vfp, *bx, 1);
+  R.div = na_view(divp, *bx, 0);
   R.cl = 0;
-  int tx = 32, ty = 8;
-  if (!keep_tile_fits(order, tx, ty)) { tx = 16; ty = 8; }
-  if (n[0] <= 16 && keep_tile_fits(order, 16, 16)) { tx = 16; ty = 16; }
-  if (n[0] <= 8 && keep_tile_fits(order, 8, 30)) { tx = 8; ty = 30; }
-  R.tx = tx; R.ty = ty; R.kc = n[2];
-  R.ntx = (n[0] + tx - 1) / tx; R.nty = (n[1] + ty - 1) / ty; R.nkz = 1;
-  const int ncol = R.ntx * R.nty;
-  const long long G = std::min<long long>((long long)keep_ctas_per_sm(order) * nsm, (long long)ncol * n[2]);
-  int nseg = 0, ncs = 0;
-  int4* segs = g_na_segs;
-  int* cta_seg = g_na_cta;
+  R.tx = 32; R.ty = 8; R.kc = n[2];
+  KeepGrid grid;
+  for (grid.x_threads = 256; grid.x_threads > 64; grid.x_threads /= 2)
+    if (keep_x_blocks(order, n, grid.x_threads) >= 4 * nsm) break;
+  grid.x_ctas = keep_x_blocks(order, n, grid.x_threads);
+  int nseg = 0, nsh = 0;
+  bool full = false;
+  const long long G = march_shares(march_items(&R, 1), 1, 8LL * keep_ctas_per_sm(order) * nsm, nsm);
   if (G + 1 > NA_MAX_SEGS) return AMRS_ERR_SIZE;
-  {
-    double total = 0.0;
-    for (int c = 0; c < ncol; ++c) {
-      const int txw = std::min(tx, n[0] - (c % R.ntx) * tx), tyw = std::min(ty, n[1] - (c / R.ntx) * ty);
-      total += (double)txw * tyw * n[2];
-    }
-    const double per = total / (double)G;
-    int cta = 0;
-    double acc = 0.0;
-    cta_seg[ncs++] = 0;
-    for (int c = 0; c < ncol; ++c) {
-      const int txw = std::min(tx, n[0] - (c % R.ntx) * tx), tyw = std::min(ty, n[1] - (c / R.ntx) * ty);
-      const double w = (double)txw * tyw;
-      int k = R.lo[2];
-      while (k <= R.hi[2]) {
-        if (nseg >= NA_MAX_SEGS) return AMRS_ERR_SIZE;
-        const double boundary = (cta + 1) * per;
-        long long fit = (long long)((boundary - acc) / w + 0.5);
-        if (fit < 1) fit = 1;
-        const int kend = (int)std::min<long long>(R.hi[2] + 1, k + fit);
-        segs[nseg++] = make_int4(0, c, k, kend);
-        acc += (kend - k) * w;
-        k = kend;
-        if (acc >= boundary - 0.5 * w && cta < G - 1) {
-          ++cta;
-          cta_seg[ncs++] = nseg;
-        }
-      }
-    }
-    while (ncs < G + 1) cta_seg[ncs++] = nseg;
-    cta_seg[G] = nseg;
-  }
+  g_na_share[nsh++] = 0;
+  march_schedule(&R, 1, G,
+                 [&](int4 v) {
+                   if (nseg < NA_MAX_SEGS) g_na_segs[nseg++] = v;
+                   else full = true;
+                 },
+                 [&] { g_na_share[nsh++] = nseg; });
+  if (full) return AMRS_ERR_SIZE;
+  const int cw = march_cta_warps(G, nsm);
+  grid.march_threads = 32 * cw;
+  grid.march_ctas = (int)((G + cw - 1) / cw);
   const int gq = std::max(order / 2, 2);
   long long pcell[2] = {0, (long long)(n[0] + 2 * gq) * (n[1] + 2 * gq) * (n[2] + 2 * gq)};
   long long vcell[2] = {0, (long long)(n[0] + 2) * (n[1] + 2) * (n[2] + 2)};
-  int fwork[2] = {0, 0};
+  int fwork[2] = {0, grid.x_ctas};
   DClosures cl;
   cl.gamma = closures->gamma; cl.cv = closures->cv; cl.cp = closures->cp; cl.Rspec = closures->Rspec;
   cl.visc_law = closures->visc_law; cl.cond_law = closures->cond_law;
@@ -226,16 +206,16 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   cl.source = 0;  // no source term on this path
   cl.force[0] = cl.force[1] = cl.force[2] = 0.0;
 
-  // table region layout: box | closures | pcell | vcell | fwork | err | segs | cta_seg
+  // table region layout: box | closures | pcell | vcell | fwork | range flag | segs | shares
   size_t t = 0;
   const size_t o_box = t; t = al(t + sizeof(BoxRec));
   const size_t o_cl = t; t = al(t + sizeof(DClosures));
   const size_t o_p = t; t = al(t + sizeof(pcell));
   const size_t o_v = t; t = al(t + sizeof(vcell));
   const size_t o_w = t; t = al(t + sizeof(fwork));
-  const size_t o_err = t; t = al(t + sizeof(int));
+  const size_t o_rng = t; t = al(t + sizeof(int));
   const size_t o_seg = t; t = al(t + sizeof(int4) * nseg);
-  const size_t o_cs = t; t = al(t + sizeof(int) * ncs);
+  const size_t o_sh = t; t = al(t + sizeof(int) * nsh);
   if (t > NA_TABLE_BYTES) return AMRS_ERR_SIZE;
   char* host = g_na_host;
   std::memset(host, 0, t);
@@ -244,9 +224,9 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   std::memcpy(&host[o_p], pcell, sizeof(pcell));
   std::memcpy(&host[o_v], vcell, sizeof(vcell));
   std::memcpy(&host[o_w], fwork, sizeof(fwork));
-  std::memcpy(&host[o_seg], segs, sizeof(int4) * nseg);
-  std::memcpy(&host[o_cs], cta_seg, sizeof(int) * ncs);
-  // The copy also clears the error flag, which must start at zero.  From
+  std::memcpy(&host[o_seg], g_na_segs, sizeof(int4) * nseg);
+  std::memcpy(&host[o_sh], g_na_share, sizeof(int) * nsh);
+  // The copy also clears the range flag, which must start at zero.  From
   // pageable host memory it waits for the stream's earlier work and returns
   // once the staging is consumed, so the static host buffer can be reused.
   if (cudaMemcpyAsync(tab, host, t, cudaMemcpyHostToDevice, st) != cudaSuccess) return AMRS_ERR_CUDA;
@@ -257,21 +237,16 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   tb.vcell = reinterpret_cast<const long long*>(tab + o_v);
   tb.fwork = reinterpret_cast<const int*>(tab + o_w);
   tb.seg = reinterpret_cast<const int4*>(tab + o_seg);
-  tb.cta_seg = reinterpret_cast<const int*>(tab + o_cs);
+  tb.share = reinterpret_cast<const int*>(tab + o_sh);
+  tb.nshare = nsh - 1;
   tb.cls = reinterpret_cast<const DClosures*>(tab + o_cl);
   tb.n = 1;
   tb.gq = gq;
-  TmaDesc tma{};
-  tma.maps = nullptr;
-  tma.enabled = 0;
+  tb.range = reinterpret_cast<int*>(tab + o_rng);
   DProg prog{};
-  // The face kernel takes a flag word that only its TMA staging's bounded
-  // waits write; this path stages with plain loads (tma.enabled = 0), so
-  // nothing can raise it and there is nothing to read back.
-  int* err = reinterpret_cast<int*>(tab + o_err);
   if (launch_prims(tb, 0, pcell[1], nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;
   if (sc.rhs_visc && launch_visc(tb, vcell[1], nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;
-  if (launch_keep_face(order, sc.rhs_visc != 0, false, tb, 0, 1, 2, prog, 1, tma, err, (int)G, nsm, st) != cudaSuccess)
+  if (launch_keep_face(order, sc.rhs_visc != 0, false, tb, 0, 1, 2, prog, 1, grid, st) != cudaSuccess)
     return AMRS_ERR_CUDA;
   return AMRS_OK;
 }

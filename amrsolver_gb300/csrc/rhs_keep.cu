@@ -1,24 +1,28 @@
 // KEEP split-form + viscous RHS and the fused RK-stage epilogue.
 //
-// Three kernels per stage (all flattened over a box list):
-//   prims_kernel     cons2prim over grow(box, gq)            (src/rhs/CNS_hydro_K.h:15-34)
-//   visc_cell_kernel cell-centred viscous fluxes, grow(box,1) (src/rhs/CNS_hydro_K.h:108-172)
-//   keep_face_kernel KEEP face fluxes (src/rhs/CentralKEEP.h:40-145), viscous face
-//                    averages (src/rhs/CNS_hydro_K.h:254-261), flux divergence
-//                    (src/tim/CNS_advance.cpp:384-390) and the stage's BLAS-1
-//                    program (src/tim/CNS_advance.cpp:51-166), fused.
+// Four kernels per stage (all flattened over a box list):
+//   prims_kernel      cons2prim over grow(box, gq)            (src/rhs/CNS_hydro_K.h:15-34)
+//   visc_cell_kernel  cell-centred viscous fluxes, grow(box,1) (src/rhs/CNS_hydro_K.h:108-172)
+//   keep_march_kernel y and z: KEEP face fluxes (src/rhs/CentralKEEP.h:40-145),
+//                     viscous face averages (src/rhs/CNS_hydro_K.h:254-261) and
+//                     their parts of the divergence (src/tim/CNS_advance.cpp:384-390)
+//   keep_x_kernel     x: the same, the sum of the three parts and the stage's
+//                     BLAS-1 program (src/tim/CNS_advance.cpp:51-166)
 //
-// GB300's FP64 pipe (about 1 TFLOP/s) is ~60x slower than its HBM relative
-// to this kernel's 9 flop/byte, so primitives and viscous cell fluxes are
-// produced once per cell into HBM scratch instead of being recomputed for
-// every tile halo.  The face kernel streams z-planes through shared memory
-// (2-deep ring, filled by TMA when the layout allows) and evaluates every
-// KEEP pair term once: a pair (a+l, a) feeds l faces, so it is stored in
-// shared memory (x, y) or carried in registers (z) and reused.
-#include <atomic>
+// Bound: GB300's FP64 pipe (one warp instruction per 16 clocks and SM, ~60x
+// slower than its HBM relative to this path's 9 flop/byte).  So nothing is
+// computed twice (primitives and viscous cell fluxes go through HBM; a pair
+// term (a+l, a) that feeds l faces is kept in a register along the march or in
+// shared memory along x), all products run on the integer pipe, and the work
+// is cut so that warps never wait for each other while they hold FP64 work:
+// the march's warps are independent, the x kernel's blocks are small (64
+// registers, 32 warps per SM).  One kernel for all three directions, streaming
+// z-planes through shared memory, held the FP64 pipe 73% busy (16 warps per SM,
+// two barriers per plane) with 272 FP64 instructions per cell; 128^3, KEEP4 +
+// viscous, per stage: 1257 us before, 427 + 348 us now with 185, FP64 pipe 82-85%
+// busy (in between, with one kernel for x and y tiles and a z march: 890 us).
 #include "amrs_boxes.cuh"
 #include "amrs_kernels.h"
-#include "tma.cuh"
 
 namespace amrs {
 
@@ -44,6 +48,7 @@ __global__ void __launch_bounds__(256) prims_kernel(BoxTable tb, int s_in) {
     for (int n = 0; n < 5; ++n) u[n] = U.p[o + n * U.ns];
     double q[NQ];
     cons2prim(u, q, tb.cls[R.cl]);
+    if (tb.range && !keep_range(q)) *tb.range = 1;
     const long long oq = R.q.off(i, j, k);
 #pragma unroll
     for (int n = 0; n < NQ; ++n) R.q.p[oq + n * R.q.ns] = q[n];
@@ -100,22 +105,11 @@ __global__ void __launch_bounds__(256) visc_cell_kernel(BoxTable tb) {
 }
 
 // ------------------------------------------------ fused face kernel -----
-// Products of the divergence epilogue on the integer pipe, one bit per
-// direction (see kmul).
+// Products of the divergence on the integer pipe (see kmul): bit 0 x, 1 y and z
+// (on the FP64 pipe the 128^3 step takes 3.36 ms instead of 3.24).
 #ifndef AMRS_DIV_IMUL
-#define AMRS_DIV_IMUL 0x4
+#define AMRS_DIV_IMUL 0x3
 #endif
-
-template <int ORDER> struct KeepCfg {
-  static constexpr int H = ORDER / 2;
-  static constexpr int QS_CAP = (ORDER == 6) ? 544 : 480;  // (tx+6)*(ty+2H) capacity
-  static constexpr int T_CAP = 352;                         // pair-term tile capacity per level
-  static constexpr int F_CAP = 288;                         // face-flux tile capacity
-  static constexpr int NLEV = (H > 1) ? H - 1 : 1;          // stored separations l = 2..H
-  static constexpr int SMEM_DOUBLES = 2 * NQ * QS_CAP + 2 * NLEV * 5 * T_CAP + 2 * 5 * F_CAP;
-};
-
-template <int ORDER> int keep_smem_bytes() { return KeepCfg<ORDER>::SMEM_DOUBLES * 8 + 256; }
 
 __device__ __forceinline__ void keep_coeffs(int order, double c[3]) {
   // CPU-branch coefficients of the reference (src/CNS.cpp:241-252)
@@ -124,363 +118,272 @@ __device__ __forceinline__ void keep_coeffs(int order, double c[3]) {
   else { c[0] = 1.0; c[1] = 0.0; c[2] = 0.0; }
 }
 
-__device__ __forceinline__ void ld_q(const DArr& Q, int i, int j, int k, double* q) {
-  const long long o = Q.off(i, j, k);
+// ---- x direction: one slot per thread.  Slot f of a row computes the pair
+// terms T_l(f-1) = pair (f-1+l, f-1), l = 1..H; the face flux F(f) adds the
+// terms T_l(f-l) .. T_l(f-2) of the H-1 slots below (shared memory), and
+// cell f the flux F(f+1) of the slot above.  The slots of a box's rows
+// (nx + H each: the first H-1 only feed the ones above) lie end to end in
+// x, y, z order; a block takes blockDim of them and its neighbours overlap by H, so
+// tiles leave no idle lanes whatever nx is.  The cell then adds the y and z parts
+// the march left and applies the stage program.
+template <int ORDER, bool VISC, bool SRC, bool FAST>
+__device__ __forceinline__ void keep_x_body(const BoxTable& tb, int s_in, int s_s1, int s_out, const DProg& prog,
+                                            int rhs_only, double* smem) {
+  constexpr int H = ORDER / 2;
+  const int tid = threadIdx.x, nth = blockDim.x;
+  double coef[3];
+  keep_coeffs(ORDER, coef);
+  const int b = find_box_i(tb.fwork, tb.n, blockIdx.x);
+  const BoxRec& R = tb.box[b];
+  const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1, nz = R.hi[2] - R.lo[2] + 1;
+  const int row_slots = nx + H;
+  // (a box's grown cells fit 31 bits, and with them the slots)
+  const int g = (blockIdx.x - tb.fwork[b]) * (nth - H) + tid;
+  const bool in = g < row_slots * ny * nz;
+  const int row = in ? g / row_slots : 0;
+  const int s = in ? g - row * row_slots : 0;
+  const int kk = row / ny;
+  const int i = R.lo[0] + s - (H - 1), j = R.lo[1] + row - kk * ny, k = R.lo[2] + kk;
+  double* ts = smem;                    // [H-1][5][nth]: T_l(f-1) of each slot, l = 2..H
+  double* fs = smem + (H - 1) * 5 * nth;  // [5][nth]: F(f)
+  double F[5];
+  if (in) {
+    const double* Q = R.q.p + R.q.off(i - 1, j, k);
+    const long long qn = R.q.ns;
+    double q2[NQ], q1[NQ];
 #pragma unroll
-  for (int n = 0; n < NQ; ++n) q[n] = Q.p[o + n * Q.ns];
-}
-__device__ __forceinline__ void ld_qs(const double* buf, int idx, int QS, double* q) {
+    for (int n = 0; n < NQ; ++n) q2[n] = Q[n * qn];
 #pragma unroll
-  for (int n = 0; n < NQ; ++n) q[n] = buf[n * QS + idx];
+    for (int l = H; l >= 2; --l) {
+      double T[5];
+#pragma unroll
+      for (int n = 0; n < NQ; ++n) q1[n] = Q[l + n * qn];
+      keep_pair<0, FAST>(q1, q2, coef[l - 1], T);
+#pragma unroll
+      for (int n = 0; n < 5; ++n) ts[((l - 2) * 5 + n) * nth + tid] = T[n];
+    }
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) q1[n] = Q[1 + n * qn];
+    keep_pair<0, FAST>(q1, q2, coef[0], F);
+  }
+  if (H >= 2) __syncthreads();
+  const bool face = in && s >= H - 1 && tid >= H - 1;
+  if (face) {
+#pragma unroll
+    for (int l = 2; l <= H; ++l)
+#pragma unroll
+      for (int m = 0; m < l; ++m) {
+        const double* t = ts + (l - 2) * 5 * nth + tid - (l - 1 - m);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) F[n] = F[n] + t[n * nth];
+      }
+    if (VISC) {
+      const double* V = R.vf.p + R.vf.off(i, j, k);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) F[1 + n] = fma(0.5, V[n * R.vf.ns - 1] + V[n * R.vf.ns], F[1 + n]);
+    }
+#pragma unroll
+    for (int n = 0; n < 5; ++n) fs[n * nth + tid] = F[n];
+  }
+  __syncthreads();
+  if (face && s < row_slots - 1 && tid < nth - 1) {
+    const DArr& Uin = R.slot[s_in];
+    const DArr& U1 = R.slot[s_s1];
+    const DArr& Uo = R.slot[s_out];
+    const double* D = R.div.p + R.div.off(i, j, k);
+    const long long dn = R.div.ns, oin = Uin.off(i, j, k), o1 = U1.off(i, j, k), oo = Uo.off(i, j, k);
+    const bool src = SRC && tb.cls[R.cl].source != 0;  // SRC: a list with a source term
+#pragma unroll
+    for (int n = 0; n < 5; ++n) {
+      double ds = kmul<AMRS_DIV_IMUL & 1>(R.dxinv[0], F[n] - fs[n * nth + tid + 1]) + D[n * dn] + D[(5 + n) * dn];
+      if (src) ds = add_source(tb.cls[R.cl], Uin.p, oin, Uin.ns, n, ds);
+      if (rhs_only) {
+        Uo.p[oo + n * Uo.ns] = ds;
+      } else {
+        double reg[3];
+        reg[0] = U1.p[o1 + n * U1.ns];
+        reg[1] = Uin.p[oin + n * Uin.ns];
+        reg[2] = ds;
+        apply_prog(prog, reg);
+        Uo.p[oo + n * Uo.ns] = reg[1];
+      }
+    }
+  }
 }
 
-// One work item = one (tx x ty) column tile of one box over a chunk of z.
+// ---- y and z directions: one thread per column, a warp marching its 32 columns
+// over a run of cells with the shared pair terms in registers.  Writes
+// dxinv (F(m) - F(m+1)) of its direction.  Segment sg: (box, 2 * block + DIR - 1,
+// m0, m1), columns consecutive in x, then in z (y march) or y (z march).
+template <int ORDER, int DIR, bool VISC, bool FAST>
+__device__ __forceinline__ void keep_march(const BoxTable& tb, const int4& sg, const double coef[3]) {
+  constexpr int H = ORDER / 2;
+  const BoxRec& R = tb.box[sg.x];
+  const int nx = R.hi[0] - R.lo[0] + 1, nt = DIR == 1 ? R.hi[2] - R.lo[2] + 1 : R.hi[1] - R.lo[1] + 1;
+  const int c = (sg.y >> 1) * 32 + (threadIdx.x & 31);
+  if (c >= nx * nt) return;
+  const int m0 = sg.z, m1 = sg.w;  // cells [m0, m1) along DIR
+  const int ct = c / nx, ci = R.lo[0] + c - ct * nx;
+  const int j0 = DIR == 1 ? m0 : R.lo[1] + ct, k0 = DIR == 1 ? R.lo[2] + ct : m0;
+  const double dxi = R.dxinv[DIR];
+  const long long qk = DIR == 1 ? R.q.js : R.q.ks, qn = R.q.ns;
+  const long long vk = DIR == 1 ? R.vf.js : R.vf.ks, vn = R.vf.ns;
+  const long long dk = DIR == 1 ? R.div.js : R.div.ks, dn = R.div.ns;
+  // pointers at cell m0 of the column
+  const double* Q = R.q.p + R.q.off(ci, j0, k0);
+  const double* V = VISC ? R.vf.p + R.vf.off(ci, j0, k0) + 4 * DIR * vn : nullptr;
+  double* D = R.div.p + R.div.off(ci, j0, k0) + 5 * (DIR - 1) * dn;
+  // code-6 y walls: faces of second order (halfsten 1, coefficient 1)
+  auto reduced = [&](int f) { return DIR == 1 && R.walls && (f <= R.red_lo || (f >= R.red_hi && f <= R.hi[1])); };
+  // carries: tc[l][m] = T_l(c+1-l+m) for m=0..l-2 (l>=2); ring of Q(c..c+H-1)
+  double tc[3][2][5];
+  double ring[3][NQ];
+  double fl[5], vl[4];  // flux and viscous cell flux below the current cell
+  {
+    // the flux at face m0 (between m0-1 and m0) and the carries
+    double qcol[2 * H][NQ];  // cells m0-H .. m0+H-1
+#pragma unroll
+    for (int p = 0; p < 2 * H; ++p)
+#pragma unroll
+      for (int n = 0; n < NQ; ++n) qcol[p][n] = Q[(p - H) * qk + n * qn];
+    const bool red = reduced(m0);
+    keep_pair<DIR, FAST>(qcol[H], qcol[H - 1], red ? 1.0 : coef[0], fl);  // T_1(m0-1)
+#pragma unroll
+    for (int l = 2; l <= H; ++l) {
+#pragma unroll
+      for (int m = 0; m < l; ++m) {
+        const int a = -l + m;  // T_l(m0+a), pair (m0+a+l, m0+a)
+        double T[5];
+        keep_pair<DIR, FAST>(qcol[H + a + l], qcol[H + a], coef[l - 1], T);
+        if (!red) {
+#pragma unroll
+          for (int n = 0; n < 5; ++n) fl[n] = fl[n] + T[n];
+        }
+        if (m >= 1) {
+#pragma unroll
+          for (int n = 0; n < 5; ++n) tc[l - 1][m - 1][n] = T[n];
+        }
+      }
+    }
+    if (VISC) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        vl[n] = V[n * vn];
+        fl[1 + n] = fma(0.5, V[n * vn - vk] + vl[n], fl[1 + n]);
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < H; ++p)
+#pragma unroll
+      for (int n = 0; n < NQ; ++n) ring[p][n] = qcol[H + p][n];
+  }
+#pragma unroll 1
+  for (int m = m0; m < m1; ++m) {
+    // T_l(m) = pair (m+l, m), l = 1..H: the flux at face m+1
+    double qtop[NQ], F[5];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) qtop[n] = Q[H * qk + n * qn];
+    const bool red = reduced(m + 1);
+    keep_pair<DIR, FAST>(H == 1 ? qtop : ring[1], ring[0], red ? 1.0 : coef[0], F);
+#pragma unroll
+    for (int l = 2; l <= H; ++l) {
+      // F += T_l(m+1-l+p), p = 0..l-1 (p = l-1 is the new term), then the
+      // carries drop T_l(m+1-l) and append T_l(m)
+      double Tn[5];
+      if (!red) {
+#pragma unroll
+        for (int p = 0; p < l - 1; ++p)
+#pragma unroll
+          for (int n = 0; n < 5; ++n) F[n] = F[n] + tc[l - 1][p][n];
+      }
+      keep_pair<DIR, FAST>(l == H ? qtop : ring[l], ring[0], coef[l - 1], Tn);
+      if (!red) {
+#pragma unroll
+        for (int n = 0; n < 5; ++n) F[n] = F[n] + Tn[n];
+      }
+#pragma unroll
+      for (int p = 0; p < l - 2; ++p)
+#pragma unroll
+        for (int n = 0; n < 5; ++n) tc[l - 1][p][n] = tc[l - 1][p + 1][n];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) tc[l - 1][l - 2][n] = Tn[n];
+    }
+    if (VISC) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const double c1 = V[vk + n * vn];
+        F[1 + n] = fma(0.5, vl[n] + c1, F[1 + n]);
+        vl[n] = c1;
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 5; ++n) {
+      D[n * dn] = kmul<(AMRS_DIV_IMUL >> 1) & 1>(dxi, fl[n] - F[n]);
+      fl[n] = F[n];
+    }
+#pragma unroll
+    for (int p = 0; p < H - 1; ++p)
+#pragma unroll
+      for (int n = 0; n < NQ; ++n) ring[p][n] = ring[p + 1][n];
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) ring[H - 1][n] = qtop[n];
+    Q += qk;
+    V += vk;
+    D += dk;
+  }
+}
+
+// Resident CTAs of the march: 128 registers hold the carries of orders 2 and 4
+// (three CTAs per SM spill and are 2% slower over a step), order 6 takes all 255
+// (two CTAs: 288 instead of 272 us per step of 45 x 33 x 27).
+template <int ORDER> constexpr int march_ctas() { return ORDER == 6 ? 1 : 2; }
+
+// range flag of the stage (BoxTable::range), uniform over the grid
+__device__ __forceinline__ bool fast_range(const BoxTable& tb) { return tb.range && *tb.range == 0; }
+
+template <int ORDER, bool VISC, bool FAST>
+__device__ __forceinline__ void keep_march_warp(const BoxTable& tb) {
+  // balanced static schedule: this warp's segments cover an equal share of
+  // the (column block x cell) work of the whole list
+  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (w >= tb.nshare) return;
+  double coef[3];
+  keep_coeffs(ORDER, coef);
+  const int send = tb.share[w + 1];
+#pragma unroll 1
+  for (int sgi = tb.share[w]; sgi < send; ++sgi) {
+    const int4 sg = tb.seg[sgi];
+    if (sg.y & 1) keep_march<ORDER, 2, VISC, FAST>(tb, sg, coef);
+    else keep_march<ORDER, 1, VISC, FAST>(tb, sg, coef);
+  }
+}
+
+template <int ORDER, bool VISC>
+__global__ void __launch_bounds__(F_THREADS, march_ctas<ORDER>()) keep_march_kernel(BoxTable tb) {
+  if (list_idle(tb)) return;
+  if (fast_range(tb)) keep_march_warp<ORDER, VISC, true>(tb);
+  else keep_march_warp<ORDER, VISC, false>(tb);
+}
+
 template <int ORDER, bool VISC, bool SRC>
-__global__ void __launch_bounds__(F_THREADS, (ORDER == 6) ? 1 : 2)
-keep_face_kernel(BoxTable tb, int s_in, int s_s1, int s_out, DProg prog_in, int rhs_only, TmaDesc tma,
-                 int* err) {
-  using C = KeepCfg<ORDER>;
-  constexpr int H = C::H;
+__global__ void __launch_bounds__(F_THREADS, 4)
+keep_x_kernel(BoxTable tb, int s_in, int s_s1, int s_out, DProg prog_in, int rhs_only) {
   if (list_idle(tb)) return;  // uniform over the CTA: before any barrier
   const DProg prog = resolve_prog(prog_in);
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  double* smem = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  double* qsbuf = smem;                                   // [2][NQ][QS_CAP]
-  double* tsx = qsbuf + 2 * NQ * C::QS_CAP;               // [NLEV][5][T_CAP]
-  double* tsy = tsx + C::NLEV * 5 * C::T_CAP;             // [NLEV][5][T_CAP]
-  double* fsx = tsy + C::NLEV * 5 * C::T_CAP;             // [5][F_CAP]
-  double* fsy = fsx + 5 * C::F_CAP;                       // [5][F_CAP]
-  __shared__ __align__(8) unsigned long long mbar[2];
-
-  const int tid = threadIdx.x;
-  double coef[3];
-  keep_coeffs(ORDER, coef);
-  unsigned int phase_bits = 0u;
-  const bool use_tma = tma.enabled != 0;
-  if (use_tma) {
-    if (tid == 0) { mbar_init(&mbar[0], 1); mbar_init(&mbar[1], 1); fence_mbar_init(); }
-    __syncthreads();
-  }
-
-  // balanced static schedule: this CTA's segments cover an equal share of
-  // the (tile column x plane) work of the whole list
-  const int sbeg = tb.cta_seg[blockIdx.x], send = tb.cta_seg[blockIdx.x + 1];
-  for (int sgi = sbeg; sgi < send; ++sgi) {
-    const int4 sg = tb.seg[sgi];
-    const int b = sg.x;
-    const BoxRec& R = tb.box[b];
-    const int tyi = sg.y / R.ntx, txi = sg.y - (sg.y / R.ntx) * R.ntx;
-    const int TX = R.tx, TY = R.ty;
-    const int x0 = R.lo[0] + txi * TX, y0 = R.lo[1] + tyi * TY;
-    const int txw = min(TX, R.hi[0] + 1 - x0), tyw = min(TY, R.hi[1] + 1 - y0);
-    const int k0 = sg.z;
-    const int k1 = sg.w;
-    const int QP = TX + 6, QR = TY + 2 * H, QS = QP * QR;
-    const int TXP = TX + H;  // row pitch of x pair terms
-    const DArr Q = R.q, VF = R.vf;
-    const DArr Uin = R.slot[s_in], U1 = R.slot[s_s1], Uo = R.slot[s_out];
-    const double dxi0 = R.dxinv[0], dxi1 = R.dxinv[1], dxi2 = R.dxinv[2];
-    const bool src = SRC && tb.cls[R.cl].source != 0;  // SRC: a list with a source term
-    // allocation bounds of Q (grow(box,3))
-    const int qlo0 = R.lo[0] - NGHOST, qhi0 = R.hi[0] + NGHOST;
-    const int qlo1 = R.lo[1] - NGHOST, qhi1 = R.hi[1] + NGHOST;
-
-    // own column (one per thread while tid < txw*tyw)
-    const bool has_col = tid < txw * tyw;
-    const int ca = has_col ? tid % txw : 0;
-    const int cb = has_col ? tid / txw : 0;
-    const int ci = x0 + ca, cj = y0 + cb;
-
-    // z carries: Tz[l][m] = T_l(k+1-l+m) for m=0..l-2 (l>=2); ring of Q(k+1..k+H-1)
-    double tz[3][2][5];
-    double ring[3][NQ];
-    double fzprev[5];
-    double fzk[4];
-    if (has_col) {
-      // prologue: F_z at face k0 (between k0-1 and k0) and carries
-      double qcol[2 * 3][NQ];  // planes k0-H .. k0+H-1
-#pragma unroll
-      for (int p = 0; p < 2 * H; ++p) ld_q(Q, ci, cj, k0 - H + p, qcol[p]);
-      double F[5];
-      // l = 1: T_1(k0-1) = pair (k0, k0-1)
-      keep_pair<2>(qcol[H], qcol[H - 1], coef[0], F);
-#pragma unroll
-      for (int l = 2; l <= H; ++l) {
-#pragma unroll
-        for (int m = 0; m < l; ++m) {
-          const int a = -l + m;  // T_l(k0+a), pair (k0+a+l, k0+a)
-          double T[5];
-          keep_pair<2>(qcol[H + a + l], qcol[H + a], coef[l - 1], T);
-#pragma unroll
-          for (int n = 0; n < 5; ++n) F[n] = F[n] + T[n];
-          if (m >= 1) {
-#pragma unroll
-            for (int n = 0; n < 5; ++n) tz[l - 1][m - 1][n] = T[n];
-          }
-        }
-      }
-      if (VISC) {
-        const long long om = VF.off(ci, cj, k0 - 1), o0 = VF.off(ci, cj, k0);
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-          const double a = VF.p[om + (8 + n) * VF.ns], c0 = VF.p[o0 + (8 + n) * VF.ns];
-          F[1 + n] = fma(0.5, a + c0, F[1 + n]);
-          fzk[n] = c0;
-        }
-      }
-#pragma unroll
-      for (int n = 0; n < 5; ++n) fzprev[n] = F[n];
-#pragma unroll
-      for (int p = 0; p < H - 1; ++p)
-#pragma unroll
-        for (int n = 0; n < NQ; ++n) ring[p][n] = qcol[H + 1 + p][n];
-    }
-
-    // first plane into the ring
-    int buf = 0;
-    if (use_tma) {
-      if (tid == 0) tma_load_plane(tma, b, &mbar[0], qsbuf, x0 - 3 - qlo0, y0 - H - qlo1, k0 - (R.lo[2] - NGHOST), QS * NQ * 8);
-    }
-
-    // Per plane k two barriers: A publishes plane k (and closes the faces
-    // of plane k-1), B closes the pair terms of plane k.  Between A and B:
-    // the divergence of plane k-1 (phase 3) and the pair terms of plane k
-    // (phase 1); after B: the faces of plane k (phase 2).  One extra
-    // iteration k = k1 runs the last plane's phase 3.
-    double fznew[5];
-    for (int k = k0; k <= k1; ++k) {
-      const bool plane = k < k1;
-      double* qs = qsbuf + buf * NQ * C::QS_CAP;
-      // ---- phase 0: plane k of Q into shared memory
-      if (plane) {
-        if (use_tma) {
-          if (!mbar_wait(&mbar[buf], (phase_bits >> buf) & 1u)) { if (tid == 0) atomicExch(err, 1); }
-          phase_bits ^= (1u << buf);
-        } else {
-          // buffer buf held plane k-2, whose readers finished before the last barrier A
-          const int nel = NQ * QS;
-          for (int e = tid; e < nel; e += F_THREADS) {
-            const int n = e / QS;
-            const int r = e - n * QS;
-            const int yy = r / QP, xx = r - (r / QP) * QP;
-            const int gi = x0 - 3 + xx, gj = y0 - H + yy;
-            double v = 0.0;
-            if (gi >= qlo0 && gi <= qhi0 && gj >= qlo1 && gj <= qhi1) v = Q(gi, gj, k, n);
-            qs[e] = v;
-          }
-        }
-      }
-      __syncthreads();  // A
-      // the next plane into the other buffer: its plane k-1 was last read
-      // by the faces of plane k-1, which every thread finished before A
-      if (plane && use_tma && tid == 0 && k + 1 < k1) {
-        fence_proxy_async();
-        tma_load_plane(tma, b, &mbar[buf ^ 1], qsbuf + (buf ^ 1) * NQ * C::QS_CAP, x0 - 3 - qlo0, y0 - H - qlo1,
-                       k + 1 - (R.lo[2] - NGHOST), QS * NQ * 8);
-      }
-
-      // ---- phase 3 of plane k-1: divergence + stage program for the own cell
-      if (k > k0 && has_col) {
-        const int kc = k - 1;
-        const long long oin = Uin.off(ci, cj, kc), o1 = U1.off(ci, cj, kc), oo = Uo.off(ci, cj, kc);
-#pragma unroll
-        for (int n = 0; n < 5; ++n) {
-          const double* fx = fsx + n * C::F_CAP + cb * (TX + 1) + ca;
-          const double* fy = fsy + n * C::F_CAP + cb * TX + ca;
-          double ds = kmul<AMRS_DIV_IMUL & 1>(dxi0, fx[0] - fx[1]) + kmul<(AMRS_DIV_IMUL >> 1) & 1>(dxi1, fy[0] - fy[TX]) +
-                      kmul<(AMRS_DIV_IMUL >> 2) & 1>(dxi2, fzprev[n] - fznew[n]);
-          if (src) ds = add_source(tb.cls[R.cl], Uin.p, oin, Uin.ns, n, ds);
-          if (rhs_only) {
-            Uo.p[oo + n * Uo.ns] = ds;
-          } else {
-            double reg[3];
-            reg[0] = U1.p[o1 + n * U1.ns];
-            reg[1] = Uin.p[oin + n * Uin.ns];
-            reg[2] = ds;
-            apply_prog(prog, reg);
-            Uo.p[oo + n * Uo.ns] = reg[1];
-          }
-          fzprev[n] = fznew[n];
-        }
-      }
-      if (!plane) break;
-
-      // ---- phase 1: stored pair terms (x, y) and the z face above plane k
-      if (has_col) {
-        double qk[NQ], qtop[NQ];
-        ld_qs(qs, (cb + H) * QP + (ca + 3), QS, qk);
-        ld_q(Q, ci, cj, k + H, qtop);
-        // T_l(k) = pair (k+l, k), l = 1..H
-        double T1[5];
-        keep_pair<2>(H == 1 ? qtop : ring[0], qk, coef[0], T1);
-#pragma unroll
-        for (int n = 0; n < 5; ++n) fznew[n] = T1[n];
-#pragma unroll
-        for (int l = 2; l <= H; ++l) {
-          double Tn[5];
-          keep_pair<2>(l == H ? qtop : ring[l - 1], qk, coef[l - 1], Tn);
-          // F += T_l(k+1-l+m), m = 0..l-1 (m = l-1 is the new term)
-#pragma unroll
-          for (int m = 0; m < l - 1; ++m)
-#pragma unroll
-            for (int n = 0; n < 5; ++n) fznew[n] = fznew[n] + tz[l - 1][m][n];
-#pragma unroll
-          for (int n = 0; n < 5; ++n) fznew[n] = fznew[n] + Tn[n];
-          // shift carries: drop T_l(k+1-l), append T_l(k)
-#pragma unroll
-          for (int m = 0; m < l - 2; ++m)
-#pragma unroll
-            for (int n = 0; n < 5; ++n) tz[l - 1][m][n] = tz[l - 1][m + 1][n];
-#pragma unroll
-          for (int n = 0; n < 5; ++n) tz[l - 1][l - 2][n] = Tn[n];
-        }
-        if (VISC) {
-          const long long o1 = VF.off(ci, cj, k + 1);
-#pragma unroll
-          for (int n = 0; n < 4; ++n) {
-            const double c1 = VF.p[o1 + (8 + n) * VF.ns];
-            fznew[1 + n] = fma(0.5, fzk[n] + c1, fznew[1 + n]);
-            fzk[n] = c1;
-          }
-        }
-        // ring shift: Q(k+2..k+H) become Q(k+1..k+H-1) of the next plane
-#pragma unroll
-        for (int p = 0; p < H - 2; ++p)
-#pragma unroll
-          for (int n = 0; n < NQ; ++n) ring[p][n] = ring[p + 1][n];
-        if (H >= 2) {
-#pragma unroll
-          for (int n = 0; n < NQ; ++n) ring[H - 2][n] = qtop[n];
-        }
-      }
-      if (H >= 2) {
-        // x: T_l(a, row) for a in [-l, txw-1]; y: T_l(col, b) for b in [-l, tyw-1]
-        int nxit = 0, nyit = 0;
-#pragma unroll
-        for (int l = 2; l <= H; ++l) { nxit += (txw + l) * tyw; nyit += txw * (tyw + l); }
-        for (int e = tid; e < nxit + nyit; e += F_THREADS) {
-          double q1[NQ], q2[NQ], T[5];
-          if (e < nxit) {
-            int r = e, l = 2;
-#pragma unroll
-            for (int ll = 2; ll < H; ++ll) {
-              if (r >= (txw + ll) * tyw) { r -= (txw + ll) * tyw; l = ll + 1; }
-            }
-            const int w2 = txw + l;
-            const int row = r / w2, a = r - row * w2 - l;
-            const int base = (row + H) * QP + 3;
-            ld_qs(qs, base + a + l, QS, q1);
-            ld_qs(qs, base + a, QS, q2);
-            keep_pair<0>(q1, q2, coef[l - 1], T);
-            double* dst = tsx + (l - 2) * 5 * C::T_CAP + row * TXP + (a + l);
-#pragma unroll
-            for (int n = 0; n < 5; ++n) dst[n * C::T_CAP] = T[n];
-          } else {
-            int r = e - nxit, l = 2;
-#pragma unroll
-            for (int ll = 2; ll < H; ++ll) {
-              if (r >= txw * (tyw + ll)) { r -= txw * (tyw + ll); l = ll + 1; }
-            }
-            const int bb = r / txw - l, col = r - (r / txw) * txw;
-            ld_qs(qs, (bb + l + H) * QP + col + 3, QS, q1);
-            ld_qs(qs, (bb + H) * QP + col + 3, QS, q2);
-            keep_pair<1>(q1, q2, coef[l - 1], T);
-            double* dst = tsy + (l - 2) * 5 * C::T_CAP + (bb + l) * TX + col;
-#pragma unroll
-            for (int n = 0; n < 5; ++n) dst[n * C::T_CAP] = T[n];
-          }
-        }
-      }
-      __syncthreads();
-
-      // ---- phase 2: x faces f in [0, txw] and y faces f in [0, tyw]
-      {
-        const int nxf = (txw + 1) * tyw, nyf = txw * (tyw + 1);
-        // items in reverse thread order: the last, partial round of faces
-        // falls on the last warps, while the partial round of pair terms
-        // before the barrier fell on the first ones (measured 0.2% faster)
-        for (int e = F_THREADS - 1 - tid; e < nxf + nyf; e += F_THREADS) {
-          double F[5], q1[NQ], q2[NQ];
-          if (e < nxf) {
-            const int row = e / (txw + 1), f = e - row * (txw + 1);
-            const int base = (row + H) * QP + 3;
-            ld_qs(qs, base + f, QS, q1);
-            ld_qs(qs, base + f - 1, QS, q2);
-            keep_pair<0>(q1, q2, coef[0], F);
-#pragma unroll
-            for (int l = 2; l <= H; ++l)
-#pragma unroll
-              for (int m = 0; m < l; ++m) {
-                const double* src = tsx + (l - 2) * 5 * C::T_CAP + row * TXP + (f - l + m + l);
-#pragma unroll
-                for (int n = 0; n < 5; ++n) F[n] = F[n] + src[n * C::T_CAP];
-              }
-            if (VISC) {
-              const long long oR = VF.off(x0 + f, y0 + row, k);
-#pragma unroll
-              for (int n = 0; n < 4; ++n) F[1 + n] = fma(0.5, VF.p[oR - 1 + n * VF.ns] + VF.p[oR + n * VF.ns], F[1 + n]);
-            }
-            double* dst = fsx + row * (TX + 1) + f;
-#pragma unroll
-            for (int n = 0; n < 5; ++n) dst[n * C::F_CAP] = F[n];
-          } else {
-            const int r = e - nxf;
-            const int f = r / txw, col = r - (r / txw) * txw;
-            ld_qs(qs, (f + H) * QP + col + 3, QS, q1);
-            ld_qs(qs, (f - 1 + H) * QP + col + 3, QS, q2);
-            const int jf = y0 + f;
-            if (R.walls && (jf <= R.red_lo || (jf >= R.red_hi && jf <= R.hi[1]))) {
-              // next to a code-6 y wall: second-order KEEP (halfsten 1, coefficient 1)
-              keep_pair<1>(q1, q2, 1.0, F);
-            } else {
-              keep_pair<1>(q1, q2, coef[0], F);
-#pragma unroll
-              for (int l = 2; l <= H; ++l)
-#pragma unroll
-                for (int m = 0; m < l; ++m) {
-                  const double* src = tsy + (l - 2) * 5 * C::T_CAP + (f - l + m + l) * TX + col;
-#pragma unroll
-                  for (int n = 0; n < 5; ++n) F[n] = F[n] + src[n * C::T_CAP];
-                }
-            }
-            if (VISC) {
-              const long long oR = VF.off(x0 + col, y0 + f, k);
-#pragma unroll
-              for (int n = 0; n < 4; ++n)
-                F[1 + n] = fma(0.5, VF.p[oR - VF.js + (4 + n) * VF.ns] + VF.p[oR + (4 + n) * VF.ns], F[1 + n]);
-            }
-            double* dst = fsy + f * TX + col;
-#pragma unroll
-            for (int n = 0; n < 5; ++n) dst[n * C::F_CAP] = F[n];
-          }
-        }
-      }
-      // phase 3 of this plane (its divergence) runs in the next iteration,
-      // after the barrier that also publishes the next plane
-      buf ^= 1;
-    }
-    // the TMA ring is drained at the last plane; nothing is in flight here
-  }
+  double* smem = reinterpret_cast<double*>(smem_raw);
+  if (tb.range_next && blockIdx.x == 0 && threadIdx.x == 0) *tb.range_next = 0;
+  if (fast_range(tb)) keep_x_body<ORDER, VISC, SRC, true>(tb, s_in, s_s1, s_out, prog, rhs_only, smem);
+  else keep_x_body<ORDER, VISC, SRC, false>(tb, s_in, s_s1, s_out, prog, rhs_only, smem);
 }
 
 // explicit instantiations + launchers
 template <int ORDER, bool VISC, bool SRC>
 static cudaError_t launch_face_t(const BoxTable& tb, int s_in, int s_s1, int s_out, const DProg& prog, int rhs_only,
-                                 const TmaDesc& tma, int* err, int grid, cudaStream_t st) {
-  const int smem = keep_smem_bytes<ORDER>();
-  // the shared-memory opt-in is a per-device function attribute: set it once
-  // for each device this process launches on (devices 0..63 tracked)
-  static std::atomic<unsigned long long> attr_set{0ull};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (dev >= 64 || !(attr_set.load() & bit)) {
-    e = cudaFuncSetAttribute(keep_face_kernel<ORDER, VISC, SRC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr_set.fetch_or(bit);
-  }
-  keep_face_kernel<ORDER, VISC, SRC><<<grid, F_THREADS, smem, st>>>(tb, s_in, s_s1, s_out, prog, rhs_only, tma, err);
+                                 const KeepGrid& g, cudaStream_t st) {
+  keep_march_kernel<ORDER, VISC><<<g.march_ctas, g.march_threads, 0, st>>>(tb);
+  keep_x_kernel<ORDER, VISC, SRC><<<g.x_ctas, g.x_threads, (ORDER / 2) * 5 * 8 * g.x_threads, st>>>(
+      tb, s_in, s_s1, s_out, prog, rhs_only);
   return cudaGetLastError();
 }
 
@@ -503,11 +406,9 @@ cudaError_t launch_visc(const BoxTable& tb, long long ncells, int nsm, cudaStrea
 }
 
 cudaError_t launch_keep_face(int order, bool visc, bool src, const BoxTable& tb, int s_in, int s_s1, int s_out,
-                             const DProg& prog, int rhs_only, const TmaDesc& tma, int* err, int grid, int nsm,
-                             cudaStream_t st) {
-  (void)nsm;
-  if (grid <= 0) return cudaSuccess;
-#define AMRS_FACE(O, V, S) launch_face_t<O, V, S>(tb, s_in, s_s1, s_out, prog, rhs_only, tma, err, grid, st)
+                             const DProg& prog, int rhs_only, const KeepGrid& g, cudaStream_t st) {
+  if (g.x_ctas <= 0) return cudaSuccess;
+#define AMRS_FACE(O, V, S) launch_face_t<O, V, S>(tb, s_in, s_s1, s_out, prog, rhs_only, g, st)
 #define AMRS_FACE_VS(O) \
   (visc ? (src ? AMRS_FACE(O, true, true) : AMRS_FACE(O, true, false)) \
         : (src ? AMRS_FACE(O, false, true) : AMRS_FACE(O, false, false)))
@@ -518,16 +419,20 @@ cudaError_t launch_keep_face(int order, bool visc, bool src, const BoxTable& tb,
 #undef AMRS_FACE
 }
 
-int keep_ctas_per_sm(int order) { return order == 6 ? 1 : 2; }
+int keep_ctas_per_sm(int order) { return order == 6 ? march_ctas<6>() : march_ctas<4>(); }
+
+int keep_x_blocks(int order, const int n[3], int threads) {
+  const int H = order / 2;
+  const long long slots = (long long)(n[0] + H) * n[1] * n[2];
+  return (int)((slots - H + threads - H - 1) / (threads - H));
+}
 
 bool keep_tile_fits(int order, int tx, int ty) {
   if (tx < 8 || ty < 1 || (tx % 2) || tx * ty > F_THREADS) return false;
   const int H = order / 2;
-  int qcap = order == 6 ? KeepCfg<6>::QS_CAP : KeepCfg<4>::QS_CAP;
-  if ((tx + 6) * (ty + 2 * H) > qcap) return false;
-  if ((tx + H) * ty > KeepCfg<4>::T_CAP || tx * (ty + H) > KeepCfg<4>::T_CAP) return false;
-  if ((tx + 1) * ty > KeepCfg<4>::F_CAP || tx * (ty + 1) > KeepCfg<4>::F_CAP) return false;
-  return true;
+  if ((tx + 6) * (ty + 2 * H) > (order == 6 ? 544 : 480)) return false;
+  if ((tx + H) * ty > 352 || tx * (ty + H) > 352) return false;
+  return (tx + 1) * ty <= 288 && tx * (ty + 1) <= 288;
 }
 
 }  // namespace amrs

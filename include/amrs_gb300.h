@@ -178,7 +178,7 @@ amrs_status amrs_rhs_box(amrs_handle* h, const amrs_box* bx, const double dxinv[
  * KEEP 2/4/6 with or without viscous terms, no JST and no source term
  * (AMRS_ERR_SCHEME otherwise, also for transport laws other than 0/1),
  * boxes of at most 32 cells per direction (AMRS_ERR_SIZE beyond); the array
- * (6.9 MB) lives on every device that loads the library until exit; every
+ * (9.6 MB) lives on every device that loads the library until exit; every
  * call shares it, so calls that overlap on the GPU race.  The kernels run on
  * the current device: a `stream` of another device is refused
  * (AMRS_ERR_STATE).  The first call on a device looks the array's address
@@ -259,9 +259,11 @@ amrs_status amrs_boxlist_create(amrs_handle* h, int32_t nboxes, const amrs_box* 
                                 int32_t nclosures, const amrs_closures* closures, amrs_boxlist** out);
 amrs_status amrs_boxlist_destroy(amrs_boxlist* bl);
 
-/* Tile shape (threads per tile = tx*ty <= 256) and z-chunk per box, as
- * chosen by the autotuner; tx must be a multiple of 8.  Applies to every
- * box whose valid extents match (nx,ny,nz) exactly; nx=ny=nz=0 sets the default. */
+/* Tile shape (tx*ty <= 256) and z-chunk per box, as chosen by the autotuner;
+ * tx must be even and at least 8.  Applies to every box whose valid extents
+ * match (nx,ny,nz) exactly; nx=ny=nz=0 sets the default.  The tiles are recorded
+ * (amrs_boxlist_get_tiles); the face kernels deal columns and rows to warps
+ * whatever they are, so results and speed do not depend on them. */
 amrs_status amrs_boxlist_set_tile(amrs_boxlist* bl, int32_t nx, int32_t ny, int32_t nz, int32_t tx, int32_t ty,
                                   int32_t kchunk);
 
@@ -296,13 +298,14 @@ amrs_status amrs_boxlist_fill_halo(amrs_boxlist* bl, int32_t slot, void* stream)
 /* Per-box tiles in one call: tiles[3*b + {0,1,2}] = (tx, ty, kchunk) of
  * box b (the autotuner's output). */
 amrs_status amrs_boxlist_set_tiles(amrs_boxlist* bl, const int32_t* tiles);
-/* Work distribution of the fused face kernel (no counterpart in the
- * reference, whose MFIter loop launches box by box): the (tile column x
- * plane) work of all boxes is cut into `waves` x (resident CTAs) equal shares
- * (1 <= waves <= 8; default 1).  One wave gives each CTA the longest z run
- * (the fewest z prologues); more waves give shorter runs that later CTAs
- * pick up as earlier ones finish.  The autotuner sweeps it with the tile
- * shapes.  Host-synchronising; recorded graphs of the list are re-recorded. */
+/* Work distribution of the fused face kernels (no counterpart in the
+ * reference, whose MFIter loop launches box by box): the (column block x cell)
+ * work of the y and z marches of all boxes is cut into equal shares, one per
+ * warp, up to `waves` x (resident warps) of them (1 <= waves <= 8; default 1).
+ * One wave gives each warp the longest run (the fewest prologues); more waves
+ * give shorter runs that later CTAs pick up as earlier ones finish.  The
+ * autotuner sweeps it.  Host-synchronising; recorded graphs of the list are
+ * re-recorded. */
 amrs_status amrs_boxlist_set_schedule(amrs_boxlist* bl, int32_t waves);
 /* CTAs of the list's face-kernel schedule (0 for the face-array path). */
 int32_t amrs_boxlist_face_grid(amrs_boxlist* bl);
