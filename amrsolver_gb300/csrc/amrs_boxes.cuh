@@ -33,9 +33,8 @@ struct BoxTable {
   const long long* pcell;  // prefix of primitive-region cells, size n+1
   const long long* vcell;  // prefix of viscous-region cells, size n+1
   const int* fwork;        // prefix of the KEEP x kernel's blocks, size n+1
-  const int4* seg;         // KEEP march segments: (box, 2 * column block + (dir - 1), m0, m1)
-  const int* share;        // segments of warp w: [share[w], share[w+1])
-  int nshare;
+  const long long* mitem;  // prefix of the KEEP marches' items (march_items), size n+1
+  int nshare;              // equal shares (warps) the items are cut into
   const DClosures* cls;
   int n;
   int gq;                  // ghost depth of the primitive region

@@ -223,7 +223,7 @@ struct List {
   std::vector<amrs_box> boxes;
   std::vector<BoxRec> hbox;
   std::vector<FaceRec> hface;
-  std::vector<long long> pcell, vcell, gcell, valid, fpre[3], spre[3];
+  std::vector<long long> pcell, vcell, gcell, valid, mitem, fpre[3], spre[3];
   std::vector<int> fwork;
   std::vector<DClosures> cls;
   bool source = false;    // some closures carry a source term
@@ -338,6 +338,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   const bool need_slope = h->sc.rhs_euler && h->sc.flux_euler == 0;
   const bool need_jst = h->sc.rhs_euler && h->sc.art_diss == 1;
   L.pcell.assign(n + 1, 0); L.vcell.assign(n + 1, 0); L.gcell.assign(n + 1, 0); L.valid.assign(n + 1, 0);
+  L.mitem.assign(n + 1, 0);
   L.fwork.assign(n + 1, 0);
   for (int d = 0; d < 3; ++d) { L.fpre[d].assign(n + 1, 0); L.spre[d].assign(n + 1, 0); }
   // scratch layout: per box, Q [NQ x grow3], VF [NVF x grow1], faces, pf, lam, sen, slopes
@@ -423,6 +424,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     L.gcell[b + 1] = L.gcell[b] + grown_cells(B, 3);
     L.valid[b + 1] = L.valid[b] + grown_cells(B, 0);
     const int nb[3] = {bn(B, 0), bn(B, 1), bn(B, 2)};
+    L.mitem[b + 1] = L.mitem[b] + march_items(R);
     L.fwork[b + 1] = L.fwork[b] + (L.fused ? keep_x_blocks(order, nb, L.grid.x_threads) : 0);
     for (int d = 0; d < 3; ++d) {
       const long long nf = (long long)(bn(B, 0) + (d == 0)) * (bn(B, 1) + (d == 1)) * (bn(B, 2) + (d == 2));
@@ -435,18 +437,16 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   L.tot_work = L.fwork[n];
   for (int d = 0; d < 3; ++d) { L.tot_f[d] = L.fpre[d][n]; L.tot_s[d] = L.spre[d][n]; }
 
-  // balanced static schedule of the y and z marches
-  std::vector<int4> segs;
-  std::vector<int> share;
+  // shares and CTAs of the y and z marches
   L.face_grid = 0;
+  L.tb.nshare = 0;
   if (L.fused) {
     const long long resident = 8LL * keep_ctas_per_sm(order) * h->nsm;
-    const long long G = march_shares(march_items(L.hbox.data(), n), L.waves, resident, h->nsm);
-    share.push_back(0);
-    march_schedule(L.hbox.data(), n, G, [&](int4 v) { segs.push_back(v); }, [&] { share.push_back((int)segs.size()); });
+    const int G = (int)march_shares(L.mitem[n], L.waves, resident, h->nsm);
     const int w = march_cta_warps(G, h->nsm);
+    L.tb.nshare = G;
     L.grid.march_threads = 32 * w;
-    L.grid.march_ctas = (int)((G + w - 1) / w);
+    L.grid.march_ctas = (G + w - 1) / w;
     L.face_grid = L.grid.march_ctas;
     L.grid.x_ctas = L.fwork[n];
   }
@@ -464,8 +464,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   for (int d = 0; d < 3; ++d) { o_f[d] = t; t = align_up(t + 8 * (n + 1), 128); }
   for (int d = 0; d < 3; ++d) { o_s[d] = t; t = align_up(t + 8 * (n + 1), 128); }
   const size_t o_w = t; t = align_up(t + 4 * (n + 1), 128);
-  const size_t o_seg = t; t = align_up(t + sizeof(int4) * segs.size(), 128);
-  const size_t o_sh = t; t = align_up(t + 4 * share.size(), 128);
+  const size_t o_mi = t; t = align_up(t + 8 * (n + 1), 128);
   const size_t o_rng = t; t = align_up(t + 2 * sizeof(int), 128);
   if (t > L.dtab_bytes) {
     if (L.dtab) { cudaFree(L.dtab); L.dtab = nullptr; L.dtab_bytes = 0; }
@@ -485,17 +484,14 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     std::memcpy(&host[o_s[d]], L.spre[d].data(), 8 * (n + 1));
   }
   std::memcpy(&host[o_w], L.fwork.data(), 4 * (n + 1));
-  if (!segs.empty()) std::memcpy(&host[o_seg], segs.data(), sizeof(int4) * segs.size());
-  if (!share.empty()) std::memcpy(&host[o_sh], share.data(), 4 * share.size());
+  std::memcpy(&host[o_mi], L.mitem.data(), 8 * (n + 1));
   CK(cudaMemcpy(L.dtab, host.data(), t, cudaMemcpyHostToDevice));
   char* D = static_cast<char*>(L.dtab);
   L.tb.box = reinterpret_cast<const BoxRec*>(D + o_box);
   L.tb.pcell = reinterpret_cast<const long long*>(D + o_p);
   L.tb.vcell = reinterpret_cast<const long long*>(D + o_v);
   L.tb.fwork = reinterpret_cast<const int*>(D + o_w);
-  L.tb.seg = reinterpret_cast<const int4*>(D + o_seg);
-  L.tb.share = reinterpret_cast<const int*>(D + o_sh);
-  L.tb.nshare = share.empty() ? 0 : (int)share.size() - 1;
+  L.tb.mitem = reinterpret_cast<const long long*>(D + o_mi);
   L.tb.cls = reinterpret_cast<const DClosures*>(D + o_cls);
   L.tb.n = n;
   L.tb.gq = L.gq;

@@ -1,5 +1,5 @@
-// Balanced static schedule of the KEEP marches (keep_march_kernel), shared by
-// the box lists and the allocation-free entry point.
+// Work distribution of the KEEP marches (keep_march_kernel), shared by the box
+// lists and the allocation-free entry point.
 #pragma once
 #include "amrs_boxes.cuh"
 
@@ -7,18 +7,16 @@ namespace amrs {
 
 // Columns of box R crossed by the march along dir (1 y, 2 z), in blocks of one
 // warp, and the cells of a column.
-inline int march_blocks(const BoxRec& R, int dir) {
+__host__ __device__ inline int march_blocks(const BoxRec& R, int dir) {
   const int t = dir == 1 ? 2 : 1;
   return ((R.hi[0] - R.lo[0] + 1) * (R.hi[t] - R.lo[t] + 1) + 31) / 32;
 }
-inline int march_cells(const BoxRec& R, int dir) { return R.hi[dir] - R.lo[dir] + 1; }
+__host__ __device__ inline int march_cells(const BoxRec& R, int dir) { return R.hi[dir] - R.lo[dir] + 1; }
 
-// (Column block x cell) items of both marches over the boxes.
-inline long long march_items(const BoxRec* box, int n) {
-  long long s = 0;
-  for (int b = 0; b < n; ++b)
-    for (int d = 1; d <= 2; ++d) s += (long long)march_blocks(box[b], d) * march_cells(box[b], d);
-  return s;
+// (Column block x cell) items of both marches of a box, in the order
+// keep_march_kernel deals them to warps: y march, z march; block; cell.
+inline long long march_items(const BoxRec& R) {
+  return (long long)march_blocks(R, 1) * march_cells(R, 1) + (long long)march_blocks(R, 2) * march_cells(R, 2);
 }
 
 // Shares (warps) the items are cut into.  Every segment of a share pays a
@@ -38,32 +36,6 @@ inline long long march_shares(long long items, int waves, long long resident, in
 inline int march_cta_warps(long long shares, int nsm) {
   const long long w = shares / nsm;
   return w < 1 ? 1 : (w > 8 ? 8 : (int)w);
-}
-
-// Cuts the items into G equal shares: runs of segments (box, 2 * block + (dir - 1),
-// m0, m1).  seg(int4) appends a segment, share() ends the current warp's share.
-template <class Seg, class Share>
-inline void march_schedule(const BoxRec* box, int n, long long G, Seg&& seg, Share&& share) {
-  const double per = (double)march_items(box, n) / (double)G;
-  long long w = 0, done = 0;
-  for (int b = 0; b < n; ++b)
-    for (int d = 1; d <= 2; ++d)
-      for (int c = 0; c < march_blocks(box[b], d); ++c) {
-        int m = box[b].lo[d];
-        while (m <= box[b].hi[d]) {
-          long long fit = (long long)((double)(w + 1) * per - (double)done + 0.5);
-          if (fit < 1) fit = 1;
-          const int end = (int)(box[b].hi[d] + 1 - m < fit ? box[b].hi[d] + 1 : m + fit);
-          seg(make_int4(b, 2 * c + d - 1, m, end));
-          done += end - m;
-          m = end;
-          if ((double)done >= (double)(w + 1) * per - 0.5 && w < G - 1) {
-            ++w;
-            share();
-          }
-        }
-      }
-  for (; w < G; ++w) share();
 }
 
 }  // namespace amrs

@@ -6,12 +6,12 @@
 // allocator) and forbids allocations behind the pool's back, or one that
 // reserves a fixed device-memory budget up front.  For them this entry point
 // keeps the scratch that amrs_rhs_box takes from its handle (primitive and
-// viscous-flux fields, the box table and the face-kernel schedule) in one
+// viscous-flux fields, the y and z divergence parts and the box table) in one
 // fixed static device array, and needs no handle.
 //
 // Limits and sharing rules:
 //  * boxes of at most 32 cells in every direction (the array holds
-//    NQ x 38^3 + 12 x 34^3 + 10 x 32^3 doubles plus a 96 KiB table region, 9.6 MB);
+//    NQ x 38^3 + 12 x 34^3 + 10 x 32^3 doubles plus an 8 KiB table region, 9.5 MB);
 //    larger boxes return AMRS_ERR_SIZE;
 //  * the array exists once per device that loads the library and stays
 //    allocated until the process exits;
@@ -39,7 +39,7 @@ namespace {
 constexpr int NA_MAX_EDGE = 32;
 constexpr size_t NA_Q = (size_t)NQ * (NA_MAX_EDGE + 6) * (NA_MAX_EDGE + 6) * (NA_MAX_EDGE + 6);
 constexpr size_t NA_VF = (size_t)NVF * (NA_MAX_EDGE + 2) * (NA_MAX_EDGE + 2) * (NA_MAX_EDGE + 2);
-constexpr size_t NA_TABLE_BYTES = 96 * 1024;
+constexpr size_t NA_TABLE_BYTES = 8 * 1024;
 constexpr size_t NA_DIV = (size_t)2 * NCONS * NA_MAX_EDGE * NA_MAX_EDGE * NA_MAX_EDGE;
 constexpr size_t NA_DOUBLES = NA_Q + NA_VF + NA_DIV + NA_TABLE_BYTES / 8;
 
@@ -52,11 +52,8 @@ static __device__ __align__(256) double g_noalloc_scratch[NA_DOUBLES];
 namespace {
 
 std::mutex g_na_mu;
-// host staging of the table region and of the schedule (no heap use)
-constexpr int NA_MAX_SEGS = 4096;
+// host staging of the table region (no heap use)
 alignas(128) char g_na_host[NA_TABLE_BYTES];
-int4 g_na_segs[NA_MAX_SEGS];
-int g_na_share[NA_MAX_SEGS + 1];
 constexpr int NA_MAX_DEVICES = 64;
 double* g_na_ptr[NA_MAX_DEVICES] = {nullptr};
 int g_na_nsm[NA_MAX_DEVICES] = {0};
@@ -158,7 +155,7 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   char* tab = reinterpret_cast<char*>(divp + NA_DIV);
   const int order = sc.order_keep;
 
-  // box record, tile and balanced schedule (as the handle path builds them)
+  // box record and launch shape (as the handle path builds them)
   BoxRec R{};
   for (int d = 0; d < 3; ++d) {
     R.lo[d] = bx->lo[d];
@@ -178,21 +175,11 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   for (grid.x_threads = 256; grid.x_threads > 64; grid.x_threads /= 2)
     if (keep_x_blocks(order, n, grid.x_threads) >= 4 * nsm) break;
   grid.x_ctas = keep_x_blocks(order, n, grid.x_threads);
-  int nseg = 0, nsh = 0;
-  bool full = false;
-  const long long G = march_shares(march_items(&R, 1), 1, 8LL * keep_ctas_per_sm(order) * nsm, nsm);
-  if (G + 1 > NA_MAX_SEGS) return AMRS_ERR_SIZE;
-  g_na_share[nsh++] = 0;
-  march_schedule(&R, 1, G,
-                 [&](int4 v) {
-                   if (nseg < NA_MAX_SEGS) g_na_segs[nseg++] = v;
-                   else full = true;
-                 },
-                 [&] { g_na_share[nsh++] = nseg; });
-  if (full) return AMRS_ERR_SIZE;
+  const long long mitem[2] = {0, march_items(R)};
+  const int G = (int)march_shares(mitem[1], 1, 8LL * keep_ctas_per_sm(order) * nsm, nsm);
   const int cw = march_cta_warps(G, nsm);
   grid.march_threads = 32 * cw;
-  grid.march_ctas = (int)((G + cw - 1) / cw);
+  grid.march_ctas = (G + cw - 1) / cw;
   const int gq = std::max(order / 2, 2);
   long long pcell[2] = {0, (long long)(n[0] + 2 * gq) * (n[1] + 2 * gq) * (n[2] + 2 * gq)};
   long long vcell[2] = {0, (long long)(n[0] + 2) * (n[1] + 2) * (n[2] + 2)};
@@ -206,7 +193,7 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   cl.source = 0;  // no source term on this path
   cl.force[0] = cl.force[1] = cl.force[2] = 0.0;
 
-  // table region layout: box | closures | pcell | vcell | fwork | range flag | segs | shares
+  // table region layout: box | closures | pcell | vcell | fwork | range flag | march items
   size_t t = 0;
   const size_t o_box = t; t = al(t + sizeof(BoxRec));
   const size_t o_cl = t; t = al(t + sizeof(DClosures));
@@ -214,8 +201,7 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   const size_t o_v = t; t = al(t + sizeof(vcell));
   const size_t o_w = t; t = al(t + sizeof(fwork));
   const size_t o_rng = t; t = al(t + sizeof(int));
-  const size_t o_seg = t; t = al(t + sizeof(int4) * nseg);
-  const size_t o_sh = t; t = al(t + sizeof(int) * nsh);
+  const size_t o_mi = t; t = al(t + sizeof(mitem));
   if (t > NA_TABLE_BYTES) return AMRS_ERR_SIZE;
   char* host = g_na_host;
   std::memset(host, 0, t);
@@ -224,8 +210,7 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   std::memcpy(&host[o_p], pcell, sizeof(pcell));
   std::memcpy(&host[o_v], vcell, sizeof(vcell));
   std::memcpy(&host[o_w], fwork, sizeof(fwork));
-  std::memcpy(&host[o_seg], g_na_segs, sizeof(int4) * nseg);
-  std::memcpy(&host[o_sh], g_na_share, sizeof(int) * nsh);
+  std::memcpy(&host[o_mi], mitem, sizeof(mitem));
   // The copy also clears the range flag, which must start at zero.  From
   // pageable host memory it waits for the stream's earlier work and returns
   // once the staging is consumed, so the static host buffer can be reused.
@@ -236,9 +221,8 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   tb.pcell = reinterpret_cast<const long long*>(tab + o_p);
   tb.vcell = reinterpret_cast<const long long*>(tab + o_v);
   tb.fwork = reinterpret_cast<const int*>(tab + o_w);
-  tb.seg = reinterpret_cast<const int4*>(tab + o_seg);
-  tb.share = reinterpret_cast<const int*>(tab + o_sh);
-  tb.nshare = nsh - 1;
+  tb.mitem = reinterpret_cast<const long long*>(tab + o_mi);
+  tb.nshare = G;
   tb.cls = reinterpret_cast<const DClosures*>(tab + o_cl);
   tb.n = 1;
   tb.gq = gq;

@@ -21,8 +21,11 @@
 // two barriers per plane) with 272 FP64 instructions per cell; 128^3, KEEP4 +
 // viscous, per stage: 1257 us before, 427 + 348 us now with 185, FP64 pipe 82-85%
 // busy (in between, with one kernel for x and y tiles and a z march: 890 us).
+#include <type_traits>
+
 #include "amrs_boxes.cuh"
 #include "amrs_kernels.h"
+#include "keep_schedule.h"
 
 namespace amrs {
 
@@ -213,26 +216,27 @@ __device__ __forceinline__ void keep_x_body(const BoxTable& tb, int s_in, int s_
 
 // ---- y and z directions: one thread per column, a warp marching its 32 columns
 // over a run of cells with the shared pair terms in registers.  Writes
-// dxinv (F(m) - F(m+1)) of its direction.  Segment sg: (box, 2 * block + DIR - 1,
-// m0, m1), columns consecutive in x, then in z (y march) or y (z march).
+// dxinv (F(m) - F(m+1)) of its direction over cells [m0, m1) of column block
+// `blk`, columns consecutive in x, then in z (y march) or y (z march).
 template <int ORDER, int DIR, bool VISC, bool FAST>
-__device__ __forceinline__ void keep_march(const BoxTable& tb, const int4& sg, const double coef[3]) {
+__device__ __forceinline__ void keep_march(const BoxRec& R, int blk, int m0, int m1, const double coef[3]) {
   constexpr int H = ORDER / 2;
-  const BoxRec& R = tb.box[sg.x];
   const int nx = R.hi[0] - R.lo[0] + 1, nt = DIR == 1 ? R.hi[2] - R.lo[2] + 1 : R.hi[1] - R.lo[1] + 1;
-  const int c = (sg.y >> 1) * 32 + (threadIdx.x & 31);
+  const int c = blk * 32 + (threadIdx.x & 31);
   if (c >= nx * nt) return;
-  const int m0 = sg.z, m1 = sg.w;  // cells [m0, m1) along DIR
   const int ct = c / nx, ci = R.lo[0] + c - ct * nx;
   const int j0 = DIR == 1 ? m0 : R.lo[1] + ct, k0 = DIR == 1 ? R.lo[2] + ct : m0;
   const double dxi = R.dxinv[DIR];
-  const long long qk = DIR == 1 ? R.q.js : R.q.ks, qn = R.q.ns;
-  const long long vk = DIR == 1 ? R.vf.js : R.vf.ks, vn = R.vf.ns;
-  const long long dk = DIR == 1 ? R.div.js : R.div.ks, dn = R.div.ns;
+  // the scratch arrays' strides fit 32 bits (a box's grown cells do): orders 2
+  // and 4, at their 128 registers, keep half as many for them
+  using Stride = typename std::conditional<ORDER == 6, long long, int>::type;
+  const Stride qk = (Stride)(DIR == 1 ? R.q.js : R.q.ks), vk = (Stride)(DIR == 1 ? R.vf.js : R.vf.ks),
+               dk = (Stride)(DIR == 1 ? R.div.js : R.div.ks);
+  const Stride qn = (Stride)R.q.ns, vn = (Stride)R.vf.ns, dn = (Stride)R.div.ns;
   // pointers at cell m0 of the column
   const double* Q = R.q.p + R.q.off(ci, j0, k0);
-  const double* V = VISC ? R.vf.p + R.vf.off(ci, j0, k0) + 4 * DIR * vn : nullptr;
-  double* D = R.div.p + R.div.off(ci, j0, k0) + 5 * (DIR - 1) * dn;
+  const double* V = VISC ? R.vf.p + R.vf.off(ci, j0, k0) + 4ll * DIR * vn : nullptr;
+  double* D = R.div.p + R.div.off(ci, j0, k0) + 5ll * (DIR - 1) * dn;
   // code-6 y walls: faces of second order (halfsten 1, coefficient 1)
   auto reduced = [&](int f) { return DIR == 1 && R.walls && (f <= R.red_lo || (f >= R.red_hi && f <= R.hi[1])); };
   // carries: tc[l][m] = T_l(c+1-l+m) for m=0..l-2 (l>=2); ring of Q(c..c+H-1)
@@ -245,7 +249,7 @@ __device__ __forceinline__ void keep_march(const BoxTable& tb, const int4& sg, c
 #pragma unroll
     for (int p = 0; p < 2 * H; ++p)
 #pragma unroll
-      for (int n = 0; n < NQ; ++n) qcol[p][n] = Q[(p - H) * qk + n * qn];
+      for (int n = 0; n < NQ; ++n) qcol[p][n] = Q[(long long)(p - H) * qk + (long long)n * qn];
     const bool red = reduced(m0);
     keep_pair<DIR, FAST>(qcol[H], qcol[H - 1], red ? 1.0 : coef[0], fl);  // T_1(m0-1)
 #pragma unroll
@@ -268,8 +272,8 @@ __device__ __forceinline__ void keep_march(const BoxTable& tb, const int4& sg, c
     if (VISC) {
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
-        vl[n] = V[n * vn];
-        fl[1 + n] = fma(0.5, V[n * vn - vk] + vl[n], fl[1 + n]);
+        vl[n] = V[(long long)n * vn];
+        fl[1 + n] = fma(0.5, V[(long long)n * vn - vk] + vl[n], fl[1 + n]);
       }
     }
 #pragma unroll
@@ -282,7 +286,7 @@ __device__ __forceinline__ void keep_march(const BoxTable& tb, const int4& sg, c
     // T_l(m) = pair (m+l, m), l = 1..H: the flux at face m+1
     double qtop[NQ], F[5];
 #pragma unroll
-    for (int n = 0; n < NQ; ++n) qtop[n] = Q[H * qk + n * qn];
+    for (int n = 0; n < NQ; ++n) qtop[n] = Q[(long long)H * qk + (long long)n * qn];
     const bool red = reduced(m + 1);
     keep_pair<DIR, FAST>(H == 1 ? qtop : ring[1], ring[0], red ? 1.0 : coef[0], F);
 #pragma unroll
@@ -311,14 +315,14 @@ __device__ __forceinline__ void keep_march(const BoxTable& tb, const int4& sg, c
     if (VISC) {
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
-        const double c1 = V[vk + n * vn];
+        const double c1 = V[vk + (long long)n * vn];
         F[1 + n] = fma(0.5, vl[n] + c1, F[1 + n]);
         vl[n] = c1;
       }
     }
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
-      D[n * dn] = kmul<(AMRS_DIV_IMUL >> 1) & 1>(dxi, fl[n] - F[n]);
+      D[(long long)n * dn] = kmul<(AMRS_DIV_IMUL >> 1) & 1>(dxi, fl[n] - F[n]);
       fl[n] = F[n];
     }
 #pragma unroll
@@ -343,18 +347,31 @@ __device__ __forceinline__ bool fast_range(const BoxTable& tb) { return tb.range
 
 template <int ORDER, bool VISC, bool FAST>
 __device__ __forceinline__ void keep_march_warp(const BoxTable& tb) {
-  // balanced static schedule: this warp's segments cover an equal share of
-  // the (column block x cell) work of the whole list
+  // warp w takes items [w N / G, (w+1) N / G) of the list: a run of segments,
+  // each within one column block
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   if (w >= tb.nshare) return;
   double coef[3];
   keep_coeffs(ORDER, coef);
-  const int send = tb.share[w + 1];
+  const long long N = tb.mitem[tb.n];
+  const long long at = w * N / tb.nshare;
+  int left = (int)((w + 1) * N / tb.nshare - at);
+  int b = find_box_ll(tb.mitem, tb.n, at);
+  int r = (int)(at - tb.mitem[b]);
 #pragma unroll 1
-  for (int sgi = tb.share[w]; sgi < send; ++sgi) {
-    const int4 sg = tb.seg[sgi];
-    if (sg.y & 1) keep_march<ORDER, 2, VISC, FAST>(tb, sg, coef);
-    else keep_march<ORDER, 1, VISC, FAST>(tb, sg, coef);
+  while (left > 0) {
+    const BoxRec& R = tb.box[b];
+    const int ny = march_cells(R, 1), nz = march_cells(R, 2);
+    const int ytot = march_blocks(R, 1) * ny, ztot = march_blocks(R, 2) * nz;
+    if (r == ytot + ztot) { ++b; r = 0; continue; }
+    const bool z = r >= ytot;
+    const int p = z ? r - ytot : r, cells = z ? nz : ny;
+    const int blk = p / cells, m = p - blk * cells;
+    const int run = min(left, cells - m), m0 = R.lo[z ? 2 : 1] + m;
+    left -= run;
+    r += run;
+    if (z) keep_march<ORDER, 2, VISC, FAST>(R, blk, m0, m0 + run, coef);
+    else keep_march<ORDER, 1, VISC, FAST>(R, blk, m0, m0 + run, coef);
   }
 }
 

@@ -178,7 +178,7 @@ amrs_status amrs_rhs_box(amrs_handle* h, const amrs_box* bx, const double dxinv[
  * KEEP 2/4/6 with or without viscous terms, no JST and no source term
  * (AMRS_ERR_SCHEME otherwise, also for transport laws other than 0/1),
  * boxes of at most 32 cells per direction (AMRS_ERR_SIZE beyond); the array
- * (9.6 MB) lives on every device that loads the library until exit; every
+ * (9.5 MB) lives on every device that loads the library until exit; every
  * call shares it, so calls that overlap on the GPU race.  The kernels run on
  * the current device: a `stream` of another device is refused
  * (AMRS_ERR_STATE).  The first call on a device looks the array's address
