@@ -335,16 +335,31 @@ __device__ __forceinline__ DProg resolve_prog(DProg p) {
   return p;
 }
 
-__device__ __forceinline__ void apply_prog(const DProg& p, double reg[3]) {
+// Its products on the integer pipe (dmul_rn), or no product where the factor is
+// one.  The registers are picked by selects (an indexed array would live in
+// local memory).
+__device__ __forceinline__ double prog_mul(double a, double x) {
+  return __double_as_longlong(a) == 0x3FF0000000000000ll ? x : dmul_rn(a, x);
+}
+__device__ __forceinline__ double prog_pick(int r, double s1, double s2, double ds) {
+  return r == 0 ? s1 : (r == 1 ? s2 : ds);
+}
+// the program on registers S1, S2 and dS; the stage result is S2
+__device__ __forceinline__ double apply_prog(const DProg& p, double s1, double s2, double ds) {
 #pragma unroll
   for (int o = 0; o < 3; ++o) {
     if (o >= p.nops) break;
     const DOp& q = p.ops[o];
-    if (q.kind == 0) reg[q.dst] = q.a * reg[q.x] + q.b * reg[q.y];
-    else if (q.kind == 1) reg[q.dst] = reg[q.dst] + q.a * reg[q.x];
-    else if (q.kind == 2) reg[q.dst] = reg[q.x] + q.a * reg[q.dst];
-    else reg[q.dst] = reg[q.x];
+    const double x = prog_pick(q.x, s1, s2, ds);
+    double r = x;
+    if (q.kind == 0) r = prog_mul(q.a, x) + prog_mul(q.b, prog_pick(q.y, s1, s2, ds));
+    else if (q.kind == 1) r = prog_pick(q.dst, s1, s2, ds) + prog_mul(q.a, x);
+    else if (q.kind == 2) r = x + prog_mul(q.a, prog_pick(q.dst, s1, s2, ds));
+    if (q.dst == 0) s1 = r;
+    else if (q.dst == 1) s2 = r;
+    else ds = r;
   }
+  return s2;
 }
 
 }  // namespace amrs

@@ -22,7 +22,8 @@ cudaError_t launch_keep_face(int order, bool visc, bool src, const BoxTable& tb,
 bool keep_tile_fits(int order, int tx, int ty);
 int keep_ctas_per_sm(int order);
 
-// ---- face-array (reference-structured) path (rhs_plain.cu)
+// ---- face-array (reference-structured) path (rhs_plain.cu); `visc`: the viscous
+// averages are added to the fluxes before they are stored
 // Face flux scratch per box: three nodal arrays, described per box in FaceRec.
 struct FaceRec {
   DArr f[3];    // face fluxes, nodal in direction d, NCONS comps, over [lo,hi] (+1 in d)
@@ -42,20 +43,20 @@ struct FaceTable {
 cudaError_t launch_keep_faces_plain(int order, const BoxTable& tb, const FaceTable& ft, long long nfaces[3],
                                     int nsm, cudaStream_t st);
 cudaError_t launch_weno(const BoxTable& tb, const FaceTable& ft, int s_in, long long ngcells, long long nfaces[3],
-                        bool ref_order, int nsm, cudaStream_t st);
+                        bool ref_order, bool visc, int nsm, cudaStream_t st);
 // physical fluxes and lambda only (the forward values the WENO adjoint reads)
 cudaError_t launch_weno_point(const BoxTable& tb, const FaceTable& ft, int s_in, long long ngcells, int nsm,
                               cudaStream_t st);
 // the WENO face kernel alone (point fluxes already current)
 cudaError_t launch_weno_faces(const BoxTable& tb, const FaceTable& ft, int s_in, long long nfaces[3], bool ref_order,
-                              int nsm, cudaStream_t st);
+                              bool visc, int nsm, cudaStream_t st);
 // MUSCL slopes and face-state terms alone (the reverse pass recomputes them)
 cudaError_t launch_slopes(const BoxTable& tb, const FaceTable& ft, const long long* spre_d[3], long long nslope[3],
                           int nsm, cudaStream_t st);
 cudaError_t launch_riemann(const BoxTable& tb, const FaceTable& ft, const long long* spre_d[3],
-                           long long nslope[3], long long nfaces[3], int nsm, cudaStream_t st);
+                           long long nslope[3], long long nfaces[3], bool visc, int nsm, cudaStream_t st);
 // WENO5-reconstructed primitive states + the two-shock solver (riemann_weno = 1)
-cudaError_t launch_weno_riemann(const BoxTable& tb, const FaceTable& ft, long long nfaces[3], int nsm,
+cudaError_t launch_weno_riemann(const BoxTable& tb, const FaceTable& ft, long long nfaces[3], bool visc, int nsm,
                                 cudaStream_t st);
 // JST sensor and spectral radius alone (the reverse pass recomputes them)
 cudaError_t launch_jst_sensor(const BoxTable& tb, const FaceTable& ft, long long nvalid, int nsm, cudaStream_t st);

@@ -539,19 +539,23 @@ amrs_status list_stage(amrs_handle* h, List& L, const DProg& prog, int s_in, int
     return AMRS_OK;
   }
   long long nf[3] = {L.tot_f[0], L.tot_f[1], L.tot_f[2]};
-  // face arrays start from zero (pure viscous runs add to them)
-  for (int b = 0; b < L.n; ++b)
-    for (int d = 0; d < 3; ++d) {
-      const FaceRec& F = L.hface[b];
-      CK(cudaMemsetAsync(F.f[d].p, 0, (size_t)F.f[d].ns * NCONS * 8, st));
-    }
+  // the Euler kernels write every face; without them the viscous averages (or
+  // the divergence) start from zero.  The viscous averages join the Euler
+  // kernel's store unless JST's dissipation comes between.
+  if (!sc.rhs_euler)
+    for (int b = 0; b < L.n; ++b)
+      for (int d = 0; d < 3; ++d) {
+        const FaceRec& F = L.hface[b];
+        CK(cudaMemsetAsync(F.f[d].p, 0, (size_t)F.f[d].ns * NCONS * 8, st));
+      }
+  const bool visc_in = sc.rhs_visc && sc.rhs_euler && sc.flux_euler != 1 && sc.art_diss == 0;
   if (sc.rhs_euler) {
     if (sc.flux_euler == 1) CK(launch_keep_faces_plain(sc.order_keep, L.tb, L.ft, nf, nsm, st));
-    else if (sc.flux_euler == 2) CK(launch_weno(L.tb, L.ft, s_in, L.tot_g, nf, sc.weno_fast == 0, nsm, st));
-    else if (sc.flux_euler == 3) CK(launch_weno_riemann(L.tb, L.ft, nf, nsm, st));
+    else if (sc.flux_euler == 2) CK(launch_weno(L.tb, L.ft, s_in, L.tot_g, nf, sc.weno_fast == 0, visc_in, nsm, st));
+    else if (sc.flux_euler == 3) CK(launch_weno_riemann(L.tb, L.ft, nf, visc_in, nsm, st));
     else {
       long long ns[3] = {L.tot_s[0], L.tot_s[1], L.tot_s[2]};
-      CK(launch_riemann(L.tb, L.ft, L.d_spre, ns, nf, nsm, st));
+      CK(launch_riemann(L.tb, L.ft, L.d_spre, ns, nf, visc_in, nsm, st));
     }
     if (sc.art_diss == 1) {
       for (int b = 0; b < L.n; ++b) {
@@ -562,7 +566,7 @@ amrs_status list_stage(amrs_handle* h, List& L, const DProg& prog, int s_in, int
       CK(launch_jst(L.tb, L.ft, s_in, L.tot_g, L.tot_valid, nf, nsm, st));
     }
   }
-  if (sc.rhs_visc) CK(launch_visc_face_add(L.tb, L.ft, nf, nsm, st));
+  if (sc.rhs_visc && !visc_in) CK(launch_visc_face_add(L.tb, L.ft, nf, nsm, st));
   CK(launch_div_stage(L.tb, L.ft, s_in, s_s1, s_out, prog, rhs_only, L.tot_valid, nsm, st));
   if (h->check_nonfinite) CK(launch_nonfinite_check(L.tb, L.ft.vpre, s_out, L.tot_valid, h->derr + 1, nsm, st));
   return AMRS_OK;
@@ -1897,17 +1901,17 @@ amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const dou
     if (e == cudaSuccess && L.fused)
       e = launch_keep_face(sc.order_keep, sc.rhs_visc != 0, L.source, L.tb, 0, 1, 2, p, 0, L.grid, st);
     else if (e == cudaSuccess && sc.flux_euler == 2)
-      e = launch_weno_faces(L.tb, L.ft, 0, nf, sc.weno_fast == 0, h->nsm, st);
+      e = launch_weno_faces(L.tb, L.ft, 0, nf, sc.weno_fast == 0, sc.rhs_visc != 0, h->nsm, st);
     else if (e == cudaSuccess && sc.flux_euler == 3)
-      e = launch_weno_riemann(L.tb, L.ft, nf, h->nsm, st);
+      e = launch_weno_riemann(L.tb, L.ft, nf, sc.rhs_visc != 0, h->nsm, st);
     else if (e == cudaSuccess && sc.flux_euler == 0) {
       long long ns[3] = {L.tot_s[0], L.tot_s[1], L.tot_s[2]};
-      e = launch_riemann(L.tb, L.ft, L.d_spre, ns, nf, h->nsm, st);
+      e = launch_riemann(L.tb, L.ft, L.d_spre, ns, nf, sc.rhs_visc != 0, h->nsm, st);
     } else if (e == cudaSuccess)
       e = launch_keep_faces_plain(sc.order_keep, L.tb, L.ft, nf, h->nsm, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[3], st);
     if (e == cudaSuccess && !L.fused) {
-      if (sc.rhs_visc) e = launch_visc_face_add(L.tb, L.ft, nf, h->nsm, st);
+      if (sc.rhs_visc && sc.flux_euler == 1) e = launch_visc_face_add(L.tb, L.ft, nf, h->nsm, st);
       if (e == cudaSuccess) e = launch_div_stage(L.tb, L.ft, 0, 1, 2, p, 0, L.tot_valid, h->nsm, st);
     }
     if (e == cudaSuccess) e = cudaEventRecord(ev[4], st);

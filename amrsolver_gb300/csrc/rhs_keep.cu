@@ -196,21 +196,31 @@ __device__ __forceinline__ void keep_x_body(const BoxTable& tb, int s_in, int s_
     const double* D = R.div.p + R.div.off(i, j, k);
     const long long dn = R.div.ns, oin = Uin.off(i, j, k), o1 = U1.off(i, j, k), oo = Uo.off(i, j, k);
     const bool src = SRC && tb.cls[R.cl].source != 0;  // SRC: a list with a source term
+    // all loads of a kind before the products: their range tests are branches
+    // that loads do not cross
+    double ds[5], y[5], z[5];
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
-      double ds = kmul<AMRS_DIV_IMUL & 1>(R.dxinv[0], F[n] - fs[n * nth + tid + 1]) + D[n * dn] + D[(5 + n) * dn];
-      if (src) ds = add_source(tb.cls[R.cl], Uin.p, oin, Uin.ns, n, ds);
-      if (rhs_only) {
-        Uo.p[oo + n * Uo.ns] = ds;
-      } else {
-        double reg[3];
-        reg[0] = U1.p[o1 + n * U1.ns];
-        reg[1] = Uin.p[oin + n * Uin.ns];
-        reg[2] = ds;
-        apply_prog(prog, reg);
-        Uo.p[oo + n * Uo.ns] = reg[1];
-      }
+      y[n] = D[n * dn];
+      z[n] = D[(5 + n) * dn];
     }
+#pragma unroll
+    for (int n = 0; n < 5; ++n) {
+      ds[n] = kmul<AMRS_DIV_IMUL & 1>(R.dxinv[0], F[n] - fs[n * nth + tid + 1]) + y[n] + z[n];
+      if (src) ds[n] = add_source(tb.cls[R.cl], Uin.p, oin, Uin.ns, n, ds[n]);
+    }
+    if (!rhs_only) {
+      double s1[5], s2[5];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) {
+        s1[n] = U1.p[o1 + n * U1.ns];
+        s2[n] = Uin.p[oin + n * Uin.ns];
+      }
+#pragma unroll
+      for (int n = 0; n < 5; ++n) ds[n] = apply_prog(prog, s1[n], s2[n], ds[n]);
+    }
+#pragma unroll
+    for (int n = 0; n < 5; ++n) Uo.p[oo + n * Uo.ns] = ds[n];
   }
 }
 

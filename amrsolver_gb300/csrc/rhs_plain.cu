@@ -109,6 +109,15 @@ __global__ void __launch_bounds__(256) keep_faces_plain_kernel(BoxTable tb, Face
   }
 }
 
+// Viscous face average added to component n >= 1 of an Euler flux at face f
+// (src/rhs/CNS_hydro_K.h:254-261; the mass component adds zero).
+__device__ __forceinline__ double visc_average(const BoxRec& R, const FaceIdx& f, int n, double flx) {
+  const DArr& V = R.vf;
+  const long long s = (f.d == 0) ? 1 : (f.d == 1 ? V.js : V.ks);
+  const double* v = V.p + V.off(f.i, f.j, f.k) + (4 * f.d + n - 1) * V.ns;
+  return fma(0.5, v[-s] + v[0], flx);
+}
+
 // ------------------------------------------------------------- WENO5 ----
 // Physical Euler fluxes + max eigenvalue: src/rhs/High_resolution.h:83-121.
 #ifndef AMRS_WPF_IMUL
@@ -353,7 +362,7 @@ static __device__ __noinline__ double weno_llf_plain(const double* p0, long long
 // (11 of the products and the quotients on the integer pipe, one thread per
 // face) and after: 256^3 54.0 -> 29.4 ms, 64^3 874 -> 464 us, the tube 78 -> 41 us;
 // with 2 CTAs per SM 30.1 ms at 256^3, with 4 (64 registers) 32.6 ms.
-template <bool REF_ORDER>
+template <bool REF_ORDER, bool VISC>
 __global__ void __launch_bounds__(256, 3) weno_face_kernel(BoxTable tb, FaceTable ft, int s_in, long long total) {
   if (list_idle(tb)) return;
   const int n = blockIdx.y;
@@ -403,6 +412,7 @@ __global__ void __launch_bounds__(256, 3) weno_face_kernel(BoxTable tb, FaceTabl
                          fma(0.5, p[1], -h[1]), ok);
       if (!ok) flx = weno_llf_plain(p0, st, u0, su, me);
     }
+    if (VISC && n > 0) flx = visc_average(R, f, n, flx);
     const DArr Fd = FR.f[f.d];
     Fd.p[Fd.off(f.i, f.j, f.k) + n * Fd.ns] = flx;
   }
@@ -853,6 +863,7 @@ __device__ __forceinline__ void riemann_prob(const double gamma, const double sm
 // integer pipe about half full; two CTAs per SM (128 registers) beat three
 // (2.94 against 3.10 ms per step at 96^3).  48^3, with the hardware's roots and
 // products and checked integer quotients before: 194 -> 86 us.
+template <bool VISC>
 __global__ void __launch_bounds__(256, 2) riemann_face_kernel(BoxTable tb, FaceTable ft, long long total) {
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -890,11 +901,10 @@ __global__ void __launch_bounds__(256, 2) riemann_face_kernel(BoxTable tb, FaceT
     riemann_prob(gam, 1.0e-40, in, F);
     const DArr Fd = ft.fr[f.b].f[d];
     const long long of = Fd.off(f.i, f.j, f.k);
-    Fd.p[of + URHO * Fd.ns] = F[0];
-    Fd.p[of + UN * Fd.ns] = F[1];
-    Fd.p[of + UT1 * Fd.ns] = F[2];
-    Fd.p[of + UT2 * Fd.ns] = F[3];
-    Fd.p[of + UET * Fd.ns] = F[4];
+    const int comp_of[5] = {URHO, UN, UT1, UT2, UET};
+#pragma unroll
+    for (int n = 0; n < 5; ++n)
+      Fd.p[of + comp_of[n] * Fd.ns] = VISC && n > 0 ? visc_average(R, f, comp_of[n], F[n]) : F[n];
   }
 }
 
@@ -905,6 +915,7 @@ __global__ void __launch_bounds__(256, 2) riemann_face_kernel(BoxTable tb, FaceT
 // i-3..i+1; right state: the mirror i+2..i-2), rho and p floored at 1e-40
 // as the MUSCL states are (src/rhs/Riemann.h:260-272), and riemann_prob
 // gives the flux.  One thread per face.
+template <bool VISC>
 __global__ void __launch_bounds__(256) weno_riemann_face_kernel(BoxTable tb, FaceTable ft, long long total) {
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -936,11 +947,10 @@ __global__ void __launch_bounds__(256) weno_riemann_face_kernel(BoxTable tb, Fac
     riemann_prob(cl.gamma, 1.0e-40, in, F);
     const DArr Fd = ft.fr[f.b].f[d];
     const long long of = Fd.off(f.i, f.j, f.k);
-    Fd.p[of + URHO * Fd.ns] = F[0];
-    Fd.p[of + UN * Fd.ns] = F[1];
-    Fd.p[of + UT1 * Fd.ns] = F[2];
-    Fd.p[of + UT2 * Fd.ns] = F[3];
-    Fd.p[of + UET * Fd.ns] = F[4];
+    const int comp_of[5] = {URHO, UN, UT1, UT2, UET};
+#pragma unroll
+    for (int n = 0; n < 5; ++n)
+      Fd.p[of + comp_of[n] * Fd.ns] = VISC && n > 0 ? visc_average(R, f, comp_of[n], F[n]) : F[n];
   }
 }
 
@@ -1033,36 +1043,41 @@ __global__ void __launch_bounds__(256) visc_face_add_kernel(BoxTable tb, FaceTab
 }
 
 // --------------------------------------- divergence + stage program ----
-// src/tim/CNS_advance.cpp:384-390, then the BLAS-1 program of the stage.
-__global__ void __launch_bounds__(256) div_stage_kernel(BoxTable tb, FaceTable ft, int s_in, int s_s1, int s_out,
-                                                        DProg prog_in, int rhs_only, long long total) {
+// src/tim/CNS_advance.cpp:384-390, then the BLAS-1 program of the stage; one
+// thread per cell and component (blockIdx.y), every load issued before the first
+// product (their range tests are branches that loads do not cross).  Bound: the
+// loads' latency and the FP64 pipe (25 to 35 instructions per cell with every
+// product on the integer pipe, 60 to 75 before).  256^3: 2.07 -> 1.46 ms per stage
+// (products moved, loads in program order: 1.87; one thread per cell: 2.97).
+__global__ void __launch_bounds__(256, 5) div_stage_kernel(BoxTable tb, FaceTable ft, int s_in, int s_s1, int s_out,
+                                                           DProg prog_in, int rhs_only, long long total) {
   if (list_idle(tb)) return;
   const DProg prog = resolve_prog(prog_in);
+  const int n = blockIdx.y;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(ft.vpre, tb.n, g);
     const BoxRec& R = tb.box[b];
-    int i, j, k;
-    decode_cell(R, (int)(g - ft.vpre[b]), 0, i, j, k);
     const FaceRec& FR = ft.fr[b];
-    const DArr Fx = FR.f[0], Fy = FR.f[1], Fz = FR.f[2];
-    const long long ox = Fx.off(i, j, k), oy = Fy.off(i, j, k), oz = Fz.off(i, j, k);
-    const DArr Uin = R.slot[s_in], U1 = R.slot[s_s1], Uo = R.slot[s_out];
-    const DClosures& cl = tb.cls[R.cl];
-    const long long oin = Uin.off(i, j, k);
-    for (int n = 0; n < 5; ++n) {
-      double ds = R.dxinv[0] * (Fx.p[ox + n * Fx.ns] - Fx.p[ox + 1 + n * Fx.ns]) +
-                  R.dxinv[1] * (Fy.p[oy + n * Fy.ns] - Fy.p[oy + Fy.js + n * Fy.ns]) +
-                  R.dxinv[2] * (Fz.p[oz + n * Fz.ns] - Fz.p[oz + Fz.ks + n * Fz.ns]);
-      if (cl.source) ds = add_source(cl, Uin.p, oin, Uin.ns, n, ds);
-      if (rhs_only) {
-        Uo(i, j, k, n) = ds;
-      } else {
-        double reg[3] = {U1(i, j, k, n), Uin(i, j, k, n), ds};
-        apply_prog(prog, reg);
-        Uo(i, j, k, n) = reg[1];
-      }
+    const int loc = (int)(g - ft.vpre[b]);
+    const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
+    const int t = loc / nx, i = loc - t * nx, k = t / ny, j = t - k * ny;  // in the box
+    // face arrays: rows of nx + 1, nx, nx (nodal in their direction)
+    const double* px = FR.f[0].p + n * FR.f[0].ns + (loc + t);
+    const double* py = FR.f[1].p + n * FR.f[1].ns + (loc + k * nx);
+    const double* pz = FR.f[2].p + n * FR.f[2].ns + loc;
+    const DArr &Uin = R.slot[s_in], &U1 = R.slot[s_s1], &Uo = R.slot[s_out];
+    const int gi = i + R.lo[0], gj = j + R.lo[1], gk = k + R.lo[2];
+    const double x0 = px[0], x1 = px[1], y0 = py[0], y1 = py[nx], z0 = pz[0], z1 = pz[nx * ny];
+    double s1 = 0.0, s2 = 0.0;
+    if (!rhs_only) {
+      s1 = U1(gi, gj, gk, n);
+      s2 = Uin(gi, gj, gk, n);
     }
+    double ds = dmul_rn(R.dxinv[0], x0 - x1) + dmul_rn(R.dxinv[1], y0 - y1) + dmul_rn(R.dxinv[2], z0 - z1);
+    const DClosures& cl = tb.cls[R.cl];
+    if (cl.source) ds = add_source(cl, Uin.p, Uin.off(gi, gj, gk), Uin.ns, n, ds);
+    Uo(gi, gj, gk, n) = rhs_only ? ds : apply_prog(prog, s1, s2, ds);
   }
 }
 
@@ -1084,19 +1099,20 @@ cudaError_t launch_weno_point(const BoxTable& tb, const FaceTable& ft, int s_in,
 }
 
 cudaError_t launch_weno_faces(const BoxTable& tb, const FaceTable& ft, int s_in, long long nfaces[3], bool ref_order,
-                              int nsm, cudaStream_t st) {
+                              bool visc, int nsm, cudaStream_t st) {
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
   const dim3 grid(grid_for(tot, nsm), NCONS);
-  if (ref_order) weno_face_kernel<true><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
-  else weno_face_kernel<false><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
+  if (ref_order && visc) weno_face_kernel<true, true><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
+  else if (ref_order) weno_face_kernel<true, false><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
+  else if (visc) weno_face_kernel<false, true><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
+  else weno_face_kernel<false, false><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_weno(const BoxTable& tb, const FaceTable& ft, int s_in, long long ngcells, long long nfaces[3],
-                        bool ref_order, int nsm, cudaStream_t st) {
+                        bool ref_order, bool visc, int nsm, cudaStream_t st) {
   weno_flux_lambda_kernel<<<grid_for(ngcells, nsm), 256, 0, st>>>(tb, ft, s_in, ngcells);
-  launch_weno_faces(tb, ft, s_in, nfaces, ref_order, nsm, st);
-  return cudaGetLastError();
+  return launch_weno_faces(tb, ft, s_in, nfaces, ref_order, visc, nsm, st);
 }
 
 cudaError_t launch_slopes(const BoxTable& tb, const FaceTable& ft, const long long* spre_d[3], long long nslope[3],
@@ -1108,19 +1124,21 @@ cudaError_t launch_slopes(const BoxTable& tb, const FaceTable& ft, const long lo
 }
 
 cudaError_t launch_riemann(const BoxTable& tb, const FaceTable& ft, const long long* spre_d[3], long long nslope[3],
-                           long long nfaces[3], int nsm, cudaStream_t st) {
+                           long long nfaces[3], bool visc, int nsm, cudaStream_t st) {
   const long long ts = nslope[0] + nslope[1] + nslope[2];
   slope_kernel<<<grid_for(ts, nsm), 256, 0, st>>>(tb, ft, spre_d[0], spre_d[1], spre_d[2], nslope[0], nslope[1],
                                                   nslope[2]);
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
-  riemann_face_kernel<<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
+  if (visc) riemann_face_kernel<true><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
+  else riemann_face_kernel<false><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
   return cudaGetLastError();
 }
 
-cudaError_t launch_weno_riemann(const BoxTable& tb, const FaceTable& ft, long long nfaces[3], int nsm,
+cudaError_t launch_weno_riemann(const BoxTable& tb, const FaceTable& ft, long long nfaces[3], bool visc, int nsm,
                                 cudaStream_t st) {
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
-  weno_riemann_face_kernel<<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
+  if (visc) weno_riemann_face_kernel<true><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
+  else weno_riemann_face_kernel<false><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
   return cudaGetLastError();
 }
 
@@ -1147,7 +1165,7 @@ cudaError_t launch_visc_face_add(const BoxTable& tb, const FaceTable& ft, long l
 
 cudaError_t launch_div_stage(const BoxTable& tb, const FaceTable& ft, int s_in, int s_s1, int s_out,
                              const DProg& prog, int rhs_only, long long nvalid, int nsm, cudaStream_t st) {
-  div_stage_kernel<<<grid_for(nvalid, nsm), 256, 0, st>>>(tb, ft, s_in, s_s1, s_out, prog, rhs_only, nvalid);
+  div_stage_kernel<<<dim3(grid_for(nvalid, nsm), NCONS), 256, 0, st>>>(tb, ft, s_in, s_s1, s_out, prog, rhs_only, nvalid);
   return cudaGetLastError();
 }
 
