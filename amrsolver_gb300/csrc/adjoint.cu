@@ -98,14 +98,15 @@ __device__ __forceinline__ void keep_pair_vjp(const double* q1, const double* q2
 // One thread per (direction, separation, pair): pairs (a, a+l) along d
 // with a in [lo-l, hi] and transverse indices in the valid box.
 template <int ORDER>
-__global__ void __launch_bounds__(256) adj_pair_kernel(BoxTable tb, AdjRec ar, long long total) {
+__global__ void __launch_bounds__(256) adj_pair_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total) {
+  dep_begin();
   constexpr int H = ORDER / 2;
   double coef[3];
   if (ORDER == 6) { coef[0] = 6.0 / 4; coef[1] = -6.0 / 20; coef[2] = 2.0 / 60; }
   else if (ORDER == 4) { coef[0] = 4.0 / 3; coef[1] = -2.0 / 12; coef[2] = 0.0; }
   else { coef[0] = 1.0; coef[1] = 0.0; coef[2] = 0.0; }
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const int n0 = R.hi[0] - R.lo[0] + 1, n1 = R.hi[1] - R.lo[1] + 1, n2 = R.hi[2] - R.lo[2] + 1;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
@@ -170,9 +171,10 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(BoxTable tb, AdjRec ar, l
 // shuffles, then the warps in order) into ar.part; adj_param_sum_kernel adds
 // the blocks' sums in block order.  No atomics: the result is the same bits
 // on every run.
-__global__ void __launch_bounds__(256) adj_visc_kernel(BoxTable tb, AdjRec ar, long long total, double* pbar) {
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+__global__ void __launch_bounds__(256) adj_visc_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, double* pbar) {
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const int nx = R.hi[0] - R.lo[0] + 3, ny = R.hi[1] - R.lo[1] + 3;
   double mu_acc = 0.0, la_acc = 0.0;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(256) adj_visc_kernel(BoxTable tb, AdjRec ar, l
 
 // pbar += the per-block sums of adj_visc_kernel, in block order.
 __global__ void adj_param_sum_kernel(const double* part, int nblocks, double* pbar) {
+  dep_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double m = 0.0, a = 0.0;
   for (int b = 0; b < nblocks; ++b) {
@@ -298,10 +301,11 @@ __global__ void adj_param_sum_kernel(const double* part, int nblocks, double* pb
 
 // Qbar gather + cons2prim VJP for every cell of grow(box,3).
 template <int ORDER>
-__global__ void __launch_bounds__(256) adj_gather_kernel(BoxTable tb, AdjRec ar, long long total, int gpair) {
+__global__ void __launch_bounds__(256) adj_gather_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, int gpair) {
+  dep_begin();
   constexpr int H = ORDER / 2;
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const int g3 = NGHOST;
   const int nx = R.hi[0] - R.lo[0] + 1 + 2 * g3, ny = R.hi[1] - R.lo[1] + 1 + 2 * g3;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -384,6 +388,7 @@ __global__ void __launch_bounds__(256) adj_gather_kernel(BoxTable tb, AdjRec ar,
 // stage input's valid values (register S2 before the program) and of dSdt.
 __global__ void __launch_bounds__(256) adj_prog_kernel(BoxRec R, DProg prog, DArr wbar, DArr s1bar, DArr inbar,
                                                        DArr vbar, long long total, int accumulate) {
+  dep_begin();
   const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
@@ -459,6 +464,7 @@ __device__ __forceinline__ int images(int c, int lo, int hi, int bcl, int bch, i
 }
 
 __global__ void __launch_bounds__(256) adj_halo_kernel(HaloBox hb, long long total) {
+  dep_begin();
   const int nx = hb.hi[0] - hb.lo[0] + 1, ny = hb.hi[1] - hb.lo[1] + 1;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
@@ -485,6 +491,7 @@ __global__ void __launch_bounds__(256) adj_halo_kernel(HaloBox hb, long long tot
 // ubar(URHO) += vbar(UMX+d) f_d and ubar(UMX+d) += vbar(UET) f_d.
 __global__ void __launch_bounds__(256) adj_source_kernel(BoxRec R, double f0, double f1, double f2, DArr vbar,
                                                          DArr ubar, long long total) {
+  dep_begin();
   const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
   const double f[3] = {f0, f1, f2};
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -529,40 +536,40 @@ cudaError_t launch_rhs_vjp(int order, const BoxTable& tb, const AdjRecHost& ah, 
   for (int d = 0; d < 3; ++d)
     for (int l = 1; l <= H; ++l) npair += (n0 + (d == 0) * l) * (n1 + (d == 1) * l) * (n2 + (d == 2) * l);
   // order 0: no KEEP pairs (the viscous part of another scheme's RHS)
-  if (order == 2) adj_pair_kernel<2><<<grid256(npair, nsm), 256, 0, st>>>(tb, ar, npair);
-  else if (order == 4) adj_pair_kernel<4><<<grid256(npair, nsm), 256, 0, st>>>(tb, ar, npair);
-  else if (order == 6) adj_pair_kernel<6><<<grid256(npair, nsm), 256, 0, st>>>(tb, ar, npair);
+  if (order == 2) launch_dep(adj_pair_kernel<2>, grid256(npair, nsm), 256, 0, st, tb, ar, npair);
+  else if (order == 4) launch_dep(adj_pair_kernel<4>, grid256(npair, nsm), 256, 0, st, tb, ar, npair);
+  else if (order == 6) launch_dep(adj_pair_kernel<6>, grid256(npair, nsm), 256, 0, st, tb, ar, npair);
   const long long nv = (n0 + 2) * (n1 + 2) * (n2 + 2);
   if (ah.visc) {
     const int nbv = grid256(nv, nsm);  // at most 8 blocks per SM: ah.part holds 2 x 8 x nsm doubles
-    adj_visc_kernel<<<nbv, 256, 0, st>>>(tb, ar, nv, pbar);
-    if (pbar) adj_param_sum_kernel<<<1, 32, 0, st>>>(ah.part, nbv, pbar);
+    launch_dep(adj_visc_kernel, nbv, 256, 0, st, tb, ar, nv, pbar);
+    if (pbar) launch_dep(adj_param_sum_kernel, 1, 32, 0, st, ah.part, nbv, pbar);
   }
   const long long ng = (n0 + 6) * (n1 + 6) * (n2 + 6);
-  if (order == 0) adj_gather_kernel<0><<<grid256(ng, nsm), 256, 0, st>>>(tb, ar, ng, 0);
-  else if (order == 2) adj_gather_kernel<2><<<grid256(ng, nsm), 256, 0, st>>>(tb, ar, ng, H);
-  else if (order == 4) adj_gather_kernel<4><<<grid256(ng, nsm), 256, 0, st>>>(tb, ar, ng, H);
-  else adj_gather_kernel<6><<<grid256(ng, nsm), 256, 0, st>>>(tb, ar, ng, H);
+  if (order == 0) launch_dep(adj_gather_kernel<0>, grid256(ng, nsm), 256, 0, st, tb, ar, ng, 0);
+  else if (order == 2) launch_dep(adj_gather_kernel<2>, grid256(ng, nsm), 256, 0, st, tb, ar, ng, H);
+  else if (order == 4) launch_dep(adj_gather_kernel<4>, grid256(ng, nsm), 256, 0, st, tb, ar, ng, H);
+  else launch_dep(adj_gather_kernel<6>, grid256(ng, nsm), 256, 0, st, tb, ar, ng, H);
   return cudaGetLastError();
 }
 
 cudaError_t launch_adj_prog(const BoxRec& R, const DProg& prog, const DArr& wbar, const DArr& s1bar, const DArr& inbar,
                             const DArr& vbar, int accumulate, int nsm, cudaStream_t st) {
   const long long n = (long long)(R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1);
-  adj_prog_kernel<<<grid256(n, nsm), 256, 0, st>>>(R, prog, wbar, s1bar, inbar, vbar, n, accumulate);
+  launch_dep(adj_prog_kernel, grid256(n, nsm), 256, 0, st, R, prog, wbar, s1bar, inbar, vbar, n, accumulate);
   return cudaGetLastError();
 }
 
 cudaError_t launch_source_vjp(const BoxRec& R, const double force[3], const DArr& vbar, const DArr& ubar, int nsm,
                               cudaStream_t st) {
   const long long n = (long long)(R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1);
-  adj_source_kernel<<<grid256(n, nsm), 256, 0, st>>>(R, force[0], force[1], force[2], vbar, ubar, n);
+  launch_dep(adj_source_kernel, grid256(n, nsm), 256, 0, st, R, force[0], force[1], force[2], vbar, ubar, n);
   return cudaGetLastError();
 }
 
 cudaError_t launch_adj_halo(const HaloBox& hb, int nsm, cudaStream_t st) {
   const long long n = (long long)(hb.hi[0] - hb.lo[0] + 1) * (hb.hi[1] - hb.lo[1] + 1) * (hb.hi[2] - hb.lo[2] + 1);
-  adj_halo_kernel<<<grid256(n, nsm), 256, 0, st>>>(hb, n);
+  launch_dep(adj_halo_kernel, grid256(n, nsm), 256, 0, st, hb, n);
   return cudaGetLastError();
 }
 

@@ -43,10 +43,11 @@ __device__ __forceinline__ bool valid_cell(const BoxRec& R, int i, int j, int k)
   return i >= R.lo[0] && i <= R.hi[0] && j >= R.lo[1] && j <= R.hi[1] && k >= R.lo[2] && k <= R.hi[2];
 }
 
-__global__ void __launch_bounds__(256) jst_vjp_face_kernel(BoxTable tb, FaceRec fr, DArr vbar, JBuf jb, int d,
+__global__ void __launch_bounds__(256) jst_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, JBuf jb, int d,
                                                            long long total) {
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const DArr U = R.slot[0];
   const DArr S = fr.sen, L = fr.lam;
   const int di = d == 0, dj = d == 1, dk = d == 2;
@@ -101,10 +102,11 @@ __global__ void __launch_bounds__(256) jst_vjp_face_kernel(BoxTable tb, FaceRec 
   }
 }
 
-__global__ void __launch_bounds__(256) jst_vjp_sensor_kernel(BoxTable tb, JBuf j0, JBuf j1, JBuf j2, double* cs_buf,
+__global__ void __launch_bounds__(256) jst_vjp_sensor_kernel(const __grid_constant__ BoxTable tb, JBuf j0, JBuf j1, JBuf j2, double* cs_buf,
                                                              long long total) {
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const DArr q = R.q;
   const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
   const JBuf jb[3] = {j0, j1, j2};
@@ -156,10 +158,11 @@ __global__ void __launch_bounds__(256) jst_vjp_sensor_kernel(BoxTable tb, JBuf j
   }
 }
 
-__global__ void __launch_bounds__(256) jst_vjp_gather_kernel(BoxTable tb, DArr ubar, JBuf j0, JBuf j1, JBuf j2,
+__global__ void __launch_bounds__(256) jst_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, JBuf j0, JBuf j1, JBuf j2,
                                                              const double* cs_buf, long long nvalid, long long total) {
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const int mx = R.hi[0] - R.lo[0] + 5, my = R.hi[1] - R.lo[1] + 5;
   const int vx = R.hi[0] - R.lo[0] + 1, vy = R.hi[1] - R.lo[1] + 1;
   const JBuf jb[3] = {j0, j1, j2};
@@ -252,12 +255,12 @@ cudaError_t launch_jst_vjp(const BoxTable& tb, const FaceRec& fr, const DArr& vb
     jb[d].nx = n[0] + (d == 0);
     jb[d].ny = n[1] + (d == 1);
     p += jb[d].nf * JSLOT;
-    jst_vjp_face_kernel<<<grid_j(jb[d].nf, nsm), 256, 0, st>>>(tb, fr, vbar, jb[d], d, jb[d].nf);
+    launch_dep(jst_vjp_face_kernel, grid_j(jb[d].nf, nsm), 256, 0, st, tb, fr, vbar, jb[d], d, jb[d].nf);
   }
   const long long nvalid = (long long)n[0] * n[1] * n[2];
-  jst_vjp_sensor_kernel<<<grid_j(nvalid, nsm), 256, 0, st>>>(tb, jb[0], jb[1], jb[2], p, nvalid);
+  launch_dep(jst_vjp_sensor_kernel, grid_j(nvalid, nsm), 256, 0, st, tb, jb[0], jb[1], jb[2], p, nvalid);
   const long long tot = (long long)(n[0] + 4) * (n[1] + 4) * (n[2] + 4);
-  jst_vjp_gather_kernel<<<grid_j(tot, nsm), 256, 0, st>>>(tb, ubar, jb[0], jb[1], jb[2], p, nvalid, tot);
+  launch_dep(jst_vjp_gather_kernel, grid_j(tot, nsm), 256, 0, st, tb, ubar, jb[0], jb[1], jb[2], p, nvalid, tot);
   return cudaGetLastError();
 }
 

@@ -64,12 +64,13 @@ struct SBuf {
 // chain per face, and 16 warps hide its latency better than 8 with all the
 // registers it would otherwise take (measured: 7.97 against 8.97 ms per
 // SSPRK3 step VJP at 64^3).
-__global__ void __launch_bounds__(256, 2) muscl_vjp_face_kernel(BoxTable tb, FaceRec fr, DArr vbar, FBuf fs, int d,
+__global__ void __launch_bounds__(256, 2) muscl_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FBuf fs, int d,
                                                              long long total) {
-  const BoxRec& R = tb.box[0];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
   const DArr q = R.q;
   const DArr S = fr.slope[d];
-  const DClosures& cl = tb.cls[R.cl];
+  const DClosures& cl = box_cls(tb, R);
   const int di = d == 0, dj = d == 1, dk = d == 2;
   const int QN = QU + d, QT1 = (d == 0) ? QV : QU, QT2 = (d == 2) ? QV : QW;
   const int UN = UMX + d, UT1 = (d == 0) ? UMY : UMX, UT2 = (d == 2) ? UMY : UMZ;
@@ -142,11 +143,12 @@ __device__ __forceinline__ void mc_vjp(double l, double r, double db, double& lb
   }
 }
 
-__global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(BoxTable tb, FaceRec fr, FBuf fs, SBuf ss, int d,
+__global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, FBuf fs, SBuf ss, int d,
                                                               long long total) {
-  const BoxRec& R = tb.box[0];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
   const DArr q = R.q;
-  const DClosures& cl = tb.cls[R.cl];
+  const DClosures& cl = box_cls(tb, R);
   const int di = d == 0, dj = d == 1, dk = d == 2;
   const int QN = QU + d, QT1 = (d == 0) ? QV : QU, QT2 = (d == 2) ? QV : QW;
   const long long s = (d == 0) ? 1 : (d == 1 ? q.js : q.ks);
@@ -268,10 +270,11 @@ __global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(Bo
   }
 }
 
-__global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_gather_kernel(BoxTable tb, DArr ubar, SBuf s0, SBuf s1, SBuf s2,
+__global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, SBuf s0, SBuf s1, SBuf s2,
                                                                long long total) {
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const int nx = R.hi[0] - R.lo[0] + 5, ny = R.hi[1] - R.lo[1] + 5;
   const SBuf sb[3] = {s0, s1, s2};
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -362,11 +365,11 @@ cudaError_t launch_muscl_vjp(const BoxTable& tb, const FaceRec& fr, const DArr& 
     fb.nf = face_count(n, d);
     fb.nx = n[0] + (d == 0);
     fb.ny = n[1] + (d == 1);
-    muscl_vjp_face_kernel<<<grid_m(fb.nf, nsm), 256, 0, st>>>(tb, fr, vbar, fb, d, fb.nf);
-    muscl_vjp_slope_kernel<<<grid_m(sb[d].nc, nsm), 256, 0, st>>>(tb, fr, fb, sb[d], d, sb[d].nc);
+    launch_dep(muscl_vjp_face_kernel, grid_m(fb.nf, nsm), 256, 0, st, tb, fr, vbar, fb, d, fb.nf);
+    launch_dep(muscl_vjp_slope_kernel, grid_m(sb[d].nc, nsm), 256, 0, st, tb, fr, fb, sb[d], d, sb[d].nc);
   }
   const long long tot = (long long)(n[0] + 4) * (n[1] + 4) * (n[2] + 4);
-  muscl_vjp_gather_kernel<<<grid_m(tot, nsm), 256, 0, st>>>(tb, ubar, sb[0], sb[1], sb[2], tot);
+  launch_dep(muscl_vjp_gather_kernel, grid_m(tot, nsm), 256, 0, st, tb, ubar, sb[0], sb[1], sb[2], tot);
   return cudaGetLastError();
 }
 

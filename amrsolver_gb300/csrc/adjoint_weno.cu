@@ -42,9 +42,10 @@ __device__ __forceinline__ double vget0(const DArr& v, const BoxRec& R, int i, i
 }
 
 // One thread per face of direction d.
-__global__ void __launch_bounds__(256) weno_vjp_face_kernel(BoxTable tb, FaceRec fr, DArr vbar, FaceBuf fb, int d,
+__global__ void __launch_bounds__(256) weno_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FaceBuf fb, int d,
                                                             long long total) {
-  const BoxRec& R = tb.box[0];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
   const int di = d == 0, dj = d == 1, dk = d == 2;
   const DArr U = R.slot[0];
   const DArr PF = fr.pf[d];
@@ -102,10 +103,11 @@ __global__ void __launch_bounds__(256) weno_vjp_face_kernel(BoxTable tb, FaceRec
 
 // Gather + VJP of cons2eulerflux_lambda (src/rhs/High_resolution.h:83-121)
 // for direction d, over cells [lo-3, hi+3] along d and the valid range across.
-__global__ void __launch_bounds__(256) weno_vjp_gather_kernel(BoxTable tb, DArr ubar, FaceBuf fb, int d, int m0,
+__global__ void __launch_bounds__(256) weno_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, FaceBuf fb, int d, int m0,
                                                               int m1, long long total) {
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const DArr U = R.slot[0];
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
@@ -224,10 +226,10 @@ cudaError_t launch_weno_vjp(const BoxTable& tb, const FaceRec& fr, const DArr& v
     fb.nx = n[0] + (d == 0);
     fb.ny = n[1] + (d == 1);
     fb.nf = (long long)fb.nx * fb.ny * (n[2] + (d == 2));
-    weno_vjp_face_kernel<<<grid_n(fb.nf, nsm), 256, 0, st>>>(tb, fr, vbar, fb, d, fb.nf);
+    launch_dep(weno_vjp_face_kernel, grid_n(fb.nf, nsm), 256, 0, st, tb, fr, vbar, fb, d, fb.nf);
     const int m0 = n[0] + (d == 0 ? 6 : 0), m1 = n[1] + (d == 1 ? 6 : 0), m2 = n[2] + (d == 2 ? 6 : 0);
     const long long tot = (long long)m0 * m1 * m2;
-    weno_vjp_gather_kernel<<<grid_n(tot, nsm), 256, 0, st>>>(tb, ubar, fb, d, m0, m1, tot);
+    launch_dep(weno_vjp_gather_kernel, grid_n(tot, nsm), 256, 0, st, tb, ubar, fb, d, m0, m1, tot);
   }
   return cudaGetLastError();
 }

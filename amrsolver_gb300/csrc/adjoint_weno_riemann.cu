@@ -42,10 +42,11 @@ __device__ __forceinline__ double vget_r(const DArr& v, const BoxRec& R, int i, 
 // Three CTAs per SM (85 registers, the rest spilled): 24 warps hide the
 // latency of the reverse solver's chain (measured: 11.96 against 13.96 ms
 // per SSPRK3 step VJP at 64^3 with the unconstrained 255 registers).
-__global__ void __launch_bounds__(256, 3) wr_vjp_face_kernel(BoxTable tb, DArr vbar, RBuf rb, int d, long long total) {
-  const BoxRec& R = tb.box[0];
+__global__ void __launch_bounds__(256, 3) wr_vjp_face_kernel(const __grid_constant__ BoxTable tb, DArr vbar, RBuf rb, int d, long long total) {
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
   const DArr q = R.q;
-  const DClosures& cl = tb.cls[R.cl];
+  const DClosures& cl = box_cls(tb, R);
   const int di = d == 0, dj = d == 1, dk = d == 2;
   const int UN = UMX + d, UT1 = (d == 0) ? UMY : UMX, UT2 = (d == 2) ? UMY : UMZ;
   const int comp[5] = {QRHO, QU + d, QPRES, (d == 0) ? QV : QU, (d == 2) ? QV : QW};
@@ -103,10 +104,11 @@ __global__ void __launch_bounds__(256, 3) wr_vjp_face_kernel(BoxTable tb, DArr v
 
 // Cells lo-3 .. hi+3 along d (the stencils of faces lo .. hi+1), the valid
 // range across.
-__global__ void __launch_bounds__(256) wr_vjp_gather_kernel(BoxTable tb, DArr ubar, RBuf rb, int d, int m0, int m1,
+__global__ void __launch_bounds__(256) wr_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, RBuf rb, int d, int m0, int m1,
                                                             long long total) {
-  const BoxRec& R = tb.box[0];
-  const DClosures& cl = tb.cls[R.cl];
+  dep_begin();
+  const BoxRec& R = box_rec(tb, 0);
+  const DClosures& cl = box_cls(tb, R);
   const int comp[5] = {QRHO, QU + d, QPRES, (d == 0) ? QV : QU, (d == 2) ? QV : QW};
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
@@ -164,10 +166,10 @@ cudaError_t launch_weno_riemann_vjp(const BoxTable& tb, const DArr& vbar, const 
     rb.nx = n[0] + (d == 0);
     rb.ny = n[1] + (d == 1);
     rb.nf = (long long)rb.nx * rb.ny * (n[2] + (d == 2));
-    wr_vjp_face_kernel<<<grid_r(rb.nf, nsm), 256, 0, st>>>(tb, vbar, rb, d, rb.nf);
+    launch_dep(wr_vjp_face_kernel, grid_r(rb.nf, nsm), 256, 0, st, tb, vbar, rb, d, rb.nf);
     const int m0 = n[0] + (d == 0 ? 6 : 0), m1 = n[1] + (d == 1 ? 6 : 0), m2 = n[2] + (d == 2 ? 6 : 0);
     const long long tot = (long long)m0 * m1 * m2;
-    wr_vjp_gather_kernel<<<grid_r(tot, nsm), 256, 0, st>>>(tb, ubar, rb, d, m0, m1, tot);
+    launch_dep(wr_vjp_gather_kernel, grid_r(tot, nsm), 256, 0, st, tb, ubar, rb, d, m0, m1, tot);
   }
   return cudaGetLastError();
 }

@@ -46,7 +46,23 @@ struct BoxTable {
   // the FP64 pipe) and clears the other of the pair, the next stage's
   int* range;
   int* range_next;
+  long long tot_p, tot_v, tot_m;  // cells of the primitive and viscous regions, march items
+  // a list of one box carries its record and closures in the launch itself, so
+  // that a kernel's first load is already data and per-box calls copy nothing
+  int one;
+  BoxRec rec;
+  DClosures rec_cls;
 };
+
+__device__ __forceinline__ const BoxRec& box_rec(const BoxTable& tb, int b) { return tb.one ? tb.rec : tb.box[b]; }
+__device__ __forceinline__ const DClosures& box_cls(const BoxTable& tb, const BoxRec& R) {
+  return tb.one ? tb.rec_cls : tb.cls[R.cl];
+}
+// entry b of a prefix table
+template <class T>
+__device__ __forceinline__ T box_base(const BoxTable& tb, const T* prefix, int b) {
+  return tb.one ? T(0) : prefix[b];
+}
 
 __device__ __forceinline__ bool list_idle(const BoxTable& tb) { return tb.active && *tb.active == 0; }
 

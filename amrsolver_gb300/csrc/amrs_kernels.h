@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "amrs_boxes.cuh"
+#include "launch.cuh"
 
 namespace amrs {
 
@@ -38,7 +39,12 @@ struct FaceTable {
   const long long* fpre[3];  // prefix of face counts per direction
   const long long* gpre;     // prefix of grow(box,3) cell counts
   const long long* vpre;     // prefix of valid cell counts
+  long long ftot[3];         // faces per direction
+  FaceRec rec;               // of a list of one box (BoxTable::one)
 };
+__device__ __forceinline__ const FaceRec& face_rec(const BoxTable& tb, const FaceTable& ft, int b) {
+  return tb.one ? ft.rec : ft.fr[b];
+}
 
 cudaError_t launch_keep_faces_plain(int order, const BoxTable& tb, const FaceTable& ft, long long nfaces[3],
                                     int nsm, cudaStream_t st);

@@ -293,11 +293,6 @@ struct amrs_handle {
   double force[3] = {0.0, 0.0, 0.0};
   void* adj = nullptr;               // adjoint scratch (pair and viscous cotangents), grow-only
   size_t adj_bytes = 0;
-  BoxRec* dring = nullptr;           // per-call box records of per-box calls (device ring)
-  BoxRec* hring = nullptr;           // pinned staging of the ring
-  cudaEvent_t ring_ev[64];
-  int ring_used[64] = {0};
-  int ring_pos = 0, ring_cur = -1;
   std::mutex mu;
 };
 
@@ -505,6 +500,14 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   }
   L.ft.gpre = reinterpret_cast<const long long*>(D + o_g);
   L.ft.vpre = reinterpret_cast<const long long*>(D + o_va);
+  for (int d = 0; d < 3; ++d) L.ft.ftot[d] = L.tot_f[d];
+  L.tb.tot_p = L.tot_p;
+  L.tb.tot_v = L.tot_v;
+  L.tb.tot_m = L.mitem[n];
+  L.tb.one = n == 1;
+  L.tb.rec = L.hbox[0];
+  L.tb.rec_cls = L.cls[L.hbox[0].cl];
+  if (need_faces) L.ft.rec = L.hface[0];
   return AMRS_OK;
 }
 
@@ -578,18 +581,11 @@ bool same_box(const amrs_box& a, const amrs_box& b) {
   return true;
 }
 
-// Per-box calls reuse one single-box list; its tables are rebuilt only when
-// the box or the arrays change.
-// Per-box calls: the geometry tables (prefixes, schedule, scratch, tensor
-// maps) of the single-box list are rebuilt only when the box or its cell
-// size changes; the per-call box record (state pointers) goes through a ring
-// of device records filled from pinned staging by an async copy on the
-// call's stream.  A ring entry is reused only after the event recorded
-// behind the kernels of its previous call has completed.
-constexpr int RING = 64;
-
+// Per-box calls reuse one single-box list: its geometry tables (prefixes,
+// scratch) are rebuilt only when the box or its cell size changes, and the
+// call's arrays go into the record its launches carry.
 amrs_status one_box(amrs_handle* h, const amrs_box* bx, const double dxinv[3], const amrs_array4* slots, int nslots,
-                    cudaStream_t st, const double* dx_override = nullptr) {
+                    const double* dx_override = nullptr) {
   List*& L = h->one;
   bool same = L && L->n == 1 && same_box(L->boxes[0], *bx) && L->nslots == nslots;
   if (same) {
@@ -604,33 +600,14 @@ amrs_status one_box(amrs_handle* h, const amrs_box* bx, const double dxinv[3], c
     CK(cudaDeviceSynchronize());
     if (amrs_status s = list_build(h, *L, 1, bx, dxinv, nslots, slots, nullptr, 0, nullptr, nullptr)) return s;
   }
-  if (!h->dring) {
-    CK(cudaMalloc(&h->dring, sizeof(BoxRec) * RING));
-    CK(cudaMallocHost(&h->hring, sizeof(BoxRec) * RING));
-    for (int i = 0; i < RING; ++i) {
-      CK(cudaEventCreateWithFlags(&h->ring_ev[i], cudaEventDisableTiming));
-      h->ring_used[i] = 0;
-    }
-  }
-  const int i = h->ring_pos;
-  h->ring_pos = (i + 1) % RING;
-  if (h->ring_used[i]) CK(cudaEventSynchronize(h->ring_ev[i]));
-  BoxRec R = L->hbox[0];
+  // the record of this call's arrays travels with its launches
+  BoxRec& R = L->tb.rec;
+  R = L->hbox[0];
   for (int s = 0; s < nslots; ++s) R.slot[s] = to_darr(slots[s]);
   set_walls(R, h->wall, h->sc);
   if (dx_override)
     for (int d = 0; d < 3; ++d) R.dx[d] = dx_override[d];
-  h->hring[i] = R;
-  CK(cudaMemcpyAsync(&h->dring[i], &h->hring[i], sizeof(BoxRec), cudaMemcpyHostToDevice, st));
-  L->tb.box = &h->dring[i];
-  h->ring_cur = i;
   return AMRS_OK;
-}
-
-// Mark the current ring entry as in use by the work queued on `st`.
-void ring_release(amrs_handle* h, cudaStream_t st) {
-  const int i = h->ring_cur;
-  if (i >= 0 && cudaEventRecord(h->ring_ev[i], st) == cudaSuccess) h->ring_used[i] = 1;
 }
 
 }  // namespace
@@ -690,11 +667,6 @@ amrs_status amrs_destroy(amrs_handle* h) {
   cudaSetDevice(h->device);
   delete h->one;
   if (h->adj) cudaFree(h->adj);
-  if (h->dring) {
-    cudaFree(h->dring);
-    cudaFreeHost(h->hring);
-    for (int i = 0; i < 64; ++i) cudaEventDestroy(h->ring_ev[i]);
-  }
   if (h->derr) cudaFree(h->derr);
   if (h->dred) cudaFree(h->dred);
   delete h;
@@ -757,10 +729,9 @@ amrs_status amrs_rhs_box(amrs_handle* h, const amrs_box* bx, const double dxinv[
   CK(cudaSetDevice(h->device));
   amrs_array4 slots[3] = {state, state, dsdt};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3)) return s;
   DProg p{};
   amrs_status rs = list_stage(h, *h->one, p, 0, 1, 2, 1, st);
-  ring_release(h, st);
   return rs;
 }
 
@@ -777,9 +748,8 @@ amrs_status amrs_rk_stage_box(amrs_handle* h, const amrs_box* bx, const double d
   CK(cudaSetDevice(h->device));
   amrs_array4 slots[3] = {stage_in, s1, out};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3)) return s;
   amrs_status rs = list_stage(h, *h->one, to_dprog(prog), 0, 1, 2, 0, st);
-  ring_release(h, st);
   return rs;
 }
 
@@ -872,10 +842,9 @@ amrs_status amrs_est_timestep_box(amrs_handle* h, const amrs_box* bx, const doub
   const double dxinv[3] = {1.0 / dx[0], 1.0 / dx[1], 1.0 / dx[2]};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // cns_estdt divides dx by the wave speed: the record carries dx exactly as given
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st, dx)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, dx)) return s;
   List& L = *h->one;
   cudaError_t e = launch_estdt(L.tb, 0, L.tot_valid, cfl, h->dred, dt_device, h->nsm, st);
-  ring_release(h, st);
   if (e != cudaSuccess) return cuda_fail(e, "launch_estdt");
   return AMRS_OK;
 }
@@ -894,12 +863,11 @@ amrs_status amrs_prim_stats_box(amrs_handle* h, const amrs_box* bx, const double
   CK(cudaSetDevice(h->device));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   amrs_array4 slots[3] = {state, state, state};
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3)) return s;
   List& L = *h->one;
   cudaError_t e = cudaSuccess;
   if (!L.d_stats) e = cudaMalloc(&L.d_stats, 32 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = launch_prim_stats(L.tb, L.ft.vpre, 0, dt, dx, L.tot_valid, L.d_stats, out, h->nsm, st);
-  ring_release(h, st);
   if (e != cudaSuccess) return cuda_fail(e, "amrs_prim_stats_box");
   return AMRS_OK;
 }
@@ -1573,14 +1541,13 @@ amrs_status amrs_rhs_vjp_box(amrs_handle* h, const amrs_box* bx, const double dx
   CK(cudaSetDevice(h->device));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   amrs_array4 slots[3] = {state, state, state};
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3)) return s;
   List& L = *h->one;
   AdjScratch S;
-  if (amrs_status s = adj_prepare(h, *bx, S, st)) { ring_release(h, st); return s; }
+  if (amrs_status s = adj_prepare(h, *bx, S, st)) return s;
   S.ah.vbar = to_darr(vbar);
   S.ah.ubar = to_darr(ubar);
   cudaError_t e = rhs_vjp_launch(h, L, *bx, S, param_bar, st);
-  ring_release(h, st);
   if (e != cudaSuccess) return cuda_fail(e, "amrs_rhs_vjp_box");
   return AMRS_OK;
 }
@@ -1638,9 +1605,9 @@ amrs_status amrs_rk_stage_vjp_box(amrs_handle* h, const amrs_box* bx, const doub
   std::lock_guard<std::mutex> lk(h->mu);
   CK(cudaSetDevice(h->device));
   amrs_array4 slots[3] = {stage_in, stage_in, stage_in};
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3)) return s;
   AdjScratch S;
-  if (amrs_status s = adj_prepare(h, *bx, S, st)) { ring_release(h, st); return s; }
+  if (amrs_status s = adj_prepare(h, *bx, S, st)) return s;
   const BoxRec R = h->one->hbox[0];
   // 1. reverse of the BLAS-1 program: cotangents of S1, of the stage input
   //    (register S2) and of dSdt
@@ -1669,7 +1636,6 @@ amrs_status amrs_rk_stage_vjp_box(amrs_handle* h, const amrs_box* bx, const doub
     ident.nops = 0;
     e = launch_adj_prog(R, to_dprog(&ident), S.ubar_tmp, S.vbar_tmp, to_darr(inbar), S.vbar_tmp, 1, h->nsm, st);
   }
-  ring_release(h, st);
   if (e != cudaSuccess) return cuda_fail(e, "amrs_rk_stage_vjp_box");
   return AMRS_OK;
 }
@@ -1687,9 +1653,9 @@ amrs_status amrs_rk_stage_vjp_box_ghosted(amrs_handle* h, const amrs_box* bx, co
   std::lock_guard<std::mutex> lk(h->mu);
   CK(cudaSetDevice(h->device));
   amrs_array4 slots[3] = {stage_in, stage_in, stage_in};
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3)) return s;
   AdjScratch S;
-  if (amrs_status s = adj_prepare(h, *bx, S, st)) { ring_release(h, st); return s; }
+  if (amrs_status s = adj_prepare(h, *bx, S, st)) return s;
   const BoxRec R = h->one->hbox[0];
   cudaError_t e = cudaMemsetAsync(S.ubar_tmp.p, 0, (size_t)S.ubar_tmp.ns * NCONS * sizeof(double), st);
   // 1. reverse of the BLAS-1 program: S1 cotangent added to s1bar, the stage
@@ -1709,7 +1675,6 @@ amrs_status amrs_rk_stage_vjp_box_ghosted(amrs_handle* h, const amrs_box* bx, co
     ident.nops = 0;
     e = launch_adj_prog(R, to_dprog(&ident), S.ubar_tmp, S.vbar_tmp, to_darr(ubar), S.vbar_tmp, 1, h->nsm, st);
   }
-  ring_release(h, st);
   if (e != cudaSuccess) return cuda_fail(e, "amrs_rk_stage_vjp_box_ghosted");
   return AMRS_OK;
 }
@@ -1877,14 +1842,14 @@ amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const dou
   CK(cudaSetDevice(h->device));
   amrs_array4 slots[3] = {stage_in, s1, out};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (amrs_status s = one_box(h, bx, dxinv, slots, 3, st)) return s;
+  if (amrs_status s = one_box(h, bx, dxinv, slots, 3)) return s;
   List& L = *h->one;
   const amrs_scheme& sc = L.sc;
   // the face-array path is profiled for WENO5 (point fluxes timed with the
   // primitives), MUSCL-Riemann (slopes timed with the faces), WENO5-Riemann
   // and the unshared KEEP baseline
   const bool plain_ok = sc.rhs_euler && !sc.art_diss && sc.flux_euler >= 0 && sc.flux_euler <= 3;
-  if (!L.fused && !plain_ok) { ring_release(h, st); return AMRS_ERR_SCHEME; }
+  if (!L.fused && !plain_ok) return AMRS_ERR_SCHEME;
   const DProg p = to_dprog(prog);
   cudaEvent_t ev[5];
   for (int i = 0; i < 5; ++i) CK(cudaEventCreate(&ev[i]));
@@ -1929,7 +1894,6 @@ amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const dou
     if (e != cudaSuccess) rs = cuda_fail(e, "amrs_profile_stage_box");
   }
   for (int i = 0; i < 5; ++i) cudaEventDestroy(ev[i]);
-  ring_release(h, st);
   if (rs) return rs;
   for (int i = 0; i < 4; ++i) ms[i] = acc[i] / reps;
   return AMRS_OK;

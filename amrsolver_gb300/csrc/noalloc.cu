@@ -225,6 +225,12 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   tb.nshare = G;
   tb.cls = reinterpret_cast<const DClosures*>(tab + o_cl);
   tb.n = 1;
+  tb.tot_p = pcell[1];
+  tb.tot_v = vcell[1];
+  tb.tot_m = mitem[1];
+  tb.one = 1;
+  tb.rec = R;
+  tb.rec_cls = cl;
   tb.gq = gq;
   tb.range = reinterpret_cast<int*>(tab + o_rng);
   DProg prog{};

@@ -30,15 +30,16 @@
 namespace amrs {
 
 // ------------------------------------------------------------- prims ----
-__global__ void __launch_bounds__(256) prims_kernel(BoxTable tb, int s_in) {
+__global__ void __launch_bounds__(256) prims_kernel(const __grid_constant__ BoxTable tb, int s_in) {
+  dep_begin();
   if (list_idle(tb)) return;
-  const long long total = tb.pcell[tb.n];
+  const long long total = tb.tot_p;
   const int g = tb.gq;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
        c += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(tb.pcell, tb.n, c);
-    const BoxRec& R = tb.box[b];
-    const int l = (int)(c - tb.pcell[b]);
+    const BoxRec& R = box_rec(tb, b);
+    const int l = (int)(c - box_base(tb, tb.pcell, b));
     const int nx = R.hi[0] - R.lo[0] + 1 + 2 * g, ny = R.hi[1] - R.lo[1] + 1 + 2 * g;
     const int i = l % nx + R.lo[0] - g;
     const int t = l / nx;
@@ -50,7 +51,7 @@ __global__ void __launch_bounds__(256) prims_kernel(BoxTable tb, int s_in) {
 #pragma unroll
     for (int n = 0; n < 5; ++n) u[n] = U.p[o + n * U.ns];
     double q[NQ];
-    cons2prim(u, q, tb.cls[R.cl]);
+    cons2prim(u, q, box_cls(tb, R));
     if (tb.range && !keep_range(q)) *tb.range = 1;
     const long long oq = R.q.off(i, j, k);
 #pragma unroll
@@ -59,14 +60,15 @@ __global__ void __launch_bounds__(256) prims_kernel(BoxTable tb, int s_in) {
 }
 
 // ------------------------------------------------- viscous cell fluxes ----
-__global__ void __launch_bounds__(256) visc_cell_kernel(BoxTable tb) {
+__global__ void __launch_bounds__(256) visc_cell_kernel(const __grid_constant__ BoxTable tb) {
+  dep_begin();
   if (list_idle(tb)) return;
-  const long long total = tb.vcell[tb.n];
+  const long long total = tb.tot_v;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
        c += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(tb.vcell, tb.n, c);
-    const BoxRec& R = tb.box[b];
-    const int l = (int)(c - tb.vcell[b]);
+    const BoxRec& R = box_rec(tb, b);
+    const int l = (int)(c - box_base(tb, tb.vcell, b));
     const int nx = R.hi[0] - R.lo[0] + 3, ny = R.hi[1] - R.lo[1] + 3;
     const int i = l % nx + R.lo[0] - 1;
     const int t = l / nx;
@@ -97,9 +99,9 @@ __global__ void __launch_bounds__(256) visc_cell_kernel(BoxTable tb) {
         q1[n] = Q.p[o + s1 + n * sn];
         q2[n] = Q.p[o + 2 * s1 + n * sn];
       }
-      viscous_wall_cell(loc, qc, qxm, qxp, q1, q2, qzm, qzp, R.dxinv, tb.cls[R.cl], f);
+      viscous_wall_cell(loc, qc, qxm, qxp, q1, q2, qzm, qzp, R.dxinv, box_cls(tb, R), f);
     } else {
-      viscous_cell(qc, qxm, qxp, qym, qyp, qzm, qzp, R.dxinv, tb.cls[R.cl], f);
+      viscous_cell(qc, qxm, qxp, qym, qyp, qzm, qzp, R.dxinv, box_cls(tb, R), f);
     }
     const long long ov = R.vf.off(i, j, k);
 #pragma unroll
@@ -137,11 +139,11 @@ __device__ __forceinline__ void keep_x_body(const BoxTable& tb, int s_in, int s_
   double coef[3];
   keep_coeffs(ORDER, coef);
   const int b = find_box_i(tb.fwork, tb.n, blockIdx.x);
-  const BoxRec& R = tb.box[b];
+  const BoxRec& R = box_rec(tb, b);
   const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1, nz = R.hi[2] - R.lo[2] + 1;
   const int row_slots = nx + H;
   // (a box's grown cells fit 31 bits, and with them the slots)
-  const int g = (blockIdx.x - tb.fwork[b]) * (nth - H) + tid;
+  const int g = (blockIdx.x - box_base(tb, tb.fwork, b)) * (nth - H) + tid;
   const bool in = g < row_slots * ny * nz;
   const int row = in ? g / row_slots : 0;
   const int s = in ? g - row * row_slots : 0;
@@ -195,7 +197,7 @@ __device__ __forceinline__ void keep_x_body(const BoxTable& tb, int s_in, int s_
     const DArr& Uo = R.slot[s_out];
     const double* D = R.div.p + R.div.off(i, j, k);
     const long long dn = R.div.ns, oin = Uin.off(i, j, k), o1 = U1.off(i, j, k), oo = Uo.off(i, j, k);
-    const bool src = SRC && tb.cls[R.cl].source != 0;  // SRC: a list with a source term
+    const bool src = SRC && box_cls(tb, R).source != 0;  // SRC: a list with a source term
     // all loads of a kind before the products: their range tests are branches
     // that loads do not cross
     double ds[5], y[5], z[5];
@@ -207,7 +209,7 @@ __device__ __forceinline__ void keep_x_body(const BoxTable& tb, int s_in, int s_
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
       ds[n] = kmul<AMRS_DIV_IMUL & 1>(R.dxinv[0], F[n] - fs[n * nth + tid + 1]) + y[n] + z[n];
-      if (src) ds[n] = add_source(tb.cls[R.cl], Uin.p, oin, Uin.ns, n, ds[n]);
+      if (src) ds[n] = add_source(box_cls(tb, R), Uin.p, oin, Uin.ns, n, ds[n]);
     }
     if (!rhs_only) {
       double s1[5], s2[5];
@@ -363,14 +365,14 @@ __device__ __forceinline__ void keep_march_warp(const BoxTable& tb) {
   if (w >= tb.nshare) return;
   double coef[3];
   keep_coeffs(ORDER, coef);
-  const long long N = tb.mitem[tb.n];
+  const long long N = tb.tot_m;
   const long long at = w * N / tb.nshare;
   int left = (int)((w + 1) * N / tb.nshare - at);
   int b = find_box_ll(tb.mitem, tb.n, at);
-  int r = (int)(at - tb.mitem[b]);
+  int r = (int)(at - box_base(tb, tb.mitem, b));
 #pragma unroll 1
   while (left > 0) {
-    const BoxRec& R = tb.box[b];
+    const BoxRec& R = box_rec(tb, b);
     const int ny = march_cells(R, 1), nz = march_cells(R, 2);
     const int ytot = march_blocks(R, 1) * ny, ztot = march_blocks(R, 2) * nz;
     if (r == ytot + ztot) { ++b; r = 0; continue; }
@@ -386,7 +388,8 @@ __device__ __forceinline__ void keep_march_warp(const BoxTable& tb) {
 }
 
 template <int ORDER, bool VISC>
-__global__ void __launch_bounds__(F_THREADS, march_ctas<ORDER>()) keep_march_kernel(BoxTable tb) {
+__global__ void __launch_bounds__(F_THREADS, march_ctas<ORDER>()) keep_march_kernel(const __grid_constant__ BoxTable tb) {
+  dep_begin();
   if (list_idle(tb)) return;
   if (fast_range(tb)) keep_march_warp<ORDER, VISC, true>(tb);
   else keep_march_warp<ORDER, VISC, false>(tb);
@@ -394,7 +397,8 @@ __global__ void __launch_bounds__(F_THREADS, march_ctas<ORDER>()) keep_march_ker
 
 template <int ORDER, bool VISC, bool SRC>
 __global__ void __launch_bounds__(F_THREADS, 4)
-keep_x_kernel(BoxTable tb, int s_in, int s_s1, int s_out, DProg prog_in, int rhs_only) {
+keep_x_kernel(const __grid_constant__ BoxTable tb, int s_in, int s_s1, int s_out, DProg prog_in, int rhs_only) {
+  dep_begin();
   if (list_idle(tb)) return;  // uniform over the CTA: before any barrier
   const DProg prog = resolve_prog(prog_in);
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -408,8 +412,8 @@ keep_x_kernel(BoxTable tb, int s_in, int s_s1, int s_out, DProg prog_in, int rhs
 template <int ORDER, bool VISC, bool SRC>
 static cudaError_t launch_face_t(const BoxTable& tb, int s_in, int s_s1, int s_out, const DProg& prog, int rhs_only,
                                  const KeepGrid& g, cudaStream_t st) {
-  keep_march_kernel<ORDER, VISC><<<g.march_ctas, g.march_threads, 0, st>>>(tb);
-  keep_x_kernel<ORDER, VISC, SRC><<<g.x_ctas, g.x_threads, (ORDER / 2) * 5 * 8 * g.x_threads, st>>>(
+  launch_dep(keep_march_kernel<ORDER, VISC>, g.march_ctas, g.march_threads, 0, st, tb);
+  launch_dep(keep_x_kernel<ORDER, VISC, SRC>, g.x_ctas, g.x_threads, (ORDER / 2) * 5 * 8 * g.x_threads, st, 
       tb, s_in, s_s1, s_out, prog, rhs_only);
   return cudaGetLastError();
 }
@@ -419,7 +423,7 @@ cudaError_t launch_prims(const BoxTable& tb, int s_in, long long ncells, int nsm
   long long blocks = (ncells + 255) / 256;
   const long long cap = (long long)nsm * 8;
   if (blocks > cap) blocks = cap;
-  prims_kernel<<<(int)blocks, 256, 0, st>>>(tb, s_in);
+  launch_dep(prims_kernel, (int)blocks, 256, 0, st, tb, s_in);
   return cudaGetLastError();
 }
 
@@ -428,7 +432,7 @@ cudaError_t launch_visc(const BoxTable& tb, long long ncells, int nsm, cudaStrea
   long long blocks = (ncells + 255) / 256;
   const long long cap = (long long)nsm * 8;
   if (blocks > cap) blocks = cap;
-  visc_cell_kernel<<<(int)blocks, 256, 0, st>>>(tb);
+  launch_dep(visc_cell_kernel, (int)blocks, 256, 0, st, tb);
   return cudaGetLastError();
 }
 

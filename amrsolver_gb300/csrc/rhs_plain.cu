@@ -28,12 +28,12 @@ struct FaceIdx {
 __device__ __forceinline__ bool decode_face(const BoxTable& tb, const FaceTable& ft, long long g, FaceIdx& f) {
   long long base = 0;
   for (int d = 0; d < 3; ++d) {
-    const long long tot = ft.fpre[d][tb.n];
+    const long long tot = ft.ftot[d];
     if (g < base + tot) {
       const long long l = g - base;
       const int b = find_box_ll(ft.fpre[d], tb.n, l);
-      const BoxRec& R = tb.box[b];
-      const int loc = (int)(l - ft.fpre[d][b]);
+      const BoxRec& R = box_rec(tb, b);
+      const int loc = (int)(l - box_base(tb, ft.fpre[d], b));
       const int nx = R.hi[0] - R.lo[0] + 1 + (d == 0), ny = R.hi[1] - R.lo[1] + 1 + (d == 1);
       f.b = b;
       f.d = d;
@@ -66,7 +66,8 @@ static int grid_for(long long n, int nsm) {
 // src/rhs/CentralKEEP.h:40-145, one face per thread, pairs summed in the
 // reference's (l, m) order without sharing between faces.
 template <int ORDER>
-__global__ void __launch_bounds__(256) keep_faces_plain_kernel(BoxTable tb, FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256) keep_faces_plain_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   constexpr int H = ORDER / 2;
   double coef[3];
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(256) keep_faces_plain_kernel(BoxTable tb, Face
        g += (long long)gridDim.x * blockDim.x) {
     FaceIdx f;
     if (!decode_face(tb, ft, g, f)) continue;
-    const BoxRec& R = tb.box[f.b];
+    const BoxRec& R = box_rec(tb, f.b);
     const DArr Q = R.q;
     const int di = f.d == 0, dj = f.d == 1, dk = f.d == 2;
     // y faces next to a code-6 wall: second-order KEEP, coefficient 1
@@ -102,7 +103,7 @@ __global__ void __launch_bounds__(256) keep_faces_plain_kernel(BoxTable tb, Face
 #pragma unroll
         for (int n = 0; n < 5; ++n) F[n] = F[n] + T[n];
       }
-    const DArr Fd = ft.fr[f.b].f[f.d];
+    const DArr Fd = face_rec(tb, ft, f.b).f[f.d];
     const long long of = Fd.off(f.i, f.j, f.k);
 #pragma unroll
     for (int n = 0; n < 5; ++n) Fd.p[of + n * Fd.ns] = F[n];
@@ -123,18 +124,19 @@ __device__ __forceinline__ double visc_average(const BoxRec& R, const FaceIdx& f
 #ifndef AMRS_WPF_IMUL
 #define AMRS_WPF_IMUL 0x0B
 #endif
-__global__ void __launch_bounds__(256) weno_flux_lambda_kernel(BoxTable tb, FaceTable ft, int s_in, long long total) {
+__global__ void __launch_bounds__(256) weno_flux_lambda_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(ft.gpre, tb.n, g);
-    const BoxRec& R = tb.box[b];
-    const FaceRec& FR = ft.fr[b];
+    const BoxRec& R = box_rec(tb, b);
+    const FaceRec& FR = face_rec(tb, ft, b);
     int i, j, k;
-    decode_cell(R, (int)(g - ft.gpre[b]), NGHOST, i, j, k);
+    decode_cell(R, (int)(g - box_base(tb, ft.gpre, b)), NGHOST, i, j, k);
     const DArr U = R.slot[s_in];
     const long long o = U.off(i, j, k);
-    const double gam = tb.cls[R.cl].gamma;
+    const double gam = box_cls(tb, R).gamma;
     const double rhoinv = ddiv_rn(1.0, U.p[o]);
     const double momx = U.p[o + U.ns], momy = U.p[o + 2 * U.ns], momz = U.p[o + 3 * U.ns];
     const double rhoet = U.p[o + 4 * U.ns];
@@ -363,15 +365,16 @@ static __device__ __noinline__ double weno_llf_plain(const double* p0, long long
 // face) and after: 256^3 54.0 -> 29.4 ms, 64^3 874 -> 464 us, the tube 78 -> 41 us;
 // with 2 CTAs per SM 30.1 ms at 256^3, with 4 (64 registers) 32.6 ms.
 template <bool REF_ORDER, bool VISC>
-__global__ void __launch_bounds__(256, 3) weno_face_kernel(BoxTable tb, FaceTable ft, int s_in, long long total) {
+__global__ void __launch_bounds__(256, 3) weno_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   const int n = blockIdx.y;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     FaceIdx f;
     if (!decode_face(tb, ft, g, f)) continue;
-    const BoxRec& R = tb.box[f.b];
-    const FaceRec& FR = ft.fr[f.b];
+    const BoxRec& R = box_rec(tb, f.b);
+    const FaceRec& FR = face_rec(tb, ft, f.b);
     const DArr U = R.slot[s_in];
     const DArr PF = FR.pf[f.d];
     const DArr L = FR.lam;
@@ -588,9 +591,10 @@ __device__ __forceinline__ void slope_terms(const SlopeQ& q, double gR, double t
 // products per cell and direction; the limiters' comparisons and scalings by
 // two were 40 further FP64 instructions).  48^3, inviscid: 64 -> 28 us; four CTAs
 // per SM 2.5% faster than two over the step.
-__global__ void __launch_bounds__(256, 4) slope_kernel(BoxTable tb, FaceTable ft, const long long* spre0,
+__global__ void __launch_bounds__(256, 4) slope_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, const long long* spre0,
                                                     const long long* spre1, const long long* spre2,
                                                     long long tot0, long long tot1, long long tot2) {
+  dep_begin();
   if (list_idle(tb)) return;
   const long long total = tot0 + tot1 + tot2;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -602,15 +606,15 @@ __global__ void __launch_bounds__(256, 4) slope_kernel(BoxTable tb, FaceTable ft
     else if (g < tot0 + tot1) { d = 1; l = g - tot0; pre = spre1; }
     else { d = 2; l = g - tot0 - tot1; pre = spre2; }
     const int b = find_box_ll(pre, tb.n, l);
-    const BoxRec& R = tb.box[b];
-    const int loc = (int)(l - pre[b]);
+    const BoxRec& R = box_rec(tb, b);
+    const int loc = (int)(l - box_base(tb, pre, b));
     const int nx = R.hi[0] - R.lo[0] + 1 + 2 * (d == 0), ny = R.hi[1] - R.lo[1] + 1 + 2 * (d == 1);
     const int i = loc % nx + R.lo[0] - (d == 0);
     const int t = loc / nx;
     const int j = t % ny + R.lo[1] - (d == 1);
     const int k = t / ny + R.lo[2] - (d == 2);
     const DArr q = R.q;
-    const DClosures& cl = tb.cls[R.cl];
+    const DClosures& cl = box_cls(tb, R);
     const long long s = (d == 0) ? 1 : (d == 1 ? q.js : q.ks);
     const double* Q = q.p + q.off(i, j, k);
     const int QN = QU + d, QT1 = (d == 0) ? QV : QU, QT2 = (d == 2) ? QV : QW;
@@ -629,7 +633,7 @@ __global__ void __launch_bounds__(256, 4) slope_kernel(BoxTable tb, FaceTable ft
     v.Tup = up ? Q[2 * s + QT * q.ns] : v.T;
     double o[NSLOPE];
     slope_terms(v, cl.gamma * cl.Rspec, d == 0 ? 2.e-40 : 1.e-40, up, o);
-    const DArr S = ft.fr[b].slope[d];
+    const DArr S = face_rec(tb, ft, b).slope[d];
     double* so = S.p + S.off(i, j, k);
 #pragma unroll
     for (int n = 0; n < SL_AL; ++n) so[n * S.ns] = o[n];
@@ -864,17 +868,18 @@ __device__ __forceinline__ void riemann_prob(const double gamma, const double sm
 // (2.94 against 3.10 ms per step at 96^3).  48^3, with the hardware's roots and
 // products and checked integer quotients before: 194 -> 86 us.
 template <bool VISC>
-__global__ void __launch_bounds__(256, 2) riemann_face_kernel(BoxTable tb, FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256, 2) riemann_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     FaceIdx f;
     if (!decode_face(tb, ft, g, f)) continue;
-    const BoxRec& R = tb.box[f.b];
+    const BoxRec& R = box_rec(tb, f.b);
     const int d = f.d;
     const DArr q = R.q;
-    const DArr S = ft.fr[f.b].slope[d];
-    const DClosures& cl = tb.cls[R.cl];
+    const DArr S = face_rec(tb, ft, f.b).slope[d];
+    const DClosures& cl = box_cls(tb, R);
     const int QN = QU + d, QT1 = (d == 0) ? QV : QU, QT2 = (d == 2) ? QV : QW;
     const int UN = UMX + d, UT1 = (d == 0) ? UMY : UMX, UT2 = (d == 2) ? UMY : UMZ;
     const int im = f.i - (d == 0), jm = f.j - (d == 1), km = f.k - (d == 2);
@@ -899,7 +904,7 @@ __global__ void __launch_bounds__(256, 2) riemann_face_kernel(BoxTable tb, FaceT
                            fma(-0.5, D(os, SL_T2), Q(oq, QT2))};
     double F[5];
     riemann_prob(gam, 1.0e-40, in, F);
-    const DArr Fd = ft.fr[f.b].f[d];
+    const DArr Fd = face_rec(tb, ft, f.b).f[d];
     const long long of = Fd.off(f.i, f.j, f.k);
     const int comp_of[5] = {URHO, UN, UT1, UT2, UET};
 #pragma unroll
@@ -916,16 +921,17 @@ __global__ void __launch_bounds__(256, 2) riemann_face_kernel(BoxTable tb, FaceT
 // as the MUSCL states are (src/rhs/Riemann.h:260-272), and riemann_prob
 // gives the flux.  One thread per face.
 template <bool VISC>
-__global__ void __launch_bounds__(256) weno_riemann_face_kernel(BoxTable tb, FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256) weno_riemann_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     FaceIdx f;
     if (!decode_face(tb, ft, g, f)) continue;
-    const BoxRec& R = tb.box[f.b];
+    const BoxRec& R = box_rec(tb, f.b);
     const int d = f.d;
     const DArr q = R.q;
-    const DClosures& cl = tb.cls[R.cl];
+    const DClosures& cl = box_cls(tb, R);
     const int QN = QU + d, QT1 = (d == 0) ? QV : QU, QT2 = (d == 2) ? QV : QW;
     const int UN = UMX + d, UT1 = (d == 0) ? UMY : UMX, UT2 = (d == 2) ? UMY : UMZ;
     const long long sq = (d == 0) ? 1 : (d == 1 ? q.js : q.ks);
@@ -945,7 +951,7 @@ __global__ void __launch_bounds__(256) weno_riemann_face_kernel(BoxTable tb, Fac
                            rmax(rgt[0], 1.0e-40), rgt[1], rmax(rgt[2], 1.0e-40), rgt[3], rgt[4]};
     double F[5];
     riemann_prob(cl.gamma, 1.0e-40, in, F);
-    const DArr Fd = ft.fr[f.b].f[d];
+    const DArr Fd = face_rec(tb, ft, f.b).f[d];
     const long long of = Fd.off(f.i, f.j, f.k);
     const int comp_of[5] = {URHO, UN, UT1, UT2, UET};
 #pragma unroll
@@ -964,25 +970,26 @@ __device__ __forceinline__ double discon_sensor(double pp, double pl, double pr)
 
 // Sensor and spectral radius on the valid box (src/rhs/CNS_hydro_K.h:46-75);
 // the arrays are zeroed beforehand, as the reference zeroes its MultiFabs.
-__global__ void __launch_bounds__(256) jst_sensor_kernel(BoxTable tb, FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256) jst_sensor_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(ft.vpre, tb.n, g);
-    const BoxRec& R = tb.box[b];
+    const BoxRec& R = box_rec(tb, b);
     int i, j, k;
-    decode_cell(R, (int)(g - ft.vpre[b]), 0, i, j, k);
+    decode_cell(R, (int)(g - box_base(tb, ft.vpre, b)), 0, i, j, k);
     const DArr q = R.q;
     const long long o = q.off(i, j, k);
     auto P = [&](long long off) { return q.p[off + QPRES * q.ns]; };
     const double pp = P(o);
-    const FaceRec& FR = ft.fr[b];
+    const FaceRec& FR = face_rec(tb, ft, b);
     const long long os = FR.sen.off(i, j, k);
     FR.sen.p[os] = discon_sensor(pp, P(o - 1), P(o + 1));
     FR.sen.p[os + FR.sen.ns] = discon_sensor(pp, P(o - q.js), P(o + q.js));
     FR.sen.p[os + 2 * FR.sen.ns] = discon_sensor(pp, P(o - q.ks), P(o + q.ks));
     const double ux = q.p[o + QU * q.ns], uy = q.p[o + QV * q.ns], uz = q.p[o + QW * q.ns];
-    const double cs = dsqrt_rn(ddiv_rn(tb.cls[R.cl].gamma * pp, q.p[o + QRHO * q.ns]));
+    const double cs = dsqrt_rn(ddiv_rn(box_cls(tb, R).gamma * pp, q.p[o + QRHO * q.ns]));
     FR.lam.p[os] = fabs(ux) + cs;
     FR.lam.p[os + FR.lam.ns] = fabs(uy) + cs;
     FR.lam.p[os + 2 * FR.lam.ns] = fabs(uz) + cs;
@@ -992,15 +999,16 @@ __global__ void __launch_bounds__(256) jst_sensor_kernel(BoxTable tb, FaceTable 
 // JST dissipation subtracted from face fluxes (src/rhs/CNS_hydro_K.h:78-104);
 // y and z read component 0 of sensor and lambda, and the z fourth
 // difference uses k-1 three times, as in the reference.
-__global__ void __launch_bounds__(256) jst_face_kernel(BoxTable tb, FaceTable ft, int s_in, long long total) {
+__global__ void __launch_bounds__(256) jst_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     FaceIdx f;
     if (!decode_face(tb, ft, g, f)) continue;
-    const BoxRec& R = tb.box[f.b];
-    const FaceRec& FR = ft.fr[f.b];
-    const DClosures& cl = tb.cls[R.cl];
+    const BoxRec& R = box_rec(tb, f.b);
+    const FaceRec& FR = face_rec(tb, ft, f.b);
+    const DClosures& cl = box_cls(tb, R);
     const DArr U = R.slot[s_in];
     const long long s = (f.d == 0) ? 1 : (f.d == 1 ? U.js : U.ks);
     const long long sl = (f.d == 0) ? 1 : (f.d == 1 ? FR.sen.js : FR.sen.ks);
@@ -1022,17 +1030,18 @@ __global__ void __launch_bounds__(256) jst_face_kernel(BoxTable tb, FaceTable ft
 
 // ---------------------------------------------- viscous face average ----
 // src/rhs/CNS_hydro_K.h:254-261 (mass component adds zero and is skipped).
-__global__ void __launch_bounds__(256) visc_face_add_kernel(BoxTable tb, FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256) visc_face_add_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     FaceIdx f;
     if (!decode_face(tb, ft, g, f)) continue;
-    const BoxRec& R = tb.box[f.b];
+    const BoxRec& R = box_rec(tb, f.b);
     const DArr V = R.vf;
     const long long s = (f.d == 0) ? 1 : (f.d == 1 ? V.js : V.ks);
     const long long ov = V.off(f.i, f.j, f.k);
-    const DArr Fd = ft.fr[f.b].f[f.d];
+    const DArr Fd = face_rec(tb, ft, f.b).f[f.d];
     const long long of = Fd.off(f.i, f.j, f.k);
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -1049,17 +1058,18 @@ __global__ void __launch_bounds__(256) visc_face_add_kernel(BoxTable tb, FaceTab
 // loads' latency and the FP64 pipe (25 to 35 instructions per cell with every
 // product on the integer pipe, 60 to 75 before).  256^3: 2.07 -> 1.46 ms per stage
 // (products moved, loads in program order: 1.87; one thread per cell: 2.97).
-__global__ void __launch_bounds__(256, 5) div_stage_kernel(BoxTable tb, FaceTable ft, int s_in, int s_s1, int s_out,
+__global__ void __launch_bounds__(256, 5) div_stage_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, int s_s1, int s_out,
                                                            DProg prog_in, int rhs_only, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   const DProg prog = resolve_prog(prog_in);
   const int n = blockIdx.y;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(ft.vpre, tb.n, g);
-    const BoxRec& R = tb.box[b];
-    const FaceRec& FR = ft.fr[b];
-    const int loc = (int)(g - ft.vpre[b]);
+    const BoxRec& R = box_rec(tb, b);
+    const FaceRec& FR = face_rec(tb, ft, b);
+    const int loc = (int)(g - box_base(tb, ft.vpre, b));
     const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
     const int t = loc / nx, i = loc - t * nx, k = t / ny, j = t - k * ny;  // in the box
     // face arrays: rows of nx + 1, nx, nx (nodal in their direction)
@@ -1075,7 +1085,7 @@ __global__ void __launch_bounds__(256, 5) div_stage_kernel(BoxTable tb, FaceTabl
       s2 = Uin(gi, gj, gk, n);
     }
     double ds = dmul_rn(R.dxinv[0], x0 - x1) + dmul_rn(R.dxinv[1], y0 - y1) + dmul_rn(R.dxinv[2], z0 - z1);
-    const DClosures& cl = tb.cls[R.cl];
+    const DClosures& cl = box_cls(tb, R);
     if (cl.source) ds = add_source(cl, Uin.p, Uin.off(gi, gj, gk), Uin.ns, n, ds);
     Uo(gi, gj, gk, n) = rhs_only ? ds : apply_prog(prog, s1, s2, ds);
   }
@@ -1086,15 +1096,15 @@ cudaError_t launch_keep_faces_plain(int order, const BoxTable& tb, const FaceTab
                                     cudaStream_t st) {
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
   const int grid = grid_for(tot, nsm);
-  if (order == 2) keep_faces_plain_kernel<2><<<grid, 256, 0, st>>>(tb, ft, tot);
-  else if (order == 4) keep_faces_plain_kernel<4><<<grid, 256, 0, st>>>(tb, ft, tot);
-  else keep_faces_plain_kernel<6><<<grid, 256, 0, st>>>(tb, ft, tot);
+  if (order == 2) launch_dep(keep_faces_plain_kernel<2>, grid, 256, 0, st, tb, ft, tot);
+  else if (order == 4) launch_dep(keep_faces_plain_kernel<4>, grid, 256, 0, st, tb, ft, tot);
+  else launch_dep(keep_faces_plain_kernel<6>, grid, 256, 0, st, tb, ft, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_weno_point(const BoxTable& tb, const FaceTable& ft, int s_in, long long ngcells, int nsm,
                               cudaStream_t st) {
-  weno_flux_lambda_kernel<<<grid_for(ngcells, nsm), 256, 0, st>>>(tb, ft, s_in, ngcells);
+  launch_dep(weno_flux_lambda_kernel, grid_for(ngcells, nsm), 256, 0, st, tb, ft, s_in, ngcells);
   return cudaGetLastError();
 }
 
@@ -1102,23 +1112,23 @@ cudaError_t launch_weno_faces(const BoxTable& tb, const FaceTable& ft, int s_in,
                               bool visc, int nsm, cudaStream_t st) {
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
   const dim3 grid(grid_for(tot, nsm), NCONS);
-  if (ref_order && visc) weno_face_kernel<true, true><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
-  else if (ref_order) weno_face_kernel<true, false><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
-  else if (visc) weno_face_kernel<false, true><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
-  else weno_face_kernel<false, false><<<grid, 256, 0, st>>>(tb, ft, s_in, tot);
+  if (ref_order && visc) launch_dep(weno_face_kernel<true, true>, grid, 256, 0, st, tb, ft, s_in, tot);
+  else if (ref_order) launch_dep(weno_face_kernel<true, false>, grid, 256, 0, st, tb, ft, s_in, tot);
+  else if (visc) launch_dep(weno_face_kernel<false, true>, grid, 256, 0, st, tb, ft, s_in, tot);
+  else launch_dep(weno_face_kernel<false, false>, grid, 256, 0, st, tb, ft, s_in, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_weno(const BoxTable& tb, const FaceTable& ft, int s_in, long long ngcells, long long nfaces[3],
                         bool ref_order, bool visc, int nsm, cudaStream_t st) {
-  weno_flux_lambda_kernel<<<grid_for(ngcells, nsm), 256, 0, st>>>(tb, ft, s_in, ngcells);
+  launch_dep(weno_flux_lambda_kernel, grid_for(ngcells, nsm), 256, 0, st, tb, ft, s_in, ngcells);
   return launch_weno_faces(tb, ft, s_in, nfaces, ref_order, visc, nsm, st);
 }
 
 cudaError_t launch_slopes(const BoxTable& tb, const FaceTable& ft, const long long* spre_d[3], long long nslope[3],
                           int nsm, cudaStream_t st) {
   const long long ts = nslope[0] + nslope[1] + nslope[2];
-  slope_kernel<<<grid_for(ts, nsm), 256, 0, st>>>(tb, ft, spre_d[0], spre_d[1], spre_d[2], nslope[0], nslope[1],
+  launch_dep(slope_kernel, grid_for(ts, nsm), 256, 0, st, tb, ft, spre_d[0], spre_d[1], spre_d[2], nslope[0], nslope[1],
                                                   nslope[2]);
   return cudaGetLastError();
 }
@@ -1126,46 +1136,46 @@ cudaError_t launch_slopes(const BoxTable& tb, const FaceTable& ft, const long lo
 cudaError_t launch_riemann(const BoxTable& tb, const FaceTable& ft, const long long* spre_d[3], long long nslope[3],
                            long long nfaces[3], bool visc, int nsm, cudaStream_t st) {
   const long long ts = nslope[0] + nslope[1] + nslope[2];
-  slope_kernel<<<grid_for(ts, nsm), 256, 0, st>>>(tb, ft, spre_d[0], spre_d[1], spre_d[2], nslope[0], nslope[1],
+  launch_dep(slope_kernel, grid_for(ts, nsm), 256, 0, st, tb, ft, spre_d[0], spre_d[1], spre_d[2], nslope[0], nslope[1],
                                                   nslope[2]);
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
-  if (visc) riemann_face_kernel<true><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
-  else riemann_face_kernel<false><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
+  if (visc) launch_dep(riemann_face_kernel<true>, grid_for(tot, nsm), 256, 0, st, tb, ft, tot);
+  else launch_dep(riemann_face_kernel<false>, grid_for(tot, nsm), 256, 0, st, tb, ft, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_weno_riemann(const BoxTable& tb, const FaceTable& ft, long long nfaces[3], bool visc, int nsm,
                                 cudaStream_t st) {
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
-  if (visc) weno_riemann_face_kernel<true><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
-  else weno_riemann_face_kernel<false><<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
+  if (visc) launch_dep(weno_riemann_face_kernel<true>, grid_for(tot, nsm), 256, 0, st, tb, ft, tot);
+  else launch_dep(weno_riemann_face_kernel<false>, grid_for(tot, nsm), 256, 0, st, tb, ft, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_jst_sensor(const BoxTable& tb, const FaceTable& ft, long long nvalid, int nsm, cudaStream_t st) {
-  jst_sensor_kernel<<<grid_for(nvalid, nsm), 256, 0, st>>>(tb, ft, nvalid);
+  launch_dep(jst_sensor_kernel, grid_for(nvalid, nsm), 256, 0, st, tb, ft, nvalid);
   return cudaGetLastError();
 }
 
 cudaError_t launch_jst(const BoxTable& tb, const FaceTable& ft, int s_in, long long ngcells, long long nvalid,
                        long long nfaces[3], int nsm, cudaStream_t st) {
   (void)ngcells;
-  jst_sensor_kernel<<<grid_for(nvalid, nsm), 256, 0, st>>>(tb, ft, nvalid);
+  launch_dep(jst_sensor_kernel, grid_for(nvalid, nsm), 256, 0, st, tb, ft, nvalid);
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
-  jst_face_kernel<<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, s_in, tot);
+  launch_dep(jst_face_kernel, grid_for(tot, nsm), 256, 0, st, tb, ft, s_in, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_visc_face_add(const BoxTable& tb, const FaceTable& ft, long long nfaces[3], int nsm,
                                  cudaStream_t st) {
   const long long tot = nfaces[0] + nfaces[1] + nfaces[2];
-  visc_face_add_kernel<<<grid_for(tot, nsm), 256, 0, st>>>(tb, ft, tot);
+  launch_dep(visc_face_add_kernel, grid_for(tot, nsm), 256, 0, st, tb, ft, tot);
   return cudaGetLastError();
 }
 
 cudaError_t launch_div_stage(const BoxTable& tb, const FaceTable& ft, int s_in, int s_s1, int s_out,
                              const DProg& prog, int rhs_only, long long nvalid, int nsm, cudaStream_t st) {
-  div_stage_kernel<<<dim3(grid_for(nvalid, nsm), NCONS), 256, 0, st>>>(tb, ft, s_in, s_s1, s_out, prog, rhs_only, nvalid);
+  launch_dep(div_stage_kernel, dim3(grid_for(nvalid, nsm), NCONS), 256, 0, st, tb, ft, s_in, s_s1, s_out, prog, rhs_only, nvalid);
   return cudaGetLastError();
 }
 

@@ -40,6 +40,7 @@ __device__ __forceinline__ bool ext_dir_ghost(int c, int lo, int hi, int bcl, in
 }
 
 __global__ void __launch_bounds__(256) halo_kernel(HaloBox hb) {
+  dep_begin();
   const int g = NGHOST;
   const int nx = hb.hi[0] - hb.lo[0] + 1 + 2 * g, ny = hb.hi[1] - hb.lo[1] + 1 + 2 * g,
             nz = hb.hi[2] - hb.lo[2] + 1 + 2 * g;
@@ -70,16 +71,16 @@ __global__ void __launch_bounds__(256) halo_kernel(HaloBox hb) {
 
 // Ghost fill of every box of a list, each box being its own domain (an
 // ensemble member or an isolated box), one launch for all boxes.
-__global__ void __launch_bounds__(256) halo_list_kernel(BoxTable tb, const long long* gpre, int slot, int bl0, int bl1,
+__global__ void __launch_bounds__(256) halo_list_kernel(const __grid_constant__ BoxTable tb, const long long* gpre, long long total, int slot, int bl0, int bl1,
                                                         int bl2, int bh0, int bh1, int bh2) {
+  dep_begin();
   if (list_idle(tb)) return;
-  const long long total = gpre[tb.n];
   const int g = NGHOST;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
        c += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(gpre, tb.n, c);
-    const BoxRec& R = tb.box[b];
-    const int l = (int)(c - gpre[b]);
+    const BoxRec& R = box_rec(tb, b);
+    const int l = (int)(c - box_base(tb, gpre, b));
     const int nx = R.hi[0] - R.lo[0] + 1 + 2 * g, ny = R.hi[1] - R.lo[1] + 1 + 2 * g;
     const int i = l % nx + R.lo[0] - g;
     const int t = l / nx;
@@ -110,25 +111,25 @@ __global__ void __launch_bounds__(256) halo_list_kernel(BoxTable tb, const long 
 // grow(box,3), in the gpre order).  Sources are valid cells only, so the
 // fill has no order dependence between boxes and is bit-identical to the
 // fill of one box covering the domain.
-__global__ void __launch_bounds__(256) halo_level_kernel(BoxTable tb, const long long* gpre, const int* owner,
+__global__ void __launch_bounds__(256) halo_level_kernel(const __grid_constant__ BoxTable tb, const long long* gpre, long long total, const int* owner,
                                                          int slot, LevelDomain dom) {
+  dep_begin();
   if (list_idle(tb)) return;
-  const long long total = gpre[tb.n];
   const int g = NGHOST;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
        c += (long long)gridDim.x * blockDim.x) {
     const int src = owner[c];
     if (src < 0) continue;  // a valid cell
     const int b = find_box_ll(gpre, tb.n, c);
-    const BoxRec& R = tb.box[b];
-    const int l = (int)(c - gpre[b]);
+    const BoxRec& R = box_rec(tb, b);
+    const int l = (int)(c - box_base(tb, gpre, b));
     const int nx = R.hi[0] - R.lo[0] + 1 + 2 * g, ny = R.hi[1] - R.lo[1] + 1 + 2 * g;
     const int i = l % nx + R.lo[0] - g;
     const int t = l / nx;
     const int j = t % ny + R.lo[1] - g;
     const int k = t / ny + R.lo[2] - g;
     const DArr U = R.slot[slot];
-    const DArr S = tb.box[src].slot[slot];
+    const DArr S = box_rec(tb, src).slot[slot];
     for (int n = 0; n < NCONS; ++n) {
       bool flip = false;
       const int si = map_coord(i, dom.lo[0], dom.hi[0], dom.bc_lo[0], dom.bc_hi[0], n, 0, flip);
@@ -145,7 +146,7 @@ cudaError_t launch_halo_level(const BoxTable& tb, const long long* gpre, const i
   long long blocks = (total + 255) / 256;
   if (blocks > (long long)nsm * 8) blocks = (long long)nsm * 8;
   if (blocks < 1) blocks = 1;
-  halo_level_kernel<<<(int)blocks, 256, 0, st>>>(tb, gpre, owner, slot, dom);
+  launch_dep(halo_level_kernel, (int)blocks, 256, 0, st, tb, gpre, total, owner, slot, dom);
   return cudaGetLastError();
 }
 
@@ -154,7 +155,7 @@ cudaError_t launch_halo_list(const BoxTable& tb, const long long* gpre, long lon
   long long blocks = (total + 255) / 256;
   if (blocks > (long long)nsm * 8) blocks = (long long)nsm * 8;
   if (blocks < 1) blocks = 1;
-  halo_list_kernel<<<(int)blocks, 256, 0, st>>>(tb, gpre, slot, bc_lo[0], bc_lo[1], bc_lo[2], bc_hi[0], bc_hi[1],
+  launch_dep(halo_list_kernel, (int)blocks, 256, 0, st, tb, gpre, total, slot, bc_lo[0], bc_lo[1], bc_lo[2], bc_hi[0], bc_hi[1],
                                                 bc_hi[2]);
   return cudaGetLastError();
 }
@@ -163,7 +164,7 @@ cudaError_t launch_halo(const HaloBox& hb, cudaStream_t st) {
   const long long total = (long long)(hb.hi[0] - hb.lo[0] + 7) * (hb.hi[1] - hb.lo[1] + 7) * (hb.hi[2] - hb.lo[2] + 7);
   long long blocks = (total + 255) / 256;
   if (blocks > 4096) blocks = 4096;
-  halo_kernel<<<(int)blocks, 256, 0, st>>>(hb);
+  launch_dep(halo_kernel, (int)blocks, 256, 0, st, hb);
   return cudaGetLastError();
 }
 
@@ -210,6 +211,7 @@ __device__ void bcnormal_isothermal_cell(const DArr& U, int i, int j, int k, int
 // row were filled by the library's fill before).
 __global__ void __launch_bounds__(256) bcnormal_box_kernel(DArr U, int lo0, int lo1, int lo2, int hi0, int hi1,
                                                            int hi2, int wlo, int whi, DClosures c, DBcNormal bn) {
+  dep_begin();
   const int g = NGHOST;
   const int nx = hi0 - lo0 + 1 + 2 * g, nz = hi2 - lo2 + 1 + 2 * g;
   const long long total = (long long)nx * nz * 2 * g;
@@ -230,18 +232,19 @@ __global__ void __launch_bounds__(256) bcnormal_box_kernel(DArr U, int lo0, int 
 // Every box of a level whose y extent touches a code-6 side of the domain:
 // the box's own ghost rows beyond that side (its first interior row and the
 // ghost columns of it were filled by halo_level_kernel).
-__global__ void __launch_bounds__(256) bcnormal_list_kernel(BoxTable tb, int slot, LevelDomain dom, DBcNormal bn) {
+__global__ void __launch_bounds__(256) bcnormal_list_kernel(const __grid_constant__ BoxTable tb, int slot, LevelDomain dom, DBcNormal bn) {
+  dep_begin();
   if (list_idle(tb)) return;
   const int g = NGHOST;
   for (int b = blockIdx.y; b < tb.n; b += gridDim.y) {
-    const BoxRec& R = tb.box[b];
+    const BoxRec& R = box_rec(tb, b);
     const bool wlo = dom.bc_lo[1] == 6 && R.lo[1] == dom.lo[1];
     const bool whi = dom.bc_hi[1] == 6 && R.hi[1] == dom.hi[1];
     if (!wlo && !whi) continue;
     const int nx = R.hi[0] - R.lo[0] + 1 + 2 * g, nz = R.hi[2] - R.lo[2] + 1 + 2 * g;
     const long long total = (long long)nx * nz * 2 * g;
     const DArr U = R.slot[slot];
-    const DClosures& c = tb.cls[R.cl];
+    const DClosures& c = box_cls(tb, R);
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
       const int i = (int)(t % nx) + R.lo[0] - g;
@@ -264,7 +267,7 @@ cudaError_t launch_bcnormal_box(const DArr& u, const int lo[3], const int hi[3],
   const long long total = (long long)(hi[0] - lo[0] + 7) * (hi[2] - lo[2] + 7) * 2 * NGHOST;
   long long blocks = (total + 255) / 256;
   if (blocks > 4096) blocks = 4096;
-  bcnormal_box_kernel<<<(int)blocks, 256, 0, st>>>(u, lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], wlo, whi, cl, bn);
+  launch_dep(bcnormal_box_kernel, (int)blocks, 256, 0, st, u, lo[0], lo[1], lo[2], hi[0], hi[1], hi[2], wlo, whi, cl, bn);
   return cudaGetLastError();
 }
 
@@ -273,7 +276,7 @@ cudaError_t launch_bcnormal_list(const BoxTable& tb, int slot, const LevelDomain
   if (bn.kind != 1 || (dom.bc_lo[1] != 6 && dom.bc_hi[1] != 6)) return cudaSuccess;
   const int gy = tb.n < nsm * 4 ? tb.n : nsm * 4;
   dim3 grid(8, (unsigned)(gy < 1 ? 1 : gy));
-  bcnormal_list_kernel<<<grid, 256, 0, st>>>(tb, slot, dom, bn);
+  launch_dep(bcnormal_list_kernel, grid, 256, 0, st, tb, slot, dom, bn);
   return cudaGetLastError();
 }
 
@@ -282,8 +285,9 @@ cudaError_t launch_bcnormal_list(const BoxTable& tb, int slot, const LevelDomain
 // with min over cells.  Positive doubles order like their bit patterns, so
 // the block minima meet in one unsigned 64-bit atomicMin; the result is the
 // exact minimum whatever the order.
-__global__ void __launch_bounds__(256) estdt_kernel(BoxTable tb, int s_in, long long total,
+__global__ void __launch_bounds__(256) estdt_kernel(const __grid_constant__ BoxTable tb, int s_in, long long total,
                                                      unsigned long long* bits) {
+  dep_begin();
   if (list_idle(tb)) return;  // uniform over the grid
   unsigned long long best = ~0ull;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -293,13 +297,13 @@ __global__ void __launch_bounds__(256) estdt_kernel(BoxTable tb, int s_in, long 
       // valid-cell prefix = pcell when gq == 0; recompute from box sizes
       long long acc = 0;
       for (b = 0; b < tb.n; ++b) {
-        const BoxRec& R = tb.box[b];
+        const BoxRec& R = box_rec(tb, b);
         const long long nc = (long long)(R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1);
         if (g < acc + nc) { g -= acc; break; }
         acc += nc;
       }
       if (b == tb.n) break;
-      const BoxRec& R = tb.box[b];
+      const BoxRec& R = box_rec(tb, b);
       const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
       const int l = (int)g;
       g += acc;
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(256) estdt_kernel(BoxTable tb, int s_in, long 
       const int j = t % ny + R.lo[1];
       const int k = t / ny + R.lo[2];
       const DArr S = R.slot[s_in];
-      const DClosures& cl = tb.cls[R.cl];
+      const DClosures& cl = box_cls(tb, R);
       const long long o = S.off(i, j, k);
       const double rho = S.p[o], mx = S.p[o + S.ns], my = S.p[o + 2 * S.ns], mz = S.p[o + 2 * S.ns];
       const double rhoinv = ddiv_rn(1.0, rmax(rho, 1.0e-40));
@@ -344,9 +348,12 @@ __global__ void __launch_bounds__(256) estdt_kernel(BoxTable tb, int s_in, long 
   }
 }
 
-__global__ void estdt_init(unsigned long long* bits) { *bits = ~0ull; }
+__global__ void estdt_init(unsigned long long* bits) {
+  dep_begin();
+  *bits = ~0ull; }
 
 __global__ void estdt_final(const unsigned long long* bits, double cfl, double* out) {
+  dep_begin();
   const unsigned long long b = *bits;
   const double dt = (b == ~0ull) ? 1.7976931348623157e308 : __longlong_as_double((long long)b);
   *out = dt * cfl;
@@ -354,12 +361,12 @@ __global__ void estdt_final(const unsigned long long* bits, double cfl, double* 
 
 cudaError_t launch_estdt(const BoxTable& tb, int s_in, long long nvalid, double cfl, unsigned long long* bits,
                          double* dt_out, int nsm, cudaStream_t st) {
-  estdt_init<<<1, 1, 0, st>>>(bits);
+  launch_dep(estdt_init, 1, 1, 0, st, bits);
   long long blocks = (nvalid + 255) / 256;
   if (blocks > (long long)nsm * 4) blocks = (long long)nsm * 4;
   if (blocks < 1) blocks = 1;
-  estdt_kernel<<<(int)blocks, 256, 0, st>>>(tb, s_in, nvalid, bits);
-  estdt_final<<<1, 1, 0, st>>>(bits, cfl, dt_out);
+  launch_dep(estdt_kernel, (int)blocks, 256, 0, st, tb, s_in, nvalid, bits);
+  launch_dep(estdt_final, 1, 1, 0, st, bits, cfl, dt_out);
   return cudaGetLastError();
 }
 
@@ -368,6 +375,7 @@ cudaError_t launch_estdt(const BoxTable& tb, int s_in, long long nvalid, double 
 // CNS::advance steps with the reference's single-level dt control
 // (computeInitialDt / computeNewDt, src/CNS.cpp:282-377) without host syncs.
 __global__ void run_estdt_reset(RunCtl* c) {
+  dep_begin();
   if (c->active) c->bits = ~0ull;
 }
 
@@ -375,6 +383,7 @@ __global__ void run_estdt_reset(RunCtl* c) {
 // dx/(|u|+c), change_max * dt), the last step clamped to stop_time with
 // eps = 0.001 dt as the reference does), then whether to go on.
 __global__ void run_step_done(RunCtl* c, cudaGraphConditionalHandle cond) {
+  dep_begin();
   if (c->active) {
     c->time = c->time + c->dt;
     c->step += 1;
@@ -394,6 +403,7 @@ __global__ void run_step_done(RunCtl* c, cudaGraphConditionalHandle cond) {
 
 // Initial dt (computeInitialDt: cfl * min dx/(|u|+c)) and whether to start.
 __global__ void run_begin(RunCtl* c) {
+  dep_begin();
   if (c->use_cfl) {
     const unsigned long long b = c->bits;
     c->dt = ((b == ~0ull) ? 1.7976931348623157e308 : __longlong_as_double((long long)b)) * c->cfl;
@@ -403,20 +413,21 @@ __global__ void run_begin(RunCtl* c) {
 
 // Valid cells of slot `from` into slot `to` for every box (the step's result
 // back into the S1 slot the next step reads).
-__global__ void __launch_bounds__(256) copy_slot_kernel(BoxTable tb, int from, int to, long long total) {
+__global__ void __launch_bounds__(256) copy_slot_kernel(const __grid_constant__ BoxTable tb, int from, int to, long long total) {
+  dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     long long acc = 0;
     int b = 0;
     for (; b < tb.n; ++b) {
-      const BoxRec& R = tb.box[b];
+      const BoxRec& R = box_rec(tb, b);
       const long long nc = (long long)(R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1);
       if (g < acc + nc) break;
       acc += nc;
     }
     if (b == tb.n) break;
-    const BoxRec& R = tb.box[b];
+    const BoxRec& R = box_rec(tb, b);
     const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
     const int l = (int)(g - acc);
     const int i = l % nx + R.lo[0];
@@ -434,16 +445,17 @@ __global__ void __launch_bounds__(256) copy_slot_kernel(BoxTable tb, int from, i
 // *flag when any component is a NaN or an infinity (exponent bits all ones,
 // tested on the integer bits, so the FP64 pipe is not used).  One extra
 // read of the slot (40 B per cell); run only when the caller opted in.
-__global__ void __launch_bounds__(256) nonfinite_check_kernel(BoxTable tb, const long long* vpre, int slot,
+__global__ void __launch_bounds__(256) nonfinite_check_kernel(const __grid_constant__ BoxTable tb, const long long* vpre, int slot,
                                                               long long total, int* flag) {
+  dep_begin();
   if (list_idle(tb)) return;
   int bad = 0;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(vpre, tb.n, g);
-    const BoxRec& R = tb.box[b];
+    const BoxRec& R = box_rec(tb, b);
     const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
-    const long long l = g - vpre[b];
+    const long long l = g - box_base(tb, vpre, b);
     const int i = (int)(l % nx) + R.lo[0];
     const long long t = l / nx;
     const int j = (int)(t % ny) + R.lo[1], k = (int)(t / ny) + R.lo[2];
@@ -463,7 +475,7 @@ cudaError_t launch_nonfinite_check(const BoxTable& tb, const long long* vpre, in
   long long blocks = (nvalid + 255) / 256;
   if (blocks > (long long)nsm * 4) blocks = (long long)nsm * 4;
   if (blocks < 1) blocks = 1;
-  nonfinite_check_kernel<<<(int)blocks, 256, 0, st>>>(tb, vpre, slot, nvalid, flag);
+  launch_dep(nonfinite_check_kernel, (int)blocks, 256, 0, st, tb, vpre, slot, nvalid, flag);
   return cudaGetLastError();
 }
 
@@ -490,13 +502,15 @@ __device__ __forceinline__ double ord_dec(unsigned long long e) {
 constexpr int NSTAT = 21;  // min[6], max[6], table[3][3]
 
 __global__ void prim_stats_init(unsigned long long* cells) {
+  dep_begin();
   const int t = threadIdx.x;
   if (t < NSTAT) cells[t] = t < 6 ? ~0ull : 0ull;
 }
 
-__global__ void __launch_bounds__(256) prim_stats_kernel(BoxTable tb, const long long* vpre, int slot, double dt,
+__global__ void __launch_bounds__(256) prim_stats_kernel(const __grid_constant__ BoxTable tb, const long long* vpre, int slot, double dt,
                                                          double dx0, double dx1, double dx2, long long total,
                                                          unsigned long long* cells) {
+  dep_begin();
   double mn[6], mx[6], t[9];
 #pragma unroll
   for (int n = 0; n < 6; ++n) { mn[n] = __longlong_as_double(0x7ff0000000000000ll); mx[n] = -mn[n]; }
@@ -506,10 +520,10 @@ __global__ void __launch_bounds__(256) prim_stats_kernel(BoxTable tb, const long
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(vpre, tb.n, g);
-    const BoxRec& R = tb.box[b];
-    const DClosures& cl = tb.cls[R.cl];
+    const BoxRec& R = box_rec(tb, b);
+    const DClosures& cl = box_cls(tb, R);
     const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
-    const long long l = g - vpre[b];
+    const long long l = g - box_base(tb, vpre, b);
     const int i = (int)(l % nx) + R.lo[0];
     const long long tt = l / nx;
     const int j = (int)(tt % ny) + R.lo[1], k = (int)(tt / ny) + R.lo[2];
@@ -565,38 +579,40 @@ __global__ void __launch_bounds__(256) prim_stats_kernel(BoxTable tb, const long
 }
 
 __global__ void prim_stats_final(const unsigned long long* cells, double* out) {
+  dep_begin();
   const int t = threadIdx.x;
   if (t < NSTAT) out[t] = ord_dec(cells[t]);
 }
 
 cudaError_t launch_prim_stats(const BoxTable& tb, const long long* vpre, int slot, double dt, const double dx[3],
                               long long nvalid, unsigned long long* cells, double* out, int nsm, cudaStream_t st) {
-  prim_stats_init<<<1, 32, 0, st>>>(cells);
+  launch_dep(prim_stats_init, 1, 32, 0, st, cells);
   long long blocks = (nvalid + 255) / 256;
   if (blocks > (long long)nsm * 4) blocks = (long long)nsm * 4;
   if (blocks < 1) blocks = 1;
-  prim_stats_kernel<<<(int)blocks, 256, 0, st>>>(tb, vpre, slot, dt, dx[0], dx[1], dx[2], nvalid, cells);
-  prim_stats_final<<<1, 32, 0, st>>>(cells, out);
+  launch_dep(prim_stats_kernel, (int)blocks, 256, 0, st, tb, vpre, slot, dt, dx[0], dx[1], dx[2], nvalid, cells);
+  launch_dep(prim_stats_final, 1, 32, 0, st, cells, out);
   return cudaGetLastError();
 }
 
 // Conserved totals of slot `slot` over the valid cells of every box:
 // per-block sums in a fixed order, then one block sums the partials in
 // block order (deterministic; not the serial sum's rounding).
-__global__ void __launch_bounds__(256) totals_partial_kernel(BoxTable tb, int slot, long long total, double* part) {
+__global__ void __launch_bounds__(256) totals_partial_kernel(const __grid_constant__ BoxTable tb, int slot, long long total, double* part) {
+  dep_begin();
   double acc[NCONS] = {0, 0, 0, 0, 0};
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     long long base = 0;
     int b = 0;
     for (; b < tb.n; ++b) {
-      const BoxRec& R = tb.box[b];
+      const BoxRec& R = box_rec(tb, b);
       const long long nc = (long long)(R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1);
       if (g < base + nc) break;
       base += nc;
     }
     if (b == tb.n) break;
-    const BoxRec& R = tb.box[b];
+    const BoxRec& R = box_rec(tb, b);
     const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
     const int l = (int)(g - base);
     const DArr S = R.slot[slot];
@@ -618,6 +634,7 @@ __global__ void __launch_bounds__(256) totals_partial_kernel(BoxTable tb, int sl
 }
 
 __global__ void totals_final_kernel(const double* part, int nblocks, double scale, double* out) {
+  dep_begin();
   if (threadIdx.x < NCONS) {
     double s = 0.0;
     for (int b = 0; b < nblocks; ++b) s += part[(long long)b * NCONS + threadIdx.x];
@@ -626,21 +643,21 @@ __global__ void totals_final_kernel(const double* part, int nblocks, double scal
 }
 
 cudaError_t launch_run_estdt(const BoxTable& tb, int s_in, long long nvalid, RunCtl* c, int nsm, cudaStream_t st) {
-  run_estdt_reset<<<1, 1, 0, st>>>(c);
+  launch_dep(run_estdt_reset, 1, 1, 0, st, c);
   long long blocks = (nvalid + 255) / 256;
   if (blocks > (long long)nsm * 4) blocks = (long long)nsm * 4;
   if (blocks < 1) blocks = 1;
-  estdt_kernel<<<(int)blocks, 256, 0, st>>>(tb, s_in, nvalid, &c->bits);
+  launch_dep(estdt_kernel, (int)blocks, 256, 0, st, tb, s_in, nvalid, &c->bits);
   return cudaGetLastError();
 }
 
 cudaError_t launch_run_step_done(RunCtl* c, cudaGraphConditionalHandle cond, cudaStream_t st) {
-  run_step_done<<<1, 1, 0, st>>>(c, cond);
+  launch_dep(run_step_done, 1, 1, 0, st, c, cond);
   return cudaGetLastError();
 }
 
 cudaError_t launch_run_begin(RunCtl* c, cudaStream_t st) {
-  run_begin<<<1, 1, 0, st>>>(c);
+  launch_dep(run_begin, 1, 1, 0, st, c);
   return cudaGetLastError();
 }
 
@@ -648,7 +665,7 @@ cudaError_t launch_copy_slot(const BoxTable& tb, int from, int to, long long nva
   long long blocks = (nvalid + 255) / 256;
   if (blocks > (long long)nsm * 8) blocks = (long long)nsm * 8;
   if (blocks < 1) blocks = 1;
-  copy_slot_kernel<<<(int)blocks, 256, 0, st>>>(tb, from, to, nvalid);
+  launch_dep(copy_slot_kernel, (int)blocks, 256, 0, st, tb, from, to, nvalid);
   return cudaGetLastError();
 }
 
@@ -661,8 +678,8 @@ int totals_blocks(long long nvalid, int nsm) {
 cudaError_t launch_totals(const BoxTable& tb, int slot, long long nvalid, double scale, double* part, double* out,
                           int nsm, cudaStream_t st) {
   const int nb = totals_blocks(nvalid, nsm);
-  totals_partial_kernel<<<nb, 256, 0, st>>>(tb, slot, nvalid, part);
-  totals_final_kernel<<<1, 32, 0, st>>>(part, nb, scale, out);
+  launch_dep(totals_partial_kernel, nb, 256, 0, st, tb, slot, nvalid, part);
+  launch_dep(totals_final_kernel, 1, 32, 0, st, part, nb, scale, out);
   return cudaGetLastError();
 }
 
@@ -906,6 +923,7 @@ cudaError_t launch_dsqrt_check(unsigned long long seed, long long count, unsigne
 // velocities (dervel: momentum / density).  out: 5 components in that order.
 __global__ void __launch_bounds__(256) plot_derive_kernel(DArr U, DArr O, int lo0, int lo1, int lo2, int nx,
                                                           int ny, long long total, double gamma, double cv) {
+  dep_begin();
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(g % nx) + lo0;
@@ -928,7 +946,7 @@ cudaError_t launch_plot_derive(const DArr& U, const DArr& O, const int lo[3], co
   long long blocks = (total + 255) / 256;
   if (blocks > (long long)nsm * 8) blocks = (long long)nsm * 8;
   if (blocks < 1) blocks = 1;
-  plot_derive_kernel<<<(int)blocks, 256, 0, st>>>(U, O, lo[0], lo[1], lo[2], n[0], n[1], total, gamma, cv);
+  launch_dep(plot_derive_kernel, (int)blocks, 256, 0, st, U, O, lo[0], lo[1], lo[2], n[0], n[1], total, gamma, cv);
   return cudaGetLastError();
 }
 
@@ -941,6 +959,7 @@ cudaError_t launch_plot_derive(const DArr& U, const DArr& O, const int lo[3], co
 __global__ void __launch_bounds__(256) avgdown_kernel(DArr fine, DArr crse, int lo0, int lo1, int lo2, int nx,
                                                       int ny, long long total, int rx, int ry, int rz, int scomp,
                                                       int ncomp, double volfrac) {
+  dep_begin();
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(g % nx) + lo0;
@@ -962,7 +981,7 @@ cudaError_t launch_avgdown(const DArr& fine, const DArr& crse, const int lo[3], 
   if (total <= 0) return cudaSuccess;
   long long blocks = (total + 255) / 256;
   if (blocks > 8LL * nsm) blocks = 8LL * nsm;
-  avgdown_kernel<<<(int)blocks, 256, 0, st>>>(fine, crse, lo[0], lo[1], lo[2], n[0], n[1], total, r[0], r[1], r[2],
+  launch_dep(avgdown_kernel, (int)blocks, 256, 0, st, fine, crse, lo[0], lo[1], lo[2], n[0], n[1], total, r[0], r[1], r[2],
                                                scomp, ncomp, volfrac);
   return cudaGetLastError();
 }
