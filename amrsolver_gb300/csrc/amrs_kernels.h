@@ -115,8 +115,8 @@ cudaError_t launch_source_vjp(const BoxRec& R, const double force[3], const DArr
 cudaError_t launch_adj_prog(const BoxRec& R, const DProg& prog, const DArr& wbar, const DArr& s1bar, const DArr& inbar,
                             const DArr& vbar, int accumulate, int nsm, cudaStream_t st);
 cudaError_t launch_adj_halo(const HaloBox& hb, int nsm, cudaStream_t st);
-cudaError_t launch_halo_list(const BoxTable& tb, const long long* gpre, long long total, int slot, const int bc_lo[3],
-                             const int bc_hi[3], int nsm, cudaStream_t st);
+cudaError_t launch_halo_list(const BoxTable& tb, const long long* gpre, const long long* vpre, long long ghosts,
+                             int slot, const int bc_lo[3], const int bc_hi[3], int nsm, cudaStream_t st);
 // Device state of a time loop over a box list (amrs_rk_run_boxlist); the
 // list's kernels read `active` through BoxTable::active.
 struct RunCtl {
@@ -144,8 +144,8 @@ struct LevelDomain {
   int lo[3], hi[3];
   int bc_lo[3], bc_hi[3];
 };
-cudaError_t launch_halo_level(const BoxTable& tb, const long long* gpre, const int* owner, long long total, int slot,
-                              const LevelDomain& dom, int nsm, cudaStream_t st);
+cudaError_t launch_halo_level(const BoxTable& tb, const long long* gpre, const long long* vpre, long long ghosts,
+                              const int* owner, int slot, const LevelDomain& dom, int nsm, cudaStream_t st);
 // A problem bcnormal evaluated on the device for y sides of code 6 (kind 1:
 // the channel problem's isothermal no-slip wall), after the library's fill.
 struct DBcNormal {

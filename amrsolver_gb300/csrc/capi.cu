@@ -1032,13 +1032,14 @@ amrs_status level_owner_table(const List& L, const LevelDomain& dom, std::vector
 // Ghost fill of one state slot of every box of a list (before a stage).
 cudaError_t list_fill(amrs_handle* h, List& L, int slot, cudaStream_t st) {
   if (L.has_bc == 2) {
-    cudaError_t e = launch_halo_level(L.tb, L.ft.gpre, L.d_owner, L.tot_g, slot, L.dom, h->nsm, st);
+    cudaError_t e = launch_halo_level(L.tb, L.ft.gpre, L.ft.vpre, L.tot_g - L.tot_valid, L.d_owner, slot, L.dom,
+                                      h->nsm, st);
     // then the problem's bcnormal beyond code-6 y sides (it reads the
     // first interior row, ghost columns included, that the fill wrote)
     if (e == cudaSuccess && L.bcn.kind) e = launch_bcnormal_list(L.tb, slot, L.dom, L.bcn, h->nsm, st);
     return e;
   }
-  return launch_halo_list(L.tb, L.ft.gpre, L.tot_g, slot, L.bc_lo, L.bc_hi, h->nsm, st);
+  return launch_halo_list(L.tb, L.ft.gpre, L.ft.vpre, L.tot_g - L.tot_valid, slot, L.bc_lo, L.bc_hi, h->nsm, st);
 }
 
 }  // namespace

@@ -12,7 +12,8 @@ namespace amrs {
 // reflection), with a sign flip for every reflect_odd mapping; this equals
 // AMReX's sequential fill (periodic images, then physical BCs direction by
 // direction).  BC types per component: src/set/CNS_setup.cpp:18-31.
-__device__ __forceinline__ int map_coord(int c, int lo, int hi, int bcl, int bch, int comp, int dir, bool& flip) {
+// `flip` collects the components (bits) whose sign changes.
+__device__ __forceinline__ int map_coord(int c, int lo, int hi, int bcl, int bch, int dir, unsigned& flip) {
   if (c >= lo && c <= hi) return c;
   const int n = hi - lo + 1;
   const bool low = c < lo;
@@ -23,12 +24,8 @@ __device__ __forceinline__ int map_coord(int c, int lo, int hi, int bcl, int bch
     return lo + r;
   }
   if (phys == 2) return low ? lo : hi;  // foextrap
-  const bool vel = comp >= UMX && comp <= UMZ;
-  const bool normal = comp == UMX + dir;
-  bool odd = false;
-  if (phys == 3 || phys == 4) odd = vel && normal;
-  else if (phys == 5) odd = vel;
-  if (odd) flip = !flip;
+  if (phys == 3 || phys == 4) flip ^= 1u << (UMX + dir);
+  else if (phys == 5) flip ^= 7u << UMX;
   return low ? 2 * lo - c - 1 : 2 * hi - c + 1;
 }
 
@@ -39,68 +36,117 @@ __device__ __forceinline__ bool ext_dir_ghost(int c, int lo, int hi, int bcl, in
   return (c < lo && (bcl == 1 || bcl == 6)) || (c > hi && (bch == 1 || bch == 6));
 }
 
-__global__ void __launch_bounds__(256) halo_kernel(HaloBox hb) {
+// Ghost cell e of a box of nx x ny x nz cells, relative to its low corner: the
+// 3 + 3 planes beyond z (ghost columns and corners included), then the rows
+// beyond y of every valid plane, then the cells beyond x of every valid row.
+// The fills deal ghost cells, not grown cells, to threads: a 32^3 box has 22,104
+// of the one and 54,872 of the other.
+__device__ __forceinline__ void ghost_cell(int e, int nx, int ny, int nz, int& i, int& j, int& k) {
+  const int mx = nx + 2 * NGHOST, plane = mx * (ny + 2 * NGHOST);
+  auto side = [](int q, int n) { return q < NGHOST ? q - NGHOST : n + q - NGHOST; };
+  if (e < 2 * NGHOST * plane) {
+    const int p = e / plane, r = e - p * plane, y = r / mx;
+    k = side(p, nz);
+    j = y - NGHOST;
+    i = r - y * mx - NGHOST;
+    return;
+  }
+  e -= 2 * NGHOST * plane;
+  const int slab = 2 * NGHOST * mx;
+  if (e < nz * slab) {
+    k = e / slab;
+    const int r = e - k * slab, q = r / mx;
+    j = side(q, ny);
+    i = r - q * mx - NGHOST;
+    return;
+  }
+  e -= nz * slab;
+  const int row = e / (2 * NGHOST);
+  i = side(e - row * 2 * NGHOST, nx);
+  k = row / ny;
+  j = row - k * ny;
+}
+__host__ __device__ __forceinline__ long long ghost_cells(long long nx, long long ny, long long nz) {
+  return (nx + 2 * NGHOST) * (ny + 2 * NGHOST) * (nz + 2 * NGHOST) - nx * ny * nz;
+}
+// The components of one ghost cell from its source cell, all loads first.
+template <int N>
+__device__ __forceinline__ void ghost_copy(double* dst, long long dn, const double* src, long long sn, unsigned flip) {
+  double v[N];
+#pragma unroll
+  for (int n = 0; n < N; ++n) v[n] = src[n * sn];
+#pragma unroll
+  for (int n = 0; n < N; ++n) dst[n * dn] = (flip >> n) & 1u ? -v[n] : v[n];
+}
+
+__global__ void __launch_bounds__(256) halo_kernel(HaloBox hb, int total) {
   dep_begin();
-  const int g = NGHOST;
-  const int nx = hb.hi[0] - hb.lo[0] + 1 + 2 * g, ny = hb.hi[1] - hb.lo[1] + 1 + 2 * g,
-            nz = hb.hi[2] - hb.lo[2] + 1 + 2 * g;
-  const long long total = (long long)nx * ny * nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
-       c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % nx) + hb.lo[0] - g;
-    const long long t = c / nx;
-    const int j = (int)(t % ny) + hb.lo[1] - g;
-    const int k = (int)(t / ny) + hb.lo[2] - g;
-    const bool inside = i >= hb.lo[0] && i <= hb.hi[0] && j >= hb.lo[1] && j <= hb.hi[1] && k >= hb.lo[2] &&
-                        k <= hb.hi[2];
-    if (inside) continue;
+  const int nx = hb.hi[0] - hb.lo[0] + 1, ny = hb.hi[1] - hb.lo[1] + 1, nz = hb.hi[2] - hb.lo[2] + 1;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+    int i, j, k;
+    ghost_cell(e, nx, ny, nz, i, j, k);
+    i += hb.lo[0];
+    j += hb.lo[1];
+    k += hb.lo[2];
     if (ext_dir_ghost(i, hb.lo[0], hb.hi[0], hb.bc_lo[0], hb.bc_hi[0]) ||
         ext_dir_ghost(j, hb.lo[1], hb.hi[1], hb.bc_lo[1], hb.bc_hi[1]) ||
         ext_dir_ghost(k, hb.lo[2], hb.hi[2], hb.bc_lo[2], hb.bc_hi[2]))
       continue;
-    for (int n = 0; n < hb.ncomp; ++n) {
-      bool flip = false;
-      const int si = map_coord(i, hb.lo[0], hb.hi[0], hb.bc_lo[0], hb.bc_hi[0], n, 0, flip);
-      const int sj = map_coord(j, hb.lo[1], hb.hi[1], hb.bc_lo[1], hb.bc_hi[1], n, 1, flip);
-      const int sk = map_coord(k, hb.lo[2], hb.hi[2], hb.bc_lo[2], hb.bc_hi[2], n, 2, flip);
-      const double v = hb.u(si, sj, sk, n);
-      hb.u(i, j, k, n) = flip ? -v : v;
+    unsigned flip = 0u;
+    const int si = map_coord(i, hb.lo[0], hb.hi[0], hb.bc_lo[0], hb.bc_hi[0], 0, flip);
+    const int sj = map_coord(j, hb.lo[1], hb.hi[1], hb.bc_lo[1], hb.bc_hi[1], 1, flip);
+    const int sk = map_coord(k, hb.lo[2], hb.hi[2], hb.bc_lo[2], hb.bc_hi[2], 2, flip);
+    double* d = hb.u.p + hb.u.off(i, j, k);
+    const double* s = hb.u.p + hb.u.off(si, sj, sk);
+    if (hb.ncomp == NCONS) {
+      ghost_copy<NCONS>(d, hb.u.ns, s, hb.u.ns, flip);
+    } else {
+      for (int n = 0; n < hb.ncomp; ++n) {
+        const double v = s[n * hb.u.ns];
+        d[n * hb.u.ns] = n < 32 && ((flip >> n) & 1u) ? -v : v;
+      }
     }
   }
 }
 
+// Box holding ghost cell e of the list: the prefixes of grown and valid cells
+// differ by that of the ghost cells.
+__device__ __forceinline__ int find_ghost_box(const BoxTable& tb, const long long* gpre, const long long* vpre,
+                                              long long e, int& rel) {
+  if (tb.one) { rel = (int)e; return 0; }
+  int lo = 0, hi = tb.n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (gpre[mid] - vpre[mid] <= e) lo = mid; else hi = mid;
+  }
+  rel = (int)(e - (gpre[lo] - vpre[lo]));
+  return lo;
+}
+
 // Ghost fill of every box of a list, each box being its own domain (an
 // ensemble member or an isolated box), one launch for all boxes.
-__global__ void __launch_bounds__(256) halo_list_kernel(const __grid_constant__ BoxTable tb, const long long* gpre, long long total, int slot, int bl0, int bl1,
-                                                        int bl2, int bh0, int bh1, int bh2) {
+__global__ void __launch_bounds__(256) halo_list_kernel(const __grid_constant__ BoxTable tb, const long long* gpre,
+                                                        const long long* vpre, long long total, int slot, int bl0,
+                                                        int bl1, int bl2, int bh0, int bh1, int bh2) {
   dep_begin();
   if (list_idle(tb)) return;
-  const int g = NGHOST;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
        c += (long long)gridDim.x * blockDim.x) {
-    const int b = find_box_ll(gpre, tb.n, c);
-    const BoxRec& R = box_rec(tb, b);
-    const int l = (int)(c - box_base(tb, gpre, b));
-    const int nx = R.hi[0] - R.lo[0] + 1 + 2 * g, ny = R.hi[1] - R.lo[1] + 1 + 2 * g;
-    const int i = l % nx + R.lo[0] - g;
-    const int t = l / nx;
-    const int j = t % ny + R.lo[1] - g;
-    const int k = t / ny + R.lo[2] - g;
-    const bool inside = i >= R.lo[0] && i <= R.hi[0] && j >= R.lo[1] && j <= R.hi[1] && k >= R.lo[2] &&
-                        k <= R.hi[2];
-    if (inside) continue;
+    int e, i, j, k;
+    const BoxRec& R = box_rec(tb, find_ghost_box(tb, gpre, vpre, c, e));
+    ghost_cell(e, R.hi[0] - R.lo[0] + 1, R.hi[1] - R.lo[1] + 1, R.hi[2] - R.lo[2] + 1, i, j, k);
+    i += R.lo[0];
+    j += R.lo[1];
+    k += R.lo[2];
     if (ext_dir_ghost(i, R.lo[0], R.hi[0], bl0, bh0) || ext_dir_ghost(j, R.lo[1], R.hi[1], bl1, bh1) ||
         ext_dir_ghost(k, R.lo[2], R.hi[2], bl2, bh2))
       continue;
-    const DArr U = R.slot[slot];
-    for (int n = 0; n < NCONS; ++n) {
-      bool flip = false;
-      const int si = map_coord(i, R.lo[0], R.hi[0], bl0, bh0, n, 0, flip);
-      const int sj = map_coord(j, R.lo[1], R.hi[1], bl1, bh1, n, 1, flip);
-      const int sk = map_coord(k, R.lo[2], R.hi[2], bl2, bh2, n, 2, flip);
-      const double v = U(si, sj, sk, n);
-      U(i, j, k, n) = flip ? -v : v;
-    }
+    unsigned flip = 0u;
+    const int si = map_coord(i, R.lo[0], R.hi[0], bl0, bh0, 0, flip);
+    const int sj = map_coord(j, R.lo[1], R.hi[1], bl1, bh1, 1, flip);
+    const int sk = map_coord(k, R.lo[2], R.hi[2], bl2, bh2, 2, flip);
+    const DArr& U = R.slot[slot];
+    ghost_copy<NCONS>(U.p + U.off(i, j, k), U.ns, U.p + U.off(si, sj, sk), U.ns, flip);
   }
 }
 
@@ -110,61 +156,58 @@ __global__ void __launch_bounds__(256) halo_list_kernel(const __grid_constant__ 
 // that owns it (owner table built on the host, one entry per cell of every
 // grow(box,3), in the gpre order).  Sources are valid cells only, so the
 // fill has no order dependence between boxes and is bit-identical to the
-// fill of one box covering the domain.
-__global__ void __launch_bounds__(256) halo_level_kernel(const __grid_constant__ BoxTable tb, const long long* gpre, long long total, const int* owner,
+// fill of one box covering the domain.  Bound: memory and its latency; with one
+// thread per grown cell that mapped its coordinates once per component, 64 boxes
+// of 32^3 took 158 us per fill, so 40 us (single box of 128^3: 37 -> 8).
+__global__ void __launch_bounds__(256) halo_level_kernel(const __grid_constant__ BoxTable tb, const long long* gpre,
+                                                         const long long* vpre, long long total, const int* owner,
                                                          int slot, LevelDomain dom) {
   dep_begin();
   if (list_idle(tb)) return;
-  const int g = NGHOST;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
        c += (long long)gridDim.x * blockDim.x) {
-    const int src = owner[c];
-    if (src < 0) continue;  // a valid cell
-    const int b = find_box_ll(gpre, tb.n, c);
+    int e, i, j, k;
+    const int b = find_ghost_box(tb, gpre, vpre, c, e);
     const BoxRec& R = box_rec(tb, b);
-    const int l = (int)(c - box_base(tb, gpre, b));
-    const int nx = R.hi[0] - R.lo[0] + 1 + 2 * g, ny = R.hi[1] - R.lo[1] + 1 + 2 * g;
-    const int i = l % nx + R.lo[0] - g;
-    const int t = l / nx;
-    const int j = t % ny + R.lo[1] - g;
-    const int k = t / ny + R.lo[2] - g;
-    const DArr U = R.slot[slot];
-    const DArr S = box_rec(tb, src).slot[slot];
-    for (int n = 0; n < NCONS; ++n) {
-      bool flip = false;
-      const int si = map_coord(i, dom.lo[0], dom.hi[0], dom.bc_lo[0], dom.bc_hi[0], n, 0, flip);
-      const int sj = map_coord(j, dom.lo[1], dom.hi[1], dom.bc_lo[1], dom.bc_hi[1], n, 1, flip);
-      const int sk = map_coord(k, dom.lo[2], dom.hi[2], dom.bc_lo[2], dom.bc_hi[2], n, 2, flip);
-      const double v = S(si, sj, sk, n);
-      U(i, j, k, n) = flip ? -v : v;
-    }
+    const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
+    ghost_cell(e, nx, ny, R.hi[2] - R.lo[2] + 1, i, j, k);
+    const int g = NGHOST;
+    const int src = owner[box_base(tb, gpre, b) + (i + g) + (nx + 2 * g) * ((j + g) + (ny + 2 * g) * (k + g))];
+    if (src < 0) continue;  // beyond an ext_dir side
+    i += R.lo[0];
+    j += R.lo[1];
+    k += R.lo[2];
+    unsigned flip = 0u;
+    const int si = map_coord(i, dom.lo[0], dom.hi[0], dom.bc_lo[0], dom.bc_hi[0], 0, flip);
+    const int sj = map_coord(j, dom.lo[1], dom.hi[1], dom.bc_lo[1], dom.bc_hi[1], 1, flip);
+    const int sk = map_coord(k, dom.lo[2], dom.hi[2], dom.bc_lo[2], dom.bc_hi[2], 2, flip);
+    const DArr& U = R.slot[slot];
+    const DArr& S = box_rec(tb, src).slot[slot];
+    ghost_copy<NCONS>(U.p + U.off(i, j, k), U.ns, S.p + S.off(si, sj, sk), S.ns, flip);
   }
 }
 
-cudaError_t launch_halo_level(const BoxTable& tb, const long long* gpre, const int* owner, long long total, int slot,
-                              const LevelDomain& dom, int nsm, cudaStream_t st) {
-  long long blocks = (total + 255) / 256;
-  if (blocks > (long long)nsm * 8) blocks = (long long)nsm * 8;
-  if (blocks < 1) blocks = 1;
-  launch_dep(halo_level_kernel, (int)blocks, 256, 0, st, tb, gpre, total, owner, slot, dom);
+static int ghost_blocks(long long total, int cap) {
+  const long long b = (total + 255) / 256;
+  return (int)(b < 1 ? 1 : (b < cap ? b : cap));
+}
+
+cudaError_t launch_halo_level(const BoxTable& tb, const long long* gpre, const long long* vpre, long long ghosts,
+                              const int* owner, int slot, const LevelDomain& dom, int nsm, cudaStream_t st) {
+  launch_dep(halo_level_kernel, ghost_blocks(ghosts, nsm * 8), 256, 0, st, tb, gpre, vpre, ghosts, owner, slot, dom);
   return cudaGetLastError();
 }
 
-cudaError_t launch_halo_list(const BoxTable& tb, const long long* gpre, long long total, int slot, const int bc_lo[3],
-                             const int bc_hi[3], int nsm, cudaStream_t st) {
-  long long blocks = (total + 255) / 256;
-  if (blocks > (long long)nsm * 8) blocks = (long long)nsm * 8;
-  if (blocks < 1) blocks = 1;
-  launch_dep(halo_list_kernel, (int)blocks, 256, 0, st, tb, gpre, total, slot, bc_lo[0], bc_lo[1], bc_lo[2], bc_hi[0], bc_hi[1],
-                                                bc_hi[2]);
+cudaError_t launch_halo_list(const BoxTable& tb, const long long* gpre, const long long* vpre, long long ghosts,
+                             int slot, const int bc_lo[3], const int bc_hi[3], int nsm, cudaStream_t st) {
+  launch_dep(halo_list_kernel, ghost_blocks(ghosts, nsm * 8), 256, 0, st, tb, gpre, vpre, ghosts, slot, bc_lo[0],
+             bc_lo[1], bc_lo[2], bc_hi[0], bc_hi[1], bc_hi[2]);
   return cudaGetLastError();
 }
 
 cudaError_t launch_halo(const HaloBox& hb, cudaStream_t st) {
-  const long long total = (long long)(hb.hi[0] - hb.lo[0] + 7) * (hb.hi[1] - hb.lo[1] + 7) * (hb.hi[2] - hb.lo[2] + 7);
-  long long blocks = (total + 255) / 256;
-  if (blocks > 4096) blocks = 4096;
-  launch_dep(halo_kernel, (int)blocks, 256, 0, st, hb);
+  const long long total = ghost_cells(hb.hi[0] - hb.lo[0] + 1, hb.hi[1] - hb.lo[1] + 1, hb.hi[2] - hb.lo[2] + 1);
+  launch_dep(halo_kernel, ghost_blocks(total, 4096), 256, 0, st, hb, (int)total);
   return cudaGetLastError();
 }
 
