@@ -1,6 +1,7 @@
 // Pieces shared by the reverse-mode kernels.
 #pragma once
 #include "amrs_boxes.cuh"
+#include "weno_int.cuh"
 
 namespace amrs {
 
@@ -36,7 +37,7 @@ __device__ __forceinline__ void cons2prim_vjp(const BoxRec& R, const DClosures& 
   ub5[4] = eib;
 }
 
-// Gradient (and, through Wout, the value) of weno5js (src/rhs/High_resolution.h:124-159):
+// Gradient and value of weno5js (src/rhs/High_resolution.h:124-159):
 //   W = sum_k w_k v_k / 6,  w_k = a_k / A,  a_k = c_k / e_k^2,  e_k = beta_k + eps
 //   dW/ds = sum_k (w_k/6) grad v_k + sum_k ebar_k grad beta_k,
 //   ebar_k = -2 w_k (v_k/6 - W) / e_k.
@@ -44,62 +45,115 @@ __device__ __forceinline__ void cons2prim_vjp(const BoxRec& R, const DClosures& 
 // D = sum_k c_k q_k^2: w_k = c_k q_k^2 / D and w_k / e_k = c_k q_k^3 / (D P),
 // so one division 1/(D P) serves the weights and the e_k quotients (D P ~ e^7
 // stays in range for e in [1e-40, 1e40]; outside it the four-division form).
-// Standalone products (those no add consumes, so contraction leaves them as
-// FP64 multiplies) may go to the integer pipe (kmul), by bit of
-// AMRS_WGRAD_IMUL: 0 g^2 and the q_k, 1 the c_k q_k^2, 2 e0 q0, D P and r P,
-// 3 the weights and w_k / e_k, 4 the v_k scalings, 5 the ebar_k, 6 the
-// beta-gradient terms, 7 the w_k / 6.
-#ifndef AMRS_WGRAD_IMUL
-#define AMRS_WGRAD_IMUL 0xD0
-#endif
-template <int M = AMRS_WGRAD_IMUL>
-__device__ __forceinline__ void weno5js_grad(const double s[5], double gr[5], double* Wout = nullptr) {
-  constexpr bool M0 = M & 1, M1 = (M >> 1) & 1, M2 = (M >> 2) & 1, M3 = (M >> 3) & 1, M4 = (M >> 4) & 1,
-                 M5 = (M >> 5) & 1, M6 = (M >> 6) & 1, M7 = (M >> 7) & 1;
+//
+// Everything is a function of the differences t_q = s_{q+1} - s_q: the smoothness
+// differences, and y_k = v_k/6 - s2 (y0 = d1/12 + d2/4, y1 = d3/12 - g/4,
+// y2 = d4/12 - d5/4), with W = s2 + sum_k w_k y_k because the weights sum to one.
+// The entries of the gradient then sum to one as well, which gives the middle
+// one.  (The reverse pass has no bit-exact counterpart.)
+struct WenoDiffs {
+  double d1, d2, d3, g, d4, d5;
+  __device__ __forceinline__ explicit WenoDiffs(const double t[4])
+      : d1(t[1] - t[0]), d2(2.0 * t[1] + d1), d3(t[2] - t[1]), g(-t[1] - t[2]), d4(t[3] - t[2]),
+        d5(-2.0 * t[2] + d4) {}
+};
+__device__ __forceinline__ void weno_grad_sums(double x0, double x1, double x2, double p1, double p2, double p3,
+                                               double p4, double p5, double p6, double gr[5]) {
+  gr[0] = (1.0 / 3.0) * x0 + (p1 + p2);
+  gr[1] = (-7.0 / 6.0) * x0 + ((-1.0 / 6.0) * x1 + (-2.0 * p1 + (-4.0 * p2 + (p3 + p4))));
+  gr[3] = (1.0 / 3.0) * x1 + ((5.0 / 6.0) * x2 + (-2.0 * p5 + (-4.0 * p6 + (p3 - p4))));
+  gr[4] = (-1.0 / 6.0) * x2 + (p5 + p6);
+  gr[2] = ((1.0 - gr[0]) - gr[4]) - (gr[1] + gr[3]);
+}
+
+// With the hardware's operations, out of line; Wy = W - s2.
+static __device__ __noinline__ void weno5js_grad_plain(const double* t, double* gr, double* Wy) {
   constexpr double eps = 1e-40;
-  const double d1 = s[0] - 2.0 * s[1] + s[2], d2 = s[0] - 4.0 * s[1] + 3.0 * s[2];
-  const double d3 = s[1] - 2.0 * s[2] + s[3], g = s[1] - s[3];
-  const double d4 = s[2] - 2.0 * s[3] + s[4], d5 = 3.0 * s[2] - 4.0 * s[3] + s[4];
-  const double g2 = kmul<M0>(g, g);
-  const double b0 = (13.0 / 12.0) * d1 * d1 + 0.25 * d2 * d2;
-  const double b1 = (13.0 / 12.0) * d3 * d3 + 0.25 * g2 * g2;
-  const double b2 = (13.0 / 12.0) * d4 * d4 + 0.25 * d5 * d5;
-  const double e0 = eps + b0, e1 = eps + b1, e2 = eps + b2;
-  const double q0 = kmul<M0>(e1, e2), q1 = kmul<M0>(e0, e2), q2 = kmul<M0>(e0, e1);
-  const double t0 = kmul<M1>(kmul<M1>(0.1, q0), q0), t1 = kmul<M1>(kmul<M1>(0.6, q1), q1),
-               t2 = kmul<M1>(kmul<M1>(0.3, q2), q2);
-  const double eq = kmul<M2>(e0, q0);
-  const double DP = kmul<M2>(t0 + t1 + t2, eq);
+  const WenoDiffs d(t);
+  const double g2 = d.g * d.g;
+  const double e0 = eps + ((13.0 / 12.0) * d.d1 * d.d1 + 0.25 * d.d2 * d.d2);
+  const double e1 = eps + ((13.0 / 12.0) * d.d3 * d.d3 + 0.25 * g2 * g2);
+  const double e2 = eps + ((13.0 / 12.0) * d.d4 * d.d4 + 0.25 * d.d5 * d.d5);
+  const double q0 = e1 * e2, q1 = e0 * e2, q2 = e0 * e1;
+  const double t0 = 0.1 * q0 * q0, t1 = 0.6 * q1 * q1, t2 = 0.3 * q2 * q2;
+  const double P = e0 * q0, DP = (t0 + t1 + t2) * P;
   double w0, w1, w2, we0, we1, we2;  // w_k and w_k / e_k
   if (DP > 1e-300 && DP < 1e300) {
-    const double r = ddiv_rn(1.0, DP), rP = kmul<M2>(r, eq);
-    w0 = kmul<M3>(t0, rP); w1 = kmul<M3>(t1, rP); w2 = kmul<M3>(t2, rP);
-    we0 = kmul<M3>(kmul<M3>(t0, q0), r); we1 = kmul<M3>(kmul<M3>(t1, q1), r); we2 = kmul<M3>(kmul<M3>(t2, q2), r);
+    const double r = 1.0 / DP, rP = r * P;
+    w0 = t0 * rP; w1 = t1 * rP; w2 = t2 * rP;
+    we0 = t0 * q0 * r; we1 = t1 * q1 * r; we2 = t2 * q2 * r;
   } else {
-    const double ie0 = ddiv_rn(1.0, e0), ie1 = ddiv_rn(1.0, e1), ie2 = ddiv_rn(1.0, e2);
-    const double a0 = 0.1 * ie0 * ie0, a1 = 0.6 * ie1 * ie1, a2 = 0.3 * ie2 * ie2;
-    const double iA = ddiv_rn(1.0, (a0 + a1 + a2));
+    const double i0 = 1.0 / e0, i1 = 1.0 / e1, i2 = 1.0 / e2;
+    const double a0 = 0.1 * i0 * i0, a1 = 0.6 * i1 * i1, a2 = 0.3 * i2 * i2;
+    const double iA = 1.0 / (a0 + a1 + a2);
     w0 = a0 * iA; w1 = a1 * iA; w2 = a2 * iA;
-    we0 = w0 * ie0; we1 = w1 * ie1; we2 = w2 * ie2;
+    we0 = w0 * i0; we1 = w1 * i1; we2 = w2 * i2;
   }
-  const double v0 = kmul<M4>(2.0 * s[0] - 7.0 * s[1] + 11.0 * s[2], 1.0 / 6.0);
-  const double v1 = kmul<M4>(-s[1] + 5.0 * s[2] + 2.0 * s[3], 1.0 / 6.0);
-  const double v2 = kmul<M4>(2.0 * s[2] + 5.0 * s[3] - s[4], 1.0 / 6.0);
-  const double W = w0 * v0 + w1 * v1 + w2 * v2;
-  if (Wout) *Wout = W;
-  const double eb0 = kmul<M5>(-2.0 * (v0 - W), we0);
-  const double eb1 = kmul<M5>(-2.0 * (v1 - W), we1);
-  const double eb2 = kmul<M5>(-2.0 * (v2 - W), we2);
-  // grad beta_k scaled by ebar_k
-  const double p1 = kmul<M6>(kmul<M6>(eb0, 13.0 / 6.0), d1), p2 = kmul<M6>(eb0 * 0.5, d2);
-  const double p3 = kmul<M6>(kmul<M6>(eb1, 13.0 / 6.0), d3), p4 = kmul<M6>(kmul<M6>(eb1, g2), g);
-  const double p5 = kmul<M6>(kmul<M6>(eb2, 13.0 / 6.0), d4), p6 = kmul<M6>(eb2 * 0.5, d5);
-  const double x0 = kmul<M7>(w0, 1.0 / 6.0), x1 = kmul<M7>(w1, 1.0 / 6.0), x2 = kmul<M7>(w2, 1.0 / 6.0);
-  gr[0] = 2.0 * x0 + p1 + p2;
-  gr[1] = -7.0 * x0 - x1 - 2.0 * p1 - 4.0 * p2 + p3 + p4;
-  gr[2] = 11.0 * x0 + 5.0 * x1 + 2.0 * x2 + p1 + 3.0 * p2 - 2.0 * p3 + p5 + 3.0 * p6;
-  gr[3] = 2.0 * x1 + 5.0 * x2 + p3 - p4 - 2.0 * p5 - 4.0 * p6;
-  gr[4] = -x2 + p5 + p6;
+  const double y0 = d.d1 * (1.0 / 12.0) + 0.25 * d.d2, y1 = d.d3 * (1.0 / 12.0) - 0.25 * d.g,
+               y2 = d.d4 * (1.0 / 12.0) - 0.25 * d.d5;
+  const double W = w0 * y0 + w1 * y1 + w2 * y2;
+  *Wy = W;
+  const double b0 = -2.0 * (y0 - W) * we0, b1 = -2.0 * (y1 - W) * we1, b2 = -2.0 * (y2 - W) * we2;
+  weno_grad_sums(w0, w1, w2, b0 * (13.0 / 6.0) * d.d1, b0 * 0.5 * d.d2, b1 * (13.0 / 6.0) * d.d3, b1 * g2 * d.g,
+                 b2 * (13.0 / 6.0) * d.d4, b2 * 0.5 * d.d5, gr);
+}
+
+// The same with its products and the division on the integer pipe (38 FP64
+// instructions are left of about 110): behind one range test per smoothness
+// difference and per y_k - Wy no product tests its own.  Differences are zero or
+// in [2^-100, 2^60), s1 - s3 below 2^35 (its fourth power enters e), so e lies in
+// [2^-133, 2^143) and D P in the normal range.  A zero difference or y_k - Wy gives
+// zero terms.  t: the four differences; Wy = W - s2.
+__device__ __forceinline__ void weno5js_grad(const double t[4], double gr[5], double& Wy) {
+  bool ok = true, slow;
+  const WenoDiffs d(t);
+  const DWords D1 = weno_diff(d.d1, ok), D2 = weno_diff(d.d2, ok), D3 = weno_diff(d.d3, ok), G = weno_diff(d.g, ok),
+               D4 = weno_diff(d.d4, ok), D5 = weno_diff(d.d5, ok);
+  ok = ok && (G.hi & 0x7FFFFFFFu) < (1058u << 20);
+  const bool z1 = is_zero(d.d1), z2 = is_zero(d.d2), z3 = is_zero(d.d3), zg = is_zero(d.g), z4 = is_zero(d.d4),
+             z5 = is_zero(d.d5);
+  auto term = [](DWords a, DWords b, bool zero) {
+    const DWords x = dmul_core(a, b);
+    return zero ? 0.0 : dfrom(x);
+  };
+  const DWords c1312{0x3FF15555u, 0x55555555u}, c112{0x3FB55555u, 0x55555555u};  // 13/12, 1/12
+  const DWords g2 = dmul_core(G, G);
+  const DWords e0 = weno_e(fma(0.25, dfrom(dmul_core(D2, D2)), dfrom(dmul_core(dmul_core(c1312, D1), D1))));
+  const DWords e1 = weno_e(fma(0.25, dfrom(dmul_core(g2, g2)), dfrom(dmul_core(dmul_core(c1312, D3), D3))));
+  const DWords e2 = weno_e(fma(0.25, dfrom(dmul_core(D5, D5)), dfrom(dmul_core(dmul_core(c1312, D4), D4))));
+  const DWords q0 = dmul_core(e1, e2), q1 = dmul_core(e0, e2), q2 = dmul_core(e0, e1);
+  const DWords t0 = dmul_core(dmul_core(DWords{0x3FB99999u, 0x9999999Au}, q0), q0);
+  const DWords t1 = dmul_core(dmul_core(DWords{0x3FE33333u, 0x33333333u}, q1), q1);
+  const DWords t2 = dmul_core(dmul_core(DWords{0x3FD33333u, 0x33333333u}, q2), q2);
+  const DWords P = dmul_core(e0, q0);
+  const DWords r = ddiv_core(DWords{0x3FF00000u, 0u}, dmul_core(dwords(dfrom(t0) + dfrom(t1) + dfrom(t2)), P), &slow);
+  ok = ok && !slow;
+  const DWords rP = dmul_core(r, P);
+  const double x0 = dfrom(dmul_core(t0, rP)), x1 = dfrom(dmul_core(t1, rP)), x2 = dfrom(dmul_core(t2, rP));
+  const double y0 = fma(0.25, d.d2, term(c112, D1, z1)), y1 = fma(-0.25, d.g, term(c112, D3, z3)),
+               y2 = fma(-0.25, d.d5, term(c112, D4, z4));
+  Wy = x0 * y0 + x1 * y1 + x2 * y2;
+  // b_k = w_k / e_k (y_k - Wy) = -ebar_k / 2; the terms ebar_k grad beta_k:
+  // p1 = -(13/3) b0 d1, p2 = -b0 d2, p4 = -2 b1 g^3, ...
+  const ZWords f0 = weno_fac(y0 - Wy, ok), f1 = weno_fac(y1 - Wy, ok), f2 = weno_fac(y2 - Wy, ok);
+  auto negated = [](DWords a) { return DWords{a.hi ^ 0x80000000u, a.lo}; };
+  const DWords b0 = negated(dmul_core(dmul_core(t0, dmul_core(q0, r)), f0.w));
+  const DWords b1 = negated(dmul_core(dmul_core(t1, dmul_core(q1, r)), f1.w));
+  const DWords b2 = negated(dmul_core(dmul_core(t2, dmul_core(q2, r)), f2.w));
+  const DWords c133{0x40115555u, 0x55555555u};  // 13/3
+  const DWords gb{b1.hi + (1u << 20), b1.lo};   // 2 b1
+  weno_grad_sums(x0, x1, x2, term(dmul_core(c133, b0), D1, f0.zero || z1), term(b0, D2, f0.zero || z2),
+                 term(dmul_core(c133, b1), D3, f1.zero || z3), term(dmul_core(gb, g2), G, f1.zero || zg),
+                 term(dmul_core(c133, b2), D4, f2.zero || z4), term(b2, D5, f2.zero || z5), gr);
+  if (!ok) {
+    double a[4], o[5], w;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) a[n] = t[n];
+    weno5js_grad_plain(a, o, &w);
+#pragma unroll
+    for (int n = 0; n < 5; ++n) gr[n] = o[n];
+    Wy = w;
+  }
 }
 
 }  // namespace amrs

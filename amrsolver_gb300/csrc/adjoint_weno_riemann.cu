@@ -17,11 +17,6 @@
 #include "amrs_kernels.h"
 #include "riemann_vjp.cuh"
 
-// Integer-pipe products of the WENO5 gradients here (see weno5js_grad).
-#ifndef AMRS_WRGRAD_IMUL
-#define AMRS_WRGRAD_IMUL 0x40
-#endif
-
 namespace amrs {
 
 namespace {
@@ -64,10 +59,12 @@ __global__ void __launch_bounds__(256, 3) wr_vjp_face_kernel(const __grid_consta
       double v[6];
 #pragma unroll
       for (int s = 0; s < 6; ++s) v[s] = q.p[o + (s - 3) * sq + comp[m] * q.ns];
-      const double sl[5] = {v[0], v[1], v[2], v[3], v[4]};
-      const double sr[5] = {v[5], v[4], v[3], v[2], v[1]};
-      weno5js_grad<AMRS_WRGRAD_IMUL>(sl, gl[m], &lraw[m]);
-      weno5js_grad<AMRS_WRGRAD_IMUL>(sr, gr[m], &rraw[m]);
+      const double tl[4] = {v[1] - v[0], v[2] - v[1], v[3] - v[2], v[4] - v[3]};
+      const double tr[4] = {v[4] - v[5], -tl[3], -tl[2], -tl[1]};
+      weno5js_grad(tl, gl[m], lraw[m]);
+      weno5js_grad(tr, gr[m], rraw[m]);
+      lraw[m] += v[2];
+      rraw[m] += v[3];
     }
     in[0] = (lraw[0] < 1.0e-40) ? 1.0e-40 : lraw[0];
     in[1] = lraw[1];

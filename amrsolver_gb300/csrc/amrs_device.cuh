@@ -144,6 +144,12 @@ __device__ __forceinline__ bool is_zero(double x) {
   const DWords w = dwords(x);
   return ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
 }
+// 0.5 x for a zero or normal x well above the smallest
+__device__ __forceinline__ double half_of(double x) {
+  const DWords w = dwords(x);
+  return dfrom(((w.hi & 0x7FFFFFFFu) | w.lo) == 0u ? w.hi : w.hi - (1u << 20), w.lo);
+}
+
 // a * b on the integer pipe without range tests, +-0 where `zero`.
 __device__ __forceinline__ double mul_core(double a, double b) { return dfrom(dmul_core(dwords(a), dwords(b))); }
 __device__ __forceinline__ double mul_zero(double a, double b, bool zero) {

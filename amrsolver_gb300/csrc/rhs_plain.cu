@@ -17,6 +17,7 @@
 // exact arithmetic, a quarter of the divisions, rounding differences only.
 #include "amrs_kernels.h"
 #include "ddiv.cuh"
+#include "weno_int.cuh"
 
 namespace amrs {
 
@@ -228,42 +229,7 @@ __device__ __forceinline__ double weno5js(const double s0, const double s1, cons
 // below half its last place) and eps below 2^-187 (the other way round); in
 // between the hardware adds them out of line.
 
-// A smoothness difference.
-__device__ __forceinline__ DWords weno_diff(double x, bool& ok) {
-  DWords w = dwords(x);
-  const bool zero = ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
-  ok = ok && (zero || w.hi * 2u - (923u << 21) < (160u << 21));
-  w.hi = zero ? (823u << 20) : w.hi;
-  return w;
-}
-static __device__ __noinline__ double dadd_hw(double a, double b) { return a + b; }
-// (eps + beta)^2
-__device__ __forceinline__ DWords weno_e2(double beta) {
-  DWords w = dwords(beta);
-  const bool big = w.hi >= (945u << 20), tiny = w.hi < (836u << 20);
-  if (!big) {
-    w = DWords{0x37A16C26u, 0x2777579Cu};  // 1e-40
-    if (!tiny) w = dwords(dadd_hw(1e-40, beta));
-  }
-  return dmul_core(w, w);
-}
-// A factor that may be zero: its words, and whether it is.
-struct ZWords {
-  DWords w;
-  bool zero;
-};
-__device__ __forceinline__ ZWords weno_fac(double x, bool& ok) {
-  ZWords z;
-  z.w = dwords(x);
-  z.zero = ((z.w.hi & 0x7FFFFFFFu) | z.w.lo) == 0u;
-  ok = ok && (z.zero || mid_range(z.w.hi));
-  return z;
-}
-// a * x for a nonzero a of the middle range.
-__device__ __forceinline__ double weno_mul(DWords a, const ZWords& x) {
-  const DWords r = dmul_core(a, x.w);
-  return dfrom(x.zero ? ((a.hi ^ x.w.hi) & 0x80000000u) : r.hi, x.zero ? 0u : r.lo);
-}
+__device__ __forceinline__ DWords weno_sq(DWords e) { return dmul_core(e, e); }
 
 __device__ __forceinline__ double weno5js_int(const double s0, const double s1, const double s2, const double s3,
                                               const double s4, bool& ok) {
@@ -273,14 +239,14 @@ __device__ __forceinline__ double weno5js_int(const double s0, const double s1, 
   const double s2x3 = weno_mul(DWords{0x40080000u, 0u}, z2);
   const DWords a = weno_diff(fma(-2.0, s1, s0) + s2, ok), b = weno_diff(fma(-4.0, s1, s0) + s2x3, ok);
   const double beta0 = fma(0.25, dfrom(dmul_core(b, b)), dfrom(dmul_core(dmul_core(c1312, a), a)));
-  const DWords alpha0 = ddiv_core(DWords{0x3FB99999u, 0x9999999Au}, weno_e2(beta0), &slow0);
+  const DWords alpha0 = ddiv_core(DWords{0x3FB99999u, 0x9999999Au}, weno_sq(weno_e(beta0)), &slow0);
   const DWords c = weno_diff(fma(-2.0, s2, s1) + s3, ok), g = weno_diff(s1 - s3, ok);
   const double beta1 = fma(0.25, dfrom(dmul_core(dmul_core(dmul_core(g, g), g), g)),
                            dfrom(dmul_core(dmul_core(c1312, c), c)));
-  const DWords alpha1 = ddiv_core(DWords{0x3FE33333u, 0x33333333u}, weno_e2(beta1), &slow1);
+  const DWords alpha1 = ddiv_core(DWords{0x3FE33333u, 0x33333333u}, weno_sq(weno_e(beta1)), &slow1);
   const DWords d = weno_diff(fma(-2.0, s3, s2) + s4, ok), f = weno_diff(fma(-4.0, s3, s2x3) + s4, ok);
   const double beta2 = fma(0.25, dfrom(dmul_core(f, f)), dfrom(dmul_core(dmul_core(c1312, d), d)));
-  const DWords alpha2 = ddiv_core(DWords{0x3FD33333u, 0x33333333u}, weno_e2(beta2), &slow2);
+  const DWords alpha2 = ddiv_core(DWords{0x3FD33333u, 0x33333333u}, weno_sq(weno_e(beta2)), &slow2);
   const DWords sum = ddiv_core(DWords{0x3FF00000u, 0u}, dwords(dfrom(alpha0) + dfrom(alpha1) + dfrom(alpha2)), &slow3);
   const ZWords z1 = weno_fac(s1, ok), z3 = weno_fac(s3, ok);
   const DWords c5{0x40140000u, 0u};
@@ -540,12 +506,6 @@ static __device__ __noinline__ void slope_plain(const SlopeQ& q, double gR, doub
     o[SL_AL] = s02 / csl + d1;
     o[SL_CL] = s02 * csl;
   }
-}
-
-// 0.5 x for a zero or normal x well above the smallest
-__device__ __forceinline__ double half_of(double x) {
-  const DWords w = dwords(x);
-  return dfrom(((w.hi & 0x7FFFFFFFu) | w.lo) == 0u ? w.hi : w.hi - (1u << 20), w.lo);
 }
 
 // The same bits on the integer pipe where the ranges hold.  c0 >= 2^-78 makes
