@@ -114,7 +114,8 @@ cudaError_t launch_source_vjp(const BoxRec& R, const double force[3], const DArr
                               cudaStream_t st);
 cudaError_t launch_adj_prog(const BoxRec& R, const DProg& prog, const DArr& wbar, const DArr& s1bar, const DArr& inbar,
                             const DArr& vbar, int accumulate, int nsm, cudaStream_t st);
-cudaError_t launch_adj_halo(const HaloBox& hb, int nsm, cudaStream_t st);
+// ghost fold in place, or (to) added to another array's valid cells
+cudaError_t launch_adj_halo(const HaloBox& hb, const DArr* to, int nsm, cudaStream_t st);
 cudaError_t launch_halo_list(const BoxTable& tb, const long long* gpre, const long long* vpre, long long ghosts,
                              int slot, const int bc_lo[3], const int bc_hi[3], int nsm, cudaStream_t st);
 // Device state of a time loop over a box list (amrs_rk_run_boxlist); the

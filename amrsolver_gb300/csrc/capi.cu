@@ -1484,7 +1484,6 @@ amrs_status adj_prepare(amrs_handle* h, const amrs_box& B, AdjScratch& S, cudaSt
   S.wbuf = reinterpret_cast<double*>(P + o_w);
   S.jbuf = reinterpret_cast<double*>(P + o_j);  // WENO or MUSCL per-face / per-cell slots
   S.ah.part = reinterpret_cast<double*>(P + o_part);
-  if (H > 0) CK(cudaMemsetAsync(P + o_pair, 0, cells(3) * 12 * 8 * 3 * H, st));
   return AMRS_OK;
 }
 
@@ -1574,7 +1573,7 @@ amrs_status amrs_fill_halo_box_adjoint(const amrs_box* domain, const int32_t bc_
   int dev = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  CK(launch_adj_halo(hb, nsm, static_cast<cudaStream_t>(stream)));
+  CK(launch_adj_halo(hb, nullptr, nsm, static_cast<cudaStream_t>(stream)));
   return AMRS_OK;
 }
 
@@ -1620,9 +1619,7 @@ amrs_status amrs_rk_stage_vjp_box(amrs_handle* h, const amrs_box* bx, const doub
     S.ah.ubar = S.ubar_tmp;
     e = rhs_vjp_launch(h, *h->one, *bx, S, param_bar, st);
   }
-  // 3. ghost fold (adjoint of FillPatch), then inbar += valid(ubar): the
-  //    reverse kernel with an empty program routes its input cotangent into
-  //    the stage-input cotangent (vbar_tmp is free here)
+  // 3. inbar += ghost fold (adjoint of FillPatch) of ubar
   if (e == cudaSuccess) {
     HaloBox hb;
     hb.u = S.ubar_tmp;
@@ -1630,12 +1627,8 @@ amrs_status amrs_rk_stage_vjp_box(amrs_handle* h, const amrs_box* bx, const doub
     for (int d = 0; d < 3; ++d) {
       hb.lo[d] = bx->lo[d]; hb.hi[d] = bx->hi[d]; hb.bc_lo[d] = bc_lo[d]; hb.bc_hi[d] = bc_hi[d];
     }
-    e = launch_adj_halo(hb, h->nsm, st);
-  }
-  if (e == cudaSuccess) {
-    amrs_stage_prog ident{};
-    ident.nops = 0;
-    e = launch_adj_prog(R, to_dprog(&ident), S.ubar_tmp, S.vbar_tmp, to_darr(inbar), S.vbar_tmp, 1, h->nsm, st);
+    const DArr to = to_darr(inbar);
+    e = launch_adj_halo(hb, &to, h->nsm, st);
   }
   if (e != cudaSuccess) return cuda_fail(e, "amrs_rk_stage_vjp_box");
   return AMRS_OK;
