@@ -14,7 +14,8 @@
 // thread, fixed summation order: deterministic):
 //   muscl_vjp_face_kernel : Fbar = dxinv_d (vbar(f) - vbar(f-1)); the
 //       riemann_prob reverse gives the cotangents of the ten state inputs,
-//       then of both cells' primitives and face-state terms (20 slots).
+//       which are those of both cells' primitives and, halved, of their
+//       face-state terms (10 slots).
 //   muscl_vjp_slope_kernel: per cell, the term cotangents of its two faces
 //       through A, B, C, the MC limiters and the characteristic differences
 //       to primitive cotangents at c-1, c, c+1 (and T at c+2 for z), plus the
@@ -35,8 +36,8 @@ namespace {
 using rpvjp::riemann_prob_vjp;
 using rpvjp::sgn1;
 
-constexpr int FSLOT = 20;  // per face: left prims (5), left terms (5), right prims (5), right terms (5)
-constexpr int SSLOT = 19;  // per cell: Qbar at c-1 (6), c (6), c+1 (6), T at c+2 (1, z only)
+constexpr int FSLOT = 10;  // per face: left prims (5), right prims (5); the terms' are +-1/2 of them
+constexpr int SSLOT = 19;  // per cell: Qbar at c-1 (6, T unused), c (6), c+1 (6, T unused), T at c+2 (1, z only)
 
 __device__ __forceinline__ double vget0(const DArr& v, const BoxRec& R, int i, int j, int k, int n) {
   if (i < R.lo[0] || i > R.hi[0] || j < R.lo[1] || j > R.hi[1] || k < R.lo[2] || k > R.hi[2]) return 0.0;
@@ -55,16 +56,11 @@ struct SBuf {
   int mx, my;
 };
 
-// Resident CTAs per SM asked of the slope and gather reverse kernels.
-#ifndef AMRS_MVJP_CTAS
-#define AMRS_MVJP_CTAS 4
-#endif
-
-// Two CTAs per SM (128 registers): the reverse solver is a long dependent
-// chain per face, and 16 warps hide its latency better than 8 with all the
-// registers it would otherwise take (measured: 7.97 against 8.97 ms per
-// SSPRK3 step VJP at 64^3).
-__global__ void __launch_bounds__(256, 2) muscl_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FBuf fs, int d,
+// Three CTAs per SM (80 registers, some spilled): the reverse solver is a long
+// dependent chain per face, and 24 warps hide its latency better than 16 with the
+// registers they would otherwise take (gradient of an SSPRK3 step at 48^3: 2510
+// against 2640 us; at 72^3 7509 against 7574).
+__global__ void __launch_bounds__(256, 3) muscl_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FBuf fs, int d,
                                                              long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
@@ -110,13 +106,9 @@ __global__ void __launch_bounds__(256, 2) muscl_vjp_face_kernel(const __grid_con
     const double rrb = (xrr < 1.0e-40) ? 0.0 : ib[5], prb = (xpr < 1.0e-40) ? 0.0 : ib[7];
     double* o = fs.p + g;
     const long long s = fs.nf;
-    // left cell: prims (rho, u_n, p, u_t1, u_t2), terms (A, B, C, d3, d4)
+    // prims (rho, u_n, p, u_t1, u_t2) of the left and of the right cell
     o[0 * s] = rlb; o[1 * s] = ib[1]; o[2 * s] = plb; o[3 * s] = ib[3]; o[4 * s] = ib[4];
-    o[5 * s] = 0.5 * rlb; o[6 * s] = 0.5 * ib[1]; o[7 * s] = 0.5 * plb; o[8 * s] = 0.5 * ib[3]; o[9 * s] = 0.5 * ib[4];
-    // right cell
-    o[10 * s] = rrb; o[11 * s] = ib[6]; o[12 * s] = prb; o[13 * s] = ib[8]; o[14 * s] = ib[9];
-    o[15 * s] = -0.5 * rrb; o[16 * s] = -0.5 * ib[6]; o[17 * s] = -0.5 * prb; o[18 * s] = -0.5 * ib[8];
-    o[19 * s] = -0.5 * ib[9];
+    o[5 * s] = rrb; o[6 * s] = ib[6]; o[7 * s] = prb; o[8 * s] = ib[8]; o[9 * s] = ib[9];
   }
 }
 
@@ -143,8 +135,11 @@ __device__ __forceinline__ void mc_vjp(double l, double r, double db, double& lb
   }
 }
 
-__global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, FBuf fs, SBuf ss, int d,
-                                                              long long total) {
+// Two, three or four CTAs per SM take the same time (2625, 2616, 2619 us for the
+// gradient of a step at 48^3).
+template <int d>
+__global__ void __launch_bounds__(256, 3) muscl_vjp_slope_kernel(const __grid_constant__ BoxTable tb,
+                                                                               FBuf fs, SBuf ss, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DArr q = R.q;
@@ -162,7 +157,7 @@ __global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(co
     const long long o = q.off(i, j, k);
     auto Q = [&](long long off, int n) { return q.p[off + n * q.ns]; };
     // forward recompute (slope_kernel)
-    const double c0 = sqrt(gR * Q(o, QT));
+    const double c0 = dsqrt_rn(gR * Q(o, QT));
     const double cs = c0 + (d == 0 ? 2.e-40 : 1.e-40);
     const double csr = c0 + 1.e-40;
     const double rc = Q(o, QRHO);
@@ -186,28 +181,28 @@ __global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(co
     };
     const double d0 = mc(l0, r0), d2 = mc(l2, r2);
     const double s02 = d0 + d2;
-    // term cotangents from the two faces of this cell
-    double Ab = 0.0, Bb = 0.0, Cb = 0.0, d3b = 0.0, d4b = 0.0, ALb = 0.0, CLb = 0.0;
-    double qb0[NQA] = {0, 0, 0, 0, 0, 0};  // direct prim cotangents at c
+    // the cotangents of the two faces' states at this cell: the primitives', and
+    // through q + terms/2 (face c+1), q - terms/2 (face c) the terms'
+    double fr5[5] = {0, 0, 0, 0, 0}, fl5[5] = {0, 0, 0, 0, 0};
     auto fidx = [&](int fi, int fj, int fk) {
       return (long long)(fi - R.lo[0]) + (long long)fs.nx * ((fj - R.lo[1]) + (long long)fs.ny * (fk - R.lo[2]));
     };
     if (c >= R.lo[d]) {  // right role at face c
       const double* f = fs.p + fidx(i, j, k);
-      const long long n = fs.nf;
-      qb0[QRHO] += f[10 * n]; qb0[QN] += f[11 * n]; qb0[QPRES] += f[12 * n]; qb0[QT1] += f[13 * n];
-      qb0[QT2] += f[14 * n];
-      Ab += f[15 * n]; Bb += f[16 * n]; Cb += f[17 * n]; d3b += f[18 * n]; d4b += f[19 * n];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) fr5[n] = f[(5 + n) * fs.nf];
     }
     if (c <= R.hi[d]) {  // left role at face c+1
       const double* f = fs.p + fidx(i + di, j + dj, k + dk);
-      const long long n = fs.nf;
-      qb0[QRHO] += f[0 * n]; qb0[QN] += f[1 * n]; qb0[QPRES] += f[2 * n]; qb0[QT1] += f[3 * n];
-      qb0[QT2] += f[4 * n];
-      if (d == 2) { ALb += f[5 * n]; CLb += f[7 * n]; }
-      else { Ab += f[5 * n]; Cb += f[7 * n]; }
-      Bb += f[6 * n]; d3b += f[8 * n]; d4b += f[9 * n];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) fl5[n] = f[n * fs.nf];
     }
+    double qb0[NQA] = {0, 0, 0, 0, 0, 0};  // direct prim cotangents at c
+    qb0[QRHO] = fr5[0] + fl5[0]; qb0[QN] = fr5[1] + fl5[1]; qb0[QPRES] = fr5[2] + fl5[2];
+    qb0[QT1] = fr5[3] + fl5[3]; qb0[QT2] = fr5[4] + fl5[4];
+    const double Bb = 0.5 * (fl5[1] - fr5[1]), d3b = 0.5 * (fl5[3] - fr5[3]), d4b = 0.5 * (fl5[4] - fr5[4]);
+    double Ab = -0.5 * fr5[0], Cb = -0.5 * fr5[2], ALb = 0.5 * fl5[0], CLb = 0.5 * fl5[2];
+    if (d != 2) { Ab += ALb; Cb += CLb; ALb = 0.0; CLb = 0.0; }
     // A = s02/csr + d1, B = (d2 - d0)/rho, C = s02*csr (z: A_L, C_L with csl).
     // The cotangents use reciprocals: the reverse pass has no bit-exact
     // counterpart (its bar is agreement with forward-mode derivatives), and
@@ -221,7 +216,7 @@ __global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(co
     double rcb = -Bb * ((d2 - d0) * irc) * irc;
     double csl = 0.0, c0l = 0.0, cslb = 0.0;
     if (d == 2 && c <= R.hi[2]) {
-      c0l = sqrt(gR * Q(o + 2 * s, QT));
+      c0l = dsqrt_rn(gR * Q(o + 2 * s, QT));
       csl = c0l + 1.e-40;
       const double icsl = ddiv_rn(1.0, csl);
       s02b += ALb * icsl + CLb * csl;
@@ -262,15 +257,15 @@ __global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_slope_kernel(co
     const long long n = ss.nc;
 #pragma unroll
     for (int m = 0; m < NQA; ++m) {
-      w[m * n] = qm[m];
+      if (m != QT) w[m * n] = qm[m];
       w[(NQA + m) * n] = qz[m];
-      w[(2 * NQA + m) * n] = qp[m];
+      if (m != QT) w[(2 * NQA + m) * n] = qp[m];
     }
-    w[(3 * NQA) * n] = (d == 2 && c <= R.hi[2] && c0l > 0.0) ? ddiv_rn(cslb * gR, (2.0 * c0l)) : 0.0;
+    if (d == 2) w[(3 * NQA) * n] = (c <= R.hi[2] && c0l > 0.0) ? ddiv_rn(cslb * gR, (2.0 * c0l)) : 0.0;
   }
 }
 
-__global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, SBuf s0, SBuf s1, SBuf s2,
+__global__ void __launch_bounds__(256, 4) muscl_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, SBuf s0, SBuf s1, SBuf s2,
                                                                long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
@@ -305,7 +300,8 @@ __global__ void __launch_bounds__(256, AMRS_MVJP_CTAS) muscl_vjp_gather_kernel(c
         const double* p = S.p + sidx(x);
         const int base = (off + 1) * NQA;
 #pragma unroll
-        for (int n = 0; n < NQA; ++n) qb[n] += p[(base + n) * S.nc];
+        for (int n = 0; n < NQA; ++n)
+          if (off == 0 || n != QT) qb[n] += p[(base + n) * S.nc];  // T only at c itself
       }
       if (d == 2) {
         int x[3] = {c[0], c[1], c[2] - 2};
@@ -366,7 +362,10 @@ cudaError_t launch_muscl_vjp(const BoxTable& tb, const FaceRec& fr, const DArr& 
     fb.nx = n[0] + (d == 0);
     fb.ny = n[1] + (d == 1);
     launch_dep(muscl_vjp_face_kernel, grid_m(fb.nf, nsm), 256, 0, st, tb, fr, vbar, fb, d, fb.nf);
-    launch_dep(muscl_vjp_slope_kernel, grid_m(sb[d].nc, nsm), 256, 0, st, tb, fr, fb, sb[d], d, sb[d].nc);
+    const int gs = grid_m(sb[d].nc, nsm);
+    if (d == 0) launch_dep(muscl_vjp_slope_kernel<0>, gs, 256, 0, st, tb, fb, sb[d], sb[d].nc);
+    else if (d == 1) launch_dep(muscl_vjp_slope_kernel<1>, gs, 256, 0, st, tb, fb, sb[d], sb[d].nc);
+    else launch_dep(muscl_vjp_slope_kernel<2>, gs, 256, 0, st, tb, fb, sb[d], sb[d].nc);
   }
   const long long tot = (long long)(n[0] + 4) * (n[1] + 4) * (n[2] + 4);
   launch_dep(muscl_vjp_gather_kernel, grid_m(tot, nsm), 256, 0, st, tb, ubar, sb[0], sb[1], sb[2], tot);

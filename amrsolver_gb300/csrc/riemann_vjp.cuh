@@ -3,6 +3,11 @@
 // checked on the CPU against the oracle's dual numbers.  Non-smooth points
 // follow the forward's branch (max, |.|, the state selection); the
 // weak-wave switch of the iteration carries no derivative.
+//
+// Bound on the device: the FP64 pipe (two thirds busy, the rest dependent chains).
+// Roots, quotients and the products no addition consumes run on the integer pipe,
+// and the reverse iterations take wave speeds, denominators and branches from the
+// forward ones instead of repeating six roots and nine quotients.
 #pragma once
 #include <cmath>
 
@@ -19,16 +24,8 @@ namespace rpvjp {
 
 using std::copysign;
 using std::fabs;
-using std::sqrt;
 
 AMRS_HD double sgn1(double x) { return x < 0.0 ? -1.0 : 1.0; }  // d|x|/dx as fabs's branch
-
-// Square roots of the reverse solver: integer-pipe (dsqrt_rn) or hardware,
-// the same correctly rounded value.
-#ifndef AMRS_RV_ISQRT
-#define AMRS_RV_ISQRT 0
-#endif
-AMRS_HD double rvsqrt(double x) { return AMRS_RV_ISQRT ? dsqrt_rn(x) : sqrt(x); }
 
 // One iteration of riemann_prob's pressure update (src/rhs/Riemann.h:163-189)
 // and its reverse.  State (P = pstar, Pm = pstnm1, UM = ustarm, UP = ustarp).
@@ -36,21 +33,36 @@ struct RPPar {
   double pl, pr, ul, ur, rl, rr, hg, cleft, cright, ccs, smallp;
 };
 
+// What the reverse of an iteration takes from its forward pass: the reciprocal
+// wave speeds, the secant's denominator and which branches were taken.
+struct RPIter {
+  double wl, wr, den;
+  unsigned br;
+};
+enum { RP_ZP = 1, RP_ZM = 2, RP_CCS = 4, RP_FLOOR = 8 };
+
 AMRS_HD void rp_iter_fwd(const RPPar& q, double P, double Pm, double UM, double UP, double& Pn,
-                                            double& UMn, double& UPn) {
-  const double wl = ddiv_rn(1., rvsqrt((q.hg * (P + q.pl) + P) * q.rl));
-  const double wr = ddiv_rn(1., rvsqrt((q.hg * (P + q.pr) + P) * q.rr));
+                                            double& UMn, double& UPn, RPIter& r) {
+  const double wl = ddiv_rn(1., dsqrt_rn(dmul_rn(q.hg * (P + q.pl) + P, q.rl)));
+  const double wr = ddiv_rn(1., dsqrt_rn(dmul_rn(q.hg * (P + q.pr) + P, q.rr)));
   UMn = q.ur - (q.pr - P) * wr;
   UPn = q.ul + (q.pl - P) * wl;
   const double dpd = fabs(Pm - P);
+  unsigned br = 0u;
   double zp = fabs(UPn - UP);
-  if (zp - 1.e-3 * q.cleft < 0.0) zp = dpd * wl;
+  if (zp - 1.e-3 * q.cleft < 0.0) { zp = dmul_rn(dpd, wl); br |= RP_ZP; }
   double zm = fabs(UMn - UM);
-  if (zm - 1.e-3 * q.cright < 0.0) zm = dpd * wr;
+  if (zm - 1.e-3 * q.cright < 0.0) { zm = dmul_rn(dpd, wr); br |= RP_ZM; }
   const double zz = zp + zm;
-  const double denom = ddiv_rn(dpd, ((zz < q.ccs) ? q.ccs : zz));
+  const bool small = zz < q.ccs;
+  r.den = small ? q.ccs : zz;
+  const double denom = ddiv_rn(dpd, r.den);
   const double pn = P - denom * (UMn - UPn);
-  Pn = (pn < q.smallp) ? q.smallp : pn;
+  const bool low = pn < q.smallp;
+  Pn = low ? q.smallp : pn;
+  r.wl = wl;
+  r.wr = wr;
+  r.br = br | (small ? RP_CCS : 0u) | (low ? RP_FLOOR : 0u);
 }
 
 // Given the cotangents of the iteration's outputs (Pn, Pm' = P, UMn, UPn),
@@ -58,38 +70,24 @@ AMRS_HD void rp_iter_fwd(const RPPar& q, double P, double Pm, double UM, double 
 struct RPBar {
   double pl, pr, ul, ur, rl, rr, ccs;
 };
-AMRS_HD void rp_iter_vjp(const RPPar& q, double P, double Pm, double UM, double UP, double Pnb,
-                                            double Pmnb, double UMnb, double UPnb, double& Pb, double& Pmb,
-                                            double& UMb, double& UPb, RPBar& g) {
-  const double al = q.hg * (P + q.pl) + P, ar = q.hg * (P + q.pr) + P;
-  const double sl = rvsqrt(al * q.rl), sr = rvsqrt(ar * q.rr);
-  const double wl = ddiv_rn(1., sl), wr = ddiv_rn(1., sr);
-  const double UMn = q.ur - (q.pr - P) * wr;
-  const double UPn = q.ul + (q.pl - P) * wl;
+AMRS_HD void rp_iter_vjp(const RPPar& q, const RPIter& r, double P, double Pm, double UM, double UP, double UMn,
+                         double UPn, double Pnb, double Pmnb, double UMnb, double UPnb, double& Pb, double& Pmb,
+                         double& UMb, double& UPb, RPBar& g) {
+  const double wl = r.wl, wr = r.wr;
   const double draw = Pm - P, dpd = fabs(draw);
-  const double zpr = UPn - UP, zp0 = fabs(zpr);
-  const bool bp = zp0 - 1.e-3 * q.cleft < 0.0;
-  const double zp = bp ? dpd * wl : zp0;
-  const double zmr = UMn - UM, zm0 = fabs(zmr);
-  const bool bm = zm0 - 1.e-3 * q.cright < 0.0;
-  const double zm = bm ? dpd * wr : zm0;
-  const double zz = zp + zm;
-  const bool bz = zz < q.ccs;
-  const double den = bz ? q.ccs : zz;
-  const double denom = ddiv_rn(dpd, den);
-  const double pn = P - denom * (UMn - UPn);
-  const bool bpn = pn < q.smallp;
+  const double zpr = UPn - UP, zmr = UMn - UM;
+  const bool bp = r.br & RP_ZP, bm = r.br & RP_ZM, bz = r.br & RP_CCS, bpn = r.br & RP_FLOOR;
+  const double iden = ddiv_rn(1.0, r.den), denom = dmul_rn(dpd, iden);
   // reverse
   double Pbar = Pmnb;  // P is also the next pstnm1
   double UMnbar = UMnb, UPnbar = UPnb, wlb = 0.0, wrb = 0.0, dpdb = 0.0;
   const double pnb = bpn ? 0.0 : Pnb;
   Pbar += pnb;
-  const double denomb = -pnb * (UMn - UPn);
+  const double denomb = dmul_rn(-pnb, UMn - UPn);
   UMnbar += -pnb * denom;
   UPnbar += pnb * denom;
-  const double iden = ddiv_rn(1.0, den);
   dpdb += denomb * iden;
-  const double denb = -denomb * denom * iden;
+  const double denb = dmul_rn(dmul_rn(-denomb, denom), iden);
   if (bz) g.ccs += denb;
   const double zzb = bz ? 0.0 : denb;
   if (bp) { dpdb += zzb * wl; wlb += zzb * dpd; }
@@ -108,13 +106,13 @@ AMRS_HD void rp_iter_vjp(const RPPar& q, double P, double Pm, double UM, double 
   g.pl += UPnbar * wl;
   Pbar -= UPnbar * wl;
   wlb += UPnbar * (q.pl - P);
-  // w = 1/rvsqrt(a r), a = hg (P + p) + P; d sqrt(x)/dx = 1/(2 sqrt(x)) = w/2
-  const double slb = -wlb * wl * wl, srb = -wrb * wr * wr;
-  const double wlsqb = 0.5 * slb * wl, wrsqb = 0.5 * srb * wr;
-  g.rl += wlsqb * al;
-  g.rr += wrsqb * ar;
-  const double alb = wlsqb * q.rl, arb = wrsqb * q.rr;
-  Pbar += alb * (q.hg + 1.0) + arb * (q.hg + 1.0);
+  // w = 1/sqrt(a r), a = hg (P + p) + P; d sqrt(x)/dx = 1/(2 sqrt(x)) = w/2
+  const double wlsqb = dmul_rn(dmul_rn(dmul_rn(-0.5 * wlb, wl), wl), wl),
+               wrsqb = dmul_rn(dmul_rn(dmul_rn(-0.5 * wrb, wr), wr), wr);
+  g.rl += wlsqb * (q.hg * (P + q.pl) + P);
+  g.rr += wrsqb * (q.hg * (P + q.pr) + P);
+  const double alb = dmul_rn(wlsqb, q.rl), arb = dmul_rn(wrsqb, q.rr);
+  Pbar += (alb + arb) * (q.hg + 1.0);
   g.pl += alb * q.hg;
   g.pr += arb * q.hg;
   Pb += Pbar;
@@ -130,8 +128,8 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   const double small = 1.e-6;
   const double hg = 0.5 * (gamma - 1.);
   // ---- forward
-  const double clsql = gamma * pl * rl, clsqr = gamma * pr * rr;
-  const double wl0 = rvsqrt(clsql), wr0 = rvsqrt(clsqr);
+  const double clsql = dmul_rn(dmul_rn(gamma, pl), rl), clsqr = dmul_rn(dmul_rn(gamma, pr), rr);
+  const double wl0 = dsqrt_rn(clsql), wr0 = dsqrt_rn(clsqr);
   const double cleft = ddiv_rn(wl0, rl), cright = ddiv_rn(wr0, rr);
   const double ccs = small * (cleft + cright);
   const double dU = ur - ul;
@@ -140,7 +138,7 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   const bool m0 = !(ps0 < smallp);
   const double p0 = m0 ? ps0 : smallp;
   const double a1l = hg * (p0 + pl) + p0, a1r = hg * (p0 + pr) + p0;
-  const double wl1 = rvsqrt(a1l * rl), wr1 = rvsqrt(a1r * rr);
+  const double wl1 = dsqrt_rn(dmul_rn(a1l, rl)), wr1 = dsqrt_rn(dmul_rn(a1r, rr));
   const double usp0 = ul - ddiv_rn((p0 - pl), wl1);
   const double usm0 = ur + ddiv_rn((p0 - pr), wr1);
   const double D1 = wl1 + wr1;
@@ -149,10 +147,11 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   const double p1 = m1 ? ps1 : smallp;
   const RPPar q{pl, pr, ul, ur, rl, rr, hg, cleft, cright, ccs, smallp};
   double P[4], Pm[4], UM[4], UP[4];
+  RPIter ri[3];
   P[0] = p1; Pm[0] = p0; UM[0] = usm0; UP[0] = usp0;
 #pragma unroll
   for (int it = 0; it < 3; ++it) {
-    rp_iter_fwd(q, P[it], Pm[it], UM[it], UP[it], P[it + 1], UM[it + 1], UP[it + 1]);
+    rp_iter_fwd(q, P[it], Pm[it], UM[it], UP[it], P[it + 1], UM[it + 1], UP[it + 1], ri[it]);
     Pm[it + 1] = P[it];
   }
   const double pstar = P[3], ustar = 0.5 * (UM[3] + UP[3]);
@@ -166,21 +165,21 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
     utr1 = 0.5 * (ut1l + ut1r); utr2 = 0.5 * (ut2l + ut2r);
   }
   const double aw = hg * (pstar + po) + pstar;
-  const double wosq = aw * ro;
+  const double wosq = dmul_rn(aw, ro);
   const double dpjmp = pstar - po;
-  const double tt = ro * dpjmp, uu = ddiv_rn(tt, wosq), dd = 1. - uu;
+  const double tt = dmul_rn(ro, dpjmp), uu = ddiv_rn(tt, wosq), dd = 1. - uu;
   const double rstar = ddiv_rn(ro, dd);
-  const double suo = sgnm * uo;
+  const double suo = sgnm < 0. ? -uo : uo;
   // kind: 0 side state, 1 star state, 2 mixed (rarefaction fan)
   int kind;
   double spin = 0.0, spout = 0.0, co = 0.0, cstar = 0.0;
   if (pstar >= po) {
-    spin = ddiv_rn(rvsqrt(wosq), ro) - suo;
+    spin = ddiv_rn(dsqrt_rn(wosq), ro) - suo;
     kind = (spin < 0.) ? 0 : ((spin >= 0.) ? 1 : 2);
     spout = spin;
   } else {
-    co = rvsqrt(ddiv_rn(gamma * po, ro));
-    cstar = rvsqrt(ddiv_rn(gamma * pstar, rstar));
+    co = dsqrt_rn(ddiv_rn(gamma * po, ro));
+    cstar = dsqrt_rn(ddiv_rn(gamma * pstar, rstar));
     spout = co - suo;
     spin = cstar - suo;
     kind = (spout < 0.) ? 0 : ((spin >= 0.) ? 1 : 2);
@@ -205,13 +204,13 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   }
   // ---- reverse of the fluxes
   const double K = ug * ug + utr1 * utr1 + utr2 * utr2;
-  const double E = 0.5 * rg * K + ddiv_rn(pg, (gamma - 1.)) + pg;
-  double rgb = fb[0] * ug + fb[1] * ug * ug + fb[2] * ug * utr1 + fb[3] * ug * utr2 + fb[4] * ug * 0.5 * K;
-  double ugb = fb[0] * rg + fb[1] * 2.0 * rg * ug + fb[2] * rg * utr1 + fb[3] * rg * utr2 +
-               fb[4] * (E + ug * rg * ug);
-  double t1b = fb[2] * rg * ug + fb[4] * ug * rg * utr1;
-  double t2b = fb[3] * rg * ug + fb[4] * ug * rg * utr2;
-  double pgb = fb[1] + fb[4] * ug * (ddiv_rn(1.0, (gamma - 1.)) + 1.0);
+  const double igm1 = ddiv_rn(1.0, (gamma - 1.)), E = 0.5 * rg * K + pg * igm1 + pg;
+  const double S = fb[0] + fb[1] * ug + fb[2] * utr1 + fb[3] * utr2, m = dmul_rn(rg, ug);
+  double rgb = dmul_rn(ug, S + 0.5 * K * fb[4]);
+  double ugb = rg * (S + ug * (fb[1] + fb[4] * ug)) + fb[4] * E;
+  double t1b = dmul_rn(m, fb[2] + fb[4] * utr1);
+  double t2b = dmul_rn(m, fb[3] + fb[4] * utr2);
+  double pgb = fb[1] + fb[4] * ug * (igm1 + 1.0);
   // ---- reverse of the selection
   double rob = 0.0, uob = 0.0, pob = 0.0, rstarb = 0.0, ustarb = 0.0, pstarb = 0.0, ccsb = 0.0;
   if (kind == 0) { rob += rgb; uob += ugb; pob += pgb; }
@@ -248,15 +247,14 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   {
     const double idd = ddiv_rn(1.0, dd), iwo = ddiv_rn(1.0, wosq);
     rob += rstarb * idd;
-    const double ddb = -rstarb * rstar * idd;
-    const double uub = -ddb;
-    const double ttb = uub * iwo;
-    const double wosqb = -uub * uu * iwo;
+    const double uub = dmul_rn(dmul_rn(rstarb, rstar), idd);
+    const double ttb = dmul_rn(uub, iwo);
+    const double wosqb = dmul_rn(-ttb, uu);
     rob += ttb * dpjmp;
-    const double dpb = ttb * ro;
+    const double dpb = dmul_rn(ttb, ro);
     pstarb += dpb;
     pob -= dpb;
-    const double awb = wosqb * ro;
+    const double awb = dmul_rn(wosqb, ro);
     rob += wosqb * aw;
     pstarb += awb * (hg + 1.0);
     pob += awb * hg;
@@ -280,7 +278,8 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
 #pragma unroll
   for (int it = 2; it >= 0; --it) {
     double Pb = 0.0, Pmb = 0.0, UMb = 0.0, UPb = 0.0;
-    rp_iter_vjp(q, P[it], Pm[it], UM[it], UP[it], Pnb, Pmnb, UMnb, UPnb, Pb, Pmb, UMb, UPb, g);
+    rp_iter_vjp(q, ri[it], P[it], Pm[it], UM[it], UP[it], UM[it + 1], UP[it + 1], Pnb, Pmnb, UMnb,
+                UPnb, Pb, Pmb, UMb, UPb, g);
     Pnb = Pb; Pmnb = Pmb; UMnb = UMb; UPnb = UPb;
   }
   // (Pnb, Pmnb, UMnb, UPnb) now hold the cotangents of (p1, p0, usm0, usp0)
@@ -289,27 +288,27 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   {
     const double ps1b = m1 ? Pnb : 0.0;
     const double iD1 = ddiv_rn(1.0, D1);
-    const double N1b = ps1b * iD1, D1b = -ps1b * ps1 * iD1;
+    const double N1b = dmul_rn(ps1b, iD1), D1b = dmul_rn(-N1b, ps1);
     double wl1b = N1b * (pr - wr1 * dU) + D1b, wr1b = N1b * (pl - wl1 * dU) + D1b;
     g.pr += N1b * wl1;
     g.pl += N1b * wr1;
-    dUb += -N1b * wr1 * wl1;
+    dUb += dmul_rn(-N1b, wr1) * wl1;
     // usm0 = ur + (p0 - pr)/wr1;  usp0 = ul - (p0 - pl)/wl1
     const double iwr1 = ddiv_rn(1.0, wr1), iwl1 = ddiv_rn(1.0, wl1);
-    const double um = UMnb * iwr1, up = UPnb * iwl1;
+    const double um = dmul_rn(UMnb, iwr1), up = dmul_rn(UPnb, iwl1);
     g.ur += UMnb;
     p0b += um;
     g.pr -= um;
-    wr1b += -um * (p0 - pr) * iwr1;
+    wr1b += dmul_rn(-um, p0 - pr) * iwr1;
     g.ul += UPnb;
     p0b -= up;
     g.pl += up;
-    wl1b += up * (p0 - pl) * iwl1;
-    // w1 = rvsqrt(a1 r), a1 = hg (p0 + p) + p0
-    const double wlsqb = 0.5 * wl1b * iwl1, wrsqb = 0.5 * wr1b * iwr1;
+    wl1b += dmul_rn(up, p0 - pl) * iwl1;
+    // w1 = sqrt(a1 r), a1 = hg (p0 + p) + p0
+    const double wlsqb = dmul_rn(0.5 * wl1b, iwl1), wrsqb = dmul_rn(0.5 * wr1b, iwr1);
     g.rl += wlsqb * a1l;
     g.rr += wrsqb * a1r;
-    const double alb = wlsqb * rl, arb = wrsqb * rr;
+    const double alb = dmul_rn(wlsqb, rl), arb = dmul_rn(wrsqb, rr);
     p0b += (alb + arb) * (hg + 1.0);
     g.pl += alb * hg;
     g.pr += arb * hg;
@@ -317,12 +316,12 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   {
     const double ps0b = m0 ? p0b : 0.0;
     const double iD0 = ddiv_rn(1.0, D0);
-    const double N0b = ps0b * iD0, D0b = -ps0b * ps0 * iD0;
+    const double N0b = dmul_rn(ps0b, iD0), D0b = dmul_rn(-N0b, ps0);
     wl0b += N0b * (pr - wr0 * dU) + D0b;
     wr0b += N0b * (pl - wl0 * dU) + D0b;
     g.pr += N0b * wl0;
     g.pl += N0b * wr0;
-    dUb += -N0b * wr0 * wl0;
+    dUb += dmul_rn(-N0b, wr0) * wl0;
   }
   // ccs = small (cleft + cright), cleft = wl0 / rl, cright = wr0 / rr
   {
@@ -335,7 +334,7 @@ AMRS_HD void riemann_prob_vjp(const double gamma, const double smallp, const dou
   }
   g.ur += dUb;
   g.ul -= dUb;
-  // w0 = rvsqrt(gamma p r)
+  // w0 = sqrt(gamma p r)
   {
     const double lb = ddiv_rn(wl0b, (2.0 * wl0)), rb2 = ddiv_rn(wr0b, (2.0 * wr0));
     g.pl += lb * gamma * rl;
