@@ -86,10 +86,10 @@ __global__ void __launch_bounds__(256, 3) weno_vjp_face_kernel(const __grid_cons
 #pragma unroll
       for (int q = 0; q < 5; ++q) {
         const double pn = PF.p[op + (q - 2) * sp + n * PF.ns];
-        const double dp = half_of(pn - pq), du = u[q + 1] - u[q];
+        const double dp = pn - pq, hdu = dmul_rn(hme, u[q + 1] - u[q]);
         pq = pn;
-        if (q < 4) tp[q] = dp + hme * du;
-        if (q > 0) tm[4 - q] = hme * du - dp;
+        if (q < 4) tp[q] = 0.5 * dp + hdu;
+        if (q > 0) tm[4 - q] = -0.5 * dp + hdu;
       }
       weno5js_grad(tp, gp, Wy);
       weno5js_grad(tm, gm, Wy);

@@ -2,7 +2,7 @@
 where one range test per value holds, and takes the hardware's operations
 elsewhere: smooth fields, exactly zero differences, a jump between uniform
 halves (some differences zero), and fields whose differences lie above and
-below the tested range.
+below the tested range, subnormal ones too.
 
 Check: <v, J w> = <J^T v, w>, J w from the oracle's dual numbers or, where some
 differences are zero, from 100 digits: there the rounding of s0 - 4 s1 + 3 s2
@@ -33,6 +33,8 @@ def _state(kind):
         f = (one, 0.25 * one, 0.0 * one, -0.5 * one, one)
     elif kind == "large":
         f = (1 + noise(0.1), 1e9 * noise(1.0), 1e9 * noise(1.0), 0.0 * one, 1e25 * (2 + noise(1.0)))
+    elif kind == "subnormal":
+        f = (1 + noise(0.1), noise(1e-309), noise(1e-310), 0.0 * one, 1 + noise(0.1))
     elif kind == "small":
         f = (1e-30 * (2 + noise(1.0)), noise(1e-3), noise(1e-90), 0.0 * one, 1e-33 * (2 + noise(1.0)))
     else:
@@ -89,7 +91,7 @@ def _exact_jvp(U, W, gamma, dxinv):
         return ((res[1] - res[0]) / step).astype(np.float64)
 
 
-@pytest.mark.parametrize("kind", ["smooth", "uniform", "jump", "large", "small"])
+@pytest.mark.parametrize("kind", ["smooth", "uniform", "jump", "large", "small", "subnormal"])
 def test_vjp_dot_product(orc, kind):
     capi.load(build_if_missing=True)
     U = _state(kind)
