@@ -42,63 +42,51 @@ __device__ __forceinline__ double fbar(const DArr& v, const BoxRec& R, int d, in
   return R.dxinv[d] * (vget(v, R, i, j, k, n) - vget(v, R, i - di, j - dj, k - dk, n));
 }
 
-// VJP of one KEEP pair term (keep_pair in amrs_device.cuh) given its
-// cotangent a[5] (already times the coefficient): contributions to the
-// primitive cotangents of point 1 (larger index) and point 2.  With
-// P = R N, the mass flux m = P/4 and the cubic factor t8 = P/8, so the
-// cotangents of R and N share one factor s = mb/4 + t8b/8 (exact scalings;
-// the reverse pass has no bit-exact counterpart).  Standalone products may
-// go to the integer pipe (kmul, AMRS_PVJP_IMUL): bit 0 the cotangents of
-// the velocity sums and of E, bit 1 those of R and N, bit 2 cv Eb.
-#ifndef AMRS_PVJP_IMUL
-#define AMRS_PVJP_IMUL 0x3
-#endif
+// VJP of one KEEP pair term (keep_pair in amrs_device.cuh) given half its
+// cotangent, a[5] (already times the coefficient): contributions to the
+// primitive cotangents of point 1 (larger index) and point 2.  With sums
+// R, N, U, E of the two ends and K = sum of the velocity products, the pair is
+// (R N) / 8 times (2, U + .., E + K) plus pressure terms, so the cotangents of
+// U and E are t4 a with t4 = R N / 4, those of R and N are N and R times one
+// factor, and the kinetic term's is that of E (exact scalings; the reverse
+// pass has no bit-exact counterpart).  Products that no addition consumes go
+// to the integer pipe: 32 FP64 instructions are left, 55 before.
 template <int D>
 __device__ __forceinline__ void keep_pair_vjp(const double* q1, const double* q2, const double a[5], double cv,
                                               double b1[NQA], double b2[NQA]) {
   constexpr int QN = QU + D;
-  constexpr bool M0 = AMRS_PVJP_IMUL & 1, M1 = (AMRS_PVJP_IMUL >> 1) & 1, M2 = (AMRS_PVJP_IMUL >> 2) & 1;
   const double R = q1[QRHO] + q2[QRHO];
-  const double N = q1[QN] + q2[QN];
-  const double Ux = q1[QU] + q2[QU], Uy = q1[QV] + q2[QV], Uz = q1[QW] + q2[QW];
-  const double E = q1[QE] + q2[QE];
-  const double P = R * N;
-  const double ke = 0.5 * (q1[QU] * q2[QU] + q1[QV] * q2[QV] + q1[QW] * q2[QW]);
-  const double t8 = 0.125 * P;
-  const double mb = a[0] + a[4] * ke;
-  const double keb = 0.25 * (a[4] * P);
-  const double t8b = a[1] * Ux + a[2] * Uy + a[3] * Uz + a[4] * E;
-  const double Uxb = kmul<M0>(a[1], t8), Uyb = kmul<M0>(a[2], t8), Uzb = kmul<M0>(a[3], t8),
-               Eb = kmul<M0>(a[4], t8);
-  const double fdivb = a[1 + D];
-  const double fgb = a[4];
-  const double sb = 0.25 * mb + 0.125 * t8b;
-  const double Rb = kmul<M1>(N, sb);
-  const double Nb = kmul<M1>(R, sb);
-  const double Pb = 0.5 * fdivb;
-  const double Ub[3] = {Uxb, Uyb, Uzb};
-  const double hk = 0.5 * keb, hg = 0.5 * fgb;
-  const double cvE = kmul<M2>(cv, Eb);
+  const double U[3] = {q1[QU] + q2[QU], q1[QV] + q2[QV], q1[QW] + q2[QW]};
+  const double N = U[D];
+  const double K = q1[QU] * q2[QU] + q1[QV] * q2[QV] + q1[QW] * q2[QW];
+  const double t4 = 0.25 * dmul_rn(R, N);
+  const double s4 =
+      0.25 * (2.0 * a[0] + (a[1] * U[0] + a[2] * U[1] + a[3] * U[2] + a[4] * ((q1[QE] + q2[QE]) + K)));
+  const double Eb = dmul_rn(a[4], t4);
+  double Ub[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) Ub[c] = dmul_rn(a[1 + c], t4);
+  Ub[D] += dmul_rn(R, s4);
+  const double Rb = dmul_rn(N, s4), cvE = dmul_rn(cv, Eb);
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
     const double* qo = s ? q1 : q2;
     double* b = s ? b2 : b1;
     b[0] = Rb;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      double t = Ub[c] + hk * qo[QU + c];
-      if (c == D) t += Nb + hg * qo[QPRES];
-      b[1 + c] = t;
-    }
+    for (int c = 0; c < 3; ++c) b[1 + c] = Ub[c] + Eb * qo[QU + c];
+    b[1 + D] += a[4] * qo[QPRES];
     b[4] = cvE;
-    b[5] = Pb + hg * qo[QN];
+    b[5] = a[1 + D] + a[4] * qo[QN];
   }
 }
 
 // One thread per (direction, separation, pair): pairs (a, a+l) along d
-// with a in [lo-l, hi] and transverse indices in the valid box.
+// with a in [lo-l, hi] and transverse indices in the valid box.  Bound: the FP64
+// pipe (76% busy at 64^3, order 4: 121 us; 158 with 55 FP64 instructions a pair).
+// Four CTAs per SM (64 registers); with two, 96 registers and 153 us.
 template <int ORDER>
-__global__ void __launch_bounds__(256) adj_pair_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total) {
+__global__ void __launch_bounds__(256, 4) adj_pair_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total) {
   dep_begin();
   constexpr int H = ORDER / 2;
   double coef[3];
@@ -122,9 +110,9 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(const __grid_constant__ B
       }
     if (!found) continue;
     const int e0 = n0 + (d == 0) * l, e1 = n1 + (d == 1) * l;
-    const int ii = (int)(r % e0);
-    const long long t = r / e0;
-    const int jj = (int)(t % e1), kk = (int)(t / e1);
+    const unsigned ru = (unsigned)r, t = ru / (unsigned)e0;  // fewer than 2^31 pairs of one direction and separation
+    const int ii = (int)(ru - t * (unsigned)e0), kk = (int)(t / (unsigned)e1);
+    const int jj = (int)(t - (unsigned)kk * (unsigned)e1);
     const int i = R.lo[0] + ii - (d == 0) * l, j = R.lo[1] + jj - (d == 1) * l, k = R.lo[2] + kk - (d == 2) * l;
     const int di = d == 0, dj = d == 1, dk = d == 2;
     // pair (a = (i,j,k), a + l e_d); faces a+1 .. a+l.  Next to a code-6 y
@@ -133,9 +121,9 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(const __grid_constant__ B
     double a[5] = {0, 0, 0, 0, 0};
     if (d == 1 && R.walls) {
       for (int m = 1; m <= l; ++m) {
-        double w = coef[l - 1];
+        double w = 0.5 * coef[l - 1];
         const int jf = j + m;
-        if (jf <= R.red_lo || (jf >= R.red_hi && jf <= R.hi[1])) w = (l == 1) ? 1.0 : 0.0;
+        if (jf <= R.red_lo || (jf >= R.red_hi && jf <= R.hi[1])) w = (l == 1) ? 0.5 : 0.0;
         if (w == 0.0) continue;
 #pragma unroll
         for (int n = 0; n < 5; ++n) a[n] += w * fbar(ar.vbar, R, d, i + m * di, j + m * dj, k + m * dk, n);
@@ -143,10 +131,10 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(const __grid_constant__ B
     } else {
       // one coefficient for all l faces: sum_m Fbar(a + m) telescopes to
       // dxinv_d (vbar(a + l) - vbar(a))
-      const double wd = coef[l - 1] * R.dxinv[d];
+      const double wd = 0.5 * coef[l - 1] * R.dxinv[d];
 #pragma unroll
       for (int n = 0; n < 5; ++n)
-        a[n] = wd * (vget(ar.vbar, R, i + l * di, j + l * dj, k + l * dk, n) - vget(ar.vbar, R, i, j, k, n));
+        a[n] = dmul_rn(wd, vget(ar.vbar, R, i + l * di, j + l * dj, k + l * dk, n) - vget(ar.vbar, R, i, j, k, n));
     }
     double q1[NQ], q2[NQ], b1[NQA], b2[NQA];
     const long long o2 = R.q.off(i, j, k), o1 = R.q.off(i + l * di, j + l * dj, k + l * dk);
@@ -170,8 +158,10 @@ __global__ void __launch_bounds__(256) adj_pair_kernel(const __grid_constant__ B
 // d/d(cond_ref) over its cells in a fixed order (grid-stride, then warp
 // shuffles, then the warps in order) into ar.part; adj_param_sum_kernel adds
 // the blocks' sums in block order.  No atomics: the result is the same bits
-// on every run.
-__global__ void __launch_bounds__(256) adj_visc_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, double* pbar) {
+// on every run.  Bound: the FP64 pipe (94 instructions a cell) behind the loads'
+// latency: four CTAs per SM 58 us at 64^3, two 65.  Its products on the integer
+// pipe gained nothing (within 0.3% of a step's gradient at 64^3).
+__global__ void __launch_bounds__(256, 4) adj_visc_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, double* pbar) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);
@@ -202,24 +192,27 @@ __global__ void __launch_bounds__(256) adj_visc_kernel(const __grid_constant__ B
     auto q = [&](long long off, int n) { return Q.p[off + n * Q.ns]; };
     const long long sx = 1, sy = Q.js, sz = Q.ks;
     const double u = q(o, QU), v = q(o, QV), w = q(o, QW), T = q(o, QT);
-    const double dudx = (q(o + sx, QU) - q(o - sx, QU)) * hx, dvdx = (q(o + sx, QV) - q(o - sx, QV)) * hx;
-    const double dwdx = (q(o + sx, QW) - q(o - sx, QW)) * hx, dTdx = (q(o + sx, QT) - q(o - sx, QT)) * hx;
+    auto central = [&](long long st, int n, double h) { return (q(o + st, n) - q(o - st, n)) * h; };
+    const double dudx = central(sx, QU, hx), dvdx = central(sx, QV, hx);
+    const double dwdx = central(sx, QW, hx), dTdx = central(sx, QT, hx);
     // y derivatives: central, or one-sided on the ghost row beyond a code-6
     // wall (ViscousWallFluxes, src/rhs/CNS_hydro_K.h:177-251)
     auto ddy = [&](int n) {
       if (R.walls && j == R.wrow_lo) return (4.0 * q(o + sy, n) - q(o + 2 * sy, n) - 3.0 * q(o, n)) * hy;
       if (R.walls && j == R.wrow_hi) return (-4.0 * q(o - sy, n) + 3.0 * q(o, n) + q(o - 2 * sy, n)) * hy;
-      return (q(o + sy, n) - q(o - sy, n)) * hy;
+      return central(sy, n, hy);
     };
     const double dudy = ddy(QU), dvdy = ddy(QV), dwdy = ddy(QW), dTdy = ddy(QT);
-    const double dudz = (q(o + sz, QU) - q(o - sz, QU)) * hz, dvdz = (q(o + sz, QV) - q(o - sz, QV)) * hz;
-    const double dwdz = (q(o + sz, QW) - q(o - sz, QW)) * hz, dTdz = (q(o + sz, QT) - q(o - sz, QT)) * hz;
+    const double dudz = central(sz, QU, hz), dvdz = central(sz, QV, hz);
+    const double dwdz = central(sz, QW, hz), dTdz = central(sz, QT, hz);
     const double div = dudx + dvdy + dwdz;
     const double mu = visc(cl, T), lam = cond(cl, T);
     const double r13 = 1.0 / 3.0;
-    const double txx = 2.0 * mu * (dudx - r13 * div), tyy = 2.0 * mu * (dvdy - r13 * div);
-    const double tzz = 2.0 * mu * (dwdz - r13 * div);
-    const double txy = mu * (dudy + dvdx), txz = mu * (dudz + dwdx), tyz = mu * (dvdz + dwdy);
+    const double mu2 = 2.0 * mu, d3 = r13 * div;
+    const double exx = dudx - d3, eyy = dvdy - d3, ezz = dwdz - d3;
+    const double exy = dudy + dvdx, exz = dudz + dwdx, eyz = dvdz + dwdy;
+    const double txx = mu2 * exx, tyy = mu2 * eyy, tzz = mu2 * ezz;
+    const double txy = mu * exy, txz = mu * exz, tyz = mu * eyz;
     const double txxb = -fb[0] - fb[3] * u;
     const double txyb = -fb[1] - fb[3] * v - fb[4] - fb[7] * u;
     const double txzb = -fb[2] - fb[3] * w - fb[8] - fb[11] * u;
@@ -229,30 +222,33 @@ __global__ void __launch_bounds__(256) adj_visc_kernel(const __grid_constant__ B
     const double ub = -(fb[3] * txx + fb[7] * txy + fb[11] * txz);
     const double vb = -(fb[3] * txy + fb[7] * tyy + fb[11] * tyz);
     const double wb = -(fb[3] * txz + fb[7] * tyz + fb[11] * tzz);
-    const double lamb = -(fb[3] * dTdx + fb[7] * dTdy + fb[11] * dTdz);
-    const double mub = txxb * 2.0 * (dudx - r13 * div) + tyyb * 2.0 * (dvdy - r13 * div) +
-                       tzzb * 2.0 * (dwdz - r13 * div) + txyb * (dudy + dvdx) + txzb * (dudz + dwdx) +
-                       tyzb * (dvdz + dwdy);
     const double divb = -(2.0 / 3.0) * mu * (txxb + tyyb + tzzb);
     double gb[12];
     const double gxy = mu * txyb, gxz = mu * txzb, gyz = mu * tyzb;
-    gb[0] = 2.0 * mu * txxb + divb;  // dudx
+    gb[0] = mu2 * txxb + divb;  // dudx
     gb[1] = gxy;                     // dvdx
     gb[2] = gxz;                     // dwdx
     gb[3] = -lam * fb[3];            // dTdx
     gb[4] = gxy;                     // dudy
-    gb[5] = 2.0 * mu * tyyb + divb;  // dvdy
+    gb[5] = mu2 * tyyb + divb;  // dvdy
     gb[6] = gyz;                     // dwdy
     gb[7] = -lam * fb[7];            // dTdy
     gb[8] = gxz;                     // dudz
     gb[9] = gyz;                     // dvdz
-    gb[10] = 2.0 * mu * tzzb + divb; // dwdz
+    gb[10] = mu2 * tzzb + divb; // dwdz
     gb[11] = -lam * fb[11];          // dTdz
     double Tb = 0.0;
-    if (cl.visc_law == 1) Tb += mub * mu * (1.5 / T - 1.0 / (cl.Tvisc_ref + T));
-    else mu_acc += mub;
-    if (cl.cond_law == 1) Tb += lamb * lam * (1.5 / T - 1.0 / (cl.Tcond_ref + T));
-    else la_acc += lamb;
+    if (cl.visc_law == 1 || pbar) {
+      const double mub =
+          2.0 * (txxb * exx + tyyb * eyy + tzzb * ezz) + txyb * exy + txzb * exz + tyzb * eyz;
+      if (cl.visc_law == 1) Tb += mub * mu * (ddiv_rn(1.5, T) - ddiv_rn(1.0, cl.Tvisc_ref + T));
+      else mu_acc += mub;
+    }
+    if (cl.cond_law == 1 || pbar) {
+      const double lamb = -(fb[3] * dTdx + fb[7] * dTdy + fb[11] * dTdz);
+      if (cl.cond_law == 1) Tb += lamb * lam * (ddiv_rn(1.5, T) - ddiv_rn(1.0, cl.Tcond_ref + T));
+      else la_acc += lamb;
+    }
     const DArr G = ar.vg;
     const long long og = G.off(i, j, k);
     G.p[og] = ub;
@@ -299,9 +295,11 @@ __global__ void adj_param_sum_kernel(const double* part, int nblocks, double* pb
   pbar[1] += a;
 }
 
-// Qbar gather + cons2prim VJP for every cell of grow(box,3).
+// Qbar gather + cons2prim VJP for every cell of grow(box,3).  Bound: the FP64 pipe
+// (82% busy: 72 of its additions at order 4 are the pairs'); 84 us at 64^3, four
+// CTAs per SM (two: 93).
 template <int ORDER>
-__global__ void __launch_bounds__(256) adj_gather_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, int gpair) {
+__global__ void __launch_bounds__(256, 4) adj_gather_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, int gpair) {
   dep_begin();
   constexpr int H = ORDER / 2;
   const BoxRec& R = box_rec(tb, 0);
@@ -396,49 +394,32 @@ __global__ void __launch_bounds__(256) adj_gather_kernel(const __grid_constant__
 }
 
 // Reverse of one stage's BLAS-1 program per valid cell: given the cotangent
-// of the stage result (register S2), produce the cotangents of S1, of the
-// stage input's valid values (register S2 before the program) and of dSdt.
-__global__ void __launch_bounds__(256) adj_prog_kernel(BoxRec R, DProg prog, DArr wbar, DArr s1bar, DArr inbar,
-                                                       DArr vbar, long long total, int accumulate) {
+// of the stage result (register S2), the cotangents of S1 (c1 times it), of the
+// stage input's valid values (c2, register S2 before the program) and of dSdt
+// (cd).  A coefficient of zero adds nothing and reads nothing.  64^3: 20 us
+// with the program reversed per value, 12 now; bound by memory.
+__global__ void __launch_bounds__(256) adj_prog_kernel(BoxRec R, double c1, double c2, double cd, DArr wbar, DArr s1bar,
+                                                       DArr inbar, DArr vbar, long long total, int accumulate) {
   dep_begin();
   const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
        g += (long long)gridDim.x * blockDim.x) {
-    const int l = (int)g;
-    const int i = l % nx + R.lo[0];
-    const int t = l / nx;
-    const int j = t % ny + R.lo[1];
-    const int k = t / ny + R.lo[2];
-    for (int n = 0; n < 5; ++n) {
-      double b[3] = {0.0, wbar(i, j, k, n), 0.0};
-      for (int o = prog.nops - 1; o >= 0; --o) {
-        const DOp& q = prog.ops[o];
-        if (q.kind == 0) {
-          const double gg = b[q.dst];
-          b[q.dst] = 0.0;
-          b[q.x] += q.a * gg;
-          b[q.y] += q.b * gg;
-        } else if (q.kind == 1) {
-          b[q.x] += q.a * b[q.dst];
-        } else if (q.kind == 2) {
-          const double gg = b[q.dst];
-          b[q.dst] = q.a * gg;
-          b[q.x] += gg;
-        } else {
-          const double gg = b[q.dst];
-          b[q.dst] = 0.0;
-          b[q.x] += gg;
-        }
-      }
-      if (accumulate) {
-        s1bar(i, j, k, n) += b[0];
-        inbar(i, j, k, n) += b[1];
-      } else {
-        s1bar(i, j, k, n) = b[0];
-        inbar(i, j, k, n) = b[1];
-      }
-      vbar(i, j, k, n) = b[2];
-    }
+    const int l = (int)g, t = l / nx;
+    const int i = l - t * nx + R.lo[0], k = t / ny + R.lo[2], j = t - (t / ny) * ny + R.lo[1];
+    double w[5];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) w[n] = wbar(i, j, k, n);
+    auto give = [&](const DArr& to, double c, bool add) {
+      if (add && c == 0.0) return;
+      double v[5];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) v[n] = add ? to(i, j, k, n) : 0.0;
+#pragma unroll
+      for (int n = 0; n < 5; ++n) to(i, j, k, n) = v[n] + (c == 0.0 ? 0.0 : c * w[n]);
+    };
+    give(s1bar, c1, accumulate);
+    give(inbar, c2, accumulate);
+    give(vbar, cd, false);
   }
 }
 
@@ -479,7 +460,8 @@ __device__ __forceinline__ int images(int c, int lo, int hi, int bcl, int bch, i
 // `to` null: in place; otherwise the folded cotangents are added to `to`.  Cells
 // more than two from every side have no images: nothing to do in place, one
 // addition otherwise (64^3: 67,000 of 262,000 cells fold; computing every cell's
-// images per component took 56 us, then a pass of 15 us added the result).
+// images per component took 56 us, then a pass of 15 us added the result; 47 us
+// component by component, 31 with five components' loads in flight).
 __global__ void __launch_bounds__(256) adj_halo_kernel(HaloBox hb, DArr to, long long total) {
   dep_begin();
   const int nx = hb.hi[0] - hb.lo[0] + 1, ny = hb.hi[1] - hb.lo[1] + 1;
@@ -494,16 +476,26 @@ __global__ void __launch_bounds__(256) adj_halo_kernel(HaloBox hb, DArr to, long
     const int nyi = images(j, hb.lo[1], hb.hi[1], hb.bc_lo[1], hb.bc_hi[1], 1, yi, ys);
     const int nzi = images(k, hb.lo[2], hb.hi[2], hb.bc_lo[2], hb.bc_hi[2], 2, zi, zs);
     if (!to.p && nxi * nyi * nzi == 1) continue;
-    for (int n = 0; n < hb.ncomp; ++n) {
-      double s = 0.0;
+    // five components at a time share the images' offsets and signs
+    for (int n0 = 0; n0 < hb.ncomp; n0 += 5) {
+      double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
       for (int a = 0; a < nzi; ++a)
         for (int b = 0; b < nyi; ++b)
           for (int c = 0; c < nxi; ++c) {
-            const double v = hb.u(xi[c], yi[b], zi[a], n);
-            s += n < 32 && (((xs[c] ^ ys[b] ^ zs[a]) >> n) & 1u) ? -v : v;
+            const double* p = hb.u.p + hb.u.off(xi[c], yi[b], zi[a]) + n0 * hb.u.ns;
+            const unsigned neg = n0 == 0 ? xs[c] ^ ys[b] ^ zs[a] : 0u;  // momenta only
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+              const double v = n0 + m < hb.ncomp ? p[m * hb.u.ns] : 0.0;
+              s[m] += (neg >> m) & 1u ? -v : v;
+            }
           }
-      if (to.p) to(i, j, k, n) += s;
-      else hb.u(i, j, k, n) = s;
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        if (n0 + m >= hb.ncomp) break;
+        if (to.p) to(i, j, k, n0 + m) += s[m];
+        else hb.u(i, j, k, n0 + m) = s[m];
+      }
     }
   }
 }
@@ -577,7 +569,27 @@ cudaError_t launch_rhs_vjp(int order, const BoxTable& tb, const AdjRecHost& ah, 
 cudaError_t launch_adj_prog(const BoxRec& R, const DProg& prog, const DArr& wbar, const DArr& s1bar, const DArr& inbar,
                             const DArr& vbar, int accumulate, int nsm, cudaStream_t st) {
   const long long n = (long long)(R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1);
-  launch_dep(adj_prog_kernel, grid256(n, nsm), 256, 0, st, R, prog, wbar, s1bar, inbar, vbar, n, accumulate);
+  // the program is linear in its registers: its reverse on the unit cotangent
+  double b[3] = {0.0, 1.0, 0.0};
+  for (int o = prog.nops - 1; o >= 0; --o) {
+    const DOp& q = prog.ops[o];
+    const double g = b[q.dst];
+    if (q.kind == 0) {
+      b[q.dst] = 0.0;
+      b[q.x] += q.a * g;
+      b[q.y] += q.b * g;
+    } else if (q.kind == 1) {
+      b[q.x] += q.a * g;
+    } else if (q.kind == 2) {
+      b[q.dst] = q.a * g;
+      b[q.x] += g;
+    } else {
+      b[q.dst] = 0.0;
+      b[q.x] += g;
+    }
+  }
+  launch_dep(adj_prog_kernel, grid256(n, nsm), 256, 0, st, R, b[0], b[1], b[2], wbar, s1bar, inbar, vbar, n,
+             accumulate);
   return cudaGetLastError();
 }
 

@@ -17,23 +17,19 @@ __device__ __forceinline__ void cons2prim_vjp(const BoxRec& R, const DClosures& 
   const long long oq = Q.off(i, j, k);
   const double rho = Q.p[oq + QRHO * Q.ns], u = Q.p[oq + QU * Q.ns], v = Q.p[oq + QV * Q.ns],
                w = Q.p[oq + QW * Q.ns], T = Q.p[oq + QT * Q.ns];
-  double rb = qb[QRHO], ub = qb[QU], vb = qb[QV], wb = qb[QW];
-  const double pb = qb[QPRES] + ddiv_rn(qb[QT], (rho * cl.Rspec));
-  rb += ddiv_rn(-qb[QT] * T, rho);
-  const double eib = (cl.gamma - 1.0) * pb;  // d/d rhoei
-  const double keb = -eib;                   // d/d rhoke
-  rb += 0.5 * (u * u + v * v + w * w) * keb;
-  ub += rho * u * keb;
-  vb += rho * v * keb;
-  wb += rho * w * keb;
   const double rinv = ddiv_rn(1.0, rho);
-  rb += -(ub * u + vb * v + wb * w) * rinv;
+  const double eib = (cl.gamma - 1.0) * (qb[QPRES] + ddiv_rn(qb[QT], rho * cl.Rspec));  // d/d rhoei
+  // d/d rhoke = -eib
+  const double reib = dmul_rn(rho, -eib);
+  const double ub = qb[QU] + reib * u, vb = qb[QV] + reib * v, wb = qb[QW] + reib * w;
+  const double rb = qb[QRHO] - 0.5 * (u * u + v * v + w * w) * eib -
+                    (qb[QT] * T + (ub * u + vb * v + wb * w)) * rinv;
   const DArr U = R.slot[0];
   const double rho_raw = U(i, j, k, URHO);
   ub5[0] = (rho_raw > 1e-40) ? rb : 0.0;
-  ub5[1] = ub * rinv;
-  ub5[2] = vb * rinv;
-  ub5[3] = wb * rinv;
+  ub5[1] = dmul_rn(ub, rinv);
+  ub5[2] = dmul_rn(vb, rinv);
+  ub5[3] = dmul_rn(wb, rinv);
   ub5[4] = eib;
 }
 
