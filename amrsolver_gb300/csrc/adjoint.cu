@@ -526,9 +526,9 @@ __global__ void __launch_bounds__(256) adj_source_kernel(BoxRec R, double f0, do
 }
 
 // ------------------------------------------------------------ launchers --
-static int grid256(long long n, int nsm) {
+static int grid256(long long n, int nsm, int ctas = GRID_CTAS) {
   long long b = (n + 255) / 256;
-  const long long cap = (long long)nsm * 8;
+  const long long cap = (long long)nsm * ctas;
   return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
@@ -554,7 +554,7 @@ cudaError_t launch_rhs_vjp(int order, const BoxTable& tb, const AdjRecHost& ah, 
   else if (order == 6) launch_dep(adj_pair_kernel<6>, grid256(npair, nsm), 256, 0, st, tb, ar, npair);
   const long long nv = (n0 + 2) * (n1 + 2) * (n2 + 2);
   if (ah.visc) {
-    const int nbv = grid256(nv, nsm);  // at most 8 blocks per SM: ah.part holds 2 x 8 x nsm doubles
+    const int nbv = grid256(nv, nsm, 8);  // at most 8 blocks per SM: ah.part holds 2 x 8 x nsm doubles
     launch_dep(adj_visc_kernel, nbv, 256, 0, st, tb, ar, nv, pbar);
     if (pbar) launch_dep(adj_param_sum_kernel, 1, 32, 0, st, ah.part, nbv, pbar);
   }

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256) jst_vjp_gather_kernel(const __grid_consta
 
 int grid_j(long long n, int nsm) {
   long long b = (n + 255) / 256;
-  const long long cap = (long long)nsm * 8;
+  const long long cap = (long long)nsm * GRID_CTAS;
   return (int)(b < 1 ? 1 : (b < cap ? b : cap));
 }
 

@@ -16,6 +16,13 @@
 
 namespace amrs {
 
+// Blocks per SM of a grid-stride launch that has more work than that: divisible by
+// 2, 3, 4, 5 and 6, so that every round of resident blocks is full whatever a
+// kernel's registers allow (with 8 the third round of a kernel with three resident
+// blocks ran with two).  A step, KEEP4 128^3: 2978 us with 8, 2928 with 12, 2922 with
+// 24, 2910 with 60; level of 32^3 boxes 3518 and 3439; WENO5 64^3 1754 and 1726.
+constexpr int GRID_CTAS = 60;
+
 // Waits until all earlier grids are complete and their writes visible.
 __device__ __forceinline__ void dep_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");

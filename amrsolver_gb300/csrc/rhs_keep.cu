@@ -30,7 +30,8 @@
 namespace amrs {
 
 // ------------------------------------------------------------- prims ----
-__global__ void __launch_bounds__(256) prims_kernel(const __grid_constant__ BoxTable tb, int s_in) {
+// Bound: the FP64 pipe (77% busy; nine instructions a cell and the copy's loads).
+__global__ void __launch_bounds__(256, 5) prims_kernel(const __grid_constant__ BoxTable tb, int s_in) {
   dep_begin();
   if (list_idle(tb)) return;
   const long long total = tb.tot_p;
@@ -60,7 +61,10 @@ __global__ void __launch_bounds__(256) prims_kernel(const __grid_constant__ BoxT
 }
 
 // ------------------------------------------------- viscous cell fluxes ----
-__global__ void __launch_bounds__(256) visc_cell_kernel(const __grid_constant__ BoxTable tb) {
+// Bound: the FP64 pipe and the integer pipes about equally (37 additions and 40
+// products a cell; 75% and half of the issue slots at 128^3, 180 us); three CTAs per
+// SM (80 registers), two 2% of a step slower, four the same.
+__global__ void __launch_bounds__(256, 3) visc_cell_kernel(const __grid_constant__ BoxTable tb) {
   dep_begin();
   if (list_idle(tb)) return;
   const long long total = tb.tot_v;
@@ -421,7 +425,7 @@ static cudaError_t launch_face_t(const BoxTable& tb, int s_in, int s_s1, int s_o
 cudaError_t launch_prims(const BoxTable& tb, int s_in, long long ncells, int nsm, cudaStream_t st) {
   if (ncells <= 0) return cudaSuccess;
   long long blocks = (ncells + 255) / 256;
-  const long long cap = (long long)nsm * 8;
+  const long long cap = (long long)nsm * GRID_CTAS;
   if (blocks > cap) blocks = cap;
   launch_dep(prims_kernel, (int)blocks, 256, 0, st, tb, s_in);
   return cudaGetLastError();
@@ -430,7 +434,7 @@ cudaError_t launch_prims(const BoxTable& tb, int s_in, long long ncells, int nsm
 cudaError_t launch_visc(const BoxTable& tb, long long ncells, int nsm, cudaStream_t st) {
   if (ncells <= 0) return cudaSuccess;
   long long blocks = (ncells + 255) / 256;
-  const long long cap = (long long)nsm * 8;
+  const long long cap = (long long)nsm * GRID_CTAS;
   if (blocks > cap) blocks = cap;
   launch_dep(visc_cell_kernel, (int)blocks, 256, 0, st, tb);
   return cudaGetLastError();
