@@ -249,6 +249,38 @@ AMRS_HD double ddiv_rn(double a, double b) {
   return x;
 }
 
+// K a for K = 3, 5, 7 or 11 and normal a with K a finite, correctly rounded: the
+// product has one or two bits more than the floor of log2 K, and rounds at them.
+template <uint32_t K>
+AMRS_HD DWords dmul_small(DWords a) {
+  constexpr uint32_t s0 = K < 4 ? 1 : (K < 8 ? 2 : 3);
+  const uint32_t mh = (a.hi & 0xFFFFFu) | 0x100000u;
+  uint64_t P = (uint64_t)a.lo * K + ((uint64_t)(mh * K) << 32);
+  const uint32_t c = (uint32_t)(P >> (53 + s0)), s = s0 + c;
+  P += (c ? (1u << s0) - 1u : (1u << (s0 - 1u)) - 1u) + ((uint32_t)(P >> s) & 1u);
+  P >>= s;
+  return DWords{(a.hi & 0xFFF00000u) + (uint32_t)(P >> 32) + ((s - 1u) << 20), (uint32_t)P};
+}
+
+// x + y of two positive normal numbers whose sum stays finite, correctly rounded:
+// significands aligned in 64 bits with ten guard bits and a sticky bit; beyond 62
+// places the smaller one is only the sticky bit.
+AMRS_HD DWords dadd_pos(DWords x, DWords y) {
+  const bool sw = y.hi > x.hi;
+  const uint32_t ah = sw ? y.hi : x.hi, al = sw ? y.lo : x.lo, bh = sw ? x.hi : y.hi, bl = sw ? x.lo : y.lo;
+  const uint32_t e = ah >> 20;
+  uint32_t d = e - (bh >> 20);
+  d = d < 62u ? d : 62u;
+  const uint64_t A = ((uint64_t)((ah & 0xFFFFFu) | 0x100000u) << 32 | al) << 10;
+  const uint64_t B = ((uint64_t)((bh & 0xFFFFFu) | 0x100000u) << 32 | bl) << 10;
+  uint64_t S = A + (B >> d);
+  S |= ((B << 1) << (63u - d)) != 0u;
+  const uint32_t c = (uint32_t)(S >> 63);
+  S = (S >> c) | (S & c);
+  S = (S + (0x1FFu + ((uint32_t)(S >> 10) & 1u))) >> 10;
+  return DWords{(uint32_t)(S >> 32) + ((e - 1u + c) << 20), (uint32_t)S};
+}
+
 // a * b for words in the domain (any exponents whose sum gives a normal
 // product).  v:t:p is the 106-bit product ma mb, p3 its upper word in
 // [2^8, 2^10); the rounding word r holds the bits below the significand with

@@ -231,14 +231,22 @@ __device__ __forceinline__ double weno5js(const double s0, const double s1, cons
 
 __device__ __forceinline__ DWords weno_sq(DWords e) { return dmul_core(e, e); }
 
+// K x for a small integer K
+template <uint32_t K>
+__device__ __forceinline__ double weno_times(const ZWords& x) {
+  const DWords r = dmul_small<K>(x.w);
+  return dfrom(x.zero ? x.w.hi : r.hi, x.zero ? 0u : r.lo);
+}
+
 __device__ __forceinline__ double weno5js_int(const double s0, const double s1, const double s2, const double s3,
                                               const double s4, bool& ok) {
   const DWords c1312{0x3FF15555u, 0x55555555u};
+  auto quarter = [](DWords w) { return DWords{w.hi - (2u << 20), w.lo}; };
   bool slow0, slow1, slow2, slow3;
   const ZWords z2 = weno_fac(s2, ok);
-  const double s2x3 = weno_mul(DWords{0x40080000u, 0u}, z2);
+  const double s2x3 = weno_times<3>(z2);
   const DWords a = weno_diff(fma(-2.0, s1, s0) + s2, ok), b = weno_diff(fma(-4.0, s1, s0) + s2x3, ok);
-  const double beta0 = fma(0.25, dfrom(dmul_core(b, b)), dfrom(dmul_core(dmul_core(c1312, a), a)));
+  const double beta0 = dfrom(dadd_pos(quarter(dmul_core(b, b)), dmul_core(dmul_core(c1312, a), a)));
   const DWords alpha0 = ddiv_core(DWords{0x3FB99999u, 0x9999999Au}, weno_sq(weno_e(beta0)), &slow0);
   const DWords c = weno_diff(fma(-2.0, s2, s1) + s3, ok), g = weno_diff(s1 - s3, ok);
   const double beta1 = fma(0.25, dfrom(dmul_core(dmul_core(dmul_core(g, g), g), g)),
@@ -247,13 +255,12 @@ __device__ __forceinline__ double weno5js_int(const double s0, const double s1, 
   const DWords d = weno_diff(fma(-2.0, s3, s2) + s4, ok), f = weno_diff(fma(-4.0, s3, s2x3) + s4, ok);
   const double beta2 = fma(0.25, dfrom(dmul_core(f, f)), dfrom(dmul_core(dmul_core(c1312, d), d)));
   const DWords alpha2 = ddiv_core(DWords{0x3FD33333u, 0x33333333u}, weno_sq(weno_e(beta2)), &slow2);
-  const DWords sum = ddiv_core(DWords{0x3FF00000u, 0u}, dwords(dfrom(alpha0) + dfrom(alpha1) + dfrom(alpha2)), &slow3);
+  const DWords sum = ddiv_core(DWords{0x3FF00000u, 0u}, dadd_pos(dadd_pos(alpha0, alpha1), alpha2), &slow3);
   const ZWords z1 = weno_fac(s1, ok), z3 = weno_fac(s3, ok);
-  const DWords c5{0x40140000u, 0u};
   // 2 s0 - 7 s1 + 11 s2, -s1 + 5 s2 + 2 s3, 2 s2 + 5 s3 - s4
-  const double vl0 = fma(2.0, s0, -weno_mul(DWords{0x401C0000u, 0u}, z1)) + weno_mul(DWords{0x40260000u, 0u}, z2);
-  const double vl1 = fma(2.0, s3, -s1 + weno_mul(c5, z2));
-  const double vl2 = fma(2.0, s2, weno_mul(c5, z3)) - s4;
+  const double vl0 = fma(2.0, s0, -weno_times<7>(z1)) + weno_times<11>(z2);
+  const double vl1 = fma(2.0, s3, -s1 + weno_times<5>(z2));
+  const double vl2 = fma(2.0, s2, weno_times<5>(z3)) - s4;
   const double S = weno_mul(alpha0, weno_fac(vl0, ok)) + weno_mul(alpha1, weno_fac(vl1, ok)) +
                    weno_mul(alpha2, weno_fac(vl2, ok));
   ok = ok && !(slow0 || slow1 || slow2 || slow3);
@@ -321,15 +328,19 @@ static __device__ __noinline__ double weno_llf_plain(const double* p0, long long
 // order; otherwise the split halves 0.5 (f +- alpha U) enter weno5js_cd doubled
 // as fma(+-alpha, U, f).
 //
-// Bound: the FP64 pipe (29 instructions per reconstruction: the differences,
-// sums and splits) with the integer pipes about as full (21 products and 4
-// quotients per reconstruction).  One component per thread instead of five in
-// a loop: the range test and the fallback then cover one flux, the kernel fits
-// three CTAs per SM (80 registers), and a small box fills the chip (256 x 8 x 8
-// tube: 1040 CTAs instead of 208).  Face kernel of the reference order, before
-// (11 of the products and the quotients on the integer pipe, one thread per
-// face) and after: 256^3 54.0 -> 29.4 ms, 64^3 874 -> 464 us, the tube 78 -> 41 us;
-// with 2 CTAs per SM 30.1 ms at 256^3, with 4 (64 registers) 32.6 ms.
+// Bound: the FP64 pipe (26 instructions per reconstruction: the differences, sums
+// and splits) with the integer ALUs about as full (16 products, 5 by small
+// integers, 3 additions of positive numbers, 4 quotients).  One component per
+// thread instead of five in a loop: the range test and the fallback then cover one
+// flux, the kernel fits three CTAs per SM (80 registers), and a small box fills the
+// chip (256 x 8 x 8 tube: 1040 CTAs instead of 208).  Face kernel of the reference
+// order, first with 11 of the products and the quotients on the integer pipe, one
+// thread per face: 256^3 54.0 ms, now 29.0 with the viscous averages in it; 64^3
+// 874 us, now 464 with them; the tube 78 us, now 39; with 2 CTAs per SM 2% more, with
+// 4 (64 registers) 11% more.  The
+// positive additions and products by small integers took a step at 256^3 from 103.0
+// to 98.3 ms: of the five positive sums, beta_0 and the weights' sums are the ones
+// that gain; with none 101.7, only the weights' 99.5, all 101.4.
 template <bool REF_ORDER, bool VISC>
 __global__ void __launch_bounds__(256, 3) weno_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, long long total) {
   dep_begin();
