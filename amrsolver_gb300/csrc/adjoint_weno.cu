@@ -43,7 +43,7 @@ __device__ __forceinline__ double vget0(const DArr& v, const BoxRec& R, int i, i
 
 // One thread per face of direction d.  Bound: the FP64 pipe.  On differences of the
 // split stencils, with the gradient's products on the integer pipe, 47 x 40 x 52
-// takes 168 us a direction, 311 with stencil values and FP64 products; the two
+// takes 170 us a direction, 311 with stencil values and FP64 products; the two
 // products per slot below stay on the FP64 pipe (1% faster than moved).  Three CTAs
 // per SM are as fast as two, four 1% slower (spills).
 __global__ void __launch_bounds__(256, 3) weno_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FaceBuf fb, int d,
@@ -111,8 +111,12 @@ __global__ void __launch_bounds__(256, 3) weno_vjp_face_kernel(const __grid_cons
 
 // Gather + VJP of cons2eulerflux_lambda (src/rhs/High_resolution.h:83-121)
 // for direction d, over cells [lo-3, hi+3] along d and the valid range across.
-__global__ void __launch_bounds__(256) weno_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, FaceBuf fb, int d, int m0,
-                                                              int m1, long long total) {
+// Bound: the FP64 pipe (66 of its additions are the slots').  Compiled per direction,
+// quotients and root on the integer pipe: 39 -> 33 us at 47 x 40 x 52; two to five
+// CTAs per SM within 0.4% of a step's gradient.
+template <int d>
+__global__ void __launch_bounds__(256, 4) weno_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar,
+                                                                   FaceBuf fb, int m0, int m1, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);
@@ -148,11 +152,11 @@ __global__ void __launch_bounds__(256) weno_vjp_gather_kernel(const __grid_const
     const double rho = U.p[o];
     const double m[3] = {U.p[o + U.ns], U.p[o + 2 * U.ns], U.p[o + 3 * U.ns]};
     const double rhoet = U.p[o + 4 * U.ns];
-    const double rhoinv = 1.0 / rho;
+    const double rhoinv = ddiv_rn(1.0, rho);
     const double uu[3] = {m[0] * rhoinv, m[1] * rhoinv, m[2] * rhoinv};
-    const double rhoekin = 0.5 * rhoinv * (m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
+    const double mm = m[0] * m[0] + m[1] * m[1] + m[2] * m[2], rhoekin = 0.5 * rhoinv * mm;
     const double P = (gam - 1.0) * (rhoet - rhoekin);
-    const double cs = sqrt(gam * P * rhoinv);
+    const double cs = dsqrt_rn(gam * P * rhoinv);
     const double ud = uu[d];
     // lambda_d = |rmax(rmax(ud + cs, ud - cs), ud)|: derivative along the taken branch
     const double ca = ud + cs, cb = ud - cs;
@@ -160,41 +164,25 @@ __global__ void __launch_bounds__(256) weno_vjp_gather_kernel(const __grid_const
     if (mx < cb) { mx = cb; dcs = -1.0; }
     if (mx < ud) { mx = ud; dcs = 0.0; }
     const double sg = (mx > 0.0) ? 1.0 : (mx < 0.0 ? -1.0 : 0.0);
-    // cotangents of the intermediates
-    double mb[3] = {0, 0, 0}, ubv[3] = {0, 0, 0};
-    double Pb = 0.0, Eb = 0.0, rinvb = 0.0;
-    // physical flux f_d: (m_d, m_x u_d (+P), m_y u_d (+P), m_z u_d (+P), (E+P) u_d)
-    mb[d] += pb[0];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      mb[a] += pb[1 + a] * ud;
-      ubv[d] += pb[1 + a] * m[a];
-    }
-    Pb += pb[1 + d];
-    Eb += pb[4] * ud;
-    Pb += pb[4] * ud;
-    ubv[d] += pb[4] * (rhoet + P);
-    // lambda_d
-    const double mxb = lb * sg;
-    ubv[d] += mxb;
-    const double csb = mxb * dcs;
+    // cotangents of the intermediates; physical flux f_d: (m_d, m_x u_d (+P),
+    // m_y u_d (+P), m_z u_d (+P), (E+P) u_d)
+    const double mxb = lb * sg, csb = mxb * dcs, hb = dmul_rn(pb[4], ud);
+    double udb = mxb + pb[1] * m[0] + pb[2] * m[1] + pb[3] * m[2] + pb[4] * (rhoet + P);
+    double Pb = pb[1 + d] + hb, rinvb = 0.0;
     if (cs > 0.0) {
-      const double h = csb * gam / (2.0 * cs);
+      const double h = ddiv_rn(csb * gam, 2.0 * cs);
       Pb += h * rhoinv;
-      rinvb += h * P;
+      rinvb = h * P;
     }
-    // u_a = m_a * rhoinv
+    // u_d = m_d * rhoinv;  P = (gam-1) (E - rhoekin), rhoekin = rhoinv (m.m) / 2
+    rinvb += udb * m[d];
+    const double eb = (gam - 1.0) * Pb, Eb = hb + eb;
+    rinvb -= 0.5 * mm * eb;
+    const double kb = dmul_rn(rhoinv, -eb);
+    double mb[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      mb[a] += ubv[a] * rhoinv;
-      rinvb += ubv[a] * m[a];
-    }
-    // P = (gam-1) (E - rhoekin), rhoekin = rhoinv (m.m) / 2
-    Eb += (gam - 1.0) * Pb;
-    const double kb = -(gam - 1.0) * Pb;
-    rinvb += 0.5 * (m[0] * m[0] + m[1] * m[1] + m[2] * m[2]) * kb;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) mb[a] += rhoinv * m[a] * kb;
+    for (int a = 0; a < 3; ++a) mb[a] = pb[1 + a] * ud + m[a] * kb;
+    mb[d] += pb[0] + udb * rhoinv;
     const double rb = -rhoinv * rhoinv * rinvb;
     // direct U cotangents through alpha*U
     const long long ob = ubar.off(c[0], c[1], c[2]);
@@ -237,7 +225,10 @@ cudaError_t launch_weno_vjp(const BoxTable& tb, const FaceRec& fr, const DArr& v
     launch_dep(weno_vjp_face_kernel, grid_n(fb.nf, nsm), 256, 0, st, tb, fr, vbar, fb, d, fb.nf);
     const int m0 = n[0] + (d == 0 ? 6 : 0), m1 = n[1] + (d == 1 ? 6 : 0), m2 = n[2] + (d == 2 ? 6 : 0);
     const long long tot = (long long)m0 * m1 * m2;
-    launch_dep(weno_vjp_gather_kernel, grid_n(tot, nsm), 256, 0, st, tb, ubar, fb, d, m0, m1, tot);
+    const int gg = grid_n(tot, nsm);
+    if (d == 0) launch_dep(weno_vjp_gather_kernel<0>, gg, 256, 0, st, tb, ubar, fb, m0, m1, tot);
+    else if (d == 1) launch_dep(weno_vjp_gather_kernel<1>, gg, 256, 0, st, tb, ubar, fb, m0, m1, tot);
+    else launch_dep(weno_vjp_gather_kernel<2>, gg, 256, 0, st, tb, ubar, fb, m0, m1, tot);
   }
   return cudaGetLastError();
 }
