@@ -833,11 +833,11 @@ __device__ __forceinline__ void riemann_prob(const double gamma, const double sm
   }
 }
 
-// MUSCL face states + Riemann flux (src/rhs/Riemann.h:251-337).  Bound: the
-// solver's serial chain of quotients and roots, with both the FP64 and the
-// integer pipe about half full; two CTAs per SM (128 registers) beat three
-// (2.94 against 3.10 ms per step at 96^3).  48^3, with the hardware's roots and
-// products and checked integer quotients before: 194 -> 86 us.
+// MUSCL face states + Riemann flux (src/rhs/Riemann.h:251-337).  Bound: the FP64
+// pipe (77% busy at 128^3, 118 instructions a face) behind the solver's serial chain
+// of quotients and roots; two CTAs per SM (128 registers) beat three (2.94 against
+// 3.10 ms per step at 96^3).  48^3, with the hardware's roots and products and
+// checked integer quotients before: 194 -> 86 us.
 template <bool VISC>
 __global__ void __launch_bounds__(256, 2) riemann_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
   dep_begin();

@@ -1031,9 +1031,8 @@ cudaError_t launch_avgdown(const DArr& fine, const DArr& crse, const int lo[3], 
 
 // ----------------------------------------------------- timeout probe ----
 // The error path of the bounded waits, without a hang: one thread waits on
-// an mbarrier that nothing arrives at, with the same bounded wait the face
-// kernel uses (at most `polls` polls), gives up, raises the error flag and
-// returns.
+// an mbarrier that nothing arrives at, with a bounded wait (at most `polls`
+// polls), gives up, raises the error flag and returns.
 __global__ void wait_timeout_probe_kernel(int* err, long long polls) {
   __shared__ unsigned long long bar;
   mbar_init(&bar, 1);

@@ -78,7 +78,7 @@ class Scheme:
 
     weno_fast (not a reference switch): 0 (default) evaluates WENO5 in the
     reference's operation order (bit-identical results); 1 forms the weights
-    over a common denominator (faster, rounding differences only).
+    over a common denominator (rounding differences only; no longer the faster form).
 
     rhs_source: cns.rhs_source; the source is the problem's user_source,
     here a constant body force per unit mass `body_force` (the channel

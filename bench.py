@@ -8,7 +8,7 @@ faces/divergence/stage update]).  Metric: cell-updates/s per RK3 step.
 Also reported on the same JSON line:
   e2e       the same step through the public API with host buffers: H2D of
             U^n from pinned memory, the step, D2H of U^{n+1}, every step;
-  roofline  the fused face kernel against the measured FP64 FMA peak (this
+  roofline  the face kernels against the measured FP64 FMA peak (this
             path is FP64-pipe bound on GB300), with its algorithmic flops from
             the oracle's operation counts;
   batched   512 uneven boxes, one SSPRK3 step: one persistent launch per
@@ -50,17 +50,17 @@ UNIT = "cell-updates/s"
 
 # --scheme: (switches, op-count key, dominant kernel, its ncu summary, kernels of ours per stage, label)
 SCHEMES = {
-    "keep4": (dict(flux_euler=1, order_keep=4, rhs_visc=1), "keep4_visc", "keep_face_kernel<4,true,false>",
-              "keep_face_kernel_tgv128.md", 4, "KEEP4 + viscous"),
+    "keep4": (dict(flux_euler=1, order_keep=4, rhs_visc=1), "keep4_visc",
+              "keep_march_kernel<4,true> + keep_x_kernel<4,true,false>", "keep_march_x_kernels_tgv128.md", 5, "KEEP4 + viscous"),
     "weno": (dict(flux_euler=2, rhs_visc=1), "weno_visc", "weno_face_kernel<true> (reference operation order)",
-             "weno_face_kernel_tgv96.md", 7, "WENO5-LLF + viscous, reference operation order"),
+             "weno_face_kernel_tgv96.md", 6, "WENO5-LLF + viscous, reference operation order"),
     "weno_fast": (dict(flux_euler=2, rhs_visc=1, weno_fast=1), "weno_visc",
-                  "weno_face_kernel<false> (common-denominator weights)", "weno_fast_face_kernel_tgv96.md", 7,
+                  "weno_face_kernel<false> (common-denominator weights)", "weno_fast_face_kernel_tgv96.md", 6,
                   "WENO5-LLF + viscous, common-denominator weights"),
     "muscl": (dict(flux_euler=0, rhs_visc=1), "muscl_visc", "slope_kernel + riemann_face_kernel",
-              "riemann_face_kernel_tgv128.md", 7, "MUSCL-Riemann + viscous"),
+              "riemann_face_kernel_tgv128.md", 6, "MUSCL-Riemann + viscous"),
     "weno_riemann": (dict(flux_euler=0, riemann_weno=1, rhs_visc=1), "weno_riemann_visc", "weno_riemann_face_kernel",
-                     "weno_riemann_face_kernel_tgv128.md", 6,
+                     "weno_riemann_face_kernel_tgv128.md", 5,
                      "WENO5-Riemann (extension) + viscous"),
 }
 

@@ -74,7 +74,8 @@ typedef struct amrs_scheme {
    * reference's operation order (src/rhs/High_resolution.h:124-159),
    * bit-identical to its CPU build.  1: each reconstruction forms its three
    * nonlinear weights over a common denominator with fused multiply-adds
-   * (one division instead of four, about 1.7x faster): the same function in
+   * (one division instead of four; slower than 0, whose products and divisions
+   * run on the integer pipe): the same function in
    * exact arithmetic, rounding differences only, which the flux
    * differencing amplifies where the RHS is small next to the split fluxes
    * (near-incompressible flow: up to ~1e-9 relative on the mass RHS). */
@@ -483,14 +484,15 @@ amrs_status amrs_probe_intpipe(amrs_handle* h, int32_t mode, double* ms);
 /* Per-kernel timing of one RK stage of one box: CUDA events around the
  * kernels on `stream`, averaged over `reps`.  ms[0] primitives (plus the
  * WENO5 point fluxes), ms[1] viscous cell fluxes, ms[2] the Euler face
- * kernel (on the fused KEEP path: faces + viscous averages + divergence +
- * stage program; on the MUSCL-Riemann path: slopes + Riemann faces), ms[3]
+ * kernels (on the fused KEEP path: march and x kernel, that is faces + viscous
+ * averages + divergence + stage program; on the MUSCL-Riemann path: slopes + Riemann faces), ms[3]
  * the whole stage.  Host-synchronising. */
 amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const double dxinv[3],
                                    const amrs_stage_prog* prog, amrs_array4 stage_in, amrs_array4 s1,
                                    amrs_array4 out, int32_t reps, void* stream, double* ms);
-/* 1 if the fused face kernel stages planes with TMA for the handle's last
- * per-box call (resp. for the box list), 0 if with plain loads, -1 if none. */
+/* 0 if the handle has made a per-box call (resp. for any box list): the face
+ * kernels read global memory with plain loads; -1 if not.  (1 stood for planes
+ * staged by TMA.) */
 int32_t amrs_debug_tma_enabled(amrs_handle* h);
 int32_t amrs_boxlist_tma_enabled(amrs_boxlist* bl);
 
