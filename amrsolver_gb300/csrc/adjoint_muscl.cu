@@ -34,7 +34,6 @@ namespace amrs {
 namespace {
 
 using rpvjp::riemann_prob_vjp;
-using rpvjp::sgn1;
 
 constexpr int FSLOT = 10;  // per face: left prims (5), right prims (5); the terms' are +-1/2 of them
 constexpr int SSLOT = 19;  // per cell: Qbar at c-1 (6, T unused), c (6), c+1 (6, T unused), T at c+2 (1, z only)
@@ -112,31 +111,47 @@ __global__ void __launch_bounds__(256, 3) muscl_vjp_face_kernel(const __grid_con
   }
 }
 
-// MC limiter (src/rhs/Riemann.h:9-17) and its reverse along the taken case.
-__device__ __forceinline__ void mc_vjp(double l, double r, double db, double& lb, double& rb) {
-  const double dcen = 0.5 * (l + r);
-  const double dsgn = copysign(1.0, dcen);
-  const double al = fabs(l), ar = fabs(r);
-  const bool rsmall = ar < al;                 // rmin(|l|, |r|) takes |r|
-  const double slop = 2.0 * (rsmall ? ar : al);
-  const bool same = l * r >= 0.0;
-  const double dlim = same ? slop : 0.0;
-  const double ac = fabs(dcen);
-  const bool take_c = ac < dlim;               // rmin(dlim, |dcen|) takes |dcen|
-  if (take_c) {
-    // dsgn * |dcen| = dcen
-    lb += 0.5 * db;
-    rb += 0.5 * db;
-  } else if (same) {
-    // dsgn * 2 min(|l|, |r|)
-    const double sb = dsgn * 2.0 * db;
-    if (rsmall) rb += sb * sgn1(r);
-    else lb += sb * sgn1(l);
+// Which case of the MC limiter (src/rhs/Riemann.h:9-17) holds for l and r:
+//   sgn(dcen) min(2 min(|l|, |r|) if l r >= 0 else 0, |dcen|), dcen = (l + r) / 2.
+// The order of magnitudes is that of the words without their signs, so the
+// comparisons stay off the FP64 pipe (with a NaN among l and r, l r is one and
+// the limiter 0 either way).
+struct McCase {
+  double dcen, slop;  // slop = 2 min(|l|, |r|)
+  bool same, rsmall, take_c, zero;  // zero: slop is
+  __device__ __forceinline__ McCase(double l, double r) {
+    auto mag = [](DWords w) { return (unsigned long long)(w.hi & 0x7FFFFFFFu) << 32 | w.lo; };
+    dcen = 0.5 * (l + r);
+    const unsigned long long al = mag(dwords(l)), ar = mag(dwords(r));
+    rsmall = ar < al;  // rmin(|l|, |r|) takes |r|
+    const unsigned long long m = rsmall ? ar : al;
+    slop = 2.0 * dfrom((uint32_t)(m >> 32), (uint32_t)m);
+    const DWords p = dwords(l * r);
+    zero = m == 0ull;
+    same = mag(p) == 0ull || (p.hi <= 0x7FF00000u && mag(p) <= 0x7FF0000000000000ull);
+    take_c = same && mag(dwords(dcen)) < mag(dwords(slop));  // rmin(dlim, |dcen|) takes |dcen|
   }
-}
+  __device__ __forceinline__ static double with_sign(double x, double s) {  // x sgn(s)
+    DWords w = dwords(x);
+    w.hi ^= dwords(s).hi & 0x80000000u;
+    return dfrom(w);
+  }
+  __device__ __forceinline__ double value() const {
+    return take_c ? dcen : with_sign(same ? slop : 0.0, dcen);
+  }
+  // the cotangents of l and r along the taken case
+  __device__ __forceinline__ void vjp(double l, double r, double db, double& lb, double& rb) const {
+    const double h = (take_c ? 0.5 : 2.0) * db;
+    // sgn(dcen) 2 db sgn(the smaller), where either zero counts as positive
+    const double s = with_sign(with_sign(h, dcen), zero ? 0.0 : (rsmall ? r : l));
+    lb = take_c ? h : (same && !rsmall ? s : 0.0);
+    rb = take_c ? h : (same && rsmall ? s : 0.0);
+  }
+};
 
-// Two, three or four CTAs per SM take the same time (2625, 2616, 2619 us for the
-// gradient of a step at 48^3).
+// Bound: the FP64 pipe (80% busy); 45 to 52 us a direction at 48^3, 35 to 38 with
+// the limiter's cases decided on words.  Two, three or four CTAs per SM take the
+// same time (2625, 2616, 2619 us for the gradient of a step then).
 template <int d>
 __global__ void __launch_bounds__(256, 3) muscl_vjp_slope_kernel(const __grid_constant__ BoxTable tb,
                                                                                FBuf fs, SBuf ss, long long total) {
@@ -170,16 +185,8 @@ __global__ void __launch_bounds__(256, 3) muscl_vjp_slope_kernel(const __grid_co
     const double l0 = ddiv_rn(0.5 * dpl, cs) - 0.5 * rc * dul, r0 = ddiv_rn(0.5 * dpr, cs) - 0.5 * rc * dur;
     const double l1 = drl - ddiv_rn(dpl, cs2), r1 = drr - ddiv_rn(dpr, cs2);
     const double l2 = ddiv_rn(0.5 * dpl, cs) + 0.5 * rc * dul, r2 = ddiv_rn(0.5 * dpr, cs) + 0.5 * rc * dur;
-    auto mc = [](double a, double b) {
-      const double dcen = 0.5 * (a + b);
-      const double dsgn = copysign(1.0, dcen);
-      const double aa = fabs(a), ab = fabs(b);
-      const double slop = 2.0 * ((ab < aa) ? ab : aa);
-      const double dlim = (a * b >= 0.0) ? slop : 0.0;
-      const double ac = fabs(dcen);
-      return dsgn * ((ac < dlim) ? ac : dlim);
-    };
-    const double d0 = mc(l0, r0), d2 = mc(l2, r2);
+    const McCase c_0(l0, r0), c_2(l2, r2);
+    const double d0 = c_0.value(), d2 = c_2.value();
     const double s02 = d0 + d2;
     // the cotangents of the two faces' states at this cell: the primitives', and
     // through q + terms/2 (face c+1), q - terms/2 (face c) the terms'
@@ -225,13 +232,12 @@ __global__ void __launch_bounds__(256, 3) muscl_vjp_slope_kernel(const __grid_co
     d0b += s02b;
     d2b += s02b;
     // limiters
-    double l0b = 0.0, r0b = 0.0, l1b = 0.0, r1b = 0.0, l2b = 0.0, r2b = 0.0, l3b = 0.0, r3b = 0.0, l4b = 0.0,
-           r4b = 0.0;
-    mc_vjp(l0, r0, d0b, l0b, r0b);
-    mc_vjp(l1, r1, d1b, l1b, r1b);
-    mc_vjp(l2, r2, d2b, l2b, r2b);
-    mc_vjp(d1l, d1r, d3b, l3b, r3b);
-    mc_vjp(d2l, d2r, d4b, l4b, r4b);
+    double l0b, r0b, l1b, r1b, l2b, r2b, l3b, r3b, l4b, r4b;
+    c_0.vjp(l0, r0, d0b, l0b, r0b);
+    McCase(l1, r1).vjp(l1, r1, d1b, l1b, r1b);
+    c_2.vjp(l2, r2, d2b, l2b, r2b);
+    McCase(d1l, d1r).vjp(d1l, d1r, d3b, l3b, r3b);
+    McCase(d2l, d2r).vjp(d2l, d2r, d4b, l4b, r4b);
     // characteristic differences
     double csb = 0.0;
     double dplb = 0.5 * (l0b + l2b) * ics - l1b * ics2, dprb = 0.5 * (r0b + r2b) * ics - r1b * ics2;
