@@ -161,6 +161,13 @@ __device__ __forceinline__ double mul_zero(double a, double b, bool zero) {
   return dfrom(zero ? (x.hi ^ y.hi) & 0x80000000u : r.hi, zero ? 0u : r.lo);
 }
 
+// The same with the sign bit of `sg` for a zero (the words of a product with a
+// zero factor are not a zero's, so nothing can be read from them).
+__device__ __forceinline__ double mul_zero(double a, double b, bool zero, uint32_t sg) {
+  const DWords r = dmul_core(dwords(a), dwords(b));
+  return dfrom(zero ? sg & 0x80000000u : r.hi, zero ? 0u : r.lo);
+}
+
 // One KEEP pair term (src/rhs/CentralKEEP.h:19-36 helpers, :76-83 body),
 // already multiplied by its coefficient: the contribution of pair
 // (point 1 = larger index, point 2 = smaller index) to the face flux in
@@ -188,7 +195,8 @@ __device__ __forceinline__ void keep_pair(const double* q1, const double* q2, do
     // P is zero exactly when unS is, and with it every term but the pressure's;
     // D's own momentum term P unS + 4 psum is positive
     const bool zP = is_zero(unS);
-    const double P = mul_core(rhoS, unS);
+    const double P = mul_core(rhoS, unS);  // not read where zP; its sign is that of unS
+    const uint32_t gP = dwords(unS).hi, gT = gP ^ dwords(c8).hi;
     double vS[3], s[3];
     bool z[3];
 #pragma unroll
@@ -199,14 +207,15 @@ __device__ __forceinline__ void keep_pair(const double* q1, const double* q2, do
       z[c] = zP || is_zero(vS[c]);
     }
     const double s3 = s[0] + s[1] + s[2];
-    T[URHO] = mul_zero(c4, P, zP);
+    T[URHO] = mul_zero(c4, P, zP, gT);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      if (c == D) T[UMX + c] = mul_core(c8, fma(4.0, psum, mul_zero(P, vS[c], zP)));
-      else T[UMX + c] = mul_zero(c8, mul_core(P, vS[c]), z[c]);
+      if (c == D) T[UMX + c] = mul_core(c8, fma(4.0, psum, mul_zero(P, vS[c], zP, 0u)));
+      else T[UMX + c] = mul_zero(c8, mul_core(P, vS[c]), z[c], gT ^ dwords(vS[c]).hi);
     }
     const double pu = mul_zero(q1[QPRES], q2[QN], is_zero(q2[QN])) + mul_zero(q2[QPRES], q1[QN], is_zero(q1[QN]));
-    const double en = fma(4.0, pu, mul_zero(P, s3, zP || is_zero(s3)) + mul_zero(P, eS, zP));
+    const double en =
+        fma(4.0, pu, mul_zero(P, s3, zP || is_zero(s3), gP ^ dwords(s3).hi) + mul_zero(P, eS, zP, gP));
     T[UET] = mul_zero(c8, en, is_zero(en));
   } else {
     const double P = rhoS * unS;
