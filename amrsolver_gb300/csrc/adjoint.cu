@@ -396,10 +396,13 @@ __global__ void __launch_bounds__(256, 4) adj_gather_kernel(const __grid_constan
 // Reverse of one stage's BLAS-1 program per valid cell: given the cotangent
 // of the stage result (register S2), the cotangents of S1 (c1 times it), of the
 // stage input's valid values (c2, register S2 before the program) and of dSdt
-// (cd).  A coefficient of zero adds nothing and reads nothing.  64^3: 20 us
+// (cd).  A register that the program does not read (its bit of `used` is clear)
+// gets nothing, and its array is not read; a coefficient that is zero still
+// multiplies, so a NaN or an infinity of the cotangent shows.  64^3: 20 us
 // with the program reversed per value, 12 now; bound by memory.
-__global__ void __launch_bounds__(256) adj_prog_kernel(BoxRec R, double c1, double c2, double cd, DArr wbar, DArr s1bar,
-                                                       DArr inbar, DArr vbar, long long total, int accumulate) {
+__global__ void __launch_bounds__(256) adj_prog_kernel(BoxRec R, double c1, double c2, double cd, int used, DArr wbar,
+                                                       DArr s1bar, DArr inbar, DArr vbar, long long total,
+                                                       int accumulate) {
   dep_begin();
   const int nx = R.hi[0] - R.lo[0] + 1, ny = R.hi[1] - R.lo[1] + 1;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -409,17 +412,18 @@ __global__ void __launch_bounds__(256) adj_prog_kernel(BoxRec R, double c1, doub
     double w[5];
 #pragma unroll
     for (int n = 0; n < 5; ++n) w[n] = wbar(i, j, k, n);
-    auto give = [&](const DArr& to, double c, bool add) {
-      if (add && c == 0.0) return;
+    auto give = [&](const DArr& to, int reg, double c, bool add) {
+      const bool any = (used >> reg) & 1;
+      if (add && !any) return;
       double v[5];
 #pragma unroll
       for (int n = 0; n < 5; ++n) v[n] = add ? to(i, j, k, n) : 0.0;
 #pragma unroll
-      for (int n = 0; n < 5; ++n) to(i, j, k, n) = v[n] + (c == 0.0 ? 0.0 : c * w[n]);
+      for (int n = 0; n < 5; ++n) to(i, j, k, n) = v[n] + (any ? c * w[n] : 0.0);
     };
-    give(s1bar, c1, accumulate);
-    give(inbar, c2, accumulate);
-    give(vbar, cd, false);
+    give(s1bar, 0, c1, accumulate);
+    give(inbar, 1, c2, accumulate);
+    give(vbar, 2, cd, false);
   }
 }
 
@@ -571,25 +575,34 @@ cudaError_t launch_adj_prog(const BoxRec& R, const DProg& prog, const DArr& wbar
   const long long n = (long long)(R.hi[0] - R.lo[0] + 1) * (R.hi[1] - R.lo[1] + 1) * (R.hi[2] - R.lo[2] + 1);
   // the program is linear in its registers: its reverse on the unit cotangent
   double b[3] = {0.0, 1.0, 0.0};
+  bool used[3] = {false, true, false};
   for (int o = prog.nops - 1; o >= 0; --o) {
     const DOp& q = prog.ops[o];
     const double g = b[q.dst];
+    const bool u = used[q.dst];
     if (q.kind == 0) {
       b[q.dst] = 0.0;
+      used[q.dst] = false;
       b[q.x] += q.a * g;
       b[q.y] += q.b * g;
+      used[q.x] = used[q.x] || u;
+      used[q.y] = used[q.y] || u;
     } else if (q.kind == 1) {
       b[q.x] += q.a * g;
+      used[q.x] = used[q.x] || u;
     } else if (q.kind == 2) {
       b[q.dst] = q.a * g;
       b[q.x] += g;
+      used[q.x] = used[q.x] || u;
     } else {
       b[q.dst] = 0.0;
+      used[q.dst] = false;
       b[q.x] += g;
+      used[q.x] = used[q.x] || u;
     }
   }
-  launch_dep(adj_prog_kernel, grid256(n, nsm), 256, 0, st, R, b[0], b[1], b[2], wbar, s1bar, inbar, vbar, n,
-             accumulate);
+  launch_dep(adj_prog_kernel, grid256(n, nsm), 256, 0, st, R, b[0], b[1], b[2], used[0] + 2 * used[1] + 4 * used[2], wbar,
+             s1bar, inbar, vbar, n, accumulate);
   return cudaGetLastError();
 }
 
