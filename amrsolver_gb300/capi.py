@@ -152,6 +152,7 @@ SIGNATURES = {
     "amrs_profile_stage_box": (_S, [_P, ctypes.POINTER(CBox), ctypes.POINTER(ctypes.c_double),
                                     ctypes.POINTER(StageProg), Array4, Array4, Array4, ctypes.c_int32, _P,
                                     ctypes.POINTER(ctypes.c_double)]),
+    "amrs_debug_keep_plain_stages": (_S, [_P, _P, ctypes.POINTER(ctypes.c_uint32)]),
     "amrs_debug_tma_enabled": (ctypes.c_int32, [_P]),
     "amrs_boxlist_tma_enabled": (ctypes.c_int32, [_P]),
 }
@@ -313,6 +314,12 @@ class Handle:
 
     def sync_check(self, stream=None):
         check(self._L.amrs_sync_check(self.h, _stream_ptr(stream)), "amrs_sync_check")
+
+    def keep_plain_stages(self):
+        """Stages of the current box that ran on the FP64 pipe (amrs_debug_keep_plain_stages)."""
+        n = ctypes.c_uint32()
+        check(self._L.amrs_debug_keep_plain_stages(self.h, None, ctypes.byref(n)), "amrs_debug_keep_plain_stages")
+        return n.value
 
     def tma_enabled(self):
         return int(self._L.amrs_debug_tma_enabled(self.h))
@@ -551,6 +558,13 @@ class BoxList:
         check(self._L.amrs_rk_step_boxlist(self.bl, order_rk, stages_rk, float(dt), s1, w1, w2, int(use_graph),
                                            _stream_ptr(stream), ctypes.byref(res)), "amrs_rk_step_boxlist")
         return res.value
+
+    def keep_plain_stages(self):
+        """Stages of this list that ran on the FP64 pipe (amrs_debug_keep_plain_stages)."""
+        n = ctypes.c_uint32()
+        check(self._L.amrs_debug_keep_plain_stages(self.handle.h, self.bl, ctypes.byref(n)),
+              "amrs_debug_keep_plain_stages")
+        return n.value
 
     def tma_enabled(self):
         return int(self._L.amrs_boxlist_tma_enabled(self.bl))

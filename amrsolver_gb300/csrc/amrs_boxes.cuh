@@ -27,6 +27,19 @@ struct BoxRec {
   int red_lo, red_hi;
 };
 
+// The KEEP path's range flag of a list, by stage numbers instead of clears, so that
+// it holds whatever launches follow each other (a recorded step of any number
+// of stages, one stage alone): the primitives' kernel takes the number `stage`,
+// passes it on in `face` and marks a cell outside keep_range by raised = stage +
+// 1; the face kernels see raised == face + 1 (every product on the FP64 pipe
+// then), and the x kernel sets stage = face + 1.  No block reads a word that another
+// block of its kernel writes.  All zero at first; `plain` counts the stages that ran on
+// the FP64 pipe.
+struct alignas(16) KeepRange {
+  unsigned face, raised;
+  unsigned stage, plain;
+};
+
 // Prefix tables for flattening launches over boxes.
 struct BoxTable {
   const BoxRec* box;
@@ -41,11 +54,8 @@ struct BoxTable {
   // device-resident time loop: every kernel of a step returns at once while
   // *active == 0 (steps after the stop time); null outside such loops
   const int* active;
-  // raised by the primitives' kernel where a cell is outside keep_range; the
-  // face kernel of the same stage reads it (raised or null: every product on
-  // the FP64 pipe) and clears the other of the pair, the next stage's
-  int* range;
-  int* range_next;
+  // whether a cell of this stage is outside keep_range; null: taken as if one were
+  KeepRange* range;
   long long tot_p, tot_v, tot_m;  // cells of the primitive and viscous regions, march items
   // a list of one box carries its record and closures in the launch itself, so
   // that a kernel's first load is already data and per-box calls copy nothing

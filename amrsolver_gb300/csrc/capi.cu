@@ -239,7 +239,6 @@ struct List {
   int tot_work = 0;
   int face_grid = 0;  // CTAs of the balanced face-kernel schedule
   KeepGrid grid;      // launch shape of the fused path's face kernels
-  int* d_range = nullptr;  // the fused path's two range flags (BoxTable::range), used by turns
   int waves = 1;      // shares of the schedule per resident CTA (amrs_boxlist_set_schedule)
   cudaGraphExec_t graph = nullptr;
   int graph_key[6] = {0, 0, 0, 0, 0, 0};
@@ -460,7 +459,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   for (int d = 0; d < 3; ++d) { o_s[d] = t; t = align_up(t + 8 * (n + 1), 128); }
   const size_t o_w = t; t = align_up(t + 4 * (n + 1), 128);
   const size_t o_mi = t; t = align_up(t + 8 * (n + 1), 128);
-  const size_t o_rng = t; t = align_up(t + 2 * sizeof(int), 128);
+  const size_t o_rng = t; t = align_up(t + sizeof(KeepRange), 128);
   if (t > L.dtab_bytes) {
     if (L.dtab) { cudaFree(L.dtab); L.dtab = nullptr; L.dtab_bytes = 0; }
     CK(cudaMalloc(&L.dtab, t));
@@ -490,9 +489,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   L.tb.cls = reinterpret_cast<const DClosures*>(D + o_cls);
   L.tb.n = n;
   L.tb.gq = L.gq;
-  L.d_range = L.fused ? reinterpret_cast<int*>(D + o_rng) : nullptr;
-  L.tb.range = L.d_range;
-  L.tb.range_next = L.d_range ? L.d_range + 1 : nullptr;
+  L.tb.range = L.fused ? reinterpret_cast<KeepRange*>(D + o_rng) : nullptr;
   L.ft.fr = reinterpret_cast<const FaceRec*>(D + o_face);
   for (int d = 0; d < 3; ++d) {
     L.ft.fpre[d] = reinterpret_cast<const long long*>(D + o_f[d]);
@@ -529,7 +526,6 @@ amrs_status list_stage(amrs_handle* h, List& L, const DProg& prog, int s_in, int
                        cudaStream_t st) {
   const amrs_scheme& sc = L.sc;
   const int nsm = h->nsm;
-  if (L.d_range) std::swap(L.tb.range, L.tb.range_next);
   // 1. primitives over the grown boxes
   if (L.gq > 0 || sc.rhs_visc) CK(launch_prims(L.tb, s_in, L.tot_p, nsm, st));
   // 2. viscous cell fluxes
@@ -1492,7 +1488,9 @@ amrs_status adj_prepare(amrs_handle* h, const amrs_box& B, AdjScratch& S, cudaSt
 // then the WENO5, MUSCL-Riemann or WENO5-Riemann Euler part.
 cudaError_t rhs_vjp_launch(amrs_handle* h, List& L, const amrs_box& B, AdjScratch& S, double* param_bar,
                            cudaStream_t st) {
-  cudaError_t e = launch_prims(L.tb, 0, L.tot_p, h->nsm, st);
+  BoxTable prims = L.tb;
+  prims.range = nullptr;  // no forward face kernel follows
+  cudaError_t e = launch_prims(prims, 0, L.tot_p, h->nsm, st);
   if (e == cudaSuccess) e = launch_rhs_vjp(S.order, L.tb, S.ah, param_bar, h->nsm, st);
   if (e == cudaSuccess && weno_scheme(h->sc)) {
     const int nb[3] = {bn(B, 0), bn(B, 1), bn(B, 2)};
@@ -1890,6 +1888,17 @@ amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const dou
   for (int i = 0; i < 5; ++i) cudaEventDestroy(ev[i]);
   if (rs) return rs;
   for (int i = 0; i < 4; ++i) ms[i] = acc[i] / reps;
+  return AMRS_OK;
+}
+
+amrs_status amrs_debug_keep_plain_stages(amrs_handle* h, amrs_boxlist* bl, uint32_t* count) {
+  if (!h || !count) return AMRS_ERR_NULL;
+  std::lock_guard<std::mutex> lk(h->mu);
+  CK(cudaSetDevice(h->device));
+  CK(cudaDeviceSynchronize());
+  const List* L = bl ? &bl->L : h->one;
+  *count = 0;
+  if (L && L->tb.range) CK(cudaMemcpy(count, &L->tb.range->plain, sizeof(*count), cudaMemcpyDeviceToHost));
   return AMRS_OK;
 }
 

@@ -200,7 +200,7 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   const size_t o_p = t; t = al(t + sizeof(pcell));
   const size_t o_v = t; t = al(t + sizeof(vcell));
   const size_t o_w = t; t = al(t + sizeof(fwork));
-  const size_t o_rng = t; t = al(t + sizeof(int));
+  const size_t o_rng = t; t = al(t + sizeof(KeepRange));
   const size_t o_mi = t; t = al(t + sizeof(mitem));
   if (t > NA_TABLE_BYTES) return AMRS_ERR_SIZE;
   char* host = g_na_host;
@@ -232,7 +232,7 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   tb.rec = R;
   tb.rec_cls = cl;
   tb.gq = gq;
-  tb.range = reinterpret_cast<int*>(tab + o_rng);
+  tb.range = reinterpret_cast<KeepRange*>(tab + o_rng);
   DProg prog{};
   if (launch_prims(tb, 0, pcell[1], nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;
   if (sc.rhs_visc && launch_visc(tb, vcell[1], nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;

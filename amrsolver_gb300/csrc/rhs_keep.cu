@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(256, 5) prims_kernel(const __grid_constant__ B
   if (list_idle(tb)) return;
   const long long total = tb.tot_p;
   const int g = tb.gq;
+  if (tb.range && blockIdx.x == 0 && threadIdx.x == 0) tb.range->face = tb.range->stage;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total;
        c += (long long)gridDim.x * blockDim.x) {
     const int b = find_box_ll(tb.pcell, tb.n, c);
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(256, 5) prims_kernel(const __grid_constant__ B
     for (int n = 0; n < 5; ++n) u[n] = U.p[o + n * U.ns];
     double q[NQ];
     cons2prim(u, q, box_cls(tb, R));
-    if (tb.range && !keep_range(q)) *tb.range = 1;
+    if (tb.range && !keep_range(q)) tb.range->raised = tb.range->stage + 1u;
     const long long oq = R.q.off(i, j, k);
 #pragma unroll
     for (int n = 0; n < NQ; ++n) R.q.p[oq + n * R.q.ns] = q[n];
@@ -358,8 +359,10 @@ __device__ __forceinline__ void keep_march(const BoxRec& R, int blk, int m0, int
 // (two CTAs: 288 instead of 272 us per step of 45 x 33 x 27).
 template <int ORDER> constexpr int march_ctas() { return ORDER == 6 ? 1 : 2; }
 
-// range flag of the stage (BoxTable::range), uniform over the grid
-__device__ __forceinline__ bool fast_range(const BoxTable& tb) { return tb.range && *tb.range == 0; }
+// every cell of the stage is inside keep_range (BoxTable::range), uniform over the grid
+__device__ __forceinline__ bool fast_range(const BoxTable& tb) {
+  return tb.range && tb.range->raised != tb.range->face + 1u;
+}
 
 template <int ORDER, bool VISC, bool FAST>
 __device__ __forceinline__ void keep_march_warp(const BoxTable& tb) {
@@ -407,8 +410,12 @@ keep_x_kernel(const __grid_constant__ BoxTable tb, int s_in, int s_s1, int s_out
   const DProg prog = resolve_prog(prog_in);
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double* smem = reinterpret_cast<double*>(smem_raw);
-  if (tb.range_next && blockIdx.x == 0 && threadIdx.x == 0) *tb.range_next = 0;
-  if (fast_range(tb)) keep_x_body<ORDER, VISC, SRC, true>(tb, s_in, s_s1, s_out, prog, rhs_only, smem);
+  const bool fast = fast_range(tb);
+  if (tb.range && blockIdx.x == 0 && threadIdx.x == 0) {
+    tb.range->stage = tb.range->face + 1u;
+    if (!fast) ++tb.range->plain;
+  }
+  if (fast) keep_x_body<ORDER, VISC, SRC, true>(tb, s_in, s_s1, s_out, prog, rhs_only, smem);
   else keep_x_body<ORDER, VISC, SRC, false>(tb, s_in, s_s1, s_out, prog, rhs_only, smem);
 }
 

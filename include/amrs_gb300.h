@@ -490,6 +490,11 @@ amrs_status amrs_probe_intpipe(amrs_handle* h, int32_t mode, double* ms);
 amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const double dxinv[3],
                                    const amrs_stage_prog* prog, amrs_array4 stage_in, amrs_array4 s1,
                                    amrs_array4 out, int32_t reps, void* stream, double* ms);
+/* Stages that the fused KEEP path of the list (null: of the handle's per-box calls
+ * of the current box) ran with every product on the FP64 pipe because a cell was
+ * outside the ranges of the integer-pipe form, since the list was built.  The
+ * results are the same bits either way.  Host-synchronising. */
+amrs_status amrs_debug_keep_plain_stages(amrs_handle* h, amrs_boxlist* bl, uint32_t* count);
 /* 0 if the handle has made a per-box call (resp. for any box list): the face
  * kernels read global memory with plain loads; -1 if not.  (1 stood for planes
  * staged by TMA.) */
