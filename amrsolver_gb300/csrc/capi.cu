@@ -213,6 +213,23 @@ void set_walls(BoxRec& R, const WallCfg& w, const amrs_scheme& sc) {
 }
 
 // -------------------------------------------------------------- list ----
+// What one launch of the KEEP face kernels covers: whole boxes b0 .. b0 + nb - 1, or
+// the planes z0 .. z1 of box b0 (z1 >= z0).  The y and z parts of the divergence
+// (BoxRec::div) need memory only between the two kernels of a piece, so all pieces
+// share it, and a list holds at most DIV_BYTES of it (or one plane of a box): 27
+// million cells, 300^3, which fill the chip many times over.  (In full it would be
+// 80 bytes a cell beside the 152 of the primitives and viscous fluxes.)
+constexpr size_t DIV_BYTES = (size_t)1 << 31;
+struct FacePiece {
+  int b0 = 0, nb = 1;
+  int z0 = 0, z1 = -1;
+  int t0 = 0;            // of its prefix tables (nb + 1 entries) in List::mitem and ::fwork
+  int nshare = 0;
+  long long items = 0;   // of the marches
+  KeepGrid grid;         // launch shape
+  bool slab() const { return z1 >= z0; }
+};
+
 // Host + device state of one box list (a level, or one box for the per-box
 // entry points).
 struct List {
@@ -225,6 +242,7 @@ struct List {
   std::vector<FaceRec> hface;
   std::vector<long long> pcell, vcell, gcell, valid, mitem, fpre[3], spre[3];
   std::vector<int> fwork;
+  std::vector<FacePiece> pieces;  // of the fused path; mitem and fwork are theirs, end to end
   std::vector<DClosures> cls;
   bool source = false;    // some closures carry a source term
   // device
@@ -236,9 +254,8 @@ struct List {
   FaceTable ft{};
   const long long* d_spre[3] = {nullptr, nullptr, nullptr};
   long long tot_p = 0, tot_v = 0, tot_g = 0, tot_valid = 0, tot_f[3] = {0, 0, 0}, tot_s[3] = {0, 0, 0};
-  int tot_work = 0;
   int face_grid = 0;  // CTAs of the balanced face-kernel schedule
-  KeepGrid grid;      // launch shape of the fused path's face kernels
+  double* div = nullptr;  // the pieces' shared part of the scratch
   int waves = 1;      // shares of the schedule per resident CTA (amrs_boxlist_set_schedule)
   cudaGraphExec_t graph = nullptr;
   int graph_key[6] = {0, 0, 0, 0, 0, 0};
@@ -314,7 +331,6 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   L.sc = h->sc;
   L.gq = prim_ghost(h->sc);
   L.fused = fused_path(h->sc);
-  L.grid = KeepGrid{};
   L.boxes.assign(boxes, boxes + n);
   L.hbox.assign(n, BoxRec{});
   L.cls.resize(std::max(ncl, 1));
@@ -332,18 +348,42 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   const bool need_slope = h->sc.rhs_euler && h->sc.flux_euler == 0;
   const bool need_jst = h->sc.rhs_euler && h->sc.art_diss == 1;
   L.pcell.assign(n + 1, 0); L.vcell.assign(n + 1, 0); L.gcell.assign(n + 1, 0); L.valid.assign(n + 1, 0);
-  L.mitem.assign(n + 1, 0);
-  L.fwork.assign(n + 1, 0);
+  L.mitem.clear();
+  L.fwork.clear();
+  L.pieces.clear();
   for (int d = 0; d < 3; ++d) { L.fpre[d].assign(n + 1, 0); L.spre[d].assign(n + 1, 0); }
-  // scratch layout: per box, Q [NQ x grow3], VF [NVF x grow1], faces, pf, lam, sen, slopes
-  size_t off = 0;
+  // scratch layout: per box, Q [NQ x grow3], VF [NVF x grow1], faces, pf, lam, sen, slopes;
+  // the pieces' divergence parts
+  size_t off = 0, div_bytes = 0, piece_bytes = 0;
   std::vector<size_t> q_off(n), vf_off(n), div_off(n), f_off(n * 3), pf_off(n), lam_off(n), sen_off(n), sl_off(n * 3);
   for (int b = 0; b < n; ++b) {
     const amrs_box& B = boxes[b];
     if (!box_ok(B)) return AMRS_ERR_BOX;
     q_off[b] = off; off = align_up(off + grown_cells(B, 3) * NQ * 8, 256);
     if (need_visc) { vf_off[b] = off; off = align_up(off + grown_cells(B, 1) * NVF * 8, 256); }
-    if (L.fused) { div_off[b] = off; off = align_up(off + grown_cells(B, 0) * 2 * NCONS * 8, 256); }
+    if (L.fused) {
+      const size_t plane = (size_t)bn(B, 0) * bn(B, 1) * 2 * NCONS * 8, all = align_up(plane * bn(B, 2), 256);
+      FacePiece p;
+      p.b0 = b;
+      if (all > DIV_BYTES) {
+        const int planes = (int)std::max<size_t>(DIV_BYTES / plane, 1);
+        for (p.z0 = B.lo[2]; p.z0 <= B.hi[2]; p.z0 = p.z1 + 1) {
+          p.z1 = std::min(B.hi[2], p.z0 + planes - 1);
+          L.pieces.push_back(p);
+        }
+        div_bytes = std::max(div_bytes, plane * planes);
+      } else {
+        if (!L.pieces.empty() && !L.pieces.back().slab() && piece_bytes + all <= DIV_BYTES) {
+          L.pieces.back().nb += 1;
+        } else {
+          L.pieces.push_back(p);
+          piece_bytes = 0;
+        }
+        div_off[b] = piece_bytes;
+        piece_bytes += all;
+        div_bytes = std::max(div_bytes, piece_bytes);
+      }
+    }
     if (need_faces)
       for (int d = 0; d < 3; ++d) {
         const long long nf = (long long)(bn(B, 0) + (d == 0)) * (bn(B, 1) + (d == 1)) * (bn(B, 2) + (d == 2));
@@ -357,22 +397,15 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     if (need_slope)
       for (int d = 0; d < 3; ++d) { sl_off[b * 3 + d] = off; off = align_up(off + grown_cells(B, 1) * NSLOPE * 8, 256); }
   }
+  const size_t div_base = off;
+  off += align_up(div_bytes, 256);
   if (off > L.dscr_bytes) {
     if (L.dscr) { cudaFree(L.dscr); L.dscr = nullptr; L.dscr_bytes = 0; }
     CK(cudaMalloc(&L.dscr, off));
     L.dscr_bytes = off;
   }
   char* S = static_cast<char*>(L.dscr);
-  if (L.fused)
-    // x kernel: narrower blocks where 256 slots would leave SMs without one
-    for (L.grid.x_threads = 256; L.grid.x_threads > 64; L.grid.x_threads /= 2) {
-      long long blocks = 0;
-      for (int b = 0; b < n; ++b) {
-        const int nb[3] = {bn(boxes[b], 0), bn(boxes[b], 1), bn(boxes[b], 2)};
-        blocks += keep_x_blocks(order, nb, L.grid.x_threads);
-      }
-      if (blocks >= 4LL * h->nsm) break;
-    }
+  L.div = reinterpret_cast<double*>(S + div_base);
   L.hface.assign(need_faces ? n : 0, FaceRec{});
   for (int b = 0; b < n; ++b) {
     const amrs_box& B = boxes[b];
@@ -396,7 +429,7 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     };
     R.q = mk(q_off[b], 3, -1, NQ);
     if (need_visc) R.vf = mk(vf_off[b], 1, -1, NVF);
-    if (L.fused) R.div = mk(div_off[b], 0, -1, 2 * NCONS);
+    if (L.fused) R.div = mk(div_base + div_off[b], 0, -1, 2 * NCONS);  // (of a box in slabs: see face_table)
     R.cl = cidx ? cidx[b] : 0;
     R.tx = tiles ? tiles[3 * b] : 32;
     R.ty = tiles ? tiles[3 * b + 1] : 8;
@@ -417,9 +450,6 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     L.vcell[b + 1] = L.vcell[b] + (need_visc ? grown_cells(B, 1) : 0);
     L.gcell[b + 1] = L.gcell[b] + grown_cells(B, 3);
     L.valid[b + 1] = L.valid[b] + grown_cells(B, 0);
-    const int nb[3] = {bn(B, 0), bn(B, 1), bn(B, 2)};
-    L.mitem[b + 1] = L.mitem[b] + march_items(R);
-    L.fwork[b + 1] = L.fwork[b] + (L.fused ? keep_x_blocks(order, nb, L.grid.x_threads) : 0);
     for (int d = 0; d < 3; ++d) {
       const long long nf = (long long)(bn(B, 0) + (d == 0)) * (bn(B, 1) + (d == 1)) * (bn(B, 2) + (d == 2));
       L.fpre[d][b + 1] = L.fpre[d][b] + nf;
@@ -428,21 +458,43 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     }
   }
   L.tot_p = L.pcell[n]; L.tot_v = L.vcell[n]; L.tot_g = L.gcell[n]; L.tot_valid = L.valid[n];
-  L.tot_work = L.fwork[n];
   for (int d = 0; d < 3; ++d) { L.tot_f[d] = L.fpre[d][n]; L.tot_s[d] = L.spre[d][n]; }
 
-  // shares and CTAs of the y and z marches
+  // the pieces' prefix tables and launch shapes
   L.face_grid = 0;
-  L.tb.nshare = 0;
-  if (L.fused) {
-    const long long resident = 8LL * keep_ctas_per_sm(order) * h->nsm;
-    const int G = (int)march_shares(L.mitem[n], L.waves, resident, h->nsm);
-    const int w = march_cta_warps(G, h->nsm);
-    L.tb.nshare = G;
-    L.grid.march_threads = 32 * w;
-    L.grid.march_ctas = (G + w - 1) / w;
-    L.face_grid = L.grid.march_ctas;
-    L.grid.x_ctas = L.fwork[n];
+  for (FacePiece& p : L.pieces) {
+    p.t0 = (int)L.mitem.size();
+    L.mitem.push_back(0);
+    L.fwork.push_back(0);
+    auto extent = [&](int b, int nb[3]) {
+      for (int d = 0; d < 3; ++d) nb[d] = bn(boxes[b], d);
+      if (p.slab()) nb[2] = p.z1 - p.z0 + 1;
+    };
+    int nb[3];
+    // x kernel: narrower blocks where 256 slots would leave SMs without one
+    for (p.grid.x_threads = 256; p.grid.x_threads > 64; p.grid.x_threads /= 2) {
+      long long blocks = 0;
+      for (int b = p.b0; b < p.b0 + p.nb; ++b) {
+        extent(b, nb);
+        blocks += keep_x_blocks(order, nb, p.grid.x_threads);
+      }
+      if (blocks >= 4LL * h->nsm) break;
+    }
+    for (int b = p.b0; b < p.b0 + p.nb; ++b) {
+      extent(b, nb);
+      BoxRec R{};
+      for (int d = 0; d < 3; ++d) R.hi[d] = nb[d] - 1;
+      L.mitem.push_back(L.mitem.back() + march_items(R));
+      L.fwork.push_back(L.fwork.back() + keep_x_blocks(order, nb, p.grid.x_threads));
+    }
+    p.items = L.mitem.back();
+    // shares and CTAs of the y and z marches
+    p.nshare = (int)march_shares(p.items, L.waves, 8LL * keep_ctas_per_sm(order) * h->nsm, h->nsm);
+    const int w = march_cta_warps(p.nshare, h->nsm);
+    p.grid.march_threads = 32 * w;
+    p.grid.march_ctas = (p.nshare + w - 1) / w;
+    p.grid.x_ctas = L.fwork.back();
+    L.face_grid += p.grid.march_ctas;
   }
 
   // device tables in one allocation
@@ -457,8 +509,8 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   size_t o_f[3], o_s[3];
   for (int d = 0; d < 3; ++d) { o_f[d] = t; t = align_up(t + 8 * (n + 1), 128); }
   for (int d = 0; d < 3; ++d) { o_s[d] = t; t = align_up(t + 8 * (n + 1), 128); }
-  const size_t o_w = t; t = align_up(t + 4 * (n + 1), 128);
-  const size_t o_mi = t; t = align_up(t + 8 * (n + 1), 128);
+  const size_t o_w = t; t = align_up(t + 4 * L.fwork.size(), 128);
+  const size_t o_mi = t; t = align_up(t + 8 * L.mitem.size(), 128);
   const size_t o_rng = t; t = align_up(t + sizeof(KeepRange), 128);
   if (t > L.dtab_bytes) {
     if (L.dtab) { cudaFree(L.dtab); L.dtab = nullptr; L.dtab_bytes = 0; }
@@ -477,8 +529,10 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
     std::memcpy(&host[o_f[d]], L.fpre[d].data(), 8 * (n + 1));
     std::memcpy(&host[o_s[d]], L.spre[d].data(), 8 * (n + 1));
   }
-  std::memcpy(&host[o_w], L.fwork.data(), 4 * (n + 1));
-  std::memcpy(&host[o_mi], L.mitem.data(), 8 * (n + 1));
+  if (L.fused) {
+    std::memcpy(&host[o_w], L.fwork.data(), 4 * L.fwork.size());
+    std::memcpy(&host[o_mi], L.mitem.data(), 8 * L.mitem.size());
+  }
   CK(cudaMemcpy(L.dtab, host.data(), t, cudaMemcpyHostToDevice));
   char* D = static_cast<char*>(L.dtab);
   L.tb.box = reinterpret_cast<const BoxRec*>(D + o_box);
@@ -500,7 +554,8 @@ amrs_status list_build(amrs_handle* h, List& L, int n, const amrs_box* boxes, co
   for (int d = 0; d < 3; ++d) L.ft.ftot[d] = L.tot_f[d];
   L.tb.tot_p = L.tot_p;
   L.tb.tot_v = L.tot_v;
-  L.tb.tot_m = L.mitem[n];
+  L.tb.nshare = L.fused ? L.pieces[0].nshare : 0;
+  L.tb.tot_m = L.fused ? L.pieces[0].items : 0;
   L.tb.one = n == 1;
   L.tb.rec = L.hbox[0];
   L.tb.rec_cls = L.cls[L.hbox[0].cl];
@@ -520,6 +575,45 @@ DProg to_dprog(const amrs_stage_prog* p) {
   return d;
 }
 
+// The list's table for one of several pieces.
+BoxTable face_table(const List& L, const FacePiece& p) {
+  BoxTable t = L.tb;
+  t.box += p.b0;
+  t.n = p.nb;
+  t.mitem += p.t0;
+  t.fwork += p.t0;
+  t.nshare = p.nshare;
+  t.tot_m = p.items;
+  t.one = p.nb == 1;
+  if (t.one) {
+    if (L.n > 1) t.rec = L.hbox[p.b0];  // (a single box's record holds the call's arrays)
+    t.rec_cls = L.cls[t.rec.cl];
+    if (p.slab()) {
+      t.rec.lo[2] = p.z0;
+      t.rec.hi[2] = p.z1;
+      DArr& d = t.rec.div;
+      d.p = L.div;
+      d.ns = d.ks * (p.z1 - p.z0 + 1);
+      d.b2 = p.z0;
+    }
+  }
+  return t;
+}
+
+// Faces, divergence and stage program of the fused path, piece by piece.
+cudaError_t keep_faces(const List& L, const DProg& prog, int s_in, int s_s1, int s_out, int rhs_only, cudaStream_t st) {
+  const amrs_scheme& sc = L.sc;
+  const bool visc = sc.rhs_visc != 0;
+  if (L.pieces.size() == 1 && !L.pieces[0].slab())
+    return launch_keep_face(sc.order_keep, visc, L.source, L.tb, s_in, s_s1, s_out, prog, rhs_only, L.pieces[0].grid, st);
+  for (const FacePiece& p : L.pieces) {
+    const cudaError_t e =
+        launch_keep_face(sc.order_keep, visc, L.source, face_table(L, p), s_in, s_s1, s_out, prog, rhs_only, p.grid, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 // One RHS evaluation (+ stage program) over the list: the kernel sequence of
 // CNS::compute_rhs (src/tim/CNS_advance.cpp:186-391).
 amrs_status list_stage(amrs_handle* h, List& L, const DProg& prog, int s_in, int s_s1, int s_out, int rhs_only,
@@ -532,8 +626,7 @@ amrs_status list_stage(amrs_handle* h, List& L, const DProg& prog, int s_in, int
   if (sc.rhs_visc) CK(launch_visc(L.tb, L.tot_v, nsm, st));
   if (L.fused) {
     // 3. fused KEEP faces + viscous averages + divergence + stage program
-    CK(launch_keep_face(sc.order_keep, sc.rhs_visc != 0, L.source, L.tb, s_in, s_s1, s_out, prog, rhs_only,
-                        L.grid, st));
+    CK(keep_faces(L, prog, s_in, s_s1, s_out, rhs_only, st));
     if (h->check_nonfinite) CK(launch_nonfinite_check(L.tb, L.ft.vpre, s_out, L.tot_valid, h->derr + 1, nsm, st));
     return AMRS_OK;
   }
@@ -1856,7 +1949,7 @@ amrs_status amrs_profile_stage_box(amrs_handle* h, const amrs_box* bx, const dou
     if (e == cudaSuccess && sc.rhs_visc) e = launch_visc(L.tb, L.tot_v, h->nsm, st);
     if (e == cudaSuccess) e = cudaEventRecord(ev[2], st);
     if (e == cudaSuccess && L.fused)
-      e = launch_keep_face(sc.order_keep, sc.rhs_visc != 0, L.source, L.tb, 0, 1, 2, p, 0, L.grid, st);
+      e = keep_faces(L, p, 0, 1, 2, 0, st);
     else if (e == cudaSuccess && sc.flux_euler == 2)
       e = launch_weno_faces(L.tb, L.ft, 0, nf, sc.weno_fast == 0, sc.rhs_visc != 0, h->nsm, st);
     else if (e == cudaSuccess && sc.flux_euler == 3)

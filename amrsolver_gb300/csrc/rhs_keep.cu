@@ -419,8 +419,9 @@ keep_x_kernel(const __grid_constant__ BoxTable tb, int s_in, int s_s1, int s_out
   double* smem = reinterpret_cast<double*>(smem_raw);
   const bool fast = fast_range(tb);
   if (tb.range && blockIdx.x == 0 && threadIdx.x == 0) {
+    // (a stage in several launches counts once)
+    if (!fast && tb.range->stage == tb.range->face) ++tb.range->plain;
     tb.range->stage = tb.range->face + 1u;
-    if (!fast) ++tb.range->plain;
   }
   if (fast) keep_x_body<ORDER, VISC, SRC, true>(tb, s_in, s_s1, s_out, prog, rhs_only, smem);
   else keep_x_body<ORDER, VISC, SRC, false>(tb, s_in, s_s1, s_out, prog, rhs_only, smem);
