@@ -3,22 +3,20 @@
 The y and z marches of the fused KEEP path cut the (column block x cell) work
 of all boxes into equal shares, one per warp, up to `waves` x (resident warps):
 one wave gives every warp the longest run, so the fewest prologues; more waves
-give shorter runs that CTAs pick up as others finish.  The tile shapes of the
-sweep are recorded with the list; the kernels deal columns and rows to warps
-whatever they are, so only the waves change the time.
+give shorter runs that CTAs pick up as others finish.  Tile shapes are not
+swept: the kernels deal columns and rows to warps whatever the list records, and
+the report's tiles are the list's own.
 
 The reference has no counterpart: its only tiling knob is MFIter over the
 boxes of max_grid_size (src/tim/CNS_advance.cpp:200).
 
 `tune_level` times whole SSPRK3 steps of the list itself (its CUDA graph,
 CUDA events, best of a few), so the balanced schedule and the interplay of
-all boxes are in every measurement.  It starts from the library's default
-tiles, sweeps the waves, then one shape for all boxes, then each of the
-classes that carry the most work, keeping a change only when it saves more
-than the timing noise; finally the winner is timed against the default once
-more and the faster of the two is applied, so the tuned list is never
-slower than the default by more than the noise.  Steps read state slot `s1`
-and write only the two work slots, so the caller's state is not changed.
+all boxes are in every measurement.  It sweeps the waves, keeping a change only
+when it saves more than the timing noise; finally the winner is timed against
+the default once more and the faster of the two is applied, so the tuned list
+is never slower than the default by more than the noise.  Steps read state slot
+`s1` and write only the two work slots, so the caller's state is not changed.
 Results are cached in JSON keyed by device, order and the box-size multiset.
 """
 from __future__ import annotations
@@ -31,7 +29,6 @@ import torch
 
 from . import capi
 
-CANDIDATES = ((32, 8), (16, 16), (24, 10), (8, 30), (16, 8), (8, 16), (8, 8), (32, 4), (24, 8))
 WAVES = (1, 2, 3, 4)
 DEFAULT_CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_lib", "autotune.json")
 
@@ -84,23 +81,19 @@ class _Timer:
 
 def tune_level(bl, shapes, s1=0, w1=1, w2=2, dt=1e-4, reps=3, max_classes=4, min_gain=0.005,
                cache_path=DEFAULT_CACHE, use_cache=True):
-    """Tune tiles per (nx, ny) class and the schedule's waves of box list `bl`
-    whose boxes have valid extents `shapes` ((nx, ny, nz) per box), apply the
-    winner and return a report: default and tuned ms per step, the choice
-    and every timed candidate."""
+    """Tune the schedule's waves of box list `bl` whose boxes have valid extents
+    `shapes` ((nx, ny, nz) per box), apply the winner and return a report: default
+    and tuned ms per step, the choice, the tiles per (nx, ny) class (the list's own)
+    and every timed candidate.  `max_classes` is accepted for callers of the tile
+    sweep and changes nothing."""
     order = bl.handle.scheme.order_keep
     key = _level_key(order, [tuple(s) for s in shapes])
     cache = load_cache(cache_path) if use_cache else {}
     timer = _Timer(bl, s1, w1, w2, dt, reps)
-    default_tiles = bl.get_tiles()
-    classes = {}
-    for b, s in enumerate(shapes):
-        classes.setdefault((s[0], s[1]), []).append(b)
-    work = {c: sum(shapes[b][0] * shapes[b][1] * shapes[b][2] for b in bs) for c, bs in classes.items()}
+    tiles = bl.get_tiles()
 
-    def apply(tiles, waves):
+    def apply(waves):
         try:
-            bl.set_tiles(tiles)
             bl.set_schedule(waves)
             return True
         except capi.AmrsError:
@@ -108,57 +101,35 @@ def tune_level(bl, shapes, s1=0, w1=1, w2=2, dt=1e-4, reps=3, max_classes=4, min
 
     if use_cache and key in cache:
         ent = cache[key]
-        tiles = [tuple(t) for t in ent["tiles"]]
-        if apply(tiles, ent["waves"]):
-            return dict(ent, cached=True)
+        try:
+            bl.set_tiles([tuple(t) for t in ent["tiles"]])
+            if apply(ent["waves"]):
+                return dict(ent, cached=True)
+        except capi.AmrsError:
+            pass
     sweep = []
 
-    def measure(tiles, waves, label):
-        if not apply(tiles, waves):
+    def measure(waves, label):
+        if not apply(waves):
             return None
         ms = timer()
         sweep.append({"candidate": label, "waves": waves, "ms": ms})
         return ms
 
-    t_default = measure(default_tiles, 1, "default")
-    best_tiles, best_w, best_ms = list(default_tiles), 1, t_default
+    best_w, best_ms = 1, measure(1, "default")
     for w in WAVES[1:]:
-        ms = measure(best_tiles, w, "default")
-        if ms is not None and ms < best_ms * (1 - min_gain):
-            best_w, best_ms = w, ms
-    for t in CANDIDATES:
-        tiles = [(t[0], t[1], kc) for (_, _, kc) in default_tiles]
-        ms = measure(tiles, best_w, "all %dx%d" % t)
-        if ms is not None and ms < best_ms * (1 - min_gain):
-            best_tiles, best_ms = tiles, ms
-    top = sorted(classes, key=lambda c: -work[c])[:max_classes]
-    for c in top:
-        for t in CANDIDATES:
-            tiles = list(best_tiles)
-            for b in classes[c]:
-                tiles[b] = (t[0], t[1], tiles[b][2])
-            if tiles == best_tiles:
-                continue
-            ms = measure(tiles, best_w, "class %dx%d -> %dx%d" % (c[0], c[1], t[0], t[1]))
-            if ms is not None and ms < best_ms * (1 - min_gain):
-                best_tiles, best_ms = tiles, ms
-    for w in WAVES:
-        if w == best_w:
-            continue
-        ms = measure(best_tiles, w, "tuned tiles")
+        ms = measure(w, "%d waves" % w)
         if ms is not None and ms < best_ms * (1 - min_gain):
             best_w, best_ms = w, ms
     # the winner against the default, timed once more each
-    t_def2 = measure(default_tiles, 1, "default (final)")
-    t_best2 = measure(best_tiles, best_w, "tuned (final)")
+    t_def2 = measure(1, "default (final)")
+    t_best2 = measure(best_w, "tuned (final)")
     if t_best2 > t_def2:
-        best_tiles, best_w, t_best2 = list(default_tiles), 1, t_def2
-    apply(best_tiles, best_w)
-    choice = {}
-    for c, bs in classes.items():
-        choice["%dx%d" % c] = list(best_tiles[bs[0]][:2])
+        best_w, t_best2 = 1, t_def2
+    apply(best_w)
+    choice = {"%dx%d" % (s[0], s[1]): list(t[:2]) for s, t in zip(shapes, tiles)}
     rep = {"default_ms": t_def2, "tuned_ms": t_best2, "tuned_over_default": t_def2 / t_best2,
-           "waves": best_w, "class_tiles": choice, "tiles": [list(t) for t in best_tiles],
+           "waves": best_w, "class_tiles": choice, "tiles": [list(t) for t in tiles],
            "candidates_timed": timer.count, "sweep": sweep, "cached": False}
     if use_cache:
         cache[key] = {k: rep[k] for k in ("default_ms", "tuned_ms", "tuned_over_default", "waves", "class_tiles",

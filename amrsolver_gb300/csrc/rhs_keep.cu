@@ -477,6 +477,8 @@ int keep_x_blocks(int order, const int n[3], int threads) {
   return (int)((slots - H + threads - H - 1) / (threads - H));
 }
 
+// The tile shapes that the tuning interface accepts (and records: no kernel reads
+// them any more): those whose planes once fitted a block's shared memory.
 bool keep_tile_fits(int order, int tx, int ty) {
   if (tx < 8 || ty < 1 || (tx % 2) || tx * ty > F_THREADS) return false;
   const int H = order / 2;

@@ -320,8 +320,7 @@ def bench_batched(torch, capi, P, nboxes=512, steps=3, warmup=2):
            "cells": cells, "batched_graph_cell_updates_per_s": cells / (ms_b * 1e-3),
            "per_box_cell_updates_per_s": cells / (ms_p * 1e-3), "ms_batched": ms_b, "ms_per_box": ms_p,
            "speedup": ms_p / ms_b}
-    # autotuner sweep over tile shapes per box class and the schedule's
-    # z coarsening, timed on this list's own graph step
+    # autotuner sweep over the schedule's waves, timed on this list's own graph step
     rep = autotune.tune_level(bl, [tuple(s.shape) for s in specs], dt=1e-4, use_cache=False)
     res["tuned"] = tuned_section(rep, cells)
     res["tuned_speedup_over_per_box"] = ms_p / rep["tuned_ms"]
