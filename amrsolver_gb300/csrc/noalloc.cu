@@ -6,12 +6,13 @@
 // allocator) and forbids allocations behind the pool's back, or one that
 // reserves a fixed device-memory budget up front.  For them this entry point
 // keeps the scratch that amrs_rhs_box takes from its handle (primitive and
-// viscous-flux fields, the y and z divergence parts and the box table) in one
-// fixed static device array, and needs no handle.
+// viscous-flux fields, the y and z divergence parts and the range flag) in one
+// fixed static device array, and needs no handle.  The box record travels in the
+// launches: a call copies nothing and does not wait.
 //
 // Limits and sharing rules:
 //  * boxes of at most 32 cells in every direction (the array holds
-//    NQ x 38^3 + 12 x 34^3 + 10 x 32^3 doubles plus an 8 KiB table region, 9.5 MB);
+//    NQ x 38^3 + 12 x 34^3 + 10 x 32^3 doubles and the flag, 9.5 MB);
 //    larger boxes return AMRS_ERR_SIZE;
 //  * the array exists once per device that loads the library and stays
 //    allocated until the process exits;
@@ -25,7 +26,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 #include <mutex>
 
 #include "../../include/amrs_gb300.h"
@@ -39,9 +39,9 @@ namespace {
 constexpr int NA_MAX_EDGE = 32;
 constexpr size_t NA_Q = (size_t)NQ * (NA_MAX_EDGE + 6) * (NA_MAX_EDGE + 6) * (NA_MAX_EDGE + 6);
 constexpr size_t NA_VF = (size_t)NVF * (NA_MAX_EDGE + 2) * (NA_MAX_EDGE + 2) * (NA_MAX_EDGE + 2);
-constexpr size_t NA_TABLE_BYTES = 8 * 1024;
 constexpr size_t NA_DIV = (size_t)2 * NCONS * NA_MAX_EDGE * NA_MAX_EDGE * NA_MAX_EDGE;
-constexpr size_t NA_DOUBLES = NA_Q + NA_VF + NA_DIV + NA_TABLE_BYTES / 8;
+constexpr size_t NA_DOUBLES = NA_Q + NA_VF + NA_DIV + sizeof(KeepRange) / 8;
+static_assert((NA_Q + NA_VF + NA_DIV) % 2 == 0, "the flag's alignment");
 
 }  // namespace
 
@@ -52,8 +52,6 @@ static __device__ __align__(256) double g_noalloc_scratch[NA_DOUBLES];
 namespace {
 
 std::mutex g_na_mu;
-// host staging of the table region (no heap use)
-alignas(128) char g_na_host[NA_TABLE_BYTES];
 constexpr int NA_MAX_DEVICES = 64;
 double* g_na_ptr[NA_MAX_DEVICES] = {nullptr};
 int g_na_nsm[NA_MAX_DEVICES] = {0};
@@ -107,8 +105,6 @@ bool na_covers(const amrs_array4& a, const amrs_box& b, int g) {
   return a.jstride >= nx && a.kstride >= a.jstride * ny && a.nstride >= a.kstride * nz;
 }
 
-size_t al(size_t x) { return (x + 127) / 128 * 128; }
-
 }  // namespace
 
 extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amrs_closures* closures,
@@ -152,7 +148,6 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   double* qp = base;
   double* vfp = base + NA_Q;
   double* divp = vfp + NA_VF;
-  char* tab = reinterpret_cast<char*>(divp + NA_DIV);
   const int order = sc.order_keep;
 
   // box record and launch shape (as the handle path builds them)
@@ -175,15 +170,12 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   for (grid.x_threads = 256; grid.x_threads > 64; grid.x_threads /= 2)
     if (keep_x_blocks(order, n, grid.x_threads) >= 4 * nsm) break;
   grid.x_ctas = keep_x_blocks(order, n, grid.x_threads);
-  const long long mitem[2] = {0, march_items(R)};
-  const int G = (int)march_shares(mitem[1], 1, 8LL * keep_ctas_per_sm(order) * nsm, nsm);
+  const long long items = march_items(R);
+  const int G = (int)march_shares(items, 1, 8LL * keep_ctas_per_sm(order) * nsm, nsm);
   const int cw = march_cta_warps(G, nsm);
   grid.march_threads = 32 * cw;
   grid.march_ctas = (G + cw - 1) / cw;
   const int gq = std::max(order / 2, 2);
-  long long pcell[2] = {0, (long long)(n[0] + 2 * gq) * (n[1] + 2 * gq) * (n[2] + 2 * gq)};
-  long long vcell[2] = {0, (long long)(n[0] + 2) * (n[1] + 2) * (n[2] + 2)};
-  int fwork[2] = {0, grid.x_ctas};
   DClosures cl;
   cl.gamma = closures->gamma; cl.cv = closures->cv; cl.cp = closures->cp; cl.Rspec = closures->Rspec;
   cl.visc_law = closures->visc_law; cl.cond_law = closures->cond_law;
@@ -193,49 +185,22 @@ extern "C" amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amr
   cl.source = 0;  // no source term on this path
   cl.force[0] = cl.force[1] = cl.force[2] = 0.0;
 
-  // table region layout: box | closures | pcell | vcell | fwork | range flag | march items
-  size_t t = 0;
-  const size_t o_box = t; t = al(t + sizeof(BoxRec));
-  const size_t o_cl = t; t = al(t + sizeof(DClosures));
-  const size_t o_p = t; t = al(t + sizeof(pcell));
-  const size_t o_v = t; t = al(t + sizeof(vcell));
-  const size_t o_w = t; t = al(t + sizeof(fwork));
-  const size_t o_rng = t; t = al(t + sizeof(KeepRange));
-  const size_t o_mi = t; t = al(t + sizeof(mitem));
-  if (t > NA_TABLE_BYTES) return AMRS_ERR_SIZE;
-  char* host = g_na_host;
-  std::memset(host, 0, t);
-  std::memcpy(&host[o_box], &R, sizeof(BoxRec));
-  std::memcpy(&host[o_cl], &cl, sizeof(DClosures));
-  std::memcpy(&host[o_p], pcell, sizeof(pcell));
-  std::memcpy(&host[o_v], vcell, sizeof(vcell));
-  std::memcpy(&host[o_w], fwork, sizeof(fwork));
-  std::memcpy(&host[o_mi], mitem, sizeof(mitem));
-  // The copy also clears the range flag, which must start at zero.  From
-  // pageable host memory it waits for the stream's earlier work and returns
-  // once the staging is consumed, so the static host buffer can be reused.
-  if (cudaMemcpyAsync(tab, host, t, cudaMemcpyHostToDevice, st) != cudaSuccess) return AMRS_ERR_CUDA;
-  BoxTable tb{};  // every field defined: tb.active stays null (no device time loop here)
-  tb.active = nullptr;
-  tb.box = reinterpret_cast<const BoxRec*>(tab + o_box);
-  tb.pcell = reinterpret_cast<const long long*>(tab + o_p);
-  tb.vcell = reinterpret_cast<const long long*>(tab + o_v);
-  tb.fwork = reinterpret_cast<const int*>(tab + o_w);
-  tb.mitem = reinterpret_cast<const long long*>(tab + o_mi);
+  // a list of one box whose launches carry everything but the flag (no tables, no
+  // device time loop)
+  BoxTable tb{};
   tb.nshare = G;
-  tb.cls = reinterpret_cast<const DClosures*>(tab + o_cl);
   tb.n = 1;
-  tb.tot_p = pcell[1];
-  tb.tot_v = vcell[1];
-  tb.tot_m = mitem[1];
+  tb.tot_p = (long long)(n[0] + 2 * gq) * (n[1] + 2 * gq) * (n[2] + 2 * gq);
+  tb.tot_v = (long long)(n[0] + 2) * (n[1] + 2) * (n[2] + 2);
+  tb.tot_m = items;
   tb.one = 1;
   tb.rec = R;
   tb.rec_cls = cl;
   tb.gq = gq;
-  tb.range = reinterpret_cast<KeepRange*>(tab + o_rng);
+  tb.range = reinterpret_cast<KeepRange*>(divp + NA_DIV);
   DProg prog{};
-  if (launch_prims(tb, 0, pcell[1], nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;
-  if (sc.rhs_visc && launch_visc(tb, vcell[1], nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;
+  if (launch_prims(tb, 0, tb.tot_p, nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;
+  if (sc.rhs_visc && launch_visc(tb, tb.tot_v, nsm, st) != cudaSuccess) return AMRS_ERR_CUDA;
   if (launch_keep_face(order, sc.rhs_visc != 0, false, tb, 0, 1, 2, prog, 1, grid, st) != cudaSuccess)
     return AMRS_ERR_CUDA;
   return AMRS_OK;

@@ -183,8 +183,9 @@ amrs_status amrs_rhs_box(amrs_handle* h, const amrs_box* bx, const double dxinv[
  * call shares it, so calls that overlap on the GPU race.  The kernels run on
  * the current device: a `stream` of another device is refused
  * (AMRS_ERR_STATE).  The first call on a device looks the array's address
- * up with that device current: make it before any stream capture.  Results
- * are identical to amrs_rhs_box. */
+ * up with that device current: make it before any stream capture.  A call
+ * copies nothing and does not wait for the device.  Results are identical to
+ * amrs_rhs_box. */
 amrs_status amrs_rhs_box_noalloc(const amrs_scheme* scheme, const amrs_closures* closures, const amrs_box* bx,
                                  const double dxinv[3], amrs_array4 state, amrs_array4 dsdt, void* stream);
 
