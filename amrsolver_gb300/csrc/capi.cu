@@ -29,6 +29,7 @@ thread_local std::string g_cuda_err;
 
 amrs_status cuda_fail(cudaError_t e, const char* where) {
   g_cuda_err = std::string(where) + ": " + cudaGetErrorString(e);
+  cudaGetLastError();  // reported: the next call's launches must not find it again
   return AMRS_ERR_CUDA;
 }
 #define CK(call)                                         \
@@ -687,7 +688,11 @@ amrs_status one_box(amrs_handle* h, const amrs_box* bx, const double dxinv[3], c
     if (L->graph) { cudaGraphExecDestroy(L->graph); L->graph = nullptr; }
     // the previous tables may still be read by queued kernels
     CK(cudaDeviceSynchronize());
-    if (amrs_status s = list_build(h, *L, 1, bx, dxinv, nslots, slots, nullptr, 0, nullptr, nullptr)) return s;
+    if (amrs_status s = list_build(h, *L, 1, bx, dxinv, nslots, slots, nullptr, 0, nullptr, nullptr)) {
+      delete L;  // half built: not to be found by the next call of this box
+      L = nullptr;
+      return s;
+    }
   }
   // the record of this call's arrays travels with its launches
   BoxRec& R = L->tb.rec;
