@@ -30,8 +30,11 @@
 // high product extends the quotient (root) to more than 80 bits.  Neither
 // operation has results half way between two doubles, so the truncated
 // 84-bit value decides the rounding unless it lies within a few units of
-// 2^-84 of a midpoint; that case (about one operand pair in 2^28) takes the
-// hardware operation.
+// 2^-84 of a midpoint; there the sign of the exact remainder at the midpoint
+// does, again in 64-bit arithmetic.  That is one random operand pair in 2^28,
+// but every 1/x for x an odd number of units in the last place below a power of
+// two, and every root of an odd number of units above one: a uniform state with
+// rho = 1 and gamma p = 1 up to rounding is full of them.
 //
 // Domain: operands with exponents in the middle half of the range (about
 // 2^-503 .. 2^504), for the product +-0 too; anything else (subnormal,
@@ -132,18 +135,18 @@ AMRS_HD DWords round_pack(uint32_t r, uint32_t k, uint32_t hi, uint32_t lo, uint
 #endif
 }
 
-// The hardware operations for inputs outside the integer paths' domains, out
-// of line: a call is a real branch taken only by lanes that need it, where an
-// inlined fallback is predicated by the compiler and issues its FP64
-// instruction on every call.
+// The operations for inputs outside the integer paths' domains (dmul_hw here,
+// ddiv_rest and dsqrt_rest below) are out of line: a call is a real branch taken
+// only by lanes that need it, where an inlined fallback is predicated by the
+// compiler and issues its FP64 instruction on every call.
 #ifdef __CUDA_ARCH__
-static __device__ __noinline__ double ddiv_hw(double a, double b) { return a / b; }
-static __device__ __noinline__ double dmul_hw(double a, double b) { return __dmul_rn(a, b); }
-static __device__ __noinline__ double dsqrt_hw(double x) { return sqrt(x); }
+#define AMRS_OUT_OF_LINE static __device__ __noinline__
+#define AMRS_SQRT(x) sqrt(x)
+AMRS_OUT_OF_LINE double dmul_hw(double a, double b) { return __dmul_rn(a, b); }
 #else
-inline double ddiv_hw(double a, double b) { return a / b; }
+#define AMRS_OUT_OF_LINE inline
+#define AMRS_SQRT(x) ::sqrt(x)
 inline double dmul_hw(double a, double b) { return a * b; }
-inline double dsqrt_hw(double x) { return ::sqrt(x); }
 #endif
 
 // Seeds of the Newton steps.  They need about 22 correct bits, not correct
@@ -203,37 +206,69 @@ AMRS_HD uint32_t seed_corr(uint32_t v, int32_t e) { return (uint32_t)(((int32_t)
 // exponent of the word in [520, 1528)
 AMRS_HD bool mid_range(uint32_t hi) { return hi * 2u - 0x41000000u < 0x7E000000u; }
 
-// a / b for words in the domain; *slow is set when the truncated quotient
-// cannot decide the rounding.  ma/mb in (1/2, 2), digits q1, q2, q3 of
+// a / b for words in the domain.  ma/mb in (1/2, 2), digits q1, q2, q3 of
 // ma 2^86 / mb = q1 2^58 + q2 2^29 + q3, each rounded down (v is):
 //   q1 <= ma 2^28 / mb,   R1 = ma 2^28 - q1 mb in [0, 2.3 mb)
 //   q2 <= R1 2^29 / mb,   R2 = R1 2^29 - q2 mb in [0, 3.8 mb)
 //   q3 <= R2 2^29 / mb    within 5 units
+// Where that leaves the rounding open, m is the last digit with which the
+// quotient would be the midpoint, and R2 2^29 - m mb (below 2^60) has the sign.
+struct DDiv {
+  uint32_t q3, rl, rh, nl, nh, Tl, Wh, Wl, s, r, E;  // R2 = (rh:rl), -mb = (nh:nl)
+  AMRS_HD DDiv(DWords a, DWords b) {
+    const uint32_t mah = (a.hi & 0xFFFFFu) | 0x100000u, mbh = (b.hi & 0xFFFFFu) | 0x100000u;
+    // v ~ 2^63 / dh, dh = the top 32 bits of mb 2^11; one Newton step
+    const uint32_t dh = shl_hi(b.lo, mbh, 11);
+    const uint32_t v0 = seed_rcp(((dh >> 8) & 0x7FFFFFu) | 0x3F800000u);
+    const int32_t e = (int32_t)(0x7FFFFFFFu - mulhi32(v0, dh));
+    const uint32_t v = v0 + seed_corr(v0, e) - 3u;  // < 2^95 / (mb 2^11)
+    const uint64_t nmb = 0ull - (((uint64_t)mbh << 32) | b.lo);
+    nl = (uint32_t)nmb;
+    nh = (uint32_t)(nmb >> 32);
+    const uint32_t q1 = mulhi32(shl_hi(a.lo, mah, 11), v) >> 3;
+    uint64_t R = madw(q1, nl, ((uint64_t)shl_hi(a.lo, mah, 28) << 32) | (a.lo << 28));
+    rl = (uint32_t)R;
+    rh = (uint32_t)(R >> 32) + q1 * nh;
+    const uint32_t q2 = mulhi32(shr_lo(rl, rh, 23), v);
+    R = madw(q2, nl, ((uint64_t)shl_hi(rl, rh, 29) << 32) | (rl << 29));
+    rl = (uint32_t)R;
+    rh = (uint32_t)(R >> 32) + q2 * nh;
+    q3 = mulhi32(shr_lo(rl, rh, 23), v);
+    const uint64_t T = madw(q2, 1u << 29, q3);
+    const uint64_t W = madw(q1, 1u << 26, T >> 32);  // in (2^53, 2^55)
+    Tl = (uint32_t)T;
+    Wh = (uint32_t)(W >> 32);
+    Wl = (uint32_t)W;
+    const uint32_t top = Wh >> 22;
+    s = 1u + top;
+    r = shr_lo(Tl, Wl, s);
+    E = (a.hi & 0xFFF00000u) - (b.hi & 0xFFF00000u) + (1021u << 20) + (top << 20);
+  }
+  AMRS_HD bool undecided() const { return r - 0x7FFFFFF8u < 8u; }
+  AMRS_HD void decide() {
+    const uint32_t m = q3 + ((0x80000000u - r) << s) - (Tl & ((1u << s) - 1u));
+    const uint64_t D = madw(m, nl, ((uint64_t)shl_hi(rl, rh, 29) << 32) | (rl << 29)) + ((uint64_t)(m * nh) << 32);
+    r = (int64_t)D < 0 ? 0x7FFFFFFFu : 0x80000000u;
+  }
+  AMRS_HD DWords pack() const { return round_pack(r, 0x80000000u, Wh >> s, shr_lo(Wl, Wh, s), E); }
+};
+AMRS_HD DWords ddiv_core(DWords a, DWords b) {
+  DDiv q(a, b);
+  if (__builtin_expect(q.undecided(), 0)) q.decide();
+  return q.pack();
+}
+// The same without the decision: *slow is set where it is needed.  For callers
+// whose operands reach it by chance only and that have a fallback anyway.
 AMRS_HD DWords ddiv_core(DWords a, DWords b, bool* slow) {
-  const uint32_t mah = (a.hi & 0xFFFFFu) | 0x100000u, mbh = (b.hi & 0xFFFFFu) | 0x100000u;
-  // v ~ 2^63 / dh, dh = the top 32 bits of mb 2^11; one Newton step
-  const uint32_t dh = shl_hi(b.lo, mbh, 11);
-  const uint32_t v0 = seed_rcp(((dh >> 8) & 0x7FFFFFu) | 0x3F800000u);
-  const int32_t e = (int32_t)(0x7FFFFFFFu - mulhi32(v0, dh));
-  const uint32_t v = v0 + seed_corr(v0, e) - 3u;  // < 2^95 / (mb 2^11)
-  const uint64_t nmb = 0ull - (((uint64_t)mbh << 32) | b.lo);
-  const uint32_t nl = (uint32_t)nmb, nh = (uint32_t)(nmb >> 32);
-  const uint32_t q1 = mulhi32(shl_hi(a.lo, mah, 11), v) >> 3;
-  uint64_t R = madw(q1, nl, ((uint64_t)shl_hi(a.lo, mah, 28) << 32) | (a.lo << 28));
-  uint32_t rl = (uint32_t)R, rh = (uint32_t)(R >> 32) + q1 * nh;
-  const uint32_t q2 = mulhi32(shr_lo(rl, rh, 23), v);
-  R = madw(q2, nl, ((uint64_t)shl_hi(rl, rh, 29) << 32) | (rl << 29));
-  rl = (uint32_t)R;
-  rh = (uint32_t)(R >> 32) + q2 * nh;
-  const uint32_t q3 = mulhi32(shr_lo(rl, rh, 23), v);
-  const uint64_t T = madw(q2, 1u << 29, q3);
-  const uint64_t W = madw(q1, 1u << 26, T >> 32);  // in (2^53, 2^55)
-  const uint32_t Wh = (uint32_t)(W >> 32), Wl = (uint32_t)W;
-  const uint32_t top = Wh >> 22, s = 1u + top;
-  const uint32_t r = shr_lo((uint32_t)T, Wl, s);
-  *slow = r - 0x7FFFFFF8u < 8u;
-  return round_pack(r, 0x80000000u, Wh >> s, shr_lo(Wl, Wh, s),
-                    (a.hi & 0xFFF00000u) - (b.hi & 0xFFF00000u) + (1021u << 20) + (top << 20));
+  const DDiv q(a, b);
+  *slow = q.undecided();
+  return q.pack();
+}
+
+// What ddiv_rn leaves: an undecided rounding, or an operand outside the domain.
+AMRS_OUT_OF_LINE double ddiv_rest(double a, double b) {
+  const DWords A = dwords(a), B = dwords(b);
+  return mid_range(A.hi) && mid_range(B.hi) ? dfrom(ddiv_core(A, B)) : a / b;
 }
 
 // a / b, correctly rounded; the integer path where its domain holds.
@@ -244,7 +279,7 @@ AMRS_HD double ddiv_rn(double a, double b) {
   if (!mid_range(A.hi) || !mid_range(B.hi) || slow) {
     // +-0 / b with b in range is +-0
     if (((A.hi << 1) | A.lo) == 0u && mid_range(B.hi)) x = dfrom((A.hi ^ B.hi) & 0x80000000u, 0u);
-    else x = ddiv_hw(a, b);
+    else x = ddiv_rest(a, b);
   }
   return x;
 }
@@ -318,38 +353,62 @@ AMRS_HD double dmul_rn(double a, double b) {
 //   s2 < R1 2^27 / (2 sqrt(n')) by 2 .. 9 (the 3 outweighs the omitted
 //   second-order term),           R2 = R1 2^54 - s2 (S1 2^28 + s2) in (0, 2^63)
 //   s3 ~ R2 / (2 sqrt(n')) within 4 units.
-AMRS_HD DWords dsqrt_core(DWords x, bool* slow) {
-  const uint32_t odd = (~x.hi >> 20) & 1u;  // the unbiased exponent is odd
-  const uint32_t mxh = (x.hi & 0xFFFFFu) | 0x100000u;
-  const uint32_t nh = shl_hi(x.lo, mxh, 10u + odd);  // top word of 4 n'
-  const uint32_t v0 = seed_rsqrt((shl_hi(x.lo, x.hi, 3) & 0x7FFFFFu) | (0x3F800000u + (odd << 23)));
-  const int32_t e = (int32_t)(0x3FFFFFFFu - mulhi32(mulhi32(v0, v0), nh));
-  const uint32_t v = v0 + seed_corr(v0, e) - 4u;
-  const uint32_t S1 = mulhi32(nh, v);
-  const uint64_t n4 = ((uint64_t)shl_hi(x.lo, mxh, 8u + odd) << 32) | (x.lo << (8u + odd));
-  const uint64_t R1 = n4 - (uint64_t)S1 * S1;
-  const uint32_t s2 = mulhi32((uint32_t)(R1 >> 4), v) - 3u;
-  const uint64_t M = madw(S1, 1u << 28, s2);
-  const uint64_t P = madw(s2, (uint32_t)M, (uint64_t)(s2 * (uint32_t)(M >> 32)) << 32);
-  const uint64_t R2 = ((uint64_t)((uint32_t)R1 << 22) << 32) - P;
-  const uint32_t s3 = mulhi32((uint32_t)(R2 >> 31), v);
-  const uint64_t T = madw(s2, 1u << 27, s3);
-  const uint64_t W = madw(S1, 1u << 22, T >> 32);
-  const uint32_t r = (uint32_t)T;
-  *slow = r - 0x7FFFFFF0u < 32u;
-  return round_pack(r, 0x80000000u, (uint32_t)(W >> 32), (uint32_t)W,
-                    (((x.hi + 0x100000u) >> 1) & 0x7FF00000u) + (510u << 20));
+// Where that leaves the rounding open, m is the last digit with which the root
+// would be the midpoint A 2^27 + m, A = S1 2^27 + s2, and the sign is that of
+// n' 2^108 - (A 2^27 + m)^2 = 2^28 (R2 2^26 - m A) - m^2.
+struct DSqrt {
+  uint32_t S1, s2, s3, r, E;
+  uint64_t R2, W;
+  AMRS_HD explicit DSqrt(DWords x) {
+    const uint32_t odd = (~x.hi >> 20) & 1u;  // the unbiased exponent is odd
+    const uint32_t mxh = (x.hi & 0xFFFFFu) | 0x100000u;
+    const uint32_t nh = shl_hi(x.lo, mxh, 10u + odd);  // top word of 4 n'
+    const uint32_t v0 = seed_rsqrt((shl_hi(x.lo, x.hi, 3) & 0x7FFFFFu) | (0x3F800000u + (odd << 23)));
+    const int32_t e = (int32_t)(0x3FFFFFFFu - mulhi32(mulhi32(v0, v0), nh));
+    const uint32_t v = v0 + seed_corr(v0, e) - 4u;
+    S1 = mulhi32(nh, v);
+    const uint64_t n4 = ((uint64_t)shl_hi(x.lo, mxh, 8u + odd) << 32) | (x.lo << (8u + odd));
+    const uint64_t R1 = n4 - (uint64_t)S1 * S1;
+    s2 = mulhi32((uint32_t)(R1 >> 4), v) - 3u;
+    const uint64_t M = madw(S1, 1u << 28, s2);
+    const uint64_t P = madw(s2, (uint32_t)M, (uint64_t)(s2 * (uint32_t)(M >> 32)) << 32);
+    R2 = ((uint64_t)((uint32_t)R1 << 22) << 32) - P;
+    s3 = mulhi32((uint32_t)(R2 >> 31), v);
+    const uint64_t T = madw(s2, 1u << 27, s3);
+    W = madw(S1, 1u << 22, T >> 32);
+    r = (uint32_t)T;
+    E = (((x.hi + 0x100000u) >> 1) & 0x7FF00000u) + (510u << 20);
+  }
+  AMRS_HD bool undecided() const { return r - 0x7FFFFFF8u < 16u; }
+  AMRS_HD void decide() {
+    const uint32_t m = s3 + (0x80000000u - r);
+    const uint64_t A = madw(S1, 1u << 27, s2);
+    const int64_t Y = (int64_t)((R2 << 26) - (madw(m, (uint32_t)A, 0ull) + ((uint64_t)(m * (uint32_t)(A >> 32)) << 32)));
+    r = Y > (int64_t)(((uint64_t)m * m) >> 28) ? 0x80000000u : 0x7FFFFFFFu;
+  }
+  AMRS_HD DWords pack() const { return round_pack(r, 0x80000000u, (uint32_t)(W >> 32), (uint32_t)W, E); }
+};
+AMRS_HD DWords dsqrt_core(DWords x) {
+  DSqrt q(x);
+  if (__builtin_expect(q.undecided(), 0)) q.decide();
+  return q.pack();
+}
+
+AMRS_HD bool dsqrt_range(uint32_t hi) { return hi - (520u << 20) < (1008u << 20); }
+AMRS_OUT_OF_LINE double dsqrt_rest(double x) {
+  const DWords X = dwords(x);
+  return dsqrt_range(X.hi) ? dfrom(dsqrt_core(X)) : AMRS_SQRT(x);
 }
 
 // sqrt(x), correctly rounded; the integer path for positive x in its domain,
 // +-0 directly, anything else by the hardware square root.
 AMRS_HD double dsqrt_rn(double x) {
   const DWords X = dwords(x);
-  bool slow;
-  double y = dfrom(dsqrt_core(X, &slow));
-  if (X.hi - (520u << 20) >= (1008u << 20) || slow) {
+  const DSqrt q(X);
+  double y = dfrom(q.pack());
+  if (!dsqrt_range(X.hi) || q.undecided()) {
     if (((X.hi << 1) | X.lo) == 0u) y = x;
-    else y = dsqrt_hw(x);
+    else y = dsqrt_rest(x);
   }
   return y;
 }

@@ -407,26 +407,14 @@ struct IntOps {
   bool ok = true;
   // a quotient of nonzero operands, the same with a dividend that may be
   // zero (positive divisor), a root
-  __device__ __forceinline__ double div(double a, double b) {
-    bool slow;
-    const double q = dfrom(ddiv_core(dwords(a), dwords(b), &slow));
-    ok = ok && !slow;
-    return q;
-  }
-  __device__ __forceinline__ double divz(double a, double b) {
+  __device__ __forceinline__ double div(double a, double b) const { return dfrom(ddiv_core(dwords(a), dwords(b))); }
+  __device__ __forceinline__ double divz(double a, double b) const {
     const DWords w = dwords(a);
-    bool slow;
-    const DWords q = ddiv_core(w, dwords(b), &slow);
+    const DWords q = ddiv_core(w, dwords(b));
     const bool zero = ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
-    ok = ok && (zero || !slow);
     return dfrom(zero ? w.hi : q.hi, zero ? w.lo : q.lo);
   }
-  __device__ __forceinline__ double root(double a) {
-    bool slow;
-    const double q = dfrom(dsqrt_core(dwords(a), &slow));
-    ok = ok && !slow;
-    return q;
-  }
+  __device__ __forceinline__ double root(double a) const { return dfrom(dsqrt_core(dwords(a))); }
   // products of nonzero factors, and of a positive factor a with any x
   __device__ __forceinline__ double mul(double a, double b) const {
     return dfrom(dmul_core(dwords(a), dwords(b)));
@@ -729,8 +717,7 @@ static __device__ __noinline__ void riemann_plain(const double gamma, const doub
 // pressure finite and, after its floor, below 2^150) need no range test in any
 // operation: every intermediate then stays well inside the normal range.
 // Comparisons of values of known sign are integer comparisons of their bits.
-// A transonic fan, a star state outside the ranges and the one quotient or
-// root in 2^28 that the truncated value cannot round take riemann_plain.
+// A transonic fan and a star state outside the ranges take riemann_plain.
 // 72 FP64 instructions (sums, the flux products) and 17 quotients, 11 roots and
 // 60 products on the integer pipe; with the products on the FP64 pipe the MUSCL
 // step at 96^3 takes 3.61 ms instead of 2.94, with any one group of them 2-13%
