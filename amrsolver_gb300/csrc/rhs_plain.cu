@@ -425,14 +425,15 @@ struct IntOps {
     const bool zero = ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u;
     return dfrom(zero ? w.hi : r.hi, zero ? w.lo : r.lo);
   }
-  // positive, in [2^-150, 2^150); zero or in [2^-100, 2^100)
+  // positive, in [2^-150, 2^150); zero or in [2^-400, 2^100); below 2^100
   __device__ __forceinline__ void pos(double x) {
     ok = ok && dwords(x).hi - (873u << 20) < (300u << 20);
   }
   __device__ __forceinline__ void vel(double x) {
     const DWords w = dwords(x);
-    ok = ok && (w.hi * 2u - (923u << 21) < (200u << 21) || ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u);
+    ok = ok && (w.hi * 2u - (623u << 21) < (500u << 21) || ((w.hi & 0x7FFFFFFFu) | w.lo) == 0u);
   }
+  __device__ __forceinline__ void below(double x) { ok = ok && dwords(x).hi * 2u < (1123u << 21); }
   // max(x, smallp) for a finite x; the result below 2^150
   __device__ __forceinline__ double floor_p(double x, double smallp) {
     const long long b = __double_as_longlong(x), s = __double_as_longlong(smallp);
@@ -453,15 +454,15 @@ static __device__ __noinline__ double mc_limiter_plain(double dlft, double drgt)
 
 // The same with one FP64 instruction (the sum): the signs, the minima and the
 // scalings by 2 and 1/2 on the words.  In range: both slopes zero or in
-// [2^-400, 2^400), so that their product's sign is that of the signs and the
-// scalings are exact; a sum of two such is zero or above 2^-453.  (Slopes of
+// [2^-500, 2^500), so that their product's sign is that of the signs and the
+// scalings are exact; a sum of two such is zero or above 2^-553.  (Slopes of
 // opposite sign, or a zero one: the limited slope is +-0 with the sign of the
 // sum.)
 __device__ __forceinline__ double mc_limiter(double dlft, double drgt) {
   const DWords l = dwords(dlft), r = dwords(drgt), c = dwords(dlft + drgt);
   const uint32_t lh = l.hi & 0x7FFFFFFFu, rh = r.hi & 0x7FFFFFFFu, ch = c.hi & 0x7FFFFFFFu;
   const bool lz = (lh | l.lo) == 0u, rz = (rh | r.lo) == 0u;
-  if (!((lz || lh - (623u << 20) < (800u << 20)) && (rz || rh - (623u << 20) < (800u << 20))))
+  if (!((lz || lh - (523u << 20) < (1000u << 20)) && (rz || rh - (523u << 20) < (1000u << 20))))
     return mc_limiter_plain(dlft, drgt);
   // 4 min(|l|, |r|) against |l + r|: the smaller half is the limited slope
   const uint64_t al = ((uint64_t)lh << 32) | l.lo, ar = ((uint64_t)rh << 32) | r.lo;
@@ -510,10 +511,12 @@ static __device__ __noinline__ void slope_plain(const SlopeQ& q, double gR, doub
 // The same bits on the integer pipe where the ranges hold.  c0 >= 2^-78 makes
 // c0 + 1e-40 = c0 + 2e-40 = c0; the halves of d0 and d2 are taken at the end
 // (the limiter and the sums scale exactly), so dp / c and rho du enter whole.
+// Normal velocities down to 2^-400: rho du is zero or above 2^-602, the sums of
+// limited slopes zero or above 2^-708.  Transverse ones meet only the limiter.
 __device__ __forceinline__ void slope_terms(const SlopeQ& q, double gR, double tiny, bool up, double o[NSLOPE]) {
   IntOps I;
 #pragma unroll
-  for (int n = 0; n < 3; ++n) { I.pos(q.rho[n]); I.pos(q.p[n]); I.vel(q.un[n]); I.vel(q.t1[n]); I.vel(q.t2[n]); }
+  for (int n = 0; n < 3; ++n) { I.pos(q.rho[n]); I.pos(q.p[n]); I.vel(q.un[n]); }
   I.pos(gR); I.pos(q.T);
   const double c = I.root(I.mul(gR, q.T));
   I.ok = I.ok && dwords(c).hi >= (945u << 20);
@@ -713,13 +716,18 @@ static __device__ __noinline__ void riemann_plain(const double gamma, const doub
 
 // The same solver, same bits, with its quotients and roots and most of its
 // products on the integer pipe.  The faces whose states are all in the tested
-// ranges (densities and pressures in 2^+-150, velocities zero or in 2^+-100, star
+// ranges (densities and pressures in 2^+-150, velocities below 2^100, star
 // pressure finite and, after its floor, below 2^150) need no range test in any
-// operation: every intermediate then stays well inside the normal range.
+// operation: every intermediate then stays well inside the normal range, but for
+// the four products of a velocity, which are on the FP64 pipe.  (Velocities as
+// small as they come are ordinary: fluid at rest beside moving fluid has them down
+// to zero within a few cells.  With a lower bound of 2^-100 a step at 96^3 in such a
+// state took 13.4 ms, with every face in riemann_plain, and takes 3.95 now; the FP64
+// products cost 0.7% elsewhere.)
 // Comparisons of values of known sign are integer comparisons of their bits.
 // A transonic fan and a star state outside the ranges take riemann_plain.
-// 72 FP64 instructions (sums, the flux products) and 17 quotients, 11 roots and
-// 60 products on the integer pipe; with the products on the FP64 pipe the MUSCL
+// 76 FP64 instructions (sums, the flux products) and 17 quotients, 11 roots and
+// 56 products on the integer pipe; with the products on the FP64 pipe the MUSCL
 // step at 96^3 takes 3.61 ms instead of 2.94, with any one group of them 2-13%
 // more.
 __device__ __forceinline__ void riemann_prob(const double gamma, const double smallp, const double in[10],
@@ -728,7 +736,7 @@ __device__ __forceinline__ void riemann_prob(const double gamma, const double sm
   const double rr = in[5], ur = in[6], pr = in[7], ut1r = in[8], ut2r = in[9];
   IntOps R;
   R.pos(rl); R.pos(pl); R.pos(rr); R.pos(pr);
-  R.vel(ul); R.vel(ur); R.vel(ut1l); R.vel(ut2l); R.vel(ut1r); R.vel(ut2r);
+  R.below(ul); R.below(ur); R.below(ut1l); R.below(ut2l); R.below(ut1r); R.below(ut2r);
   auto bits = [](double x) { return __double_as_longlong(x); };
   const double hg = 0.5 * (gamma - 1.);
   R.pos(gamma); R.pos(hg);
@@ -739,7 +747,7 @@ __device__ __forceinline__ void riemann_prob(const double gamma, const double sm
   const double ccsmall = R.mul(1.e-6, cleft + cright);
   const double du = ur - ul;
   auto star = [&]() {
-    const double num = R.mul(wl, pr) + R.mul(wr, pl) - R.mulz(R.mul(wr, wl), du);
+    const double num = R.mul(wl, pr) + R.mul(wr, pl) - R.mul(wr, wl) * du;
     return R.floor_p(R.divz(num, wl + wr), smallp);
   };
   auto wsq = [&](double ps, double p, double r) { return R.mul(R.mul(hg, ps + p) + ps, r); };
@@ -804,12 +812,12 @@ __device__ __forceinline__ void riemann_prob(const double gamma, const double sm
   } else if (bits(spin) < 0) {
     R.ok = false;  // inside a transonic fan
   }
-  const double m = R.mulz(rg, ug);
+  const double m = rg * ug;
   out[0] = m;
   out[1] = m * ug + pg;
   out[2] = m * utrans1;
   out[3] = m * utrans2;
-  out[4] = ug * (fma(0.5, R.mulz(rg, ug * ug + utrans1 * utrans1 + utrans2 * utrans2), R.div(pg, gamma - 1.)) + pg);
+  out[4] = ug * (fma(0.5, rg * (ug * ug + utrans1 * utrans1 + utrans2 * utrans2), R.div(pg, gamma - 1.)) + pg);
   if (!R.ok) {
     double a[10], o[5];
 #pragma unroll
