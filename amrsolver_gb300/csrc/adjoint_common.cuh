@@ -96,18 +96,21 @@ static __device__ __noinline__ void weno5js_grad_plain(const double* t, double* 
 
 // The same with its products and the division on the integer pipe (38 FP64
 // instructions are left of about 110): behind one range test per smoothness
-// difference and per y_k - Wy no product tests its own.  Differences are zero or
-// in [2^-100, 2^60), s1 - s3 below 2^35 (its fourth power enters e), so e lies in
-// [2^-133, 2^143) and D P in the normal range.  A zero difference or y_k - Wy gives
-// zero terms.  t: the four differences; Wy = W - s2.
+// difference and per y_k - Wy no product tests its own.  Differences are below 2^60,
+// s1 - s3 below 2^35 (its fourth power enters e), so e lies in [2^-133, 2^143) and D P
+// in the normal range.  A zero y_k - Wy gives zero terms, and so does a difference
+// below 2^-240: its terms are below 2^-170, beside entries that sum to one (ebar_k is
+// at most 2^134 |y_k - Wy|, and that at most 2^-66 where e_k is about eps).  The y_k
+// are twelvefold, Y0 = d1 + 3 d2 and so on, and 1/12 goes with 1/(D P).  t: the four
+// differences; Wy = W - s2.
 __device__ __forceinline__ void weno5js_grad(const double t[4], double gr[5], double& Wy) {
   bool ok = true, slow;
   const WenoDiffs d(t);
   const DWords D1 = weno_diff(d.d1, ok), D2 = weno_diff(d.d2, ok), D3 = weno_diff(d.d3, ok), G = weno_diff(d.g, ok),
                D4 = weno_diff(d.d4, ok), D5 = weno_diff(d.d5, ok);
   ok = ok && (G.hi & 0x7FFFFFFFu) < (1058u << 20);
-  const bool z1 = is_zero(d.d1), z2 = is_zero(d.d2), z3 = is_zero(d.d3), zg = is_zero(d.g), z4 = is_zero(d.d4),
-             z5 = is_zero(d.d5);
+  const bool z1 = weno_tiny(d.d1), z2 = weno_tiny(d.d2), z3 = weno_tiny(d.d3), zg = weno_tiny(d.g), z4 = weno_tiny(d.d4),
+             z5 = weno_tiny(d.d5);
   auto term = [](DWords a, DWords b, bool zero) {
     const DWords x = dmul_core(a, b);
     return zero ? 0.0 : dfrom(x);
@@ -124,18 +127,18 @@ __device__ __forceinline__ void weno5js_grad(const double t[4], double gr[5], do
   const DWords P = dmul_core(e0, q0);
   const DWords r = ddiv_core(DWords{0x3FF00000u, 0u}, dmul_core(dwords(dfrom(t0) + dfrom(t1) + dfrom(t2)), P), &slow);
   ok = ok && !slow;
-  const DWords rP = dmul_core(r, P);
+  const DWords rP = dmul_core(r, P), r12 = dmul_core(r, c112);
   const double x0 = dfrom(dmul_core(t0, rP)), x1 = dfrom(dmul_core(t1, rP)), x2 = dfrom(dmul_core(t2, rP));
-  const double y0 = fma(0.25, d.d2, term(c112, D1, z1)), y1 = fma(-0.25, d.g, term(c112, D3, z3)),
-               y2 = fma(-0.25, d.d5, term(c112, D4, z4));
-  Wy = x0 * y0 + x1 * y1 + x2 * y2;
+  const double y0 = fma(3.0, d.d2, d.d1), y1 = fma(-3.0, d.g, d.d3), y2 = fma(-3.0, d.d5, d.d4);
+  const double S = x0 * y0 + x1 * y1 + x2 * y2;
+  Wy = S * (1.0 / 12.0);
   // b_k = w_k / e_k (y_k - Wy) = -ebar_k / 2; the terms ebar_k grad beta_k:
   // p1 = -(13/3) b0 d1, p2 = -b0 d2, p4 = -2 b1 g^3, ...
-  const ZWords f0 = weno_fac(y0 - Wy, ok), f1 = weno_fac(y1 - Wy, ok), f2 = weno_fac(y2 - Wy, ok);
+  const ZWords f0 = weno_fac(y0 - S, ok), f1 = weno_fac(y1 - S, ok), f2 = weno_fac(y2 - S, ok);
   auto negated = [](DWords a) { return DWords{a.hi ^ 0x80000000u, a.lo}; };
-  const DWords b0 = negated(dmul_core(dmul_core(t0, dmul_core(q0, r)), f0.w));
-  const DWords b1 = negated(dmul_core(dmul_core(t1, dmul_core(q1, r)), f1.w));
-  const DWords b2 = negated(dmul_core(dmul_core(t2, dmul_core(q2, r)), f2.w));
+  const DWords b0 = negated(dmul_core(dmul_core(t0, dmul_core(q0, r12)), f0.w));
+  const DWords b1 = negated(dmul_core(dmul_core(t1, dmul_core(q1, r12)), f1.w));
+  const DWords b2 = negated(dmul_core(dmul_core(t2, dmul_core(q2, r12)), f2.w));
   const DWords c133{0x40115555u, 0x55555555u};  // 13/3
   const DWords gb{b1.hi + (1u << 20), b1.lo};   // 2 b1
   weno_grad_sums(x0, x1, x2, term(dmul_core(c133, b0), D1, f0.zero || z1), term(b0, D2, f0.zero || z2),

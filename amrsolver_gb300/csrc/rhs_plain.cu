@@ -223,9 +223,8 @@ __device__ __forceinline__ double weno5js(const double s0, const double s1, cons
 // integer pipe from end to end: they stay in the operands' words (dmul_core,
 // ddiv_core), and `ok` collects one range test per value that enters in place
 // of a test in every operation; where it ends up false the caller takes the
-// plain form.  The smoothness differences are zero or in [2^-100, 2^60); a
-// zero enters its square (or fourth power) as 2^-200, and the result, at most
-// 2^-400, changes no sum it enters.  eps + beta is beta from 2^-78 up (eps is
+// plain form.  The smoothness differences are below 2^60 (weno_diff).  eps + beta is
+// beta from 2^-78 up (eps is
 // below half its last place) and eps below 2^-187 (the other way round); in
 // between the hardware adds them out of line.
 
