@@ -86,7 +86,8 @@ __device__ __forceinline__ void keep_pair_vjp(const double* q1, const double* q2
 // pipe (76% busy at 64^3, order 4: 121 us; 158 with 55 FP64 instructions a pair).
 // Four CTAs per SM (64 registers); with two, 96 registers and 153 us.
 template <int ORDER>
-__global__ void __launch_bounds__(256, 4) adj_pair_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total) {
+__global__ void __launch_bounds__(256, 4)
+adj_pair_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total) {
   dep_begin();
   constexpr int H = ORDER / 2;
   double coef[3];
@@ -161,7 +162,8 @@ __global__ void __launch_bounds__(256, 4) adj_pair_kernel(const __grid_constant_
 // on every run.  Bound: the FP64 pipe (94 instructions a cell) behind the loads'
 // latency: four CTAs per SM 58 us at 64^3, two 65.  Its products on the integer
 // pipe gained nothing (within 0.3% of a step's gradient at 64^3).
-__global__ void __launch_bounds__(256, 4) adj_visc_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, double* pbar) {
+__global__ void __launch_bounds__(256, 4)
+adj_visc_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, double* pbar) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);
@@ -299,7 +301,8 @@ __global__ void adj_param_sum_kernel(const double* part, int nblocks, double* pb
 // (82% busy: 72 of its additions at order 4 are the pairs'); 84 us at 64^3, four
 // CTAs per SM (two: 93).
 template <int ORDER>
-__global__ void __launch_bounds__(256, 4) adj_gather_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, int gpair) {
+__global__ void __launch_bounds__(256, 4)
+adj_gather_kernel(const __grid_constant__ BoxTable tb, AdjRec ar, long long total, int gpair) {
   dep_begin();
   constexpr int H = ORDER / 2;
   const BoxRec& R = box_rec(tb, 0);

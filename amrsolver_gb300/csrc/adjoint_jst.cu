@@ -43,8 +43,8 @@ __device__ __forceinline__ bool valid_cell(const BoxRec& R, int i, int j, int k)
   return i >= R.lo[0] && i <= R.hi[0] && j >= R.lo[1] && j <= R.hi[1] && k >= R.lo[2] && k <= R.hi[2];
 }
 
-__global__ void __launch_bounds__(256) jst_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, JBuf jb, int d,
-                                                           long long total) {
+__global__ void __launch_bounds__(256)
+jst_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, JBuf jb, int d, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);
@@ -102,8 +102,9 @@ __global__ void __launch_bounds__(256) jst_vjp_face_kernel(const __grid_constant
   }
 }
 
-__global__ void __launch_bounds__(256) jst_vjp_sensor_kernel(const __grid_constant__ BoxTable tb, JBuf j0, JBuf j1, JBuf j2, double* cs_buf,
-                                                             long long total) {
+__global__ void __launch_bounds__(256)
+jst_vjp_sensor_kernel(const __grid_constant__ BoxTable tb, JBuf j0, JBuf j1, JBuf j2, double* cs_buf,
+                      long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);
@@ -158,8 +159,9 @@ __global__ void __launch_bounds__(256) jst_vjp_sensor_kernel(const __grid_consta
   }
 }
 
-__global__ void __launch_bounds__(256) jst_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, JBuf j0, JBuf j1, JBuf j2,
-                                                             const double* cs_buf, long long nvalid, long long total) {
+__global__ void __launch_bounds__(256)
+jst_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, JBuf j0, JBuf j1, JBuf j2, const double* cs_buf,
+                      long long nvalid, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);

@@ -59,8 +59,8 @@ struct SBuf {
 // dependent chain per face, and 24 warps hide its latency better than 16 with the
 // registers they would otherwise take (gradient of an SSPRK3 step at 48^3: 2510
 // against 2640 us; at 72^3 7509 against 7574).
-__global__ void __launch_bounds__(256, 3) muscl_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FBuf fs, int d,
-                                                             long long total) {
+__global__ void __launch_bounds__(256, 3)
+muscl_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FBuf fs, int d, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DArr q = R.q;
@@ -271,8 +271,8 @@ __global__ void __launch_bounds__(256, 3) muscl_vjp_slope_kernel(const __grid_co
   }
 }
 
-__global__ void __launch_bounds__(256, 4) muscl_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, SBuf s0, SBuf s1, SBuf s2,
-                                                               long long total) {
+__global__ void __launch_bounds__(256, 4)
+muscl_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, SBuf s0, SBuf s1, SBuf s2, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);

@@ -46,8 +46,8 @@ __device__ __forceinline__ double vget0(const DArr& v, const BoxRec& R, int i, i
 // takes 170 us a direction, 311 with stencil values and FP64 products; the two
 // products per slot below stay on the FP64 pipe (1% faster than moved).  Three CTAs
 // per SM are as fast as two, four 1% slower (spills).
-__global__ void __launch_bounds__(256, 3) weno_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FaceBuf fb, int d,
-                                                            long long total) {
+__global__ void __launch_bounds__(256, 3)
+weno_vjp_face_kernel(const __grid_constant__ BoxTable tb, FaceRec fr, DArr vbar, FaceBuf fb, int d, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const int di = d == 0, dj = d == 1, dk = d == 2;

@@ -37,7 +37,8 @@ __device__ __forceinline__ double vget_r(const DArr& v, const BoxRec& R, int i, 
 // Three CTAs per SM (85 registers, the rest spilled): 24 warps hide the
 // latency of the reverse solver's chain (measured: 11.96 against 13.96 ms
 // per SSPRK3 step VJP at 64^3 with the unconstrained 255 registers).
-__global__ void __launch_bounds__(256, 3) wr_vjp_face_kernel(const __grid_constant__ BoxTable tb, DArr vbar, RBuf rb, int d, long long total) {
+__global__ void __launch_bounds__(256, 3)
+wr_vjp_face_kernel(const __grid_constant__ BoxTable tb, DArr vbar, RBuf rb, int d, long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DArr q = R.q;
@@ -101,8 +102,9 @@ __global__ void __launch_bounds__(256, 3) wr_vjp_face_kernel(const __grid_consta
 
 // Cells lo-3 .. hi+3 along d (the stencils of faces lo .. hi+1), the valid
 // range across.
-__global__ void __launch_bounds__(256) wr_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, RBuf rb, int d, int m0, int m1,
-                                                            long long total) {
+__global__ void __launch_bounds__(256)
+wr_vjp_gather_kernel(const __grid_constant__ BoxTable tb, DArr ubar, RBuf rb, int d, int m0, int m1,
+                     long long total) {
   dep_begin();
   const BoxRec& R = box_rec(tb, 0);
   const DClosures& cl = box_cls(tb, R);

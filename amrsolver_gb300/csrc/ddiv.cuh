@@ -44,8 +44,9 @@
 // Bound: the integer pipes' issue rate.  Cycles per warp operation and SM with
 // 16 warps resident and nothing else running (GB300), against the earlier
 // form (64-bit fixed-point Newton iterations and a 128-bit product) and the
-// hardware operation: product 14 (29, 20), division 29 (80, 144), square root
-// 31 (81, 150); without the range checks (the *_core functions) 11 and 18.
+// hardware operation: product 14 (28, 19), division 27 (76, 137), square root
+// 29 (77, 143); without the range checks (the *_core functions) 10, 20 and 25, a
+// division that leaves undecided roundings to its caller 17.
 // Beside a saturated FP64 stream of 16 FMAs, four products cost 4% (hardware
 // products 30%) and four divisions 6% (earlier form 41%).
 #pragma once

@@ -19,8 +19,10 @@
 // registers, 32 warps per SM).  One kernel for all three directions, streaming
 // z-planes through shared memory, held the FP64 pipe 73% busy (16 warps per SM,
 // two barriers per plane) with 272 FP64 instructions per cell; 128^3, KEEP4 +
-// viscous, per stage: 1257 us before, 427 + 348 us now with 185, FP64 pipe 82-85%
-// busy (in between, with one kernel for x and y tiles and a z march: 890 us).
+// viscous, per stage: 1257 us before, 430 + 320 us now with 167, FP64 pipe 72-79%
+// busy (in between, with one kernel for x and y tiles and a z march: 890 us).  With a
+// cell outside keep_range every product is on the FP64 pipe: a step with fluid at
+// rest takes 4.09 ms instead of 2.88 (4.75 with the one kernel).
 #include <type_traits>
 
 #include "amrs_boxes.cuh"
@@ -30,7 +32,7 @@
 namespace amrs {
 
 // ------------------------------------------------------------- prims ----
-// Bound: the FP64 pipe (77% busy; nine instructions a cell and the copy's loads).
+// Bound: the FP64 pipe (74% busy; nine instructions a cell and the copy's loads).
 __global__ void __launch_bounds__(256, 5) prims_kernel(const __grid_constant__ BoxTable tb, int s_in) {
   dep_begin();
   if (list_idle(tb)) return;
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(256, 5) prims_kernel(const __grid_constant__ B
 
 // ------------------------------------------------- viscous cell fluxes ----
 // Bound: the FP64 pipe and the integer pipes about equally (37 additions and 40
-// products a cell; 75% and half of the issue slots at 128^3, 180 us); three CTAs per
+// products a cell; 77% and half of the issue slots at 128^3, 170 us); three CTAs per
 // SM (80 registers), two 2% of a step slower, four the same.
 __global__ void __launch_bounds__(256, 3) visc_cell_kernel(const __grid_constant__ BoxTable tb) {
   dep_begin();
@@ -402,7 +404,8 @@ __device__ __forceinline__ void keep_march_warp(const BoxTable& tb) {
 }
 
 template <int ORDER, bool VISC>
-__global__ void __launch_bounds__(F_THREADS, march_ctas<ORDER>()) keep_march_kernel(const __grid_constant__ BoxTable tb) {
+__global__ void __launch_bounds__(F_THREADS, march_ctas<ORDER>())
+keep_march_kernel(const __grid_constant__ BoxTable tb) {
   dep_begin();
   if (list_idle(tb)) return;
   if (fast_range(tb)) keep_march_warp<ORDER, VISC, true>(tb);

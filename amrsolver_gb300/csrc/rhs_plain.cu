@@ -67,7 +67,8 @@ static int grid_for(long long n, int nsm, int ctas = GRID_CTAS) {
 // src/rhs/CentralKEEP.h:40-145, one face per thread, pairs summed in the
 // reference's (l, m) order without sharing between faces.
 template <int ORDER>
-__global__ void __launch_bounds__(256) keep_faces_plain_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256)
+keep_faces_plain_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   constexpr int H = ORDER / 2;
@@ -125,7 +126,9 @@ __device__ __forceinline__ double visc_average(const BoxRec& R, const FaceIdx& f
 #ifndef AMRS_WPF_IMUL
 #define AMRS_WPF_IMUL 0x0B
 #endif
-__global__ void __launch_bounds__(256) weno_flux_lambda_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, long long total) {
+__global__ void __launch_bounds__(256)
+weno_flux_lambda_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in,
+                        long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -341,7 +344,9 @@ static __device__ __noinline__ double weno_llf_plain(const double* p0, long long
 // to 98.3 ms: of the five positive sums, beta_0 and the weights' sums are the ones
 // that gain; with none 101.7, only the weights' 99.5, all 101.4.
 template <bool REF_ORDER, bool VISC>
-__global__ void __launch_bounds__(256, 3) weno_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, long long total) {
+__global__ void __launch_bounds__(256, 3)
+weno_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in,
+                 long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   const int n = blockIdx.y;
@@ -552,9 +557,9 @@ __device__ __forceinline__ void slope_terms(const SlopeQ& q, double gR, double t
 // products per cell and direction; the limiters' comparisons and scalings by
 // two were 40 further FP64 instructions).  48^3, inviscid: 64 -> 28 us; four CTAs
 // per SM 2.5% faster than two over the step.
-__global__ void __launch_bounds__(256, 4) slope_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, const long long* spre0,
-                                                    const long long* spre1, const long long* spre2,
-                                                    long long tot0, long long tot1, long long tot2) {
+__global__ void __launch_bounds__(256, 4)
+slope_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, const long long* spre0,
+             const long long* spre1, const long long* spre2, long long tot0, long long tot1, long long tot2) {
   dep_begin();
   if (list_idle(tb)) return;
   const long long total = tot0 + tot1 + tot2;
@@ -828,12 +833,13 @@ __device__ __forceinline__ void riemann_prob(const double gamma, const double sm
 }
 
 // MUSCL face states + Riemann flux (src/rhs/Riemann.h:251-337).  Bound: the FP64
-// pipe (77% busy at 128^3, 118 instructions a face) behind the solver's serial chain
+// pipe (76% busy at 128^3, 122 instructions a face) behind the solver's serial chain
 // of quotients and roots; two CTAs per SM (128 registers) beat three (2.94 against
 // 3.10 ms per step at 96^3).  48^3, with the hardware's roots and products and
 // checked integer quotients before: 194 -> 86 us.
 template <bool VISC>
-__global__ void __launch_bounds__(256, 2) riemann_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256, 2)
+riemann_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -886,7 +892,8 @@ __global__ void __launch_bounds__(256, 2) riemann_face_kernel(const __grid_const
 // as the MUSCL states are (src/rhs/Riemann.h:260-272), and riemann_prob
 // gives the flux.  One thread per face.
 template <bool VISC>
-__global__ void __launch_bounds__(256) weno_riemann_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256)
+weno_riemann_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -935,7 +942,8 @@ __device__ __forceinline__ double discon_sensor(double pp, double pl, double pr)
 
 // Sensor and spectral radius on the valid box (src/rhs/CNS_hydro_K.h:46-75);
 // the arrays are zeroed beforehand, as the reference zeroes its MultiFabs.
-__global__ void __launch_bounds__(256) jst_sensor_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256)
+jst_sensor_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -964,7 +972,9 @@ __global__ void __launch_bounds__(256) jst_sensor_kernel(const __grid_constant__
 // JST dissipation subtracted from face fluxes (src/rhs/CNS_hydro_K.h:78-104);
 // y and z read component 0 of sensor and lambda, and the z fourth
 // difference uses k-1 three times, as in the reference.
-__global__ void __launch_bounds__(256) jst_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, long long total) {
+__global__ void __launch_bounds__(256)
+jst_face_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in,
+                long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -995,7 +1005,8 @@ __global__ void __launch_bounds__(256) jst_face_kernel(const __grid_constant__ B
 
 // ---------------------------------------------- viscous face average ----
 // src/rhs/CNS_hydro_K.h:254-261 (mass component adds zero and is skipped).
-__global__ void __launch_bounds__(256) visc_face_add_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
+__global__ void __launch_bounds__(256)
+visc_face_add_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -1023,8 +1034,9 @@ __global__ void __launch_bounds__(256) visc_face_add_kernel(const __grid_constan
 // loads' latency and the FP64 pipe (25 to 35 instructions per cell with every
 // product on the integer pipe, 60 to 75 before).  256^3: 2.07 -> 1.46 ms per stage
 // (products moved, loads in program order: 1.87; one thread per cell: 2.97).
-__global__ void __launch_bounds__(256, 5) div_stage_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, int s_s1, int s_out,
-                                                           DProg prog_in, int rhs_only, long long total) {
+__global__ void __launch_bounds__(256, 5)
+div_stage_kernel(const __grid_constant__ BoxTable tb, const __grid_constant__ FaceTable ft, int s_in, int s_s1,
+                 int s_out, DProg prog_in, int rhs_only, long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   const DProg prog = resolve_prog(prog_in);

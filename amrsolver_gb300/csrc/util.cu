@@ -275,7 +275,8 @@ __global__ void __launch_bounds__(256) bcnormal_box_kernel(DArr U, int lo0, int 
 // Every box of a level whose y extent touches a code-6 side of the domain:
 // the box's own ghost rows beyond that side (its first interior row and the
 // ghost columns of it were filled by halo_level_kernel).
-__global__ void __launch_bounds__(256) bcnormal_list_kernel(const __grid_constant__ BoxTable tb, int slot, LevelDomain dom, DBcNormal bn) {
+__global__ void __launch_bounds__(256)
+bcnormal_list_kernel(const __grid_constant__ BoxTable tb, int slot, LevelDomain dom, DBcNormal bn) {
   dep_begin();
   if (list_idle(tb)) return;
   const int g = NGHOST;
@@ -393,7 +394,8 @@ __global__ void __launch_bounds__(256) estdt_kernel(const __grid_constant__ BoxT
 
 __global__ void estdt_init(unsigned long long* bits) {
   dep_begin();
-  *bits = ~0ull; }
+  *bits = ~0ull;
+}
 
 __global__ void estdt_final(const unsigned long long* bits, double cfl, double* out) {
   dep_begin();
@@ -456,7 +458,8 @@ __global__ void run_begin(RunCtl* c) {
 
 // Valid cells of slot `from` into slot `to` for every box (the step's result
 // back into the S1 slot the next step reads).
-__global__ void __launch_bounds__(256) copy_slot_kernel(const __grid_constant__ BoxTable tb, int from, int to, long long total) {
+__global__ void __launch_bounds__(256)
+copy_slot_kernel(const __grid_constant__ BoxTable tb, int from, int to, long long total) {
   dep_begin();
   if (list_idle(tb)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
@@ -488,8 +491,9 @@ __global__ void __launch_bounds__(256) copy_slot_kernel(const __grid_constant__ 
 // *flag when any component is a NaN or an infinity (exponent bits all ones,
 // tested on the integer bits, so the FP64 pipe is not used).  One extra
 // read of the slot (40 B per cell); run only when the caller opted in.
-__global__ void __launch_bounds__(256) nonfinite_check_kernel(const __grid_constant__ BoxTable tb, const long long* vpre, int slot,
-                                                              long long total, int* flag) {
+__global__ void __launch_bounds__(256)
+nonfinite_check_kernel(const __grid_constant__ BoxTable tb, const long long* vpre, int slot, long long total,
+                       int* flag) {
   dep_begin();
   if (list_idle(tb)) return;
   int bad = 0;
@@ -550,9 +554,9 @@ __global__ void prim_stats_init(unsigned long long* cells) {
   if (t < NSTAT) cells[t] = t < 6 ? ~0ull : 0ull;
 }
 
-__global__ void __launch_bounds__(256) prim_stats_kernel(const __grid_constant__ BoxTable tb, const long long* vpre, int slot, double dt,
-                                                         double dx0, double dx1, double dx2, long long total,
-                                                         unsigned long long* cells) {
+__global__ void __launch_bounds__(256)
+prim_stats_kernel(const __grid_constant__ BoxTable tb, const long long* vpre, int slot, double dt, double dx0,
+                  double dx1, double dx2, long long total, unsigned long long* cells) {
   dep_begin();
   double mn[6], mx[6], t[9];
 #pragma unroll
@@ -641,7 +645,8 @@ cudaError_t launch_prim_stats(const BoxTable& tb, const long long* vpre, int slo
 // Conserved totals of slot `slot` over the valid cells of every box:
 // per-block sums in a fixed order, then one block sums the partials in
 // block order (deterministic; not the serial sum's rounding).
-__global__ void __launch_bounds__(256) totals_partial_kernel(const __grid_constant__ BoxTable tb, int slot, long long total, double* part) {
+__global__ void __launch_bounds__(256)
+totals_partial_kernel(const __grid_constant__ BoxTable tb, int slot, long long total, double* part) {
   dep_begin();
   double acc[NCONS] = {0, 0, 0, 0, 0};
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;

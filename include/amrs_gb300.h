@@ -261,7 +261,7 @@ amrs_status amrs_boxlist_create(amrs_handle* h, int32_t nboxes, const amrs_box* 
                                 int32_t nclosures, const amrs_closures* closures, amrs_boxlist** out);
 amrs_status amrs_boxlist_destroy(amrs_boxlist* bl);
 
-/* Tile shape (tx*ty <= 256) and z-chunk per box, as chosen by the autotuner;
+/* Tile shape (tx*ty <= 256) and z-chunk per box, recorded with the list;
  * tx must be even and at least 8.  Applies to every box whose valid extents
  * match (nx,ny,nz) exactly; nx=ny=nz=0 sets the default.  The tiles are recorded
  * (amrs_boxlist_get_tiles); the face kernels deal columns and rows to warps
@@ -298,7 +298,7 @@ amrs_status amrs_boxlist_set_bcnormal(amrs_boxlist* bl, const amrs_bcnormal* bn)
 amrs_status amrs_boxlist_fill_halo(amrs_boxlist* bl, int32_t slot, void* stream);
 
 /* Per-box tiles in one call: tiles[3*b + {0,1,2}] = (tx, ty, kchunk) of
- * box b (the autotuner's output). */
+ * box b. */
 amrs_status amrs_boxlist_set_tiles(amrs_boxlist* bl, const int32_t* tiles);
 /* Work distribution of the fused face kernels (no counterpart in the
  * reference, whose MFIter loop launches box by box): the (column block x cell)
