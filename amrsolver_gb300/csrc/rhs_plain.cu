@@ -227,9 +227,8 @@ __device__ __forceinline__ double weno5js(const double s0, const double s1, cons
 // ddiv_core), and `ok` collects one range test per value that enters in place
 // of a test in every operation; where it ends up false the caller takes the
 // plain form.  The smoothness differences are below 2^60 (weno_diff).  eps + beta is
-// beta from 2^-78 up (eps is
-// below half its last place) and eps below 2^-187 (the other way round); in
-// between the hardware adds them out of line.
+// beta from 2^-78 up (eps is below half its last place) and eps below 2^-187 (the
+// other way round); in between the hardware adds them out of line.
 
 __device__ __forceinline__ DWords weno_sq(DWords e) { return dmul_core(e, e); }
 
